@@ -3,9 +3,9 @@ missing: there is no fallback implementation."""
 from __future__ import annotations
 
 import ctypes as C
-from pathlib import Path
-
 import os
+from pathlib import Path
+from types import SimpleNamespace
 
 _PKG = Path(__file__).resolve().parent
 # HQ_LIBRARY selects another build of the same library (e.g. libhq_checked.so)
@@ -105,18 +105,36 @@ def lib_path() -> Path:
     return _LIB_PATH
 
 
+def _attach(lib):
+    """Prototypes of include/hq.h for ctypes callers, and lib.host: the same functions
+    as native calls on torch tensors (csrc/host/host.cpp), by their C names."""
+    import torch  # noqa: F401  (the extension links against its libraries)
+
+    try:
+        from . import _host
+    except ImportError as e:
+        raise ImportError(
+            f"{_PKG / '_host.so'} cannot be loaded ({e}) - build it with "
+            "`python -m hecbench_b200.build`") from e
+
+    for name, (res, args) in SIGNATURES.items():
+        fn = getattr(lib, name)  # AttributeError if the symbol is not exported
+        fn.restype = res
+        fn.argtypes = args
+    lib.host = SimpleNamespace(
+        empty=_host.empty, place=_host.place,
+        **{name: _host.Entry(name, C.cast(getattr(lib, name), C.c_void_p).value, check)
+           for name in _host.symbols})
+    return lib
+
+
 def load_checked_library():
     """A separate handle on libhq_checked.so (the -DHQ_BOUNDS_CHECK build), with
     the same prototypes; None when it was not built."""
     path = _PKG / "libhq_checked.so"
     if not path.exists():
         return None
-    lib = C.CDLL(str(path))
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)
-        fn.restype = res
-        fn.argtypes = args
-    return lib
+    return _attach(C.CDLL(str(path)))
 
 
 def load_library():
@@ -128,13 +146,8 @@ def load_library():
         raise ImportError(
             f"{_LIB_PATH} is missing - build it with `python -m hecbench_b200.build` "
             "(nvcc, sm_100a).  There is no CPU or PyTorch fallback.")
-    lib = C.CDLL(str(_LIB_PATH))
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)  # AttributeError if the symbol is not exported
-        fn.restype = res
-        fn.argtypes = args
-    _lib = lib
-    return lib
+    _lib = _attach(C.CDLL(str(_LIB_PATH)))
+    return _lib
 
 
 def check(fn: str, status: int) -> None:

@@ -3,38 +3,22 @@
 Each function keeps the name, argument order and in/out convention of the
 HeCBench launcher it stands in for (file:line given per function; paths
 relative to the HeCBench source tree) and forwards to the C ABI of libhq.so on
-the current torch CUDA stream.  Arguments are validated here the way the C ABI
-validates them; errors surface as HqError / TypeError, never as a silent
-fallback.
+the current torch CUDA stream (lib.host, a native extension: for a decode-time
+mat-vec the host side of the call would otherwise take longer than the kernel).
+Arguments are validated there and here the way the C ABI validates them; errors
+surface as HqError / TypeError, never as a silent fallback.
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional, Sequence
 
 import torch
 
-from ._lib import check, load_library
+from ._lib import load_library
 
 NF4_HIGH_NIBBLE_FIRST = 0
 NF4_WEIGHTS_RESIDENT = 2
 NF4_LOW_NIBBLE_FIRST = 1
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
-def _dev(t: torch.Tensor, dtype: torch.dtype, name: str) -> int:
-    if not isinstance(t, torch.Tensor):
-        raise TypeError(f"{name}: expected a torch.Tensor")
-    if not t.is_cuda:
-        raise TypeError(f"{name}: must be a CUDA tensor (there is no CPU path)")
-    if t.dtype != dtype:
-        raise TypeError(f"{name}: expected dtype {dtype}, got {t.dtype}")
-    if not t.is_contiguous():
-        raise TypeError(f"{name}: must be contiguous")
-    return t.data_ptr()
 
 
 # --------------------------------------------------------------------------
@@ -46,39 +30,22 @@ def vecquant3matmul(vec, mat, mul, scales, zeros, height: int, width: int) -> No
 
     mul[c] += sum_k (scales[c]*q[k][c] - zeros[c]) * vec[k]; `mul` is
     accumulated into, exactly like the reference (the caller zeroes it)."""
-    lib = load_library()
-    args = (
-        _dev(vec, torch.float32, "vec"), _dev(mat, torch.int32, "mat"),
-        _dev(mul, torch.float32, "mul"), _dev(scales, torch.float32, "scales"),
-        _dev(zeros, torch.float32, "zeros"), height, width)
-    with torch.cuda.device(mat.device):
-        check("hq_q3_gemv_f32", lib.hq_q3_gemv_f32(*args, _stream()))
+    load_library().host.hq_q3_gemv_f32(vec, mat, mul, scales, zeros, height, width)
 
 
 def vecquant3matmul_faster(vec, mat, mul, scales, zeros, height: int, width: int) -> None:
     """vecquant3matmul_faster (quant3MatMul-cuda/kernels.h:193-217): fp16 input."""
-    lib = load_library()
-    args = (
-        _dev(vec, torch.float16, "vec"), _dev(mat, torch.int32, "mat"),
-        _dev(mul, torch.float32, "mul"), _dev(scales, torch.float32, "scales"),
-        _dev(zeros, torch.float32, "zeros"), height, width)
-    with torch.cuda.device(mat.device):
-        check("hq_q3_gemv_f16in", lib.hq_q3_gemv_f16in(*args, _stream()))
+    load_library().host.hq_q3_gemv_f16in(vec, mat, mul, scales, zeros, height, width)
 
 
 def vecquant3_dequant(mat, scales, zeros, height: int, width: int,
                       dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """Dequantised weights W[K][width] by the fp32 rule (kernels.h:43) or the
     fp16 rule (kernels.h:121-122,137)."""
-    lib = load_library()
-    K = height * 32 // 3
-    W = torch.empty((K, width), dtype=dtype, device=mat.device)
-    fn = {torch.float32: "hq_q3_dequant_f32", torch.float16: "hq_q3_dequant_f16"}[dtype]
-    args = (
-        _dev(mat, torch.int32, "mat"), _dev(scales, torch.float32, "scales"),
-        _dev(zeros, torch.float32, "zeros"), W.data_ptr(), height, width)
-    with torch.cuda.device(mat.device):
-        check(fn, getattr(lib, fn)(*args, _stream()))
+    host = load_library().host
+    fn = {torch.float32: host.hq_q3_dequant_f32, torch.float16: host.hq_q3_dequant_f16}[dtype]
+    W = host.empty(mat, dtype, height * 32 // 3, width)
+    fn(mat, scales, zeros, W, height, width)
     return W
 
 
@@ -89,14 +56,9 @@ def vecquant3_dequant(mat, scales, zeros, height: int, width: int,
 def kQuantize(code, A, out, n: int) -> None:
     """kQuantize<256,256><<<grid,block>>>(code, A, out, n)
     (quantBnB-cuda/main.cu:90-130,176)."""
-    lib = load_library()
     if n > A.numel() or n > out.numel():
         raise ValueError("n exceeds the buffers")
-    args = (
-        _dev(code, torch.float32, "code"), _dev(A, torch.float32, "A"),
-        _dev(out, torch.uint8, "out"), n)
-    with torch.cuda.device(A.device):
-        check("hq_bnb_quantize_u8", lib.hq_bnb_quantize_u8(*args, _stream()))
+    load_library().host.hq_bnb_quantize_u8(code, A, out, n)
 
 
 def dequantize_nf4(B, absmax, lut16, n: int, blocksize: int = 64,
@@ -104,15 +66,10 @@ def dequantize_nf4(B, absmax, lut16, n: int, blocksize: int = 64,
                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """NF4 blockwise dequantize to fp16 (no counterpart in the reference tree):
     out[e] = half_rn(lut16[code_e] * absmax[e // blocksize])."""
-    lib = load_library()
+    host = load_library().host
     if out is None:
-        out = torch.empty(n, dtype=torch.float16, device=B.device)
-    args = (
-        _dev(B, torch.uint8, "B"), _dev(absmax, torch.float32, "absmax"),
-        _dev(lut16, torch.float32, "lut16"), _dev(out, torch.float16, "out"),
-        n, blocksize, nibble_order)
-    with torch.cuda.device(B.device):
-        check("hq_nf4_dequant_f16", lib.hq_nf4_dequant_f16(*args, _stream()))
+        out = host.empty(B, torch.float16, n)
+    host.hq_nf4_dequant_f16(B, absmax, lut16, out, n, blocksize, nibble_order)
     return out
 
 
@@ -123,16 +80,11 @@ def gemv_nf4(A, B, absmax, lut16, N: int, K: int, blocksize: int = 64,
     out[n] = half(sum_k A[k] * lut16[code[n][k]] * absmax[(n*K+k)//blocksize]).
     weights_resident: B, absmax and lut16 are not written by earlier work in the
     stream, so the kernel may fetch them while the preceding kernel is finishing."""
-    lib = load_library()
+    host = load_library().host
     if out is None:
-        out = torch.empty(N, dtype=torch.float16, device=B.device)
-    args = (
-        _dev(A, torch.float16, "A"), _dev(B, torch.uint8, "B"),
-        _dev(absmax, torch.float32, "absmax"), _dev(lut16, torch.float32, "lut16"),
-        _dev(out, torch.float16, "out"), N, K, blocksize,
-        nibble_order | (NF4_WEIGHTS_RESIDENT if weights_resident else 0))
-    with torch.cuda.device(B.device):
-        check("hq_nf4_gemv_f16", lib.hq_nf4_gemv_f16(*args, _stream()))
+        out = host.empty(B, torch.float16, N)
+    host.hq_nf4_gemv_f16(A, B, absmax, lut16, out, N, K, blocksize,
+                         nibble_order | (NF4_WEIGHTS_RESIDENT if weights_resident else 0))
     return out
 
 
@@ -158,14 +110,11 @@ def static_scaled_int8_quant(output, input, hidden_size: int, num_tokens: int, s
     """static_scaled_int8_quant<scalar_t>(output, input, hidden_size, num_tokens,
     scale, azp) (quantVLLM-cuda/main.cu:137-153): azp == 0 selects the form
     without zero point, as in the reference."""
-    lib = load_library()
     code = _vllm_input(input, hidden_size, num_tokens)
     if output.numel() != input.numel():
         raise ValueError("output and input differ in size")
-    with torch.cuda.device(input.device):
-        check("hq_vllm_static_scaled_int8_quant", lib.hq_vllm_static_scaled_int8_quant(
-            _dev(output, torch.int8, "output"), input.data_ptr(), code, hidden_size, num_tokens,
-            float(scale), int(azp), _stream()))
+    load_library().host.hq_vllm_static_scaled_int8_quant(output, input, code, hidden_size,
+                                                         num_tokens, float(scale), int(azp))
 
 
 def dynamic_scaled_int8_quant(output, input, hidden_size: int, num_tokens: int, scales,
@@ -174,29 +123,25 @@ def dynamic_scaled_int8_quant(output, input, hidden_size: int, num_tokens: int, 
     scales, azp) (quantVLLM-cuda/main.cu:155-172): scales float32[num_tokens]
     and, when azp (int32[num_tokens]) is given, the per-token zero points are
     written too."""
-    lib = load_library()
     code = _vllm_input(input, hidden_size, num_tokens)
     if output.numel() != input.numel() or scales.numel() < num_tokens:
         raise ValueError("output / scales are too small")
     if azp is not None and azp.numel() < num_tokens:
         raise ValueError("azp is too small")
-    with torch.cuda.device(input.device):
-        check("hq_vllm_dynamic_scaled_int8_quant", lib.hq_vllm_dynamic_scaled_int8_quant(
-            _dev(output, torch.int8, "output"), input.data_ptr(), code, hidden_size, num_tokens,
-            _dev(scales, torch.float32, "scales"),
-            0 if azp is None else _dev(azp, torch.int32, "azp"), _stream()))
+    load_library().host.hq_vllm_dynamic_scaled_int8_quant(output, input, code, hidden_size,
+                                                          num_tokens, scales, azp)
 
 
 # --------------------------------------------------------------------------
 # gemv: uniform int8 / int4 weight-only mat-vec
 # --------------------------------------------------------------------------
 
-def _gemv_out(mat, vec, n: int, out):
+def _gemv_out(host, mat, vec, n: int, out):
     rows = mat.shape[0]
     if vec.numel() != n:
         raise ValueError(f"vec has {vec.numel()} elements, a row of mat {n}")
     if out is None:
-        out = torch.empty(rows, dtype=torch.float16, device=mat.device)
+        out = host.empty(mat, torch.float16, rows)
     elif out.numel() < rows:
         raise ValueError("out is too small")
     return rows, out
@@ -205,12 +150,10 @@ def _gemv_out(mat, vec, n: int, out):
 def gemv_fp16(mat, vec, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """gemv_fp16 behind solve_gemv_with_params (gemv-cuda/kernels.h:64-123,
     gemv.cu:61-81): mat fp16 [rows][n], vec fp16 [n] -> fp16 [rows]."""
+    host = load_library().host
     n = mat.shape[1]
-    rows, out = _gemv_out(mat, vec, n, out)
-    with torch.cuda.device(mat.device):
-        check("hq_gemv_f16", load_library().hq_gemv_f16(
-            _dev(mat, torch.float16, "mat"), _dev(vec, torch.float16, "vec"),
-            _dev(out, torch.float16, "out"), rows, n, _stream()))
+    rows, out = _gemv_out(host, mat, vec, n, out)
+    host.hq_gemv_f16(mat, vec, out, rows, n)
     return out
 
 
@@ -219,12 +162,10 @@ def gemv_int8_quantized(mat, vec, scale: float, zero_point: float,
     """gemv_quantized_int8 behind solve_gemv_int8_quantized_with_params
     (gemv-cuda/kernels.h:127-200, gemv.cu:38-59): mat int8 [rows][n]; scale and
     zero_point are rounded to fp16 as the reference launcher does."""
+    host = load_library().host
     n = mat.shape[1]
-    rows, out = _gemv_out(mat, vec, n, out)
-    with torch.cuda.device(mat.device):
-        check("hq_gemv_int8_f16", load_library().hq_gemv_int8_f16(
-            _dev(mat, torch.int8, "mat"), _dev(vec, torch.float16, "vec"),
-            _dev(out, torch.float16, "out"), rows, n, float(scale), float(zero_point), _stream()))
+    rows, out = _gemv_out(host, mat, vec, n, out)
+    host.hq_gemv_int8_f16(mat, vec, out, rows, n, scale, zero_point)
     return out
 
 
@@ -233,12 +174,10 @@ def gemv_int4_quantized(mat, vec, scale: float, zero_point: float,
     """gemv_quantized_int4 behind solve_gemv_int4_quantized_with_params
     (gemv-cuda/kernels.h:205-307, gemv.cu:15-36): mat uint8 [rows][n/2], element
     2j in the low nibble of byte j (uint4_2, kernels.h:9-32)."""
+    host = load_library().host
     n = 2 * mat.shape[1]
-    rows, out = _gemv_out(mat, vec, n, out)
-    with torch.cuda.device(mat.device):
-        check("hq_gemv_int4_f16", load_library().hq_gemv_int4_f16(
-            _dev(mat, torch.uint8, "mat"), _dev(vec, torch.float16, "vec"),
-            _dev(out, torch.float16, "out"), rows, n, float(scale), float(zero_point), _stream()))
+    rows, out = _gemv_out(host, mat, vec, n, out)
+    host.hq_gemv_int4_f16(mat, vec, out, rows, n, scale, zero_point)
     return out
 
 
@@ -251,14 +190,10 @@ def zero_point(x_min, x_max, qmin: int, qmax: int, size: int, preserve_sparsity:
     """zero_point<<<...>>>(x_min, x_max, qmin, qmax, size, preserve_sparsity, scale,
     zero_point) (zeropoint-cuda/main.cu:10-18): fp32 scale and int32 zero point of
     every channel from its minimum and maximum."""
-    lib = load_library()
     if min(x_min.numel(), x_max.numel(), scale.numel(), zero_point_out.numel()) < size:
         raise ValueError("a tensor is shorter than size")
-    with torch.cuda.device(x_min.device):
-        check("hq_zero_point", lib.hq_zero_point(
-            _dev(x_min, torch.float32, "x_min"), _dev(x_max, torch.float32, "x_max"), int(qmin),
-            int(qmax), int(size), int(bool(preserve_sparsity)), _dev(scale, torch.float32, "scale"),
-            _dev(zero_point_out, torch.int32, "zero_point"), _stream()))
+    load_library().host.hq_zero_point(x_min, x_max, int(qmin), int(qmax), int(size),
+                                      int(bool(preserve_sparsity)), scale, zero_point_out)
 
 
 def quantize_q3(W, mat=None, scales=None, zeros=None):
@@ -273,20 +208,16 @@ def quantize_q3(W, mat=None, scales=None, zeros=None):
     if W.dim() != 2 or not W.is_cuda or not W.is_contiguous():
         raise ValueError("W must be a contiguous 2-D CUDA tensor")
     K, N = W.shape
-    dev = W.device
+    host = lib.host
     if mat is None:
-        mat = torch.empty((K * 3 // 32, N), dtype=torch.int32, device=dev)
+        mat = host.empty(W, torch.int32, K * 3 // 32, N)
     if scales is None:
-        scales = torch.empty(N, dtype=torch.float32, device=dev)
+        scales = host.empty(W, torch.float32, N)
     if zeros is None:
-        zeros = torch.empty(N, dtype=torch.float32, device=dev)
+        zeros = host.empty(W, torch.float32, N)
     nbytes = int(lib.hq_q3_quantize_workspace_bytes(N))
-    ws = torch.empty(max(nbytes, 4), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        check("hq_q3_quantize", lib.hq_q3_quantize(
-            W.data_ptr(), code, K, N, _dev(mat, torch.int32, "mat"),
-            _dev(scales, torch.float32, "scales"), _dev(zeros, torch.float32, "zeros"),
-            ws.data_ptr(), nbytes, _stream()))
+    ws = host.empty(W, torch.uint8, max(nbytes, 4))
+    host.hq_q3_quantize(W, code, K, N, mat, scales, zeros, ws, nbytes)
     return mat, scales, zeros
 
 
@@ -295,22 +226,18 @@ def quantize_bcq(W, nb: int = 3, group_size: int = 128, bias: bool = True):
     float16 / bfloat16 / float32 -> (bW int32[K/32][nb][M] sign planes, alpha
     float16[K/group_size][nb][M], q_bias float16[K/group_size][M] or None), the
     arrays nQWeight_fp16 takes."""
-    lib = load_library()
+    host = load_library().host
     code = _VLLM_DTYPE.get(W.dtype)
     if code is None:
         raise TypeError("W must be float16, bfloat16 or float32")
     if W.dim() != 2 or not W.is_cuda or not W.is_contiguous():
         raise ValueError("W must be a contiguous 2-D CUDA tensor")
     K, M = W.shape
-    dev = W.device
     G = K // group_size
-    bW = torch.empty((K // 32, nb, M), dtype=torch.int32, device=dev)
-    alpha = torch.empty((G, nb, M), dtype=torch.float16, device=dev)
-    qb = torch.empty((G, M), dtype=torch.float16, device=dev) if bias else None
-    with torch.cuda.device(dev):
-        check("hq_lutgemm_quantize", lib.hq_lutgemm_quantize(
-            W.data_ptr(), code, K, M, nb, group_size, bW.data_ptr(), alpha.data_ptr(),
-            qb.data_ptr() if bias else None, _stream()))
+    bW = host.empty(W, torch.int32, K // 32, nb, M)
+    alpha = host.empty(W, torch.float16, G, nb, M)
+    qb = host.empty(W, torch.float16, G, M) if bias else None
+    host.hq_lutgemm_quantize(W, code, K, M, nb, group_size, bW, alpha, qb)
     return bW, alpha, qb
 
 
@@ -320,7 +247,7 @@ def quantize_nf4(W, lut16, blocksize: int = 64, nibble_order: int = NF4_HIGH_NIB
     the reference tree): W float16 / bfloat16 / float32 -> (B uint8[n / 2], absmax
     float32[n / blocksize]); code = the nearest of the 16 ascending levels lut16 to
     w / absmax, a tie going to the lower level."""
-    lib = load_library()
+    host = load_library().host
     code = _VLLM_DTYPE.get(W.dtype)
     if code is None:
         raise TypeError("W must be float16, bfloat16 or float32")
@@ -328,13 +255,10 @@ def quantize_nf4(W, lut16, blocksize: int = 64, nibble_order: int = NF4_HIGH_NIB
         raise ValueError("W must be a contiguous CUDA tensor")
     n = W.numel()
     if B is None:
-        B = torch.empty(n // 2, dtype=torch.uint8, device=W.device)
+        B = host.empty(W, torch.uint8, n // 2)
     if absmax is None:
-        absmax = torch.empty(n // blocksize, dtype=torch.float32, device=W.device)
-    with torch.cuda.device(W.device):
-        check("hq_nf4_quantize", lib.hq_nf4_quantize(
-            W.data_ptr(), code, n, blocksize, _dev(lut16, torch.float32, "lut16"), nibble_order,
-            _dev(B, torch.uint8, "B"), _dev(absmax, torch.float32, "absmax"), _stream()))
+        absmax = host.empty(W, torch.float32, n // blocksize)
+    host.hq_nf4_quantize(W, code, n, blocksize, lut16, nibble_order, B, absmax)
     return B, absmax
 
 
@@ -353,43 +277,33 @@ def mxfp4(y, a, numel: int) -> None:
     """mxfp4<T>(y, a, numel, ...) (mxfp4-cuda/main.cu:152-176, without its timing
     loop): y = a quantized to MXFP4 and back, groups of 32, T = float16 or
     bfloat16."""
-    lib = load_library()
     code = _mx_code(a)
     if y.dtype != a.dtype or min(y.numel(), a.numel()) < numel:
         raise ValueError("y and a must have the same type and numel elements")
-    with torch.cuda.device(a.device):
-        check("hq_mxfp4_qdq", lib.hq_mxfp4_qdq(a.data_ptr(), y.data_ptr(), int(numel), code,
-                                               _stream()))
+    load_library().host.hq_mxfp4_qdq(a, y, int(numel), code)
 
 
 def mxfp4_quantize(a, codes=None, scales=None):
     """Packed MXFP4 of a float16 / bfloat16 tensor: (codes uint8[numel / 2], element
     2j in the low nibble; scales uint8[numel / 32], E8M0)."""
-    lib = load_library()
+    host = load_library().host
     code = _mx_code(a)
     n = a.numel()
     if codes is None:
-        codes = torch.empty(n // 2, dtype=torch.uint8, device=a.device)
+        codes = host.empty(a, torch.uint8, n // 2)
     if scales is None:
-        scales = torch.empty(n // 32, dtype=torch.uint8, device=a.device)
-    with torch.cuda.device(a.device):
-        check("hq_mxfp4_quantize", lib.hq_mxfp4_quantize(
-            a.data_ptr(), _dev(codes, torch.uint8, "codes"), _dev(scales, torch.uint8, "scales"),
-            n, code, _stream()))
+        scales = host.empty(a, torch.uint8, n // 32)
+    host.hq_mxfp4_quantize(a, codes, scales, n, code)
     return codes, scales
 
 
 def mxfp4_dequantize(codes, scales, dtype=torch.float16, out=None):
     """Values of a packed MXFP4 tensor in float16 or bfloat16."""
-    lib = load_library()
+    host = load_library().host
     n = codes.numel() * 2
     if out is None:
-        out = torch.empty(n, dtype=dtype, device=codes.device)
-    code = _mx_code(out)
-    with torch.cuda.device(codes.device):
-        check("hq_mxfp4_dequantize", lib.hq_mxfp4_dequantize(
-            _dev(codes, torch.uint8, "codes"), _dev(scales, torch.uint8, "scales"), out.data_ptr(),
-            n, code, _stream()))
+        out = host.empty(codes, dtype, n)
+    host.hq_mxfp4_dequantize(codes, scales, out, n, _mx_code(out))
     return out
 
 
@@ -413,34 +327,22 @@ def gemv_fused(fmt: str, x, mat, rows_out: int, *, gamma=None, eps: float = 1e-5
     (geglu-cuda/reference.h:8-16, swish-cuda/reference.h:4).  weights_resident
     (NF4): as in gemv_nf4, the weights may be fetched while the preceding kernel
     of the stream drains."""
-    lib = load_library()
+    host = load_library().host
     n = x.numel()
     if out is None:
-        out = torch.empty(rows_out, dtype=torch.float16, device=x.device)
-    xp = _dev(x, torch.float16, "x")
-    gp = 0 if gamma is None else _dev(gamma, torch.float16, "gamma")
-    op = _dev(out, torch.float16, "out")
-    with torch.cuda.device(x.device):
-        if fmt == "f16":
-            st = lib.hq_gemv_fused_f16(xp, gp, float(eps), _dev(mat, torch.float16, "mat"), op,
-                                       rows_out, n, act, _stream())
-        elif fmt == "int8":
-            st = lib.hq_gemv_fused_int8_f16(xp, gp, float(eps), _dev(mat, torch.int8, "mat"), op,
-                                            rows_out, n, float(scale), float(zero_point), act,
-                                            _stream())
-        elif fmt == "int4":
-            st = lib.hq_gemv_fused_int4_f16(xp, gp, float(eps), _dev(mat, torch.uint8, "mat"), op,
-                                            rows_out, n, float(scale), float(zero_point), act,
-                                            _stream())
-        elif fmt == "nf4":
-            st = lib.hq_gemv_fused_nf4_f16(xp, gp, float(eps), _dev(mat, torch.uint8, "mat"),
-                                           _dev(absmax, torch.float32, "absmax"),
-                                           _dev(lut16, torch.float32, "lut16"), op, rows_out, n,
-                                           blocksize, nibble_order | (2 if weights_resident else 0),
-                                           act, _stream())
-        else:
-            raise ValueError(f"unknown format {fmt!r}")
-        check("hq_gemv_fused_" + fmt, st)
+        out = host.empty(x, torch.float16, rows_out)
+    if fmt == "f16":
+        host.hq_gemv_fused_f16(x, gamma, eps, mat, out, rows_out, n, act)
+    elif fmt == "int8":
+        host.hq_gemv_fused_int8_f16(x, gamma, eps, mat, out, rows_out, n, scale, zero_point, act)
+    elif fmt == "int4":
+        host.hq_gemv_fused_int4_f16(x, gamma, eps, mat, out, rows_out, n, scale, zero_point, act)
+    elif fmt == "nf4":
+        host.hq_gemv_fused_nf4_f16(x, gamma, eps, mat, absmax, lut16, out, rows_out, n, blocksize,
+                                   nibble_order | (NF4_WEIGHTS_RESIDENT if weights_resident else 0),
+                                   act)
+    else:
+        raise ValueError(f"unknown format {fmt!r}")
     return out
 
 
@@ -502,16 +404,10 @@ def matmul(output, input, nqW: nQWeight_fp16, m: int = 1, algo: int = 0) -> None
     """matmul(void* output, void* input, nQWeight_fp16& nqW, int m, int algo)
     (lut-gemm-cuda/kernels.cu:27-31): overwrites output[0:mSize] with the
     mat-vec of one input row (like the reference, only batch 1 is computed)."""
-    lib = load_library()
     ws = nqW.workspace()
-    args = (
-        _dev(output, torch.float16, "output"), _dev(input, torch.float16, "input"),
-        nqW.bWeight.data_ptr(), nqW.alpha.data_ptr(),
-        0 if nqW.q_bias is None else nqW.q_bias.data_ptr(),
-        nqW.mSize, nqW.kSize, nqW.nb, nqW.group_size,
-        ws.data_ptr(), ws.numel())
-    with torch.cuda.device(nqW.bWeight.device):
-        check("hq_lutgemm_nqmv", lib.hq_lutgemm_nqmv(*args, _stream()))
+    load_library().host.hq_lutgemm_nqmv(output, input, nqW.bWeight, nqW.alpha, nqW.q_bias,
+                                        nqW.mSize, nqW.kSize, nqW.nb, nqW.group_size, ws,
+                                        ws.numel())
 
 
 # --------------------------------------------------------------------------
@@ -524,31 +420,17 @@ def code1x16_matvec(A, B, C_out, codebook, prob_m: int, prob_k: int,
     """code1x16_matvec (quantAQLM-cuda/main.cu:113-141).  A = codes (int16 or
     uint16, [prob_m][prob_k/8]), B = input half[prob_k], C_out = half[prob_m]
     (overwritten), codebook half[..][65536][8]; `scales` is an extension."""
-    lib = load_library()
     if A.dtype not in (torch.int16, torch.uint16):
         raise TypeError("A: expected int16/uint16 codes")
-    sizes = (C.c_int * 4)(*[int(v) for v in codebook_a_sizes])
-    args = (
-        _dev(A, A.dtype, "A"), _dev(B, torch.float16, "B"),
-        _dev(C_out, torch.float16, "C"), _dev(codebook, torch.float16, "codebook"),
-        prob_m, prob_k, sizes, codebook_stride,
-        0 if scales is None else _dev(scales, torch.float16, "scales"))
-    with torch.cuda.device(A.device):
-        check("hq_aqlm_1x16_matvec", lib.hq_aqlm_1x16_matvec(*args, _stream()))
+    load_library().host.hq_aqlm_1x16_matvec(A, B, C_out, codebook, prob_m, prob_k,
+                                            codebook_a_sizes, codebook_stride, scales)
 
 
 def code2x8_matvec(A, B, C_out, codebooks, prob_m: int, prob_k: int,
                    scales: Optional[torch.Tensor] = None) -> None:
     """AQLM 2x8 mat-vec (no counterpart in the reference tree).  A = uint8 codes
     [prob_m][prob_k/8][2], codebooks half[2][256][8]."""
-    lib = load_library()
-    args = (
-        _dev(A, torch.uint8, "A"), _dev(B, torch.float16, "B"),
-        _dev(C_out, torch.float16, "C"), _dev(codebooks, torch.float16, "codebooks"),
-        prob_m, prob_k,
-        0 if scales is None else _dev(scales, torch.float16, "scales"))
-    with torch.cuda.device(A.device):
-        check("hq_aqlm_2x8_matvec", lib.hq_aqlm_2x8_matvec(*args, _stream()))
+    load_library().host.hq_aqlm_2x8_matvec(A, B, C_out, codebooks, prob_m, prob_k, scales)
 
 
 # --------------------------------------------------------------------------
@@ -558,16 +440,16 @@ def code2x8_matvec(A, B, C_out, codebooks, prob_m: int, prob_k: int,
 _qgemm_ws = {}
 
 
-def _qgemm_workspace(lib, device, Mb: int, N: int):
+def _qgemm_workspace(lib, X, Mb: int, N: int):
     """Zero-initialised split-K scratch, one per (device, stream, Mb, N): calls on
     different streams may overlap on the GPU and must not share the fp32 partial
     sums and tile counters."""
-    key = (device, _stream(), Mb, N)
+    key = (lib.host.place(X), Mb, N)
     ws = _qgemm_ws.get(key)
     if ws is None:
-        ws = torch.zeros(lib.hq_qgemm_workspace_bytes(Mb, N), dtype=torch.uint8, device=device)
+        ws = torch.zeros(lib.hq_qgemm_workspace_bytes(Mb, N), dtype=torch.uint8, device=X.device)
         _qgemm_ws[key] = ws
-    return ws.data_ptr(), ws.numel()
+    return ws, ws.numel()
 
 
 def qgemm_reset_workspaces() -> None:
@@ -592,24 +474,17 @@ def qgemm_q3(X, mat, scales, zeros, N: int, K: int, group_size: int = 128,
     the output slice of every GPU of the node instead of `out` (hq_qgemm_q3_f16_peers);
     returns None in that form."""
     lib = load_library()
+    host = lib.host
     Mb = X.shape[0]
-    head = (
-        _dev(X, torch.float16, "X"), _dev(mat, torch.int32, "mat"),
-        _dev(scales, torch.float16, "scales"), _dev(zeros, torch.float16, "zeros"))
-    ws_ptr, ws_bytes = _qgemm_workspace(lib, X.device, Mb, N) if split_k else (0, 0)
-    st = 0 if status is None else _dev(status, torch.int32, "status")
-    with torch.cuda.device(X.device):
-        if peers is not None:
-            table, offset, world = peers
-            check("hq_qgemm_q3_f16_peers", lib.hq_qgemm_q3_f16_peers(
-                *head, int(table), int(offset), int(world), Mb, N, K, group_size, ws_ptr, ws_bytes,
-                st, _stream()))
-            return None
-        if out is None:
-            out = torch.empty((Mb, N), dtype=torch.float16, device=X.device)
-        check("hq_qgemm_q3_f16", lib.hq_qgemm_q3_f16(
-            *head, _dev(out, torch.float16, "out"), Mb, N, K, group_size, ws_ptr, ws_bytes, st,
-            _stream()))
+    ws, ws_bytes = _qgemm_workspace(lib, X, Mb, N) if split_k else (None, 0)
+    if peers is not None:
+        table, offset, world = peers
+        host.hq_qgemm_q3_f16_peers(X, mat, scales, zeros, int(table), int(offset), int(world), Mb,
+                                   N, K, group_size, ws, ws_bytes, status)
+        return None
+    if out is None:
+        out = host.empty(X, torch.float16, Mb, N)
+    host.hq_qgemm_q3_f16(X, mat, scales, zeros, out, Mb, N, K, group_size, ws, ws_bytes, status)
     return out
 
 
@@ -621,22 +496,16 @@ def qgemm_nf4(X, B, absmax, lut16, N: int, K: int, blocksize: int = 64, nibble_o
     elements); same conventions as gemv_nf4, same workspace, status and `peers`
     rules as qgemm_q3 (no counterpart in the reference tree)."""
     lib = load_library()
+    host = lib.host
     Mb = X.shape[0]
-    head = (
-        _dev(X, torch.float16, "X"), _dev(B, torch.uint8, "B"),
-        _dev(absmax, torch.float32, "absmax"), _dev(lut16, torch.float32, "lut16"))
-    ws_ptr, ws_bytes = _qgemm_workspace(lib, X.device, Mb, N) if split_k else (0, 0)
-    st = 0 if status is None else _dev(status, torch.int32, "status")
-    with torch.cuda.device(X.device):
-        if peers is not None:
-            table, offset, world = peers
-            check("hq_qgemm_nf4_f16_peers", lib.hq_qgemm_nf4_f16_peers(
-                *head, int(table), int(offset), int(world), Mb, N, K, blocksize, nibble_order,
-                ws_ptr, ws_bytes, st, _stream()))
-            return None
-        if out is None:
-            out = torch.empty((Mb, N), dtype=torch.float16, device=X.device)
-        check("hq_qgemm_nf4_f16", lib.hq_qgemm_nf4_f16(
-            *head, _dev(out, torch.float16, "out"), Mb, N, K, blocksize, nibble_order, ws_ptr,
-            ws_bytes, st, _stream()))
+    ws, ws_bytes = _qgemm_workspace(lib, X, Mb, N) if split_k else (None, 0)
+    if peers is not None:
+        table, offset, world = peers
+        host.hq_qgemm_nf4_f16_peers(X, B, absmax, lut16, int(table), int(offset), int(world), Mb,
+                                    N, K, blocksize, nibble_order, ws, ws_bytes, status)
+        return None
+    if out is None:
+        out = host.empty(X, torch.float16, Mb, N)
+    host.hq_qgemm_nf4_f16(X, B, absmax, lut16, out, Mb, N, K, blocksize, nibble_order, ws,
+                          ws_bytes, status)
     return out

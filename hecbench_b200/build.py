@@ -2,8 +2,9 @@
 
 `python -m hecbench_b200.build` compiles every .cu under csrc/ with nvcc
 (cross-compiles without a GPU) into hecbench_b200/libhq.so, and the
-streaming-read probe of bench.py (csrc/probe/) into hecbench_b200/libhq_probe.so.  The objects are
-cached under hecbench_b200/build/ and rebuilt when a source or header is newer.
+streaming-read probe of bench.py (csrc/probe/) into hecbench_b200/libhq_probe.so;
+csrc/host/ (the launch path of the Python layer) goes into hecbench_b200/_host.so with g++.
+The objects are cached under hecbench_b200/build/ and rebuilt when a source or header is newer.
 """
 from __future__ import annotations
 
@@ -19,6 +20,7 @@ CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libhq.so"
 PROBE_LIB = PKG / "libhq_probe.so"
+HOST_EXT = PKG / "_host.so"
 CHECKED_LIB = PKG / "libhq_checked.so"
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -73,7 +75,30 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {probe_src.name}:\n{r.stderr}")
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> Path:
+    """The Python extension module hecbench_b200._host (C++ only, no kernels)."""
+    import sysconfig
+
+    import torch
+
+    src = CSRC / "host" / "host.cpp"
+    if force or _newer(HOST_EXT, [src]):
+        base = Path(torch.__file__).parent
+        cuda = Path(NVCC).resolve().parent.parent
+        cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f"-I{base / 'include'}", f"-I{base / 'include/torch/csrc/api/include'}",
+               f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}", str(src), "-o",
+               str(HOST_EXT), f"-L{base / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+               "-ltorch_cuda", "-ltorch_python"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed for {src.name}:\n{r.stderr}")
+    return HOST_EXT
 
 
 def build_checked(force: bool = False) -> Path:
