@@ -217,6 +217,26 @@ def test_bcq_quantize_against_oracle(hq, oracle, dev, dtype, K, M, nb, gs, bias)
         assert np.array_equal(qb.cpu().numpy().view(np.uint16), oqb.view(np.uint16))
 
 
+@pytest.mark.parametrize("gs,bias", [(128, True), (96, False), (96, True), (32, False)])
+def test_bcq_quantize_signed_zeros_and_overflow(hq, oracle, dev, gs, bias):
+    """-0 counts as >= 0; a scale that overflows fp16 (and the infinite and NaN residuals
+    after it) follows the comparisons of the rule; group sizes that are no power of two."""
+    K, M, nb = 2 * gs, 72, 3
+    W = (np.random.default_rng(gs).standard_normal((K, M)) * 0.05).astype(np.float32)
+    W[:, 0] = -0.0
+    W[::2, 1] = -0.0
+    W[:gs, 2] *= 3e6
+    W[gs:, 3] = np.where(np.arange(gs) % 2, 7e4, -7e4)
+    W[5, 4], W[6, 5], W[7, 6] = np.inf, -np.inf, np.nan
+    bW, alpha, qb = hq.quantize_bcq(_to_torch(W, "float32", dev), nb, gs, bias)
+    with np.errstate(all="ignore"):
+        obW, oal, oqb = oracle.lutgemm_quantize(W, nb, gs, bias)
+    assert np.array_equal(bW.cpu().numpy().view(np.uint32), obW)
+    assert np.array_equal(alpha.cpu().numpy(), oal, equal_nan=True)
+    if bias:
+        assert np.array_equal(qb.cpu().numpy(), oqb, equal_nan=True)
+
+
 def test_bcq_quantize_error_shrinks_and_feeds_the_mat_vec(hq, oracle, dev):
     """More planes, smaller error; and the quantized layer through the LUT-GEMM
     mat-vec equals the mat-vec of its own dequantised weights."""
