@@ -78,6 +78,26 @@ def test_vllm_quant_matches_oracle(hq, oracle, dev, dtype, tokens, hidden):
     assert _same(res["dynazp"], q) and _same(res["dynazp_scale"], s) and _same(res["dynazp_azp"], z)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,hidden", [(300, 7), (300, 8), (297, 15), (299, 2041), (298, 2057),
+                                           (296, 4103), (1, 8191), (2, 16385), (297, 16389)])
+def test_vllm_quant_block_shapes(hq, oracle, dev, dtype, tokens, hidden):
+    """Row lengths around the chunks-per-thread and block-size choices, rows that share
+    their boundary chunks, quotients on and beside ties."""
+    rng = np.random.default_rng(hidden)
+    base = np.round(rng.standard_normal((tokens, hidden)) * 40) * 0.05     # multiples of half the static scale
+    base += rng.integers(-3, 4, (tokens, 1))                                # one-sided rows among them
+    x = {"float16": lambda a: a.astype(np.float16), "bfloat16": _bf16_bits,
+         "float32": lambda a: a.astype(np.float32)}[dtype](base)
+    res = _run_all(hq, x, dtype, dev)
+    assert _same(res["static"], oracle.vllm_static_quant(x, dtype, 0.1, 0))
+    assert _same(res["static_azp"], oracle.vllm_static_quant(x, dtype, 0.1, 54))
+    q, s, _ = oracle.vllm_dynamic_quant(x, dtype, False)
+    assert _same(res["dyn"], q) and _same(res["dyn_scale"], s)
+    q, s, z = oracle.vllm_dynamic_quant(x, dtype, True)
+    assert _same(res["dynazp"], q) and _same(res["dynazp_scale"], s) and _same(res["dynazp_azp"], z)
+
+
 def test_vllm_quant_rejects_bad_arguments(hq, dev):
     import torch
     t = torch.zeros((4, 8), dtype=torch.float64, device=dev)
