@@ -22,11 +22,11 @@
 // memory.  One CTA (448 threads) owns 128 output features and a range of K
 // blocks of 64 inputs, and runs two independent pipelines j = 0, 1 over the
 // blocks j, j + 2, ...:
-//   warps 9, 10  packed-word TMA of pipeline 0 / 1: per block lane 0 waits for
-//              the ring slot and posts the byte count, lanes 0-2 issue the
+//   warps 9, 10  packed-word TMA of pipeline 0 / 1: per block the warp waits for
+//              the ring slot, one lane posts the byte count and issues the
 //              boxes (6 rows x 128 columns of words, 128 scales, 128 zeros)
 //              into the pipeline's slots of an 8-deep shared-memory ring;
-//   warps 12, 13 X TMA of pipeline 0 / 1 (one lane): one box of 64 inputs x all
+//   warps 12, 13 X TMA of pipeline 0 / 1: one box of 64 inputs x all
 //              tokens per block into the pipeline's four X stages, in the
 //              128-byte-swizzled K-major layout (rows beyond the token count
 //              are zero-filled by the TMA unit);
@@ -38,7 +38,7 @@
 //              its lane of the pipeline's A stage (tcgen05.st 32x32b.x32), then
 //              tcgen05.wait::st, tcgen05.fence::before_thread_sync and one
 //              mbarrier arrival per warp;
-//   warps 8, 11  MMA issuer of pipeline 0 / 1 (one lane): waits for the block's
+//   warps 8, 11  MMA issuer of pipeline 0 / 1: waits for the block's
 //              "full" barrier (four unpack-warp arrivals + the X bytes), issues
 //              four tcgen05.mma.cta_group::1.kind::f16 (K = 16 each, A from
 //              tensor memory, B through a shared-memory descriptor) into the
@@ -53,12 +53,21 @@
 // stages x 32 columns = 256 of the SM's 512 columns, so two CTAs share an SM
 // (the shared-memory request is padded to keep it at two); beyond 64 tokens a
 // CTA takes all 512 columns.  No TMA load uses cluster multicast.
+//
+// What bounds it: the length of the chain word TMA -> unpack -> MMA issue ->
+// commit per 64-input block; issue slots, shared memory, tensor pipe and DRAM are
+// all below half.  The issuer and TMA warps run their loops as whole warps and
+// elect one lane for the single-thread instructions (elect_one below).  With a
+// branch on lane 0 around the loop an issuer spent 1190 cycles on a block - 330 on
+// four MMAs, 260 on two commits, 600 on waits that were already over - and its
+// unpack group waited for it half of the time.  64 x 8192 x 28672: 3-bit 66.6 us
+// with the branch, 59.8 us now; NF4 94.1 and 91.5 (its table lookups, two
+// shared-memory wavefronts per byte, take over); 64 x 28672 x 8192: 62.0 -> 55.6
+// and 86.9 -> 85.6; 64 x 4096 x 6144: 16.4 -> 14.4 and 20.3 -> 18.6.
 // Every mbarrier wait is bounded: when the limit is hit the thread records a
 // status code, stops waiting and carries on, so the kernel always terminates
 // and frees its tensor memory; the host reads the status word.
 #include <cuda.h>
-
-#include <cstdlib>
 
 #include "hq_common.cuh"
 
@@ -134,6 +143,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, bool he
   }
   return false;
 }
+// One lane of a converged warp.  The single-thread instructions (MMA, commit, TMA,
+// barrier) take their operands from uniform registers: inside a branch on
+// elect.sync, in a warp that runs the loop as a whole, the compiler keeps them
+// there; inside a branch on the lane number it moves every operand over.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -195,6 +215,16 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 
 
 
+// both fp32 products in one instruction
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float b) {
+  unsigned long long r;
+  asm("{\n .reg .b64 x, y;\n mov.b64 x, {%1, %2};\n mov.b64 y, {%3, %3};\n"
+      " mul.rn.f32x2 %0, x, y;\n}\n"
+      : "=l"(r)
+      : "f"(a.x), "f"(a.y), "f"(b));
+  return make_float2(__uint_as_float((uint32_t)r), __uint_as_float((uint32_t)(r >> 32)));
+}
+
 struct QgemmParams {
   __half* Y;
   // Sharded layers: when peer_Y is non-null the tile is stored, as soon as it is
@@ -206,9 +236,6 @@ struct QgemmParams {
   float* ws;            // fp32 [Mb][N] scratch + per-tile counters, used when ksplit > 1
   unsigned* counters;
   int* status;
-#ifdef HQ_QGEMM_TRACE
-  long long* trace;  // development: [CTA][4 roles][8] accumulated clock cycles
-#endif
   int Mb, N, K, group_size, tokens_padded, ksplit;
   // NF4 only (group_size is the absmax block size there)
   const float* absmax;
@@ -268,7 +295,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       sm + tiles_bytes + kWordRing + 8 * (2 * kXStages + kStages + 2 * kWordAhead + 1));
   __shared__ unsigned s_last;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform for the compiler
   // tensor memory: two accumulators D[128 lanes][tokens] fp32 (one per MMA
   // issuer), then kStages A tiles of 128 lanes x 32 columns (64 halves per row)
   const uint32_t tmem_cols = p.tokens_padded <= 64 ? 256u : 512u;
@@ -280,13 +308,6 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   const int kb1 = (int)(((long long)nkb_total * (blockIdx.y + 1)) / p.ksplit);
   const int nloc = kb1 - kb0;
   bool ok = true;
-#ifdef HQ_QGEMM_TRACE
-  long long tr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  long long tmark = clock64();
-#define HQ_TR(i) { const long long now_ = clock64(); tr[i] += now_ - tmark; tmark = now_; }
-#else
-#define HQ_TR(i)
-#endif
 
   if (tid == 0) {
     for (int s = 0; s < kXStages; s++) {
@@ -348,10 +369,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     uint32_t a_stage = (uint32_t)grp, a_use = 0, x_stage = (uint32_t)grp;
     uint32_t w_slot = (uint32_t)grp, w_parity = 0;
     if constexpr (FMT == kFmtQ3) {
-      HQ_TR(0)
       for (int i = grp; i < nloc; i += 2) {
         if (!mbar_wait(wfull0 + 8 * w_slot, w_parity, ok)) ok = false;
-        HQ_TR(1)
         uint32_t w[6];
         uint16_t sc_bits, z_bits;
         {
@@ -398,17 +417,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         if (lane == 0) mbar_arrive(wempty0 + 8 * w_slot);
         w_slot += 2;
         if (w_slot >= kWordAhead) { w_slot -= kWordAhead; w_parity ^= 1u; }
-        HQ_TR(2)
         // the A tile of this stage must have been released by the tensor core
         if (a_use != 0 && !mbar_wait(empty0 + 8 * a_stage, (a_use - 1u) & 1u, ok)) ok = false;
-        HQ_TR(3)
         tc_fence_after();  // orders the stores after the tensor core's reads of the stage
         tmem_store_32(a_lane + a_stage * (uint32_t)kAColumns, o);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(full0 + 8 * x_stage);
-        HQ_TR(4)
         a_stage += 2;
         if (a_stage >= kStages) { a_stage -= kStages; a_use++; }
         x_stage += 2;
@@ -448,7 +464,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
             const uint32_t off =
                 ((t == 0 ? (w[q] << 7) : (w[q] >> (8 * t - 7))) & 0x7f80u) | lane8;
             const float2 lv = *reinterpret_cast<const float2*>(lut + off);
-            o[4 * q + t] = half2_as_u32(__floats2half2_rn(lv.x * am, lv.y * am));
+            const float2 w2 = mul_f32x2(lv, am);
+            o[4 * q + t] = half2_as_u32(__floats2half2_rn(w2.x, w2.y));
           }
         }
         __syncwarp();
@@ -468,7 +485,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         if (x_stage >= kXStages) x_stage -= kXStages;
       }
     }
-  } else if ((warp == 8 || warp == 11) && lane == 0) {
+  } else if (warp == 8 || warp == 11) {
     // ------------------------------ MMA issuers ------------------------------
     // Issuer j takes blocks j, j + 2, ... (the blocks of unpack group j) and
     // accumulates into its own tensor-memory columns, so that one issuer's
@@ -480,80 +497,73 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     const uint32_t acc = tmem_d + (uint32_t)(j * p.tokens_padded);
     uint32_t st = (uint32_t)j, xs = (uint32_t)j, xuse = 0;
     uint32_t accumulate = 0;
-    HQ_TR(0)
     for (int i = j; i < nloc; i += 2) {
       if (!mbar_wait(full0 + 8 * xs, xuse & 1u, ok)) ok = false;
-      HQ_TR(1)
+      __syncwarp();
       tc_fence_after();
-      const uint32_t a_tmem = tmem_d + a_col0 + st * (uint32_t)kAColumns;
-      const uint64_t bdesc = smem_desc(b_tiles + xs * kBTile);
+      if (elect_one()) {
+        const uint32_t a_tmem = tmem_d + a_col0 + st * (uint32_t)kAColumns;
+        const uint64_t bdesc = smem_desc(b_tiles + xs * kBTile);
 #pragma unroll
-      for (int k = 0; k < kBlockK / 16; k++) {
-        umma_f16_ts(acc, a_tmem + 8 * k, bdesc + 2 * k, idesc, accumulate);
-        accumulate = 1u;
+        for (int k = 0; k < kBlockK / 16; k++)
+          umma_f16_ts(acc, a_tmem + 8 * k, bdesc + 2 * k, idesc, k ? 1u : accumulate);
+        umma_commit(empty0 + 8 * st);
+        umma_commit(xempty0 + 8 * xs);
       }
-      umma_commit(empty0 + 8 * st);
-      umma_commit(xempty0 + 8 * xs);
-      HQ_TR(2)
+      __syncwarp();
+      accumulate = 1u;
       st += 2;
       if (st >= kStages) st -= kStages;
       xs += 2;
       if (xs >= kXStages) { xs -= kXStages; xuse++; }
     }
-    umma_commit(accum_bar);
-  } else if ((warp == 9 || warp == 10) && lane < 3) {
+    // the commit covers the MMAs of the thread that executes it: elect.sync names
+    // the same lane of the full warp every time
+    if (elect_one()) umma_commit(accum_bar);
+    __syncwarp();
+  } else if (warp == 9 || warp == 10) {
     // ------------------------------ packed-word TMA ------------------------------
-    // One warp per pipeline j: lane 0 waits for the slot and posts the byte
-    // count, then lanes 0-2 issue the loads side by side (3-bit: lane 0 the word
-    // box, lanes 1 and 2 the scales and zeros; NF4: lane 0 alone).
+    // One warp per pipeline j: waits for the slot, posts the byte count and issues
+    // the loads (3-bit: the word box, the scales and the zeros).
     const int j = warp - 9;
     uint32_t slot = (uint32_t)j, use = 0;
     for (int i = j; i < nloc; i += 2) {
-      if (lane == 0) {
-        if (use != 0 && !mbar_wait(wempty0 + 8 * slot, (use - 1u) & 1u, ok)) ok = false;
-        mbar_expect_tx(wfull0 + 8 * slot, kWordSlot);
+      if (use != 0 && !mbar_wait(wempty0 + 8 * slot, (use - 1u) & 1u, ok)) ok = false;
+      __syncwarp();
+      const int g = FMT == kFmtQ3 ? ((kb0 + i) * kBlockK) / p.group_size : 0;
+      if (elect_one()) {
+        const uint32_t dst = word_ring + slot * kWordSlot, bar = wfull0 + 8 * slot;
+        mbar_expect_tx(bar, kWordSlot);
+        if constexpr (FMT == kFmtQ3) {
+          tma_load_2d(dst, &map_w, n0, 6 * (kb0 + i), bar);
+          tma_load_2d(dst + 6 * 512, &map_s, n0, g, bar);
+          tma_load_2d(dst + 6 * 512 + 256, &map_z, n0, g, bar);
+        } else {
+          tma_load_2d(dst, &map_w, 32 * (kb0 + i), n0, bar);
+        }
       }
-      __syncwarp(0x7u);
-      const uint32_t dst = word_ring + slot * kWordSlot;
-      if constexpr (FMT == kFmtQ3) {
-        const int g = ((kb0 + i) * kBlockK) / p.group_size;
-        if (lane == 0) tma_load_2d(dst, &map_w, n0, 6 * (kb0 + i), wfull0 + 8 * slot);
-        else if (lane == 1) tma_load_2d(dst + 6 * 512, &map_s, n0, g, wfull0 + 8 * slot);
-        else tma_load_2d(dst + 6 * 512 + 256, &map_z, n0, g, wfull0 + 8 * slot);
-      } else {
-        if (lane == 0) tma_load_2d(dst, &map_w, 32 * (kb0 + i), n0, wfull0 + 8 * slot);
-      }
+      __syncwarp();
       slot += 2;
       if (slot >= kWordAhead) { slot -= kWordAhead; use++; }
     }
-  } else if ((warp == 12 || warp == 13) && lane == 0) {
+  } else if (warp == 12 || warp == 13) {
     // ------------------------------ X TMA ------------------------------
     const int j = warp - 12;
     uint32_t xs = (uint32_t)j, use = 0;
     for (int i = j; i < nloc; i += 2) {
       if (use != 0 && !mbar_wait(xempty0 + 8 * xs, (use - 1u) & 1u, ok)) ok = false;
-      const uint32_t bar = full0 + 8 * xs;
-      mbar_expect_tx(bar, (uint32_t)kBTile);
-      tma_load_2d(b_tiles + xs * (uint32_t)kBTile, &map_x, (kb0 + i) * kBlockK, 0, bar);
+      __syncwarp();
+      if (elect_one()) {
+        const uint32_t bar = full0 + 8 * xs;
+        mbar_expect_tx(bar, (uint32_t)kBTile);
+        tma_load_2d(b_tiles + xs * (uint32_t)kBTile, &map_x, (kb0 + i) * kBlockK, 0, bar);
+      }
+      __syncwarp();
       xs += 2;
       if (xs >= kXStages) { xs -= kXStages; use++; }
     }
   }
 
-#ifdef HQ_QGEMM_TRACE
-  if (p.trace != nullptr) {
-    int role = -1;
-    if (tid == 0) role = 0;            // unpack group 0
-    else if (tid == 128) role = 1;     // unpack group 1
-    else if (warp == 8 && lane == 0) role = 2;   // MMA issuer 0
-    else if (warp == 11 && lane == 0) role = 3;  // MMA issuer 1
-    if (role >= 0) {
-      HQ_TR(5)
-      for (int k = 0; k < 8; k++)
-        p.trace[((size_t)(blockIdx.y * gridDim.x + blockIdx.x) * 4 + role) * 8 + k] = tr[k];
-    }
-  }
-#endif
   if (warp < 8) {
     // ------------------------------ epilogue ------------------------------
     if (!mbar_wait(accum_bar, 0, ok)) ok = false;
@@ -762,12 +772,6 @@ QgemmParams make_params(void* Y_half, int Mb, int N, int K, int group_size, void
   prm.absmax = nullptr;
   prm.lut16 = nullptr;
   prm.low_first = 0;
-#ifdef HQ_QGEMM_TRACE
-  {
-    const char* tp = getenv("HQ_QGEMM_TRACE_PTR");
-    prm.trace = tp ? reinterpret_cast<long long*>(strtoull(tp, nullptr, 0)) : nullptr;
-  }
-#endif
   return prm;
 }
 
