@@ -740,20 +740,41 @@ size_t qgemm_ws_bytes(int Mb, int N) {
   return ((size_t)Mb * N * 4 + 255) / 256 * 256 + ((size_t)(N / kTileN + 1) * 4 + 255) / 256 * 256;
 }
 
-// K split: only with a workspace, and only when the tiles alone cannot fill
-// the CTA slots of the machine (two per SM)
+// Number of parts K is cut into, for `tiles` tiles of nkb blocks.  The plain choice
+// fills the CTA slots of the machine once; another one replaces it where this
+// model, in blocks of a CTA that shares its SM, expects 5 % less:
+//  * a wave of CTAs lasts its blocks; a last wave that leaves every CTA an SM of its
+//    own takes 0.67 of that (0.27 against 0.405 us per block, 3-bit);
+//  * every wave after the first costs 9 blocks (beyond 64 tokens, where one CTA
+//    takes the SM, 16) for its start, a split 10 (14) + 0.25 per part for the fp32
+//    reduction.
+// Measured, 64 tokens, K 8192, us with one part -> three: 160 tiles 57.4 -> 48.6
+// (NF4 89.9 -> 72.4), 192 tiles 57.4 -> 49.2 (90.2 -> 73.4), 224 tiles 57.8 against
+// 59.4: not split.  100 tokens, K 4096, 96 tiles, three parts -> one: 28.7 -> 24.6
+// (NF4 34.9 -> 34.8).
+int choose_ksplit(int tiles, int nkb, bool wide, int sms) {
+  const int slots = wide ? sms : 2 * sms;
+  const int most = max(1, min(nkb / 8, 2 * slots / tiles + 3));
+  auto cost = [&](int k) {
+    const int ctas = tiles * k, waves = (ctas + slots - 1) / slots;
+    const bool alone = !wide && ctas - (waves - 1) * slots <= sms;
+    return ((nkb + k - 1) / k) * (waves - 1 + (alone ? 0.67 : 1.0)) +
+           (waves - 1) * (wide ? 16.0 : 9.0) + (k > 1 ? (wide ? 14.0 : 10.0) + 0.25 * k : 0.0);
+  };
+  int best = max(1, min(2 * sms / tiles, nkb / 8));
+  double limit = 0.95 * cost(best);
+  for (int k = 1; k <= most; k++)
+    if (cost(k) < limit) { best = k; limit = cost(k); }
+  return best;
+}
+
 QgemmParams make_params(void* Y_half, int Mb, int N, int K, int group_size, void* workspace,
                         size_t workspace_bytes, int* status_word) {
   QgemmParams prm;
   const int tiles = N / kTileN;
-  const int slots = 2 * sm_count();
-  int ksplit = 1;
-  if (workspace != nullptr && workspace_bytes >= qgemm_ws_bytes(Mb, N) && aligned16(workspace)) {
-    ksplit = slots / tiles;
-    const int nkb = K / kBlockK;
-    if (ksplit > nkb / 8) ksplit = nkb / 8;
-    if (ksplit < 1) ksplit = 1;
-  }
+  int ksplit = 1;  // K is split only with a workspace
+  if (workspace != nullptr && workspace_bytes >= qgemm_ws_bytes(Mb, N) && aligned16(workspace))
+    ksplit = choose_ksplit(tiles, K / kBlockK, Mb > 64, sm_count());
   prm.Y = reinterpret_cast<__half*>(Y_half);
   prm.peer_Y = nullptr;
   prm.y_offset = 0;

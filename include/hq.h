@@ -480,9 +480,9 @@ int hq_mxfp4_dequantize(const uint8_t* codes, const uint8_t* scales_e8m0, void* 
  * output.  No counterpart in the reference tree.  1 <= Mb <= 128,
  * N % 128 == 0, K % group_size == 0, group_size % 64 == 0.  workspace
  * (nullable) is zero-initialised device scratch of hq_qgemm_workspace_bytes
- * bytes that lets the kernel split K over several CTAs when N alone gives too
- * few tiles to fill the GPU; every call that ends with status 0 leaves it
- * zero.  Two rules follow: (1) one workspace serves one stream - calls that may
+ * bytes that lets the kernel split K over several CTAs when N alone gives a
+ * grid that does not fill the GPU evenly (the parts meet in fp32 sums, in no
+ * fixed order); every call that ends with status 0 leaves it zero.  Two rules follow: (1) one workspace serves one stream - calls that may
  * overlap on the GPU (different streams, several host threads) need a
  * workspace each, or they race on the partial sums and tile counters and give
  * wrong results without any error; (2) after a call that set the status word

@@ -71,6 +71,25 @@ def test_qgemm_nf4_matches_dequant_then_gemm(hq, dev):
     assert float(err.max()) < TOL_F16
 
 
+@pytest.mark.parametrize("Mb,K,N", [(64, 8192, 20480), (33, 8192, 24576), (100, 4096, 12288)])
+def test_qgemm_parts_of_k(hq, dev, Mb, K, N):
+    """Shapes where the number of parts K is cut into leaves the one that fills the GPU
+    once (three parts in two waves; one part beyond 64 tokens), twice on one workspace,
+    against the library's own dequantisation and a dense fp32 product in torch."""
+    import torch
+    X, B, absmax, lut16 = synth.qgemm_nf4_case(Mb, K, N, 64, 7)
+    dX, dB, dA, dL = (to_dev(a, dev) for a in (X, B, absmax, lut16))
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    Y = [hq.qgemm_nf4(dX, dB, dA, dL, N, K, 64, 0, status=status) for _ in range(2)]
+    W = hq.dequantize_nf4(dB, dA, dL, N * K, 64, 0).view(N, K)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    ref = dX.float() @ W.float().t()
+    for y in Y:
+        err = (y.float() - ref).abs() / torch.maximum(ref.abs(), ref.pow(2).mean().sqrt())
+        assert float(err.max()) < TOL_F16
+
+
 LLAMA3_70B_MLP = [(8192, 28672), (28672, 8192)]  # (K, N): up/gate and down projections
 
 
