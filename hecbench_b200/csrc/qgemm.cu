@@ -60,7 +60,7 @@
 // elect one lane for the single-thread instructions (elect_one below).  With a
 // branch on lane 0 around the loop an issuer spent 1190 cycles on a block - 330 on
 // four MMAs, 260 on two commits, 600 on waits that were already over - and its
-// unpack group waited for it half of the time.  64 x 8192 x 28672: 3-bit 66.6 us
+// unpack group waited for it half of the time.  Launched one after the other, 64 x 8192 x 28672: 3-bit 66.6 us
 // with the branch, 59.8 us now; NF4 94.1 and 91.5 (its table lookups, two
 // shared-memory wavefronts per byte, take over); 64 x 28672 x 8192: 62.0 -> 55.6
 // and 86.9 -> 85.6; 64 x 4096 x 6144: 16.4 -> 14.4 and 20.3 -> 18.6.
@@ -322,6 +322,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     mbar_init(accum_bar, 2);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // Everything up to here, and the 3-bit table, needs no earlier kernel's results.
+  // The wait stands before the tensor-memory allocation, and the next kernel is let
+  // in after it: a CTA never holds columns that an unfinished kernel still asks for.
+  // Starting early takes 2 to 3 us off a call among others: 3-bit 64 x 2048 x 28672
+  // 20.5 -> 18.2 us, 37 x 4096 x 1024 10.3 -> 7.5; NF4 37 x 28672 x 8192 82.2 -> 80.2.
+  if (FMT == kFmtNf4) pdl_wait();
   if (FMT == kFmtQ3) {
     for (int i = tid; i < 64 * 32; i += kThreads) {
       const int v = i >> 5;
@@ -335,6 +341,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       lut_s[2 * i + 1] = __float_as_uint(p.lut16[p.low_first ? hi : lo]);
     }
   }
+  if (FMT == kFmtQ3) pdl_wait();
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
@@ -345,6 +352,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();
   const uint32_t tmem_d = *tmem_slot;
 
   if (warp < 8) {
@@ -810,7 +818,8 @@ int launch_qgemm(const CUtensorMap& map_x, const CUtensorMap& map_w, const CUten
     constexpr auto kern = qgemm_kernel<FMT, false>;
     cudaError_t e = ensure_dynamic_smem<kern>(smem);
     if (e != cudaSuccess) return cuda_status(e);
-    kern<<<grid, kThreads, smem, (cudaStream_t)stream>>>(map_x, map_w, map_s, map_z, prm);
+    return cuda_status(launch_pdl(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, map_x,
+                                  map_w, map_s, map_z, prm));
   }
   return launch_status();
 }
