@@ -21,6 +21,7 @@ namespace hq {
 namespace {
 
 constexpr int kWarps1x16 = 8;
+constexpr int kWarps2x8 = 8;
 // Rows per warp: 4 when that still gives every SM two CTAs, else 2 (a 4096-row
 // layer is latency-bound: more resident warps pay more than the per-CTA staging
 // of the inputs costs: 12.5 -> 11.0 us for 1x16, 11.5 -> 8.0 us for 2x8).
@@ -47,6 +48,25 @@ __device__ __forceinline__ float dot8_ref_order(const uint4& a, const uint4& b) 
   return __half2float(__low2half(r)) + __half2float(__high2half(r));
 }
 
+// Four of a thread's 16-byte pieces of the inputs, g0, g0 + 256, ...: all loads in
+// flight, then to shared memory.
+struct InputPieces {
+  uint4 v[4];
+  __device__ __forceinline__ void load(const uint4* x, int groups, int g0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (g0 + i * 256 < groups) v[i] = ld_dependent_u4(x + g0 + i * 256);
+  }
+  __device__ __forceinline__ void store(uint4* sh_x, int groups, int g0) const {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int g = g0 + i * 256;
+      if (g < groups) sh_x[kPad * (g >> 3) + (g & 7)] = v[i];
+    }
+  }
+};
+static_assert(kWarps1x16 * 32 == 256 && kWarps2x8 * 32 == 256, "stride of InputPieces");
+
 // VPL = 16-byte code vectors per lane per row (prob_k / 64 / 32 rounded up),
 // RPW = rows per warp.  The dependent chain code -> codebook row -> FMA is what
 // bounds this kernel, so everything that does not depend on the input vector
@@ -64,6 +84,10 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
   const int groups = prob_k >> 3;    // 16-byte input groups
   const int vec_per_row = prob_k >> 6;
   const int row_begin = (blockIdx.x * kWarps1x16 + warp) * RPW;
+  // the next kernel of the stream may become resident while this grid drains;
+  // nothing is read or written before every earlier kernel has completed
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int kUnits = RPW * VPL;  // unit u = (row u / VPL, vector u % VPL)
 
   uint4 cv[kUnits];
@@ -91,10 +115,14 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
         rows[i] = ldg_nc_u4(cb + ((cw[i >> 1] >> (16 * (i & 1))) & 0xffffu));
     }
   };
+  // at most 1024 pieces of inputs: four per thread, requested before the first
+  // gather waits for its codes
+  InputPieces xin;
+  xin.load(x, groups, tid);
   uint4 rows[2][8];
   gather(0, rows[0]);
 
-  for (int g = tid; g < groups; g += blockDim.x) sh_x[kPad * (g >> 3) + (g & 7)] = x[g];
+  xin.store(sh_x, groups, tid);
   __syncthreads();
 
   float res = 0.f;
@@ -118,8 +146,6 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
   }
 }
 
-constexpr int kWarps2x8 = 8;
-
 __global__ void __launch_bounds__(kWarps2x8 * 32)
 aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
                 __half* __restrict__ out, const uint4* __restrict__ codebooks, int prob_m,
@@ -130,8 +156,14 @@ aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = prob_k >> 3;
   const int vec_per_row = prob_k >> 6;  // 16 bytes = 8 groups x 2 codes
+  pdl_launch_dependents();  // as in the 1x16 kernel
+  pdl_wait();
   for (int i = tid; i < 2 * 256 * 8; i += blockDim.x) cbs[i] = codebooks[i >> 3];
-  for (int g = tid; g < groups; g += blockDim.x) sh_x[kPad * (g >> 3) + (g & 7)] = x[g];
+  for (int g0 = tid; g0 < groups; g0 += 4 * 256) {
+    InputPieces xin;
+    xin.load(x, groups, g0);
+    xin.store(sh_x, groups, g0);
+  }
   __syncthreads();
 
   const uint4* cb0 = cbs + (lane & 7);
@@ -191,6 +223,10 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps1x16);
   const int rows_per_cta = kWarps1x16 * rows_per_warp;
   const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
+  // A grid that fills the SMs starts while the one before it drains (4096 x 4096
+  // back to back: 12.4 -> 11.0 us).  A smaller one does not: the CTAs of an early
+  // start are not spread over all SMs, and the gathers are bound by each SM's L1
+  // (1024 x 8192: 13.2 us, 18.9 with the early start).
   const int4 sizes = make_int4(cb_sizes[0], cb_sizes[1], cb_sizes[2], cb_sizes[3]);
   cudaStream_t st = (cudaStream_t)stream;
 #define HQ_AQLM_LAUNCH(VPL, RPW)                                                             \
@@ -200,10 +236,16 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
       cudaError_t e = ensure_dynamic_smem<kern>(smem);                                       \
       if (e != cudaSuccess) return cuda_status(e);                                           \
     }                                                                                        \
-    kern<<<grid, kWarps1x16 * 32, smem, st>>>(                                               \
-        reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint4*>(x_half),       \
-        reinterpret_cast<__half*>(out_half), reinterpret_cast<const uint4*>(codebook),       \
-        prob_m, prob_k, sizes, cb_stride_int4, reinterpret_cast<const __half*>(scales_half)); \
+    const auto c = reinterpret_cast<const uint4*>(codes);                                    \
+    const auto x = reinterpret_cast<const uint4*>(x_half);                                   \
+    const auto o = reinterpret_cast<__half*>(out_half);                                      \
+    const auto cb = reinterpret_cast<const uint4*>(codebook);                                \
+    const auto sc = reinterpret_cast<const __half*>(scales_half);                            \
+    if (grid >= sm_count())                                                                  \
+      return cuda_status(launch_pdl(kern, dim3(grid), dim3(kWarps1x16 * 32), smem, st, c, x, o, \
+                                    cb, prob_m, prob_k, sizes, cb_stride_int4, sc));         \
+    kern<<<grid, kWarps1x16 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sizes,            \
+                                              cb_stride_int4, sc);                           \
   }
 #define HQ_AQLM_ROWS(VPL)                                \
   if (rows_per_warp == 4) HQ_AQLM_LAUNCH(VPL, 4)         \
@@ -234,10 +276,18 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps2x8);
   const int rows_per_cta = kWarps2x8 * rows_per_warp;
   const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
-  aqlm_2x8_kernel<<<grid, kWarps2x8 * 32, smem, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint4*>(x_half),
-      reinterpret_cast<__half*>(out_half), reinterpret_cast<const uint4*>(codebooks), prob_m,
-      prob_k, reinterpret_cast<const __half*>(scales_half), rows_per_warp);
+  const auto c = reinterpret_cast<const uint4*>(codes);
+  const auto x = reinterpret_cast<const uint4*>(x_half);
+  const auto o = reinterpret_cast<__half*>(out_half);
+  const auto cb = reinterpret_cast<const uint4*>(codebooks);
+  const auto sc = reinterpret_cast<const __half*>(scales_half);
+  const cudaStream_t st = (cudaStream_t)stream;
+  // early start as for 1x16: 4096 x 8192 14.4 -> 12.6 us with a full grid, 2048 x
+  // 4096 8.2 us plain and 9.1 with it
+  if (grid >= sm_count())
+    return cuda_status(launch_pdl(kern2x8, dim3(grid), dim3(kWarps2x8 * 32), smem, st, c, x, o, cb,
+                                  prob_m, prob_k, sc, rows_per_warp));
+  kern2x8<<<grid, kWarps2x8 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sc, rows_per_warp);
   return launch_status();
 }
 
