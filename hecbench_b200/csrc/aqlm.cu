@@ -282,9 +282,10 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const auto cb = reinterpret_cast<const uint4*>(codebooks);
   const auto sc = reinterpret_cast<const __half*>(scales_half);
   const cudaStream_t st = (cudaStream_t)stream;
-  // early start as for 1x16: 4096 x 8192 14.4 -> 12.6 us with a full grid, 2048 x
-  // 4096 8.2 us plain and 9.1 with it
-  if (grid >= sm_count())
+  // early start as for 1x16, from two CTAs per SM on: 14336 x 4096 28.5 -> 26.3 us;
+  // 2048 x 4096 takes 8.2 us plain and 9.1 with it, and in a replayed graph 4096 x
+  // 4096 (256 CTAs) 8.0 and 9.5
+  if (grid >= 2 * sm_count())
     return cuda_status(launch_pdl(kern2x8, dim3(grid), dim3(kWarps2x8 * 32), smem, st, c, x, o, cb,
                                   prob_m, prob_k, sc, rows_per_warp));
   kern2x8<<<grid, kWarps2x8 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sc, rows_per_warp);
