@@ -30,14 +30,6 @@ inline int rows_per_warp_for(int prob_m, int warps) {
 }
 constexpr int kPad = 9;  // input slots per 8 groups (one pad slot: conflict-free 128-bit reads)
 
-__device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-
 __device__ __forceinline__ float dot8_ref_order(const uint4& a, const uint4& b) {
   // res2 = hfma2(a[j], b[j], res2), j = 0..3, from zero; float(res2.x) + float(res2.y)
   __half2 r = __float2half2_rn(0.f);
@@ -76,9 +68,9 @@ static_assert(kWarps1x16 * 32 == 256 && kWarps2x8 * 32 == 256, "stride of InputP
 // is multiplied.  The arithmetic (and its order) is the reference's.
 template <int VPL, int RPW>
 __global__ void __launch_bounds__(kWarps1x16 * 32)
-aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
-                 __half* __restrict__ out, const uint4* __restrict__ codebook, int prob_m,
-                 int prob_k, int4 cb_sizes, int cb_stride, const __half* __restrict__ scales) {
+aqlm_1x16_kernel(const uint4* codes, const uint4* x,
+                 __half* __restrict__ out, const uint4* codebook, int prob_m,
+                 int prob_k, int4 cb_sizes, int cb_stride, const __half* scales) {
   extern __shared__ __align__(16) uint4 sh_x[];  // padded inputs: slot 9*(g/8) + g%8
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = prob_k >> 3;    // 16-byte input groups
@@ -95,7 +87,7 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
   for (int u = 0; u < kUnits; u++) {
     const int m = row_begin + u / VPL, idx = lane + 32 * (u % VPL);
     cv[u] = (m < prob_m && idx < vec_per_row)
-                ? ldg_stream_u4(codes + (size_t)m * vec_per_row + idx)
+                ? ld_ordered_stream_u4(codes + (size_t)m * vec_per_row + idx)
                 : make_uint4(0, 0, 0, 0);
   }
   auto book = [&](int m) {
@@ -112,7 +104,7 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
       const uint32_t cw[4] = {cv[u].x, cv[u].y, cv[u].z, cv[u].w};
 #pragma unroll
       for (int i = 0; i < 8; i++)
-        rows[i] = ldg_nc_u4(cb + ((cw[i >> 1] >> (16 * (i & 1))) & 0xffffu));
+        rows[i] = ld_ordered_u4(cb + ((cw[i >> 1] >> (16 * (i & 1))) & 0xffffu));
     }
   };
   // at most 1024 pieces of inputs: four per thread, requested before the first
@@ -138,7 +130,7 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) res += __shfl_down_sync(0xffffffffu, res, o);
       if (lane == 0 && m < prob_m) {
-        if (scales != nullptr) res *= __half2float(scales[m]);
+        if (scales != nullptr) res *= __half2float(ld_ordered_f16(scales + m));
         out[m] = __float2half(res);
       }
       res = 0.f;
@@ -147,9 +139,9 @@ aqlm_1x16_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
 }
 
 __global__ void __launch_bounds__(kWarps2x8 * 32)
-aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
-                __half* __restrict__ out, const uint4* __restrict__ codebooks, int prob_m,
-                int prob_k, const __half* __restrict__ scales, int rows_per_warp) {
+aqlm_2x8_kernel(const uint4* codes, const uint4* x,
+                __half* __restrict__ out, const uint4* codebooks, int prob_m,
+                int prob_k, const __half* scales, int rows_per_warp) {
   extern __shared__ __align__(16) uint4 smem4[];
   uint4* cbs = smem4;                  // [2][256][8 replicas]
   uint4* sh_x = smem4 + 2 * 256 * 8;   // padded inputs
@@ -158,7 +150,16 @@ aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
   const int vec_per_row = prob_k >> 6;  // 16 bytes = 8 groups x 2 codes
   pdl_launch_dependents();  // as in the 1x16 kernel
   pdl_wait();
-  for (int i = tid; i < 2 * 256 * 8; i += blockDim.x) cbs[i] = codebooks[i >> 3];
+  constexpr int kThreads2x8 = kWarps2x8 * 32, kBatch = 8;  // entries requested at a time
+#pragma unroll
+  for (int i0 = 0; i0 < 2 * 256 * 8; i0 += kBatch * kThreads2x8) {
+    uint4 e[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; b++)
+      e[b] = ld_ordered_u4(codebooks + ((i0 + b * kThreads2x8 + tid) >> 3));
+#pragma unroll
+    for (int b = 0; b < kBatch; b++) cbs[i0 + b * kThreads2x8 + tid] = e[b];
+  }
   for (int g0 = tid; g0 < groups; g0 += 4 * 256) {
     InputPieces xin;
     xin.load(x, groups, g0);
@@ -175,7 +176,7 @@ aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
     const uint4* crow = codes + (size_t)m * vec_per_row;
     float res = 0.f;
     for (int idx = lane; idx < vec_per_row; idx += 32) {
-      const uint4 cv = ldg_stream_u4(crow + idx);
+      const uint4 cv = ld_ordered_stream_u4(crow + idx);
       const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
 #pragma unroll
       for (int i = 0; i < 8; i++) {
@@ -197,7 +198,7 @@ aqlm_2x8_kernel(const uint4* __restrict__ codes, const uint4* __restrict__ x,
     }
     res = warp_sum(res);
     if (lane == 0) {
-      if (scales != nullptr) res *= __half2float(scales[m]);
+      if (scales != nullptr) res *= __half2float(ld_ordered_f16(scales + m));
       out[m] = __float2half_rn(res);
     }
   }

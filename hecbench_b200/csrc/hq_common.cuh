@@ -154,12 +154,18 @@ __device__ __forceinline__ uint32_t ldg_stream_u32(const void* p) {
   return v;
 }
 
-// Loads of data that an earlier kernel of the stream may have written (the input
-// vector of a mat-vec), for kernels launched with programmatic dependent launch:
-// they must stay behind griddepcontrol.wait.  A non-coherent load (ld.global.nc,
-// which __ldg and const __restrict__ pointers produce) promises that the data is
-// read-only for the whole kernel, so the assembler may move it above the wait;
-// these are ordinary coherent loads that the compiler may not reorder.
+// Loads for kernels launched with programmatic dependent launch: whatever an earlier
+// kernel of the stream may have written has to be read behind griddepcontrol.wait,
+// and that holds for weights as well (a layer can be quantized and multiplied on one
+// stream).  A non-coherent load (ld.global.nc, which ldg_stream_*, __ldg and const
+// __restrict__ pointers produce) promises that the data is read-only for the whole
+// kernel, so the assembler may move it above the wait - it has done so; these are
+// ordinary coherent loads that the compiler may not reorder.
+//  * ld_dependent_*: input vectors; the clobber also orders them with plain loads
+//    and stores.
+//  * ld_ordered_*: weights, scales, tables, which no thread of the kernel writes:
+//    in program order with the wait and with one another (asm volatile), free to
+//    move past plain loads and stores.  The stream form does not allocate in L1.
 __device__ __forceinline__ uint4 ld_dependent_u4(const void* p) {
   uint4 v;
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -176,6 +182,36 @@ __device__ __forceinline__ float ld_dependent_f32(const float* p) {
 __device__ __forceinline__ __half ld_dependent_f16(const __half* p) {
   unsigned short v;
   asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return __ushort_as_half(v);
+}
+
+__device__ __forceinline__ uint4 ld_ordered_stream_u4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_ordered_u4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_ordered_u2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_ordered_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ __half ld_ordered_f16(const __half* p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return __ushort_as_half(v);
 }
 

@@ -80,12 +80,6 @@ __device__ __forceinline__ float lds_f32_imm(uint32_t addr) {
   asm("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(addr), "n"(IMM));
   return v;
 }
-__device__ __forceinline__ uint2 ldg_nc_u2(const void* p) {
-  uint2 v;
-  asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-
 // One launch handles NB bit planes b0 .. b0+NB-1 of nb_total (more planes than
 // fit the register budget are split over launches that accumulate into the
 // same scratch row; only the last one converts it).  RPG: packed rows that
@@ -93,8 +87,8 @@ __device__ __forceinline__ uint2 ldg_nc_u2(const void* p) {
 // column range (per_range != 0) or a single one.
 template <int TR, int NB, int RPG, int kThreads>
 __global__ void __launch_bounds__(kThreads, (kThreads == 256 ? 2 : 1))
-lutgemm_kernel(const uint32_t* __restrict__ bW, const __half* __restrict__ alpha,
-               const __half* __restrict__ q_bias, const __half* __restrict__ x,
+lutgemm_kernel(const uint32_t* bW, const __half* alpha,
+               const __half* q_bias, const __half* x,
                __half* __restrict__ out, float* __restrict__ ws, unsigned* __restrict__ counters,
                int M, int K, int rows_per_group, int cols_per_cta, int nb_total, int b0,
                int finalize, int per_range) {
@@ -159,7 +153,7 @@ lutgemm_kernel(const uint32_t* __restrict__ bW, const __half* __restrict__ alpha
 #pragma unroll
       for (int b = 0; b < NB; b++) {
         const uint32_t* src = src0 + (size_t)(r * nb_total + b) * M + (m - m0);
-        if (HQ_IN_BOUNDS(src, 16, bW, bw_bytes, 201)) wv[r][b] = ldg_stream_u4(src);
+        if (HQ_IN_BOUNDS(src, 16, bW, bw_bytes, 201)) wv[r][b] = ld_ordered_stream_u4(src);
       }
     }
   };
@@ -169,10 +163,10 @@ lutgemm_kernel(const uint32_t* __restrict__ bW, const __half* __restrict__ alpha
 #pragma unroll
       for (int b = 0; b < NB; b++) {
         const __half* src = alpha + ((size_t)g * nb_total + b0 + b) * M + m;
-        if (HQ_IN_BOUNDS(src, 8, alpha, alpha_bytes, 202)) av[gi][b] = ldg_nc_u2(src);
+        if (HQ_IN_BOUNDS(src, 8, alpha, alpha_bytes, 202)) av[gi][b] = ld_ordered_u2(src);
       }
       if (q_bias != nullptr && HQ_IN_BOUNDS(q_bias + (size_t)g * M + m, 8, q_bias, bias_bytes, 203))
-        av[gi][NB] = ldg_nc_u2(q_bias + (size_t)g * M + m);
+        av[gi][NB] = ld_ordered_u2(q_bias + (size_t)g * M + m);
     }
   };
   if (nsteps > 0 && m0 < m_end) {

@@ -245,9 +245,7 @@ struct QgemmParams {
 
 // output slice of this launch on GPU g (the table is constant during the launch)
 __device__ __forceinline__ __half* peer_slice(const QgemmParams& p, int g) {
-  return reinterpret_cast<__half*>(
-             __ldg(reinterpret_cast<const unsigned long long*>(p.peer_Y) + g)) +
-         p.y_offset;
+  return p.peer_Y[g] + p.y_offset;
 }
 
 // PEERS: the sharded form (tiles stored to every GPU's slice); a separate
@@ -448,10 +446,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       auto am_index = [&](int kb) {
         return am_pow2 ? (kb >> am_shift) : (kb * kBlockK) / p.group_size;
       };
-      float am_next = grp < nloc ? __ldg(am_row + am_index(kb0 + grp)) : 0.f;
+      float am_next = grp < nloc ? ld_ordered_f32(am_row + am_index(kb0 + grp)) : 0.f;
       for (int i = grp; i < nloc; i += 2) {
         const float am = am_next;
-        if (i + 2 < nloc) am_next = __ldg(am_row + am_index(kb0 + i + 2));
+        if (i + 2 < nloc) am_next = ld_ordered_f32(am_row + am_index(kb0 + i + 2));
         if (!mbar_wait(wfull0 + 8 * w_slot, w_parity, ok)) ok = false;
         uint32_t w[8];
         {
