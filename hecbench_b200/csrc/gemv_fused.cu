@@ -100,7 +100,7 @@ gemv_fused_kernel(const FusedParams p) {
     if (HQ_IN_BOUNDS(xg + i, 16, p.x, (size_t)n * 2, 502)) v = ld_dependent_u4(xg + i);
     if (p.gamma != nullptr) {
       uint4 g = make_uint4(0, 0, 0, 0);
-      if (HQ_IN_BOUNDS(gg + i, 16, p.gamma, (size_t)n * 2, 503)) g = __ldg(gg + i);
+      if (HQ_IN_BOUNDS(gg + i, 16, p.gamma, (size_t)n * 2, 503)) g = ld_ordered_u4(gg + i);
       uint32_t h[4] = {v.x, v.y, v.z, v.w};
       const uint32_t gh[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
@@ -140,7 +140,7 @@ gemv_fused_kernel(const FusedParams p) {
           const unsigned char* at = src + (size_t)r * row_bytes + (size_t)c * 16;
           w[u][r] = make_uint4(0, 0, 0, 0);  // a row past the end contributes zeros
           if (c < chunks && row0 + r < rows_mat && HQ_IN_BOUNDS(at, 16, p.mat, mat_bytes, 504))
-            w[u][r] = ldg_stream_u4(at);
+            w[u][r] = ld_ordered_stream_u4(at);
         }
       }
 #pragma unroll

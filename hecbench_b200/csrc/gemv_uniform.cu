@@ -39,7 +39,7 @@ using namespace rows;
 // n: inputs per row; row_bytes = n * BITS / 8 (a multiple of 16).
 template <int BITS>
 __global__ void __launch_bounds__(kThreads, 2)
-gemv_uniform_kernel(const unsigned char* __restrict__ mat, const __half* __restrict__ vec,
+gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
                     __half* __restrict__ res, int rows, int n, float scale, float zero_point) {
   extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
   __shared__ float s_part[kWarps];
@@ -50,9 +50,9 @@ gemv_uniform_kernel(const unsigned char* __restrict__ mat, const __half* __restr
   const int chunks = (int)(row_bytes / 16);   // 16-byte chunks per row
 
   // Programmatic dependent launch: the next kernel of the stream may become
-  // resident while this grid drains; everything that earlier work may have
-  // produced - the input vector - is read after the wait, and nothing is written
-  // before it.
+  // resident while this grid drains; nothing is read before the wait (the matrix
+  // may be an earlier kernel's output like the input vector), and nothing is
+  // written before it.
   pdl_launch_dependents();
   pdl_wait();
   // ---- prologue: inputs to shared memory (piece-major) and their sum ----
@@ -96,7 +96,7 @@ gemv_uniform_kernel(const unsigned char* __restrict__ mat, const __half* __restr
           const unsigned char* at = src + (size_t)r * row_bytes + (size_t)c * 16;
           w[u][r] = make_uint4(0, 0, 0, 0);  // a row past the end contributes zeros
           if (c < chunks && row0 + r < rows && HQ_IN_BOUNDS(at, 16, mat, mat_bytes, 402))
-            w[u][r] = ldg_stream_u4(at);
+            w[u][r] = ld_ordered_stream_u4(at);
         }
       }
 #pragma unroll

@@ -65,15 +65,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Loads that keep their place in the program order among the other ordered
-// loads (asm volatile): the prologue depends on WHICH request reaches the memory
-// system first.
-__device__ __forceinline__ float ldg_ordered_f32(const float* p) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-
 // 16-byte asynchronous copy global -> shared (no register holds the data)
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem)
@@ -281,15 +272,16 @@ nf4_gemv_kernel(const GemvParams p) {
 
   // The 16 levels first: the table build must not queue behind the weight loads
   // below.  (The levels count as weights: read before the wait with early_fetch.)
-  // (ordered loads: the compiler must not sink them below the weight loads)
+  // (ordered loads: the compiler must not sink them below the weight loads, and
+  // without early_fetch nothing may raise any of them above the wait)
   constexpr int kTabTurns = (256 * 4 + THREADS - 1) / THREADS;
   float lv_first[kTabTurns], lv_second[kTabTurns];
 #pragma unroll
   for (int t = 0; t < kTabTurns; t++) {
     const int entry = ((tid + t * THREADS) >> 2) & 255;
     const int hi = entry >> 4, lo = entry & 15;
-    lv_first[t] = ldg_ordered_f32(p.lut16 + (p.low_first ? lo : hi));
-    lv_second[t] = ldg_ordered_f32(p.lut16 + (p.low_first ? hi : lo));
+    lv_first[t] = ld_ordered_f32(p.lut16 + (p.low_first ? lo : hi));
+    lv_second[t] = ld_ordered_f32(p.lut16 + (p.low_first ? hi : lo));
   }
   // this lane's chunk columns; a lane beyond the row end loads nothing and
   // keeps zero codes, scales and inputs
@@ -318,8 +310,8 @@ nf4_gemv_kernel(const GemvParams p) {
         a = p.absmax + (p.cpb_shift >= 0 ? (ci[i] >> p.cpb_shift) : (ci[i] / (uint32_t)p.cpb)); \
       if (live[i] && HQ_IN_BOUNDS(wp[i], 16, p.B, p.b_bytes, 101) &&                            \
           HQ_IN_BOUNDS(a, 4, p.absmax, p.absmax_bytes, 102)) {                                  \
-        cw[STAGE][i] = ldg_stream_u4(wp[i]);                                                    \
-        cs[STAGE][i] = __ldg(a);                                                                \
+        cw[STAGE][i] = ld_ordered_stream_u4(wp[i]);                                             \
+        cs[STAGE][i] = ld_ordered_f32(a);                                                       \
       }                                                                                         \
       const bool odd = FUSE && (((STAGE) & 1) != 0);                                            \
       wp[i] += odd ? p.w_step_odd : p.w_step;                                                   \
@@ -813,7 +805,7 @@ nf4_gemv_bulk_kernel(const GemvParams p, int rows_total) {
 // carries the epoch of the latest completed gather (sync_words[1]; no check
 // when sync_words is null) and stores its value.
 __global__ void __launch_bounds__(256)
-ll_unpack_kernel(const uint2* __restrict__ ll, long long n, __half* __restrict__ out,
+ll_unpack_kernel(const uint2* ll, long long n, __half* __restrict__ out,
                  const unsigned* sync_words, unsigned max_polls, int* status) {
   pdl_launch_dependents();
   pdl_wait();

@@ -42,9 +42,9 @@ __device__ __forceinline__ int f16_window_start(int w) {
 // instantiation: the single-block form keeps its code).
 template <bool F16IN, bool MULTI>
 __global__ void __launch_bounds__(kThreads)
-q3_gemv_kernel(const void* __restrict__ vec_, const int32_t* __restrict__ mat,
-               float* __restrict__ mul, const float* __restrict__ scales,
-               const float* __restrict__ zeros, int groups, int width, int groups_per_cta,
+q3_gemv_kernel(const void* vec_, const int32_t* mat,
+               float* mul, const float* scales,
+               const float* zeros, int groups, int width, int groups_per_cta,
                int colblocks_per_cta) {
   // the next kernel of the stream may become resident while this grid runs;
   // nothing is read or written before every earlier kernel has completed
@@ -132,17 +132,17 @@ q3_gemv_kernel(const void* __restrict__ vec_, const int32_t* __restrict__ mat,
     uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0, n2 = n0;
     if (active && warp < ng) {
       const int32_t* p = base + (size_t)warp * 3 * width;
-      n0 = ldg_stream_u4(p);
-      n1 = ldg_stream_u4(p + width);
-      n2 = ldg_stream_u4(p + 2 * (size_t)width);
+      n0 = ld_ordered_stream_u4(p);
+      n1 = ld_ordered_stream_u4(p + width);
+      n2 = ld_ordered_stream_u4(p + 2 * (size_t)width);
     }
     for (int gi = warp; gi < ng; gi += kWarps) {
       const uint4 u0 = n0, u1 = n1, u2 = n2;
       if (active && gi + kWarps < ng) {
         const int32_t* p = base + (size_t)(gi + kWarps) * 3 * width;
-        n0 = ldg_stream_u4(p);
-        n1 = ldg_stream_u4(p + width);
-        n2 = ldg_stream_u4(p + 2 * (size_t)width);
+        n0 = ld_ordered_stream_u4(p);
+        n1 = ld_ordered_stream_u4(p + width);
+        n2 = ld_ordered_stream_u4(p + 2 * (size_t)width);
       }
       sumx += gsum[gi];
       const uint32_t w0s[4] = {u0.x, u0.y, u0.z, u0.w};
@@ -221,6 +221,8 @@ q3_gemv_kernel(const void* __restrict__ vec_, const int32_t* __restrict__ mat,
         }
         // undo the input pre-scaling: fp32 path 2^(49+e), fp16 path 2^(9+e)
         q = F16IN ? q * pow2f(9 + e) : (q * pow2f(49)) * pow2f(e);
+        // (no __restrict__: the parameters may alias mul for all the compiler knows, so
+        // these are ordinary loads behind the wait)
         float sc, nz;
         if (F16IN) {
           // the reference rounds both parameters to fp16 (kernels.h:121-122)

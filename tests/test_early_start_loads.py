@@ -16,7 +16,8 @@ def _blocks(text):
     return re.split(r"^}\n", text, flags=re.M)
 
 
-@pytest.mark.parametrize("name", ["aqlm.cu", "lutgemm.cu", "qgemm.cu"])
+@pytest.mark.parametrize("name", ["aqlm.cu", "gemv_fused.cu", "gemv_uniform.cu", "lutgemm.cu", "nf4.cu",
+                                  "q3_gemv.cu", "qgemm.cu"])
 def test_no_load_can_pass_the_wait(name):
     blocks = _blocks((CSRC / name).read_text())
     early = [b for b in blocks if "__global__" in b and "pdl_wait();" in b]
@@ -68,6 +69,35 @@ def _consumer(hq, family, dev):
             else:
                 hq.code2x8_matvec(a.view(torch.uint8), x, out, b, M, K, scales=s)
         return n, call, (M,)
+    if kind in ("q3mv", "nf4mv", "int4mv", "fused"):
+        N, K = 2048, 512
+        lut, x = torch.linspace(-1, 1, 16, device=dev), halves(K)
+        if kind == "q3mv":
+            parts = {"words": codes(K * 3 // 8, N).view(torch.int32).view(K * 3 // 32, N),
+                     "scales": halves(N, scale=2 ** -5 if operand == "zeros" else 1).float(),
+                     "zeros": halves(N, scale=1 if operand == "zeros" else 2 ** -5).float()}
+        elif kind == "nf4mv":
+            parts = {"codes": codes(N, K // 2), "absmax": halves(N * K // 64).float()}
+        elif kind == "int4mv":
+            parts = {"codes": codes(N, K // 2)}
+        else:
+            parts = {"gamma": halves(K), "codes": codes(N, K // 2)}
+        operand_t = parts[operand]
+
+        def call(buf, out):
+            p = {**parts, operand: buf.view(operand_t.dtype).view(operand_t.shape)}
+            if kind == "q3mv":
+                mul = torch.zeros(N, device=dev)
+                hq.vecquant3matmul_faster(x, p["words"], mul, p["scales"], p["zeros"], K * 3 // 32, N)
+                out.copy_(mul * 2 ** -2)
+            elif kind == "nf4mv":
+                hq.gemv_nf4(x, p["codes"], p["absmax"], lut, N, K, 64, out=out)
+            elif kind == "int4mv":
+                hq.gemv_int4_quantized(p["codes"], x, 2 ** -4, 7.0, out=out)
+            else:
+                hq.gemv_fused("int4", x, p["codes"], N, gamma=p["gamma"], scale=2 ** -4, zero_point=7.0,
+                              out=out)
+        return operand_t.numel() * operand_t.dtype.itemsize // 2, call, (N,)
     Mb, N, K = 20, 1024, 512
     X = halves(Mb, K)
     if kind == "q3":
@@ -92,7 +122,9 @@ def _consumer(hq, family, dev):
 @pytest.mark.gpu
 @pytest.mark.parametrize("family", ["lutgemm words", "lutgemm alpha", "lutgemm bias", "1x16 codes",
                                     "1x16 codebook", "1x16 scales", "2x8 codes", "2x8 codebook",
-                                    "2x8 scales", "q3 words", "q3 scales", "nf4 codes", "nf4 absmax"])
+                                    "2x8 scales", "q3 words", "q3 scales", "nf4 codes", "nf4 absmax",
+                                    "q3mv words", "q3mv scales", "q3mv zeros", "nf4mv codes", "nf4mv absmax",
+                                    "int4mv codes", "fused codes", "fused gamma"])
 def test_weights_written_by_the_launch_before(hq, dev, family):
     """An operand is the output of the launch right before, which itself started early:
     the numbers 0.5 to 2, or their bit patterns as codes (as absmax: 1e-4 to 2).  The
