@@ -350,6 +350,21 @@ def gemv_fused(fmt: str, x, mat, rows_out: int, *, gamma=None, eps: float = 1e-5
 # lut-gemm
 # --------------------------------------------------------------------------
 
+def _stream_scratch(cache: dict, key, nbytes: int, like: torch.Tensor) -> torch.Tensor:
+    """The zero-initialised scratch of `cache` for `key`, which names the device and
+    current stream of `like`: calls on different streams may overlap on the GPU and
+    must not share partial sums and counters.  Scratch that is first needed while the
+    stream is being captured is not kept: its clearing belongs to that graph, so an
+    eager call or another graph would find it uncleared."""
+    ws = cache.get(key)
+    if ws is None:
+        ws = torch.zeros(nbytes, dtype=torch.uint8, device=like.device)
+        with torch.cuda.device(like.device):
+            if not torch.cuda.is_current_stream_capturing():
+                cache[key] = ws
+    return ws
+
+
 class nQWeight_fp16:
     """Mirror of class nQWeight_fp16 (lut-gemm-cuda/nQWeight_fp16.h:22-45,
     nQWeight_fp16.cu:22-53): holds the bit-plane weights, fp16 alphas and the
@@ -363,7 +378,7 @@ class nQWeight_fp16:
         self.bWeight = self.alpha = self.q_bias = None
         self.num_groups = self.group_size = self.mSize = self.kSize = self.nb = 0
         self.is_row_wise_quantize = False
-        self._ws = None
+        self._ws = {}
         if bW is not None:
             self.parsing(bW, A, row, col, num_bits, is_row_wise_quantize, num_alpha_groups,
                          q_bias, device)
@@ -392,12 +407,11 @@ class nQWeight_fp16:
             raise ValueError("alpha has the wrong number of elements")
 
     def workspace(self) -> torch.Tensor:
-        """Zero-initialised fp32 scratch the kernel accumulates K tiles into; it
-        is left zero by every call."""
-        if self._ws is None:
-            nbytes = load_library().hq_lutgemm_workspace_bytes(self.mSize)
-            self._ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.bWeight.device)
-        return self._ws
+        """Zero-initialised fp32 scratch the kernel accumulates K tiles into, one per
+        device and current stream; it is left zero by every call."""
+        lib = load_library()
+        return _stream_scratch(self._ws, (lib.host.place(self.bWeight), self.mSize),
+                               lib.hq_lutgemm_workspace_bytes(self.mSize), self.bWeight)
 
 
 def matmul(output, input, nqW: nQWeight_fp16, m: int = 1, algo: int = 0) -> None:
