@@ -483,7 +483,9 @@ def qgemm_q3(X, mat, scales, zeros, N: int, K: int, group_size: int = 128,
     fp16 scales / zeros [K/group_size][N] (no counterpart in the reference tree).
     `status` (int32[1], optional) receives 1 if a bounded in-kernel wait ran out;
     call qgemm_reset_workspaces() before the next product in that case.
-    With split_k a zero-initialised scratch matrix is kept per (device, stream, Mb, N).
+    With split_k a zero-initialised scratch matrix is kept per (device, stream, Mb, N);
+    the parts of K meet in it in a fixed order for wide layers only (hq.h), so
+    split_k=False is the way to the same bits on every call for any shape.
     peers = (pointer_table, offset_elements, world): store every finished tile into
     the output slice of every GPU of the node instead of `out` (hq_qgemm_q3_f16_peers);
     returns None in that form."""

@@ -237,11 +237,26 @@ struct QgemmParams {
   unsigned* counters;
   int* status;
   int Mb, N, K, group_size, tokens_padded, ksplit;
+  int ordered;          // the parts of a tile add to the scratch in the order of K
   // NF4 only (group_size is the absmax block size there)
   const float* absmax;
   const float* lut16;
   int low_first;
 };
+
+// Waits until `turn` parts of the tile have been added to the scratch, for sums in a
+// fixed order.  CTAs start in the order of their part (blockIdx.y), so the parts
+// before this one are finished or running, and a part lasts about as long as the one
+// before it.  Bounded: past the limit (milliseconds) the sums are still right, only
+// their order is not the usual one.
+constexpr uint32_t kTurnSpins = 1u << 14;
+__device__ __forceinline__ void await_turn(const unsigned* counter, unsigned turn) {
+  for (uint32_t i = 0; i < kTurnSpins; i++) {
+    unsigned done;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(counter) : "memory");
+    if (done >= turn) return;
+  }
+}
 
 // output slice of this launch on GPU g (the table is constant during the launch)
 __device__ __forceinline__ __half* peer_slice(const QgemmParams& p, int g) {
@@ -317,7 +332,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       mbar_init(wfull0 + 8 * s, 1);
       mbar_init(wempty0 + 8 * s, kProducerThreads / 64);
     }
-    mbar_init(accum_bar, 2);
+    mbar_init(accum_bar, p.ordered ? 3 : 2);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // Everything up to here, and the 3-bit table, needs no earlier kernel's results.
@@ -568,6 +583,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       xs += 2;
       if (xs >= kXStages) { xs -= kXStages; use++; }
     }
+    // sums in a fixed order: the epilogue starts when it is this part's turn as well
+    if (j == 1 && p.ordered && elect_one()) {
+      await_turn(p.counters + blockIdx.x, blockIdx.y);
+      mbar_arrive(accum_bar);
+    }
+    __syncwarp();
   }
 
   if (warp < 8) {
@@ -758,7 +779,17 @@ size_t qgemm_ws_bytes(int Mb, int N) {
 // (NF4 89.9 -> 72.4), 192 tiles 57.4 -> 49.2 (90.2 -> 73.4), 224 tiles 57.8 against
 // 59.4: not split.  100 tokens, K 4096, 96 tiles, three parts -> one: 28.7 -> 24.6
 // (NF4 34.9 -> 34.8).
-int choose_ksplit(int tiles, int nkb, bool wide, int sms) {
+// A layer that the plain choice leaves in one or two parts gives the same bits on
+// every call (two addends have no order), and three or more parts keep that by adding
+// in turn (ordered): no slower while a spare warp watches for the turn (64 x 8192 x
+// 24576 in three parts 46.6 us either way, NF4 69.9 and 69.8).  Narrower layers, where
+// many short parts of a tile end together, add in any order: in turn, 64 x 4096 x 6144
+// would take 25.4 us for 12.7.
+struct KSplit {
+  int parts;
+  bool ordered;
+};
+KSplit choose_ksplit(int tiles, int nkb, bool wide, int sms) {
   const int slots = wide ? sms : 2 * sms;
   const int most = max(1, min(nkb / 8, 2 * slots / tiles + 3));
   auto cost = [&](int k) {
@@ -767,20 +798,21 @@ int choose_ksplit(int tiles, int nkb, bool wide, int sms) {
     return ((nkb + k - 1) / k) * (waves - 1 + (alone ? 0.67 : 1.0)) +
            (waves - 1) * (wide ? 16.0 : 9.0) + (k > 1 ? (wide ? 14.0 : 10.0) + 0.25 * k : 0.0);
   };
-  int best = max(1, min(2 * sms / tiles, nkb / 8));
+  const int plain = max(1, min(2 * sms / tiles, nkb / 8));
+  int best = plain;
   double limit = 0.95 * cost(best);
   for (int k = 1; k <= most; k++)
     if (cost(k) < limit) { best = k; limit = cost(k); }
-  return best;
+  return {best, plain <= 2 && best > 2};
 }
 
 QgemmParams make_params(void* Y_half, int Mb, int N, int K, int group_size, void* workspace,
                         size_t workspace_bytes, int* status_word) {
   QgemmParams prm;
   const int tiles = N / kTileN;
-  int ksplit = 1;  // K is split only with a workspace
+  KSplit split = {1, false};  // K is split only with a workspace
   if (workspace != nullptr && workspace_bytes >= qgemm_ws_bytes(Mb, N) && aligned16(workspace))
-    ksplit = choose_ksplit(tiles, K / kBlockK, Mb > 64, sm_count());
+    split = choose_ksplit(tiles, K / kBlockK, Mb > 64, sm_count());
   prm.Y = reinterpret_cast<__half*>(Y_half);
   prm.peer_Y = nullptr;
   prm.y_offset = 0;
@@ -795,7 +827,8 @@ QgemmParams make_params(void* Y_half, int Mb, int N, int K, int group_size, void
   prm.K = K;
   prm.group_size = group_size;
   prm.tokens_padded = (Mb + 15) / 16 * 16;
-  prm.ksplit = ksplit;
+  prm.ksplit = split.parts;
+  prm.ordered = split.ordered ? 1 : 0;
   prm.absmax = nullptr;
   prm.lut16 = nullptr;
   prm.low_first = 0;

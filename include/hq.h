@@ -481,9 +481,12 @@ int hq_mxfp4_dequantize(const uint8_t* codes, const uint8_t* scales_e8m0, void* 
  * N % 128 == 0, K % group_size == 0, group_size % 64 == 0.  workspace
  * (nullable) is zero-initialised device scratch of hq_qgemm_workspace_bytes
  * bytes that lets the kernel split K over several CTAs when N alone gives a
- * grid that does not fill the GPU evenly (the parts meet in fp32 sums, in no
- * fixed order); every call that ends with status 0 leaves it zero.  Two rules follow: (1) one workspace serves one stream - calls that may
- * overlap on the GPU (different streams, several host threads) need a
+ * grid that does not fill the GPU evenly; every call that ends with status 0
+ * leaves it zero.  The parts meet in fp32 sums.  For N > 128 * 2 * SMs / 3 (12629
+ * on 148 SMs) or K < 1536 they are added in the order of K, so a call gives the
+ * same bits every time; for narrower layers, and in the sharded form below, they
+ * are added in no fixed order.  Without a workspace every result is repeatable.
+ * Two rules follow: (1) one workspace serves one stream - calls that may overlap on the GPU (different streams, several host threads) need a
  * workspace each, or they race on the partial sums and tile counters and give
  * wrong results without any error; (2) after a call that set the status word
  * the workspace may hold partial sums and counters: clear it (cudaMemsetAsync

@@ -90,6 +90,49 @@ def test_qgemm_parts_of_k(hq, dev, Mb, K, N):
         assert float(err.max()) < TOL_F16
 
 
+@pytest.mark.parametrize("fmt", ["q3", "nf4"])
+@pytest.mark.parametrize("Mb,K,N", [(64, 8192, 20480), (5, 8192, 24576), (100, 8192, 20480),
+                                    (33, 28672, 28672), (128, 28672, 12800)])
+def test_qgemm_parts_of_k_repeat(hq, dev, fmt, Mb, K, N):
+    """Wide layers (more than two thirds of a tile per SM) in two to five parts of K: the same
+    bits from every call, also beside another stream's product and on fresh scratch, and
+    the dense fp32 product of the dequantised weights."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(K + N)
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    if fmt == "nf4":
+        lut = torch.linspace(-1, 1, 16, device=dev)
+        B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+        absmax = torch.rand(N * K // 64, generator=g, device=dev) + 0.5
+        W = hq.dequantize_nf4(B, absmax, lut, N * K, 64, 0).view(N, K)
+        ref = X.float() @ W.float().t()
+        call = lambda: hq.qgemm_nf4(X, B, absmax, lut, N, K, 64, 0, status=status)
+    else:
+        mat = torch.randint(-2**31, 2**31, (K * 3 // 32, N), generator=g, device=dev).to(torch.int32)
+        scales = (torch.rand((K // 128, N), generator=g, device=dev) * 0.01).half()
+        zeros = scales * 3.5
+        one, zero = torch.ones(N, device=dev), torch.zeros(N, device=dev)
+        W = hq.vecquant3_dequant(mat, one, zero, K * 3 // 32, N, dtype=torch.float16)
+        W = torch.addcmul(-zeros.float().repeat_interleave(128, 0), W.float(),
+                          scales.float().repeat_interleave(128, 0)).half()
+        ref = X.float() @ W.float()
+        call = lambda: hq.qgemm_q3(X, mat, scales, zeros, N, K, 128, status=status)
+    del W
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    first = call()
+    err = (first.float() - ref).abs() / torch.maximum(ref.abs(), ref.pow(2).mean().sqrt())
+    assert float(err.max()) < TOL_F16
+    outs = [call() for _ in range(6)]
+    torch.cuda.synchronize()
+    for s in (torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(s):
+            outs += [call() for _ in range(3)]
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for y in outs:
+        assert torch.equal(y, first)
+
+
 LLAMA3_70B_MLP = [(8192, 28672), (28672, 8192)]  # (K, N): up/gate and down projections
 
 
