@@ -768,17 +768,21 @@ size_t qgemm_ws_bytes(int Mb, int N) {
 }
 
 // Number of parts K is cut into, for `tiles` tiles of nkb blocks.  The plain choice
-// fills the CTA slots of the machine once; another one replaces it where this
-// model, in blocks of a CTA that shares its SM, expects 5 % less:
+// makes up to two CTAs per SM (beyond 64 tokens, where one takes the SM, that is up to
+// two waves); another one replaces it where this model, in blocks of a CTA that
+// shares its SM, expects 5 % less:
 //  * a wave of CTAs lasts its blocks; a last wave that leaves every CTA an SM of its
 //    own takes 0.67 of that (0.27 against 0.405 us per block, 3-bit);
 //  * every wave after the first costs 9 blocks (beyond 64 tokens, where one CTA
 //    takes the SM, 16) for its start, a split 10 (14) + 0.25 per part for the fp32
 //    reduction.
-// Measured, 64 tokens, K 8192, us with one part -> three: 160 tiles 57.4 -> 48.6
-// (NF4 89.9 -> 72.4), 192 tiles 57.4 -> 49.2 (90.2 -> 73.4), 224 tiles 57.8 against
-// 59.4: not split.  100 tokens, K 4096, 96 tiles, three parts -> one: 28.7 -> 24.6
-// (NF4 34.9 -> 34.8).
+// Measured against every count from one to six, both formats, 4 to 128 tokens, 16
+// layers of K 2048 to 28672: never slower than the plain choice, within 5 % of the
+// best.  us, plain -> model, 3-bit (NF4):
+//   64 x 8192 x 20480, 1 -> 3 parts: 55.0 -> 45.9 (87.5 -> 69.2); 4 tokens: 52.9 -> 41.7
+//   64 x 28672 x 20480, 1 -> 5: 180 -> 119 (287 -> 189); x 28672, 1 -> 5: 181 -> 163
+//   64 x 8192 x 28672 stays in one: 55.5, three parts 57.7
+//   100 x 4096 x 14336, 2 -> 1: 30.8 -> 22.5 (41.2 -> 31.8); x 12288, 3 -> 1: 25.5 -> 22.7
 // A layer that the plain choice leaves in one or two parts gives the same bits on
 // every call (two addends have no order), and three or more parts keep that by adding
 // in turn (ordered): no slower while a spare warp watches for the turn (64 x 8192 x
@@ -789,7 +793,10 @@ struct KSplit {
   int parts;
   bool ordered;
 };
-KSplit choose_ksplit(int tiles, int nkb, bool wide, int sms) {
+// The sharded form keeps the plain choice: split, the last CTA of a tile stores it to
+// every GPU in 8-byte pieces instead of 256-byte rows, a cost that the model does not
+// know (no timing on several GPUs).
+KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
   const int slots = wide ? sms : 2 * sms;
   const int most = max(1, min(nkb / 8, 2 * slots / tiles + 3));
   auto cost = [&](int k) {
@@ -799,6 +806,7 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, int sms) {
            (waves - 1) * (wide ? 16.0 : 9.0) + (k > 1 ? (wide ? 14.0 : 10.0) + 0.25 * k : 0.0);
   };
   const int plain = max(1, min(2 * sms / tiles, nkb / 8));
+  if (sharded) return {plain, false};
   int best = plain;
   double limit = 0.95 * cost(best);
   for (int k = 1; k <= most; k++)
@@ -806,13 +814,13 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, int sms) {
   return {best, plain <= 2 && best > 2};
 }
 
-QgemmParams make_params(void* Y_half, int Mb, int N, int K, int group_size, void* workspace,
-                        size_t workspace_bytes, int* status_word) {
+QgemmParams make_params(void* Y_half, bool sharded, int Mb, int N, int K, int group_size,
+                        void* workspace, size_t workspace_bytes, int* status_word) {
   QgemmParams prm;
   const int tiles = N / kTileN;
   KSplit split = {1, false};  // K is split only with a workspace
   if (workspace != nullptr && workspace_bytes >= qgemm_ws_bytes(Mb, N) && aligned16(workspace))
-    split = choose_ksplit(tiles, K / kBlockK, Mb > 64, sm_count());
+    split = choose_ksplit(tiles, K / kBlockK, Mb > 64, sharded, sm_count());
   prm.Y = reinterpret_cast<__half*>(Y_half);
   prm.peer_Y = nullptr;
   prm.y_offset = 0;
@@ -905,7 +913,8 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HQ_ERR_UNSUPPORTED;
   }
-  QgemmParams prm = make_params(Y_half, Mb, N, K, group_size, workspace, workspace_bytes, status_word);
+  QgemmParams prm = make_params(Y_half, po.peer_Y != nullptr, Mb, N, K, group_size, workspace,
+                                workspace_bytes, status_word);
   prm.peer_Y = reinterpret_cast<__half* const*>(po.peer_Y);
   prm.y_offset = po.y_offset;
   prm.world = po.world;
@@ -941,7 +950,8 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HQ_ERR_UNSUPPORTED;
   }
-  QgemmParams prm = make_params(Y_half, Mb, N, K, blocksize, workspace, workspace_bytes, status_word);
+  QgemmParams prm = make_params(Y_half, po.peer_Y != nullptr, Mb, N, K, blocksize, workspace,
+                                workspace_bytes, status_word);
   prm.absmax = absmax;
   prm.lut16 = lut16;
   prm.low_first = (flags & HQ_NF4_LOW_NIBBLE_FIRST) ? 1 : 0;

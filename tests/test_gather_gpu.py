@@ -241,3 +241,21 @@ def test_qgemm_peer_epilogue_equals_plain(hq, dev, fmt, Mb, N, K):
         assert torch.allclose(got[0].float(), plain.float(), rtol=2e-3, atol=2e-3)
     for b in bufs:
         assert bool((b[:offset] == 3).all()) and bool((b[offset + Mb * N:] == 3).all())
+
+
+def test_qgemm_peer_epilogue_wide_layer_in_one_part(hq, dev):
+    """A wide layer leaves the sharded epilogue in whole rows, K in one part, with
+    scratch at hand too: the bits of the product without scratch."""
+    import torch
+    Mb, K, N = 9, 8192, 20480
+    g = torch.Generator(device=dev).manual_seed(2)
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = torch.rand(N * K // 64, generator=g, device=dev) + 0.5
+    args = (X, B, absmax, torch.linspace(-1, 1, 16, device=dev), N, K, 64, 0)
+    want = hq.qgemm_nf4(*args, split_k=False)
+    bufs = [torch.zeros((Mb, N), dtype=torch.float16, device=dev) for _ in range(2)]
+    table = torch.tensor([b.data_ptr() for b in bufs], dtype=torch.int64, device=dev)
+    hq.qgemm_nf4(*args, peers=(table.data_ptr(), 0, 2))
+    torch.cuda.synchronize()
+    assert torch.equal(bufs[0], want) and torch.equal(bufs[1], want)
