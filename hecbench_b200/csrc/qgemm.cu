@@ -793,9 +793,9 @@ struct KSplit {
   int parts;
   bool ordered;
 };
-// The sharded form keeps the plain choice: split, the last CTA of a tile stores it to
-// every GPU in 8-byte pieces instead of 256-byte rows, a cost that the model does not
-// know (no timing on several GPUs).
+// The sharded form never takes more parts than the plain choice: split, the last CTA
+// of a tile stores it to every GPU in 8-byte pieces instead of 256-byte rows, a cost
+// that the model does not know (no timing on several GPUs).
 KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
   const int slots = wide ? sms : 2 * sms;
   const int most = max(1, min(nkb / 8, 2 * slots / tiles + 3));
@@ -806,10 +806,9 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
            (waves - 1) * (wide ? 16.0 : 9.0) + (k > 1 ? (wide ? 14.0 : 10.0) + 0.25 * k : 0.0);
   };
   const int plain = max(1, min(2 * sms / tiles, nkb / 8));
-  if (sharded) return {plain, false};
   int best = plain;
   double limit = 0.95 * cost(best);
-  for (int k = 1; k <= most; k++)
+  for (int k = 1; k <= (sharded ? min(most, plain) : most); k++)
     if (cost(k) < limit) { best = k; limit = cost(k); }
   return {best, plain <= 2 && best > 2};
 }
