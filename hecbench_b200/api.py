@@ -455,14 +455,10 @@ _qgemm_ws = {}
 
 
 def _qgemm_workspace(lib, X, Mb: int, N: int):
-    """Zero-initialised split-K scratch, one per (device, stream, Mb, N): calls on
-    different streams may overlap on the GPU and must not share the fp32 partial
-    sums and tile counters."""
-    key = (lib.host.place(X), Mb, N)
-    ws = _qgemm_ws.get(key)
-    if ws is None:
-        ws = torch.zeros(lib.hq_qgemm_workspace_bytes(Mb, N), dtype=torch.uint8, device=X.device)
-        _qgemm_ws[key] = ws
+    """Split-K scratch (fp32 partial sums and tile counters), one per (device, stream,
+    Mb, N)."""
+    ws = _stream_scratch(_qgemm_ws, (lib.host.place(X), Mb, N),
+                         lib.hq_qgemm_workspace_bytes(Mb, N), X)
     return ws, ws.numel()
 
 

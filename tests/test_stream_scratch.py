@@ -50,6 +50,18 @@ def test_lutgemm_scratch_of_a_capture_is_not_kept(place):
     assert w.workspace() is c                    # cleared by an eager call on this stream
 
 
+def test_qgemm_scratch_of_a_capture_is_not_kept(place, monkeypatch):
+    from hecbench_b200 import api
+    monkeypatch.setattr(api, "_qgemm_ws", {})
+    lib, X = api.load_library(), torch.zeros(2, 64)
+    place.capturing = True
+    a, n = api._qgemm_workspace(lib, X, 2, 128)
+    assert n == 4 * 2 * 128
+    place.capturing = False
+    b, _ = api._qgemm_workspace(lib, X, 2, 128)
+    assert b is not a and api._qgemm_workspace(lib, X, 2, 128)[0] is b
+
+
 @pytest.mark.gpu
 def test_one_layer_on_two_streams(hq, dev):
     """Two streams multiply by the same layer at the same time; sums meet in no fixed
@@ -96,6 +108,31 @@ def test_graph_before_its_stream_has_scratch(hq, dev):
         with torch.cuda.graph(graph, stream=s):
             hq.matmul(replayed, x, w)
         hq.matmul(eager, x, w)
+        graph.replay()
+        graph.replay()
+    torch.cuda.synchronize()
+    for o in (eager, replayed):
+        assert float((o.float() - want.float()).norm() / want.float().norm()) < 2 ** -10
+
+
+@pytest.mark.gpu
+def test_qgemm_graph_before_its_stream_has_scratch(hq, dev):
+    """As above for the batched product with K split over several CTAs."""
+    Mb, K, N = 16, 4096, 640
+    g = torch.Generator(device=dev).manual_seed(6)
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = torch.rand(N * K // 64, generator=g, device=dev)
+    args = (X, B, absmax, torch.linspace(-1, 1, 16, device=dev), N, K, 64)
+    want = hq.qgemm_nf4(*args)
+    eager, replayed = torch.zeros_like(want), torch.zeros_like(want)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            hq.qgemm_nf4(*args, out=replayed)
+        hq.qgemm_nf4(*args, out=eager)
         graph.replay()
         graph.replay()
     torch.cuda.synchronize()
