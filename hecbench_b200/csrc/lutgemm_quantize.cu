@@ -29,6 +29,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "hq_common.cuh"
 
@@ -38,8 +39,15 @@ namespace {
 constexpr int kColsPerCta = 64;   // two per lane
 constexpr int kMaxRuns = 16;      // runs of 32 inputs per group = warps per CTA (group_size <= 512)
 
+// Whether a row of the weights is less than 4 GiB, so that its length fits 32 bits (the
+// 64-bit form of the addresses costs 1 to 4 %).
+constexpr bool row_fits_32(int M, int bytes) { return (unsigned)M <= 0xffffffffu / bytes; }
+static_assert(!row_fits_32(1 << 30, 4) && row_fits_32((1 << 30) - 2, 4) && row_fits_32(INT_MAX, 2),
+              "fp32 rows of 2^30 columns on are longer");
+
 // RUNS: runs of 32 inputs per group where it is a compile-time constant, else 0.
-template <int DTYPE, int RUNS>
+// Pitch: the type that holds the bytes of a row.
+template <int DTYPE, int RUNS, typename Pitch>
 __global__ void __launch_bounds__(RUNS ? RUNS * 32 : kMaxRuns * 32)
 bcq_quantize_kernel(const void* __restrict__ W, int K, int M, int nb, int gs,
                     uint32_t* __restrict__ bW, __half* __restrict__ alpha,
@@ -57,7 +65,7 @@ bcq_quantize_kernel(const void* __restrict__ W, int K, int M, int nb, int gs,
   {
     constexpr int kBytes = DTYPE == HQ_DTYPE_F32 ? 4 : 2;
     const char* p = reinterpret_cast<const char*>(W) + ((size_t)k0 * M + min(m, M - 2)) * kBytes;
-    const uint32_t step = (uint32_t)M * kBytes;
+    const Pitch step = (Pitch)(unsigned)M * kBytes;
 #pragma unroll
     for (int t = 0; t < 32; t++) {
       const char* at = p + (unsigned long long)t * step;
@@ -180,10 +188,12 @@ int run(const void* W, int K, int M, int nb, int gs, uint32_t* bW, void* alpha, 
   const dim3 grid((M + kColsPerCta - 1) / kColsPerCta, K / gs);
   __half* al = reinterpret_cast<__half*>(alpha);
   __half* qb = reinterpret_cast<__half*>(q_bias);
-  if (gs == 128)  // the usual group: its exchange is unrolled
-    bcq_quantize_kernel<DTYPE, 4><<<grid, gs, 0, st>>>(W, K, M, nb, gs, bW, al, qb);
+  if (DTYPE == HQ_DTYPE_F32 && !row_fits_32(M, 4))
+    bcq_quantize_kernel<HQ_DTYPE_F32, 0, unsigned long long><<<grid, gs, 0, st>>>(W, K, M, nb, gs, bW, al, qb);
+  else if (gs == 128)  // the usual group: its exchange is unrolled
+    bcq_quantize_kernel<DTYPE, 4, uint32_t><<<grid, gs, 0, st>>>(W, K, M, nb, gs, bW, al, qb);
   else
-    bcq_quantize_kernel<DTYPE, 0><<<grid, gs, 0, st>>>(W, K, M, nb, gs, bW, al, qb);
+    bcq_quantize_kernel<DTYPE, 0, uint32_t><<<grid, gs, 0, st>>>(W, K, M, nb, gs, bW, al, qb);
   return launch_status();
 }
 
