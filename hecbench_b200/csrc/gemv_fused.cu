@@ -184,13 +184,14 @@ int launch(FusedParams prm, hq_stream_t stream) {
     return HQ_ERR_BAD_SHAPE;
   if (!aligned16(prm.mat) || !aligned16(prm.x) || (prm.gamma && !aligned16(prm.gamma)))
     return HQ_ERR_MISALIGNED;
-  const size_t smem = (size_t)prm.n * 2;
-  if (smem > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
+  // beyond 113 KiB only one CTA fits an SM
+  if ((size_t)prm.n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;
+  const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
+  const int grid = std::min(2 * sm_count(), (rows_mat + kWarps * kRows - 1) / (kWarps * kRows));
+  const size_t smem = smem_request((size_t)prm.n * 2, grid);
   constexpr auto kern = gemv_fused_kernel<BITS>;
   const cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
-  const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
-  const int grid = std::min(2 * sm_count(), (rows_mat + kWarps * kRows - 1) / (kWarps * kRows));
   return cuda_status(
       launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream, prm));
 }

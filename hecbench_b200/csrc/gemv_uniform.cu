@@ -127,15 +127,15 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   // 16-byte groups: n a multiple of 8 (fp16), 16 (int8), 32 (int4)
   if (rows <= 0 || n <= 0 || n % (128 / BITS) != 0) return HQ_ERR_BAD_SHAPE;
   if (!aligned16(mat) || !aligned16(vec_half)) return HQ_ERR_MISALIGNED;
-  const size_t smem = (size_t)n * 2;
-  if (smem > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
+  if ((size_t)n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
+  const int grid = std::min(2 * sm_count(), (rows + kWarps * kRows - 1) / (kWarps * kRows));
+  const size_t smem = smem_request((size_t)n * 2, grid);
   constexpr auto kern = gemv_uniform_kernel<BITS>;
   const cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
   // the launcher of the reference rounds both parameters to fp16 (gemv.cu:21-22)
   const float s = __half2float(__float2half_rn(scale));
   const float z = __half2float(__float2half_rn(zero_point));
-  const int grid = std::min(2 * sm_count(), (rows + kWarps * kRows - 1) / (kWarps * kRows));
   return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream,
                                 reinterpret_cast<const unsigned char*>(mat),
                                 reinterpret_cast<const __half*>(vec_half),

@@ -43,7 +43,9 @@ def _dev_kw(kw, dev):
     (1000, 2048, 2, True),     # GeGLU
     (512, 1024, 0, True),      # RMSNorm + plain mat-vec
     (333, 2048, 1, False),     # no normalisation, an odd number of outputs
-    (7, 8192, 0, False)])      # plain mat-vec, an odd number of rows (a lone last row)
+    (7, 8192, 0, False),       # plain mat-vec, an odd number of rows (a lone last row)
+    (4704, 1024, 0, True), (4736, 1024, 0, True), (4737, 1024, 0, False),  # one CTA per SM and around
+    (2368, 2048, 1, True)])    # the same as pairs of rows
 def test_fused_against_oracle(hq, oracle, dev, fmt, rows_out, n, act, norm):
     rows_mat = rows_out * (2 if act else 1)
     x, gamma, mat, kw = _case(fmt, rows_mat, n, seed=rows_out + n + act)

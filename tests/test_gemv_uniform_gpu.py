@@ -43,6 +43,30 @@ def test_gemv_uniform_against_oracle(hq, oracle, dev, bits, rows, n, scale, zp):
     assert oracle.rel_err(y.cpu().numpy().astype(np.float64), ref) < TOL_F16
 
 
+@pytest.mark.parametrize("bits", [8, 4, 16])
+@pytest.mark.parametrize("extra,n", [(-33, 64), (-1, 4096), (0, 1024), (1, 1024), (0, 60032)])
+def test_gemv_uniform_around_one_cta_per_sm(hq, oracle, dev, bits, extra, n):
+    """32 rows per CTA: one CTA per SM less one, exactly one, one more; rows whose inputs
+    alone take more than half an SM's shared memory.  Each call reads the output of the
+    one before as part of its input."""
+    import torch
+    rows = 32 * torch.cuda.get_device_properties(dev).multi_processor_count + extra
+    mat, vec = synth.gemv_uniform_case(rows, n, bits, seed=rows + n + bits)
+    dm, dv = to_dev(mat, dev), to_dev(vec, dev)
+    call = {16: lambda v: hq.gemv_fp16(dm, v), 8: lambda v: hq.gemv_int8_quantized(dm, v, 2 ** -9, 0.5),
+            4: lambda v: hq.gemv_int4_quantized(dm, v, 2 ** -9, 0.5)}[bits]
+    chain = [dv]
+    for _ in range(4):
+        y = call(chain[-1])
+        chain.append(torch.cat([y[:32] * 2 ** -12, chain[-1][32:]]))
+    torch.cuda.synchronize()
+    for a, b in zip(chain, chain[1:]):
+        ref = oracle.gemv_uniform_f64(mat, a.cpu().numpy(), bits, 2 ** -9, 0.5)
+        got = call(a).cpu().numpy().astype(np.float64)
+        assert oracle.rel_err(got, ref) < TOL_F16
+        assert torch.equal(b[:32], torch.from_numpy(got[:32]).to(torch.float16).to(dev) * 2 ** -12)
+
+
 def test_gemv_uniform_signed_inputs_and_extreme_codes(hq, oracle, dev):
     """Inputs of both signs (the reference only draws U(0,1)), all-minimum and
     all-maximum codes: the sign-flip / exponent-byte conversion of int8 and the
