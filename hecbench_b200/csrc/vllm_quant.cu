@@ -244,8 +244,9 @@ vllm_dynamic_vec_kernel(const T* __restrict__ in, int8_t* __restrict__ out,
 #pragma unroll
       for (int k = 0; k < 4; k++) ext.template take<!AZP>(w[k]);
     } else if (first < end) {
-      // a row boundary: the neighbour's elements are replaced by one of this row (the
-      // chunk's first or last, whichever end of the row it holds)
+      // a row boundary: the neighbour's elements are replaced by zeros for the largest
+      // magnitude, else by one of this row (the chunk's first or last, whichever end of
+      // the row it holds)
       const int own = max(skip - first, 0);
       const T* e = reinterpret_cast<const T*>(&raw[j]);
 #pragma unroll
@@ -256,9 +257,9 @@ vllm_dynamic_vec_kernel(const T* __restrict__ in, int8_t* __restrict__ out,
           const int i = EPW * k + h, at = first + i;
           T x = e[i];
           if (at < skip || at >= end) {
-            x = e[0];
+            x = AZP ? e[0] : T(0.f);
 #pragma unroll
-            for (int o = 1; o < EPC; o++) x = o == own ? e[o] : x;
+            for (int o = 1; o < EPC; o++) x = AZP && o == own ? e[o] : x;
           }
           if (EPW == 2) u |= (uint32_t)*reinterpret_cast<const unsigned short*>(&x) << (16 * h);
           else u = *reinterpret_cast<const uint32_t*>(&x);
@@ -446,11 +447,15 @@ int dynamic_launch_ept(int8_t* out, const T* x, float* scales, int* azp, int tok
   // slots of its whole-warp block without a chunk (a row of 644 chunks: 3 x 224
   // threads) among blocks of at most 256 threads, so that some of an SM's blocks
   // load while others store (8192 x 16384 fp16: 62 us, with blocks of 512 and 1024
-  // threads 79 and 91); one chunk per thread where few rows leave only the block
-  // itself to fill the SM, larger blocks where the row needs them.
+  // threads 79 and 91), larger blocks where the row needs them.  One chunk per thread
+  // where a warp covers the row and where there are too few rows to fill the SMs: below
+  // two per SM, or 24 warps per SM in all (300 x 1025 fp16, 10 warps per SM: 1.83 us,
+  // with two chunks per thread 2.46; 900 x 1025, 30: 2.21 and 2.62; 1800 x 1025, 61:
+  // 3.62 and 3.23; 900 x 2049, 55: 3.03 and 2.86).
   int cpt = 0, threads = 0;
   if (aligned16(x) && aligned8(out) && chunks <= 8L * 1024) {
-    const int lo = tokens < 2 * sm_count() ? 1 : 2;
+    const long sms = sm_count(), warps = (chunks + 31) / 32;
+    const int lo = warps == 1 || tokens < 2 * sms || tokens * warps <= 24 * sms ? 1 : 2;
     long best = 0;
     for (int c = lo; c <= 8; c++) {
       const long th = (chunks + c - 1) / c, w = (th + 31) / 32 * 32;

@@ -80,7 +80,8 @@ def test_vllm_quant_matches_oracle(hq, oracle, dev, dtype, tokens, hidden):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tokens,hidden", [(300, 7), (300, 8), (297, 15), (299, 2041), (298, 2057),
-                                           (296, 4103), (1, 8191), (2, 16385), (297, 16389)])
+                                           (296, 4103), (1, 8191), (2, 16385), (297, 16389), (710, 1025),
+                                           (711, 1025), (300, 255), (300, 257)])
 def test_vllm_quant_block_shapes(hq, oracle, dev, dtype, tokens, hidden):
     """Row lengths around the chunks-per-thread and block-size choices, rows that share
     their boundary chunks, quotients on and beside ties."""
