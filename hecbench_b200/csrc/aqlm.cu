@@ -15,6 +15,8 @@
 // 2x8: both codebooks (8 KiB) live in shared memory, replicated 8 times with
 // entry e of replica r at 16-byte slot 8*e + r, so the 8 lanes that a 128-bit
 // shared load serves per cycle (r = lane % 8) always hit distinct bank groups.
+#include <algorithm>
+
 #include "hq_common.cuh"
 
 namespace hq {
@@ -272,8 +274,6 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const size_t smem = (size_t)2 * 256 * 8 * 16 + (size_t)kPad * ((groups + 7) / 8) * 16;
   if (smem > 220 * 1024) return HQ_ERR_TOO_LARGE;
   constexpr auto kern2x8 = aqlm_2x8_kernel;
-  cudaError_t e = ensure_dynamic_smem<kern2x8>(smem);
-  if (e != cudaSuccess) return cuda_status(e);
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps2x8);
   const int rows_per_cta = kWarps2x8 * rows_per_warp;
   const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
@@ -283,11 +283,18 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const auto cb = reinterpret_cast<const uint4*>(codebooks);
   const auto sc = reinterpret_cast<const __half*>(scales_half);
   const cudaStream_t st = (cudaStream_t)stream;
-  // early start as for 1x16, from two CTAs per SM on: 14336 x 4096 28.5 -> 26.3 us;
-  // 2048 x 4096 takes 8.2 us plain and 9.1 with it, and in a replayed graph 4096 x
-  // 4096 (256 CTAs) 8.0 and 9.5
+  // Early start as for 1x16, from two CTAs per SM on.  The CTAs of an early start would
+  // go wherever there is room; shared memory is asked for so that an SM holds no more of
+  // them than the fullest SM takes anyway.  Three of up to 4992 inputs would fit: 296
+  // CTAs (4736 x 4096) 7.6 us in a graph and 10.3 as calls without the early start, 9.2
+  // and 9.3 with it, 7.5 and 7.8 held to two per SM; 9472 x 4096, 296 CTAs of 32 rows:
+  // 12.6 and 14.5, 15.4 and 15.5, 12.5 and 12.7.
+  const int per_sm = (grid + sm_count() - 1) / sm_count();
+  const size_t request = std::max(smem, (size_t)228 * 1024 / (per_sm + 1) - 1024 + 16);
+  cudaError_t e = ensure_dynamic_smem<kern2x8>(request);
+  if (e != cudaSuccess) return cuda_status(e);
   if (grid >= 2 * sm_count())
-    return cuda_status(launch_pdl(kern2x8, dim3(grid), dim3(kWarps2x8 * 32), smem, st, c, x, o, cb,
+    return cuda_status(launch_pdl(kern2x8, dim3(grid), dim3(kWarps2x8 * 32), request, st, c, x, o, cb,
                                   prob_m, prob_k, sc, rows_per_warp));
   kern2x8<<<grid, kWarps2x8 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sc, rows_per_warp);
   return launch_status();

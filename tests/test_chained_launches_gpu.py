@@ -6,12 +6,15 @@ sums of split rows meet in no fixed order, hence 5e-3 of the 2-norm after six ca
 import pytest
 
 pytestmark = pytest.mark.gpu
-SIZE = 4096
 
 
 def _calls(hq, family, dev):
     """call(x, out) and the shape of x and out."""
     import torch
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    # 2x8 starts early from two CTAs of 16 rows (64 from 64 * SMs rows on: 32 rows) per SM
+    # on, where SMs are not evenly full or hold no third CTA
+    SIZE = {"aqlm 2x8": 64 * (sms // 2 + 4), "aqlm 2x8 long": 64 * sms}.get(family, 4096)
     g = torch.Generator(device=dev)
     g.manual_seed(11)
 
@@ -30,32 +33,79 @@ def _calls(hq, family, dev):
         c = codes(SIZE, SIZE // 4).view(torch.int16)
         book = (torch.randn((1, 65536, 8), generator=g, device=dev) * 0.016).half()
         return lambda x, out: hq.code1x16_matvec(c, x, out, book, SIZE, SIZE, [SIZE] * 4, 65536), (SIZE,)
-    if family == "aqlm 2x8":
+    if family.startswith("aqlm 2x8"):
+        rows = 32 if family.endswith("long") else 16
+        assert SIZE // rows >= 2 * sms and (rows == 32) == (SIZE // 32 >= 2 * sms)
         c = codes(SIZE, SIZE // 8, 2)
-        book = (torch.randn((2, 256, 8), generator=g, device=dev) * 0.011).half()
+        book = (torch.randn((2, 256, 8), generator=g, device=dev) * (0.5 / SIZE) ** 0.5).half()
         return lambda x, out: hq.code2x8_matvec(c, x, out, book, SIZE, SIZE), (SIZE,)
+    if family == "qgemm q3":
+        words = codes(SIZE * 3 // 8, SIZE).view(torch.int32).view(SIZE * 3 // 32, SIZE)
+        scales = uniform(0.8, 1.2, SIZE // 128, SIZE).div(2.3 * SIZE ** 0.5).half()
+        zeros = scales * 3.5
+        return lambda x, out: hq.qgemm_q3(x, words, scales, zeros, SIZE, SIZE, 128, out=out), (48, SIZE)
     mat = codes(SIZE, SIZE // 2)
     absmax = uniform(0.5, 2.0, SIZE * SIZE // 64) / SIZE ** 0.5
     lut = torch.linspace(-1, 1, 16, device=dev)
     return lambda x, out: hq.qgemm_nf4(x, mat, absmax, lut, SIZE, SIZE, 64, out=out), (48, SIZE)
 
 
-@pytest.mark.parametrize("family", ["lutgemm", "aqlm 1x16", "aqlm 2x8", "qgemm"])
-def test_each_launch_waits_for_the_one_before(hq, dev, family):
+@pytest.mark.parametrize("replayed", [False, True])
+@pytest.mark.parametrize("family", ["lutgemm", "aqlm 1x16", "aqlm 2x8", "aqlm 2x8 long", "qgemm",
+                                    "qgemm q3"])
+def test_each_launch_waits_for_the_one_before(hq, dev, family, replayed):
     import torch
     call, shape = _calls(hq, family, dev)
     x0 = torch.randn(shape, generator=torch.Generator(device=dev).manual_seed(5), device=dev).half()
 
+    a0, b0 = x0.clone(), torch.zeros_like(x0)
+
     def chain(sync):
-        a, b = x0.clone(), torch.zeros_like(x0)
+        a, b = a0, b0
+        a.copy_(x0)
         for _ in range(6):
             call(a, b)
             if sync:
                 torch.cuda.synchronize()
             a, b = b, a
-        return a.float()
+        return a
 
-    want = chain(True)
+    want = chain(True).float()
     assert bool(torch.isfinite(want).all()) and float(want.norm()) > 0
+    if replayed:
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            chain(False)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=s):
+                chain(False)
     for _ in range(20):
-        assert float((chain(False) - want).norm() / want.norm()) < 5e-3
+        if replayed:
+            graph.replay()
+            got = a0
+        else:
+            got = chain(False)
+        assert float((got.float() - want).norm() / want.norm()) < 5e-3
+
+
+@pytest.mark.parametrize("per_cta,ctas_per_sm,extra", [(16, 2, -1), (16, 2, 0), (16, 2, 1), (16, 3, 0),
+                                                       (32, 2, 0), (32, 2, 1), (32, 3, 5)])
+def test_2x8_around_the_early_start(hq, dev, per_cta, ctas_per_sm, extra):
+    """Row counts around two and three CTAs per SM, 16 and 32 rows per CTA, against the
+    product of the decoded weights in fp64; the kernel rounds sums of 16 products to fp16
+    (2^-11 of a sum whose terms are a few times larger), so 1e-2 of the rms."""
+    import torch
+    m = per_cta * ctas_per_sm * torch.cuda.get_device_properties(dev).multi_processor_count + extra
+    k = 192
+    g = torch.Generator(device=dev).manual_seed(m)
+    codes = torch.randint(0, 256, (m, k // 8, 2), generator=g, device=dev, dtype=torch.uint8)
+    book = torch.randn((2, 256, 8), generator=g, device=dev).half()
+    x = torch.randn(k, generator=g, device=dev).half()
+    out = torch.full((m + 8,), 3.0, dtype=torch.float16, device=dev)
+    for _ in range(2):
+        hq.code2x8_matvec(codes, x, out[:m], book, m, k)
+    w = sum(book[i].double()[codes[..., i].long()] for i in range(2)).view(m, k)
+    want = w @ x.double()
+    assert float((out[:m].double() - want).abs().max() / want.pow(2).mean().sqrt()) < 1e-2
+    assert bool((out[m:] == 3).all())
