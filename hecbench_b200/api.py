@@ -433,11 +433,22 @@ def code1x16_matvec(A, B, C_out, codebook, prob_m: int, prob_k: int,
                     scales: Optional[torch.Tensor] = None) -> None:
     """code1x16_matvec (quantAQLM-cuda/main.cu:113-141).  A = codes (int16 or
     uint16, [prob_m][prob_k/8]), B = input half[prob_k], C_out = half[prob_m]
-    (overwritten), codebook half[..][65536][8]; `scales` is an extension."""
+    (overwritten), codebook half[..][65536][8]; `scales` is an extension.
+    prob_k <= 8192.  codebook_a_sizes: up to four numbers, those left out count as 0;
+    row m takes the codebook as many strides in as there are values <= m among the
+    first three."""
     if A.dtype not in (torch.int16, torch.uint16):
         raise TypeError("A: expected int16/uint16 codes")
-    load_library().host.hq_aqlm_1x16_matvec(A, B, C_out, codebook, prob_m, prob_k,
-                                            codebook_a_sizes, codebook_stride, scales)
+    sizes = codebook_a_sizes
+    if not isinstance(sizes, (list, tuple)):
+        sizes = list(sizes)
+    if len(sizes) < 3:
+        # a limit of 0 moves every row on: the codebook that the rows reach must be there
+        last = sum(int(v) < prob_m for v in [*sizes, 0, 0, 0][:3])
+        if (last * codebook_stride + 65536) * 8 > codebook.numel():
+            raise ValueError("codebook_a_sizes: rows beyond the last codebook")
+    load_library().host.hq_aqlm_1x16_matvec(A, B, C_out, codebook, prob_m, prob_k, sizes,
+                                            codebook_stride, scales)
 
 
 def code2x8_matvec(A, B, C_out, codebooks, prob_m: int, prob_k: int,

@@ -77,7 +77,7 @@ constexpr Param O(const char* name, at::ScalarType t) { return {Kind::kOptionalT
 constexpr Param R(const char* name) { return {Kind::kRaw, name, at::kByte}; }
 constexpr Param I() { return {Kind::kInt, nullptr, at::kByte}; }
 constexpr Param F() { return {Kind::kFloat, nullptr, at::kByte}; }
-// a sequence of four whole numbers, passed as const int[4]
+// up to four numbers, zeros for the rest, passed as const int[4]
 constexpr Param S(const char* name) { return {Kind::kFourInts, name, at::kByte}; }
 constexpr auto f32 = at::kFloat;
 constexpr auto f16 = at::kHalf;
@@ -247,13 +247,19 @@ PyObject* entry_call(PyObject* self_, PyObject* const* args, size_t nargsf, PyOb
       case Kind::kFourInts: {
         PyObject* seq = PySequence_Fast(args[k], q.name);
         if (!seq) return nullptr;
-        if (PySequence_Fast_GET_SIZE(seq) != 4) {
+        const Py_ssize_t given = PySequence_Fast_GET_SIZE(seq);
+        if (given > 4) {
           Py_DECREF(seq);
-          PyErr_Format(PyExc_ValueError, "%s: expected four numbers", q.name);
+          PyErr_Format(PyExc_ValueError, "%s: expected at most four numbers", q.name);
           return nullptr;
         }
-        for (int i = 0; i < 4; i++)
-          four[i] = (int)PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i));
+        for (int i = 0; i < 4; i++) four[i] = 0;
+        for (Py_ssize_t i = 0; i < given; i++) {  // what int() takes
+          PyObject* whole = PyNumber_Long(PySequence_Fast_GET_ITEM(seq, i));
+          if (!whole) break;
+          four[i] = (int)PyLong_AsUnsignedLongLongMask(whole);
+          Py_DECREF(whole);
+        }
         Py_DECREF(seq);
         if (PyErr_Occurred()) return nullptr;
         v[k].p = four;
