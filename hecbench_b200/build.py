@@ -86,8 +86,9 @@ def build_host(force: bool = False) -> Path:
     import torch
 
     src = CSRC / "host" / "host.cpp"
-    if force or _newer(HOST_EXT, [src]):
-        base = Path(torch.__file__).parent
+    base = Path(torch.__file__).parent
+    # rebuilt for another torch too: the extension uses its C++ interface
+    if force or _newer(HOST_EXT, [src, base / "version.py"]):
         cuda = Path(NVCC).resolve().parent.parent
         cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
