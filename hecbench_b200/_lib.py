@@ -122,7 +122,7 @@ def _attach(lib):
         fn.restype = res
         fn.argtypes = args
     lib.host = SimpleNamespace(
-        empty=_host.empty, place=_host.place,
+        empty=_host.empty, place=_host.place, capturing=_host.capturing,
         **{name: _host.Entry(name, C.cast(getattr(lib, name), C.c_void_p).value, check)
            for name in _host.symbols})
     return lib

@@ -350,7 +350,7 @@ def gemv_fused(fmt: str, x, mat, rows_out: int, *, gamma=None, eps: float = 1e-5
 # lut-gemm
 # --------------------------------------------------------------------------
 
-def _stream_scratch(cache: dict, key, nbytes: int, like: torch.Tensor) -> torch.Tensor:
+def _stream_scratch(host, cache: dict, key, nbytes: int, like: torch.Tensor) -> torch.Tensor:
     """The zero-initialised scratch of `cache` for `key`, which names the device and
     current stream of `like`: calls on different streams may overlap on the GPU and
     must not share partial sums and counters.  Scratch that is first needed while the
@@ -359,9 +359,8 @@ def _stream_scratch(cache: dict, key, nbytes: int, like: torch.Tensor) -> torch.
     ws = cache.get(key)
     if ws is None:
         ws = torch.zeros(nbytes, dtype=torch.uint8, device=like.device)
-        with torch.cuda.device(like.device):
-            if not torch.cuda.is_current_stream_capturing():
-                cache[key] = ws
+        if not host.capturing(like):
+            cache[key] = ws
     return ws
 
 
@@ -410,7 +409,7 @@ class nQWeight_fp16:
         """Zero-initialised fp32 scratch the kernel accumulates K tiles into, one per
         device and current stream; it is left zero by every call."""
         lib = load_library()
-        return _stream_scratch(self._ws, (lib.host.place(self.bWeight), self.mSize),
+        return _stream_scratch(lib.host, self._ws, (lib.host.place(self.bWeight), self.mSize),
                                lib.hq_lutgemm_workspace_bytes(self.mSize), self.bWeight)
 
 
@@ -468,7 +467,7 @@ _qgemm_ws = {}
 def _qgemm_workspace(lib, X, Mb: int, N: int):
     """Split-K scratch (fp32 partial sums and tile counters), one per (device, stream,
     Mb, N)."""
-    ws = _stream_scratch(_qgemm_ws, (lib.host.place(X), Mb, N),
+    ws = _stream_scratch(lib.host, _qgemm_ws, (lib.host.place(X), Mb, N),
                          lib.hq_qgemm_workspace_bytes(Mb, N), X)
     return ws, ws.numel()
 

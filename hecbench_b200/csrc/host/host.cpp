@@ -16,6 +16,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -341,10 +342,24 @@ PyObject* host_place(PyObject*, PyObject* t) {
   END_HANDLE_TH_ERRORS
 }
 
+// capturing(t): whether the current stream on the device of t is being captured.
+PyObject* host_capturing(PyObject*, PyObject* t) {
+  HANDLE_TH_ERRORS
+  if (!THPVariable_Check(t) || !THPVariable_Unpack(t).is_cuda()) {
+    PyErr_SetString(PyExc_TypeError, "expected a CUDA tensor (there is no CPU path)");
+    return nullptr;
+  }
+  c10::cuda::CUDAGuard guard(THPVariable_Unpack(t).device().index());
+  return PyBool_FromLong(c10::cuda::currentStreamCaptureStatusMayInitCtx() !=
+                         c10::cuda::CaptureStatus::None);
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef kMethods[] = {
     {"empty", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&host_empty)), METH_FASTCALL,
      nullptr},
     {"place", &host_place, METH_O, nullptr},
+    {"capturing", &host_capturing, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods};

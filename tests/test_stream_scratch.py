@@ -1,6 +1,5 @@
 """Scratch of calls whose partial sums meet in device memory: one per stream, and
 none kept from a stream capture."""
-import contextlib
 from types import SimpleNamespace
 
 import pytest
@@ -12,12 +11,11 @@ def place(monkeypatch):
     """The fake library's device and stream, on the CPU."""
     from hecbench_b200 import api
     state = SimpleNamespace(where=(0, 1), capturing=False)
-    fake = SimpleNamespace(host=SimpleNamespace(place=lambda t: state.where),
+    fake = SimpleNamespace(host=SimpleNamespace(place=lambda t: state.where,
+                                                capturing=lambda t: state.capturing),
                            hq_lutgemm_workspace_bytes=lambda m: 4 * m,
                            hq_qgemm_workspace_bytes=lambda m, n: 4 * m * n)
     monkeypatch.setattr(api, "load_library", lambda: fake)
-    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
     return state
 
 
