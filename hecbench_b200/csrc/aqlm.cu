@@ -9,8 +9,8 @@
 // kernel.  What changes is the memory behaviour: all code vectors of a row and
 // all their 16-byte gathers are issued before any arithmetic (up to 16 gathers
 // in flight per lane instead of 1), a warp walks several rows, and the 1 MiB
-// codebook is read through the read-only path so that it stays L2-resident
-// while the codes stream past it without allocating in L1.
+// codebook goes through L1 and stays L2-resident while the codes stream past it
+// without allocating in L1.
 //
 // 2x8: both codebooks (8 KiB) live in shared memory, replicated 8 times with
 // entry e of replica r at 16-byte slot 8*e + r, so the 8 lanes that a 128-bit
@@ -42,6 +42,8 @@ __device__ __forceinline__ float dot8_ref_order(const uint4& a, const uint4& b) 
   return __half2float(__low2half(r)) + __half2float(__high2half(r));
 }
 
+constexpr int kMaxVpl1x16 = 4;  // code vectors per lane and row: up to 8192 inputs
+
 // Four of a thread's 16-byte pieces of the inputs, g0, g0 + 256, ...: all loads in
 // flight, then to shared memory.
 struct InputPieces {
@@ -60,14 +62,16 @@ struct InputPieces {
   }
 };
 static_assert(kWarps1x16 * 32 == 256 && kWarps2x8 * 32 == 256, "stride of InputPieces");
+static_assert(kMaxVpl1x16 * 32 * 8 <= 4 * 256, "the 1x16 kernel stages its inputs in one turn");
 
 // VPL = 16-byte code vectors per lane per row (prob_k / 64 / 32 rounded up),
 // RPW = rows per warp.  The dependent chain code -> codebook row -> FMA is what
 // bounds this kernel, so everything that does not depend on the input vector
-// is issued first: the code vectors of ALL rows of the warp, then the gathers
-// of the first vector, and only then the CTA stages the inputs in shared
-// memory; afterwards the gathers of vector u + 1 are in flight while vector u
-// is multiplied.  The arithmetic (and its order) is the reference's.
+// is issued early: the code vectors of ALL rows of the warp, the inputs, then,
+// as the codes arrive, the gathers of the first vector; the inputs go to shared
+// memory while those are under way, and afterwards the gathers of vector u + 1
+// are in flight while vector u is multiplied.  The arithmetic (and its order) is
+// the reference's.
 template <int VPL, int RPW>
 __global__ void __launch_bounds__(kWarps1x16 * 32)
 aqlm_1x16_kernel(const uint4* codes, const uint4* x,
@@ -79,7 +83,8 @@ aqlm_1x16_kernel(const uint4* codes, const uint4* x,
   const int vec_per_row = prob_k >> 6;
   const int row_begin = (blockIdx.x * kWarps1x16 + warp) * RPW;
   // the next kernel of the stream may become resident while this grid drains;
-  // nothing is read or written before every earlier kernel has completed
+  // nothing is read or written before every earlier kernel has completed (codes,
+  // codebook and scales may be their output: ordered loads below)
   pdl_launch_dependents();
   pdl_wait();
   constexpr int kUnits = RPW * VPL;  // unit u = (row u / VPL, vector u % VPL)
@@ -220,16 +225,17 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
   if (!aligned16(codes) || !aligned16(x_half) || !aligned16(codebook)) return HQ_ERR_MISALIGNED;
   const int vec_per_row = prob_k / 64;
   const int vpl = (vec_per_row + 31) / 32;
-  if (vpl > 4) return HQ_ERR_TOO_LARGE;  // prob_k <= 8192
+  if (vpl > kMaxVpl1x16) return HQ_ERR_TOO_LARGE;
   const int groups = prob_k / 8;
   const size_t smem = (size_t)kPad * ((groups + 7) / 8) * 16;
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps1x16);
   const int rows_per_cta = kWarps1x16 * rows_per_warp;
   const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
   // A grid that fills the SMs starts while the one before it drains (4096 x 4096
-  // back to back: 12.4 -> 11.0 us).  A smaller one does not: the CTAs of an early
-  // start are not spread over all SMs, and the gathers are bound by each SM's L1
-  // (1024 x 8192: 13.2 us, 18.9 with the early start).
+  // back to back: 12.4 -> 11.0 us; in a replayed graph 10.7 -> 10.6, and 2368 x 4096,
+  // 148 CTAs, 6.6 -> 6.4).  A smaller one does not: the CTAs of an early start are not
+  // spread over all SMs, and the gathers are bound by each SM's L1 (1024 x 8192: 13.2
+  // us, 18.9 with the early start; 2048 x 4096 in a graph 6.6 and 10.0).
   const int4 sizes = make_int4(cb_sizes[0], cb_sizes[1], cb_sizes[2], cb_sizes[3]);
   cudaStream_t st = (cudaStream_t)stream;
 #define HQ_AQLM_LAUNCH(VPL, RPW)                                                             \

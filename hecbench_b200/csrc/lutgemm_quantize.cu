@@ -19,13 +19,12 @@
 // sums through shared memory (one barrier), every thread adds them in order,
 // takes the signs of its residuals, updates them in registers and stores its two
 // words.  The weights are read once; nothing else touches memory.
-// The bound is instruction issue (20 per weight for three planes, 80 % of the
+// The bound is instruction issue (20.2 per weight for three planes, 85 % of the
 // slots busy): the bits come from the residual's sign (one funnel shift per weight
 // instead of a comparison, a select and a merge), the update puts the sign on
 // -alpha with one logic operation, and update, bits and the next plane's
 // magnitudes share one pass.  12288 x 12288 fp16, three planes: 164 -> 101 us.
-// Packed two-lane fp32 additions were no faster (the compiler pays for the register
-// pairs with moves), neither were six CTAs per SM (spills).
+// Packed two-lane fp32 additions were no faster, neither were six CTAs per SM (spills).
 #include <cuda_bf16.h>
 
 #include <algorithm>

@@ -56,14 +56,16 @@
 //
 // What bounds it: the length of the chain word TMA -> unpack -> MMA issue ->
 // commit per 64-input block; issue slots, shared memory, tensor pipe and DRAM are
-// all below half.  The issuer and TMA warps run their loops as whole warps and
+// all below half (3-bit).  The issuer and TMA warps run their loops as whole warps and
 // elect one lane for the single-thread instructions (elect_one below).  With a
 // branch on lane 0 around the loop an issuer spent 1190 cycles on a block - 330 on
 // four MMAs, 260 on two commits, 600 on waits that were already over - and its
-// unpack group waited for it half of the time.  Launched one after the other, 64 x 8192 x 28672: 3-bit 66.6 us
-// with the branch, 59.8 us now; NF4 94.1 and 91.5 (its table lookups, two
-// shared-memory wavefronts per byte, take over); 64 x 28672 x 8192: 62.0 -> 55.6
-// and 86.9 -> 85.6; 64 x 4096 x 6144: 16.4 -> 14.4 and 20.3 -> 18.6.
+// unpack group waited for it half of the time.  Launched one after the other, 64 x
+// 8192 x 28672: 3-bit 66.6 us with the branch, 59.8 us now; NF4 94.1 and 91.5; 64 x
+// 28672 x 8192: 62.0 -> 55.6 and 86.9 -> 85.6; 64 x 4096 x 6144: 16.4 -> 14.4 and 20.3
+// -> 18.6.  NF4 has the table look-ups in the chain of a block, two shared-memory
+// wavefronts per byte: 7.3 of the 10.6 million of 37 x 28672 x 8192, which keep that
+// pipe busy for 56 % of its 80 us.
 // Every mbarrier wait is bounded: when the limit is hit the thread records a
 // status code, stops waiting and carries on, so the kernel always terminates
 // and frees its tensor memory; the host reads the status word.
@@ -143,10 +145,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, bool he
   }
   return false;
 }
-// One lane of a converged warp.  The single-thread instructions (MMA, commit, TMA,
-// barrier) take their operands from uniform registers: inside a branch on
-// elect.sync, in a warp that runs the loop as a whole, the compiler keeps them
-// there; inside a branch on the lane number it moves every operand over.
+// One lane of a converged warp, for the single-thread instructions (MMA, commit, TMA,
+// barrier).  In a warp that runs the loop as a whole with a branch on elect.sync around
+// them, the issuer's loop takes a third less time than in a branch on the lane number.
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(
@@ -247,9 +248,9 @@ struct QgemmParams {
 // Waits until `turn` parts of the tile have been added to the scratch, for sums in a
 // fixed order.  CTAs start in the order of their part (blockIdx.y), so the parts
 // before this one are finished or running, and a part lasts about as long as the one
-// before it.  Bounded: past the limit (milliseconds) the sums are still right, only
+// before it.  Bounded: past the limit (some milliseconds) the sums are still right, only
 // their order is not the usual one.
-constexpr uint32_t kTurnSpins = 1u << 14;
+constexpr uint32_t kTurnSpins = 1u << 13;  // far below what kSpinLimit gives the epilogue
 __device__ __forceinline__ void await_turn(const unsigned* counter, unsigned turn) {
   for (uint32_t i = 0; i < kTurnSpins; i++) {
     unsigned done;

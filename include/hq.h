@@ -292,14 +292,14 @@ int hq_lutgemm_nqmv_noalloc(void* out_half, const void* x_half, const uint32_t* 
  * the cumulative row ranges cb_sizes[0..3] (main.cu:43-51), cb_stride_int4 =
  * 16-byte units between codebooks.  scales (half[prob_m], nullable) is an
  * extension: the row sum is multiplied by it before rounding.
- * prob_k % 64 == 0. */
+ * prob_k % 64 == 0, prob_k <= 8192 (HQ_ERR_TOO_LARGE beyond). */
 int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half,
                         const void* codebook, int prob_m, int prob_k, const int cb_sizes[4],
                         int cb_stride_int4, const void* scales_half, hq_stream_t stream);
 
 /* AQLM 2x8 (no counterpart in the reference tree): codes
  * uint8[prob_m][prob_k/8][2], codebooks half[2][256][8], scales nullable.
- * prob_k % 64 == 0. */
+ * prob_k % 64 == 0, prob_k <= 70976 (HQ_ERR_TOO_LARGE beyond). */
 int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half,
                        const void* codebooks, int prob_m, int prob_k, const void* scales_half,
                        hq_stream_t stream);
