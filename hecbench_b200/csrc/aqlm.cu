@@ -296,7 +296,8 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   // and 9.3 with it, 7.5 and 7.8 held to two per SM; 9472 x 4096, 296 CTAs of 32 rows:
   // 12.6 and 14.5, 15.4 and 15.5, 12.5 and 12.7.
   const int per_sm = (grid + sm_count() - 1) / sm_count();
-  const size_t request = std::max(smem, (size_t)228 * 1024 / (per_sm + 1) - 1024 + 16);
+  const size_t share = (size_t)228 * 1024 / (per_sm + 1);  // 1 KiB of it is reserved per CTA
+  const size_t request = std::max(smem, share > 1024 ? share - 1024 + 16 : 0);
   cudaError_t e = ensure_dynamic_smem<kern2x8>(request);
   if (e != cudaSuccess) return cuda_status(e);
   if (grid >= 2 * sm_count())

@@ -90,14 +90,15 @@ def test_each_launch_waits_for_the_one_before(hq, dev, family, replayed):
 
 
 @pytest.mark.parametrize("per_cta,ctas_per_sm,extra", [(16, 2, -1), (16, 2, 0), (16, 2, 1), (16, 3, 0),
-                                                       (32, 2, 0), (32, 2, 1), (32, 3, 5)])
+                                                       (32, 2, 0), (32, 2, 1), (32, 3, 5),
+                                                       (32, 240, 0)])
 def test_2x8_around_the_early_start(hq, dev, per_cta, ctas_per_sm, extra):
-    """Row counts around two and three CTAs per SM, 16 and 32 rows per CTA, against the
-    product of the decoded weights in fp64; the kernel rounds sums of 16 products to fp16
+    """Row counts around two and three CTAs per SM, 16 and 32 rows per CTA, and more CTAs
+    per SM than it has KiB of shared memory, against the product of the decoded weights in fp64; the kernel rounds sums of 16 products to fp16
     (2^-11 of a sum whose terms are a few times larger), so 1e-2 of the rms."""
     import torch
     m = per_cta * ctas_per_sm * torch.cuda.get_device_properties(dev).multi_processor_count + extra
-    k = 192
+    k = 192 if ctas_per_sm < 100 else 64
     g = torch.Generator(device=dev).manual_seed(m)
     codes = torch.randint(0, 256, (m, k // 8, 2), generator=g, device=dev, dtype=torch.uint8)
     book = torch.randn((2, 256, 8), generator=g, device=dev).half()
