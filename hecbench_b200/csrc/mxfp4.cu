@@ -35,7 +35,10 @@
 // exact product by 2^k.  Warp instructions per 32 values: 4.9 packing (14.1 with binade
 // compares, magic additions and index arithmetic), 4.6 unpacking, 6.3 for the
 // quantize-dequantize (16.9).  Packing and unpacking 32 Mi bf16 values took 69.6 us and
-// takes 31.6; 64 Mi fp16 packed 37.7 -> 26.1, quantized and dequantized 54.5 -> 41.5.
+// took 31.6 after that; 64 Mi fp16 packed 37.7 -> 26.1, quantized and dequantized 54.5 -> 41.5.
+// The kernels may become resident while the launch before them drains: packed and
+// unpacked, of a pair of calls among others, 32 Mi bf16 values 29.9 -> 26.4 us, 64 Mi fp16
+// 55.8 -> 52.4, 1 Mi 8.2 -> 4.4.
 // Groups that hold an
 // infinity or a NaN, and scales whose power of two is no number of the type, go
 // through plain fp32 arithmetic.
@@ -168,14 +171,14 @@ __device__ __forceinline__ void load_group(uint32_t (&w)[16], const char* p, boo
   if (wide) {
 #pragma unroll
     for (int h = 0; h < 2; h++)
-      asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                    : "=r"(w[8 * h]), "=r"(w[8 * h + 1]), "=r"(w[8 * h + 2]), "=r"(w[8 * h + 3]),
                      "=r"(w[8 * h + 4]), "=r"(w[8 * h + 5]), "=r"(w[8 * h + 6]), "=r"(w[8 * h + 7])
                    : "l"(p + 32 * h));
   } else {
 #pragma unroll
     for (int h = 0; h < 4; h++) {
-      const uint4 v = ldg_stream_u4(p + 16 * h);
+      const uint4 v = ld_ordered_stream_u4(p + 16 * h);
       w[4 * h] = v.x, w[4 * h + 1] = v.y, w[4 * h + 2] = v.z, w[4 * h + 3] = v.w;
     }
   }
@@ -198,8 +201,10 @@ __device__ __forceinline__ void store_group(const uint32_t (&w)[16], char* p, bo
 // MODE 0: out = quantize-dequantize of in (type T); MODE 1: codes + scales
 template <bool BF16, int MODE>
 __global__ void __launch_bounds__(kThreads)
-mxfp4_kernel(const char* __restrict__ in, char* __restrict__ out, uint32_t* __restrict__ codes,
+mxfp4_kernel(const char* in, char* __restrict__ out, uint32_t* __restrict__ codes,
              uint8_t* __restrict__ scales, size_t groups, bool wide, bool wide_codes) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   const size_t g = (size_t)blockIdx.x * kThreads + threadIdx.x;
   if (g >= groups || !HQ_IN_BOUNDS(in + g * 64, 64, in, groups * 64, 601)) return;
   uint32_t w[16];
@@ -239,21 +244,23 @@ mxfp4_kernel(const char* __restrict__ in, char* __restrict__ out, uint32_t* __re
 // codes + scales -> T
 template <bool BF16>
 __global__ void __launch_bounds__(kThreads)
-mxfp4_dequant_kernel(const uint32_t* __restrict__ codes, const uint8_t* __restrict__ scales,
-                     char* __restrict__ out, size_t groups, bool wide, bool wide_codes) {
+mxfp4_dequant_kernel(const uint32_t* codes, const uint8_t* scales, char* __restrict__ out,
+                     size_t groups, bool wide, bool wide_codes) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   const size_t g = (size_t)blockIdx.x * kThreads + threadIdx.x;
   if (g >= groups || !HQ_IN_BOUNDS(codes + 4 * g, 16, codes, groups * 16, 605) ||
       !HQ_IN_BOUNDS(scales + g, 1, scales, groups, 606))
     return;
   uint32_t c[4];
   if (wide_codes) {
-    const uint4 v = ldg_stream_u4(codes + 4 * g);
+    const uint4 v = ld_ordered_stream_u4(codes + 4 * g);
     c[0] = v.x, c[1] = v.y, c[2] = v.z, c[3] = v.w;
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; j++) c[j] = ldg_stream_u32(codes + 4 * g + j);
+    for (int j = 0; j < 4; j++) c[j] = ld_ordered_stream_u32(codes + 4 * g + j);
   }
-  const int k = (int)__ldg(scales + g) - 127;
+  const int k = (int)ld_ordered_u8(scales + g) - 127;
   uint32_t w[16];
 #pragma unroll
   for (int j = 0; j < 4; j++) decode8<BF16>(c[j], k, w + 4 * j);
@@ -283,9 +290,9 @@ int hq_mxfp4_qdq(const void* in, void* out, size_t numel, int dtype, hq_stream_t
   if (!aligned16(in) || !aligned16(out)) return HQ_ERR_MISALIGNED;
   const size_t groups = numel / 32;
   const auto kern = dtype == HQ_DTYPE_BF16 ? mxfp4_kernel<true, 0> : mxfp4_kernel<false, 0>;
-  kern<<<grid_for(groups), kThreads, 0, (cudaStream_t)stream>>>(
-      (const char*)in, (char*)out, nullptr, nullptr, groups, aligned32(in) && aligned32(out), false);
-  return launch_status();
+  return cuda_status(launch_pdl(kern, dim3(grid_for(groups)), dim3(kThreads), 0, (cudaStream_t)stream,
+                                (const char*)in, (char*)out, nullptr, nullptr, groups,
+                                aligned32(in) && aligned32(out), false));
 }
 
 int hq_mxfp4_quantize(const void* in, uint8_t* codes, uint8_t* scales_e8m0, size_t numel, int dtype,
@@ -297,10 +304,9 @@ int hq_mxfp4_quantize(const void* in, uint8_t* codes, uint8_t* scales_e8m0, size
   if (!aligned16(in) || !aligned4(codes)) return HQ_ERR_MISALIGNED;
   const size_t groups = numel / 32;
   const auto kern = dtype == HQ_DTYPE_BF16 ? mxfp4_kernel<true, 1> : mxfp4_kernel<false, 1>;
-  kern<<<grid_for(groups), kThreads, 0, (cudaStream_t)stream>>>(
-      (const char*)in, nullptr, reinterpret_cast<uint32_t*>(codes), scales_e8m0, groups,
-      aligned32(in), aligned16(codes));
-  return launch_status();
+  return cuda_status(launch_pdl(kern, dim3(grid_for(groups)), dim3(kThreads), 0, (cudaStream_t)stream,
+                                (const char*)in, nullptr, reinterpret_cast<uint32_t*>(codes), scales_e8m0,
+                                groups, aligned32(in), aligned16(codes)));
 }
 
 int hq_mxfp4_dequantize(const uint8_t* codes, const uint8_t* scales_e8m0, void* out, size_t numel,
@@ -312,10 +318,9 @@ int hq_mxfp4_dequantize(const uint8_t* codes, const uint8_t* scales_e8m0, void* 
   if (!aligned4(codes) || !aligned16(out)) return HQ_ERR_MISALIGNED;
   const size_t groups = numel / 32;
   const auto kern = dtype == HQ_DTYPE_BF16 ? mxfp4_dequant_kernel<true> : mxfp4_dequant_kernel<false>;
-  kern<<<grid_for(groups), kThreads, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const uint32_t*>(codes), scales_e8m0, (char*)out, groups, aligned32(out),
-      aligned16(codes));
-  return launch_status();
+  return cuda_status(launch_pdl(kern, dim3(grid_for(groups)), dim3(kThreads), 0, (cudaStream_t)stream,
+                                reinterpret_cast<const uint32_t*>(codes), scales_e8m0, (char*)out, groups,
+                                aligned32(out), aligned16(codes)));
 }
 
 }  // extern "C"

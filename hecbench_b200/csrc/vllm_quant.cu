@@ -32,7 +32,12 @@
 //    other forms are a product by the rounded reciprocal and one fused residual
 //    correction (exact_quotient).  4096 x 5137 fp16: dynamic 24.1 -> 11.7 us, 13.4 warp
 //    instructions per 32 elements with addresses, masks and stores (22.0 before), issue
-//    slots 75 % busy; with zero point 33.3 -> 18.4; static 18.4 -> 11.3.
+//    slots 75 % busy; with zero point 33.3 -> 18.4; static 18.4 -> 11.3;
+//  * every kernel may become resident while the launch before it drains: of a call
+//    among others the launch and the last wave of the one before cost 1.7 to 2.4 us
+//    (device time per call, dynamic: 1 x 4096 fp16 4.1 -> 1.75 us, 300 x 1025 4.1 -> 2.4,
+//    4096 x 5137 14.4 -> 12.7, 8192 x 16384 63.6 -> 61.7; static 2048 x 8192 bf16 12.3 ->
+//    10.3; with zero point 2048 x 4096 fp32 13.7 -> 11.7).
 #include <cuda_bf16.h>
 
 #include <cfloat>
@@ -98,8 +103,10 @@ __device__ __forceinline__ void unpack16(const uint4& v, float (&f)[16 / sizeof(
 // ---- static forms: flat over num_tokens * hidden_size elements ----
 template <typename T, bool AZP>
 __global__ void __launch_bounds__(kThreads)
-vllm_static_kernel(const T* __restrict__ in, int8_t* __restrict__ out, size_t n, float scale,
+vllm_static_kernel(const T* in, int8_t* __restrict__ out, size_t n, float scale,
                    int azp, int vec_ok) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   constexpr int kPerLoad = 16 / sizeof(T);  // elements per 16-byte load
   constexpr int kLoads = 16 / kPerLoad;     // loads per 16 outputs
   const size_t stride = (size_t)gridDim.x * kThreads;
@@ -114,7 +121,7 @@ vllm_static_kernel(const T* __restrict__ in, int8_t* __restrict__ out, size_t n,
     uint4 raw[kLoads];
 #pragma unroll
     for (int l = 0; l < kLoads; l++)
-      raw[l] = ldg_stream_u4(reinterpret_cast<const uint4*>(in) + v * kLoads + l);
+      raw[l] = ld_ordered_stream_u4(reinterpret_cast<const uint4*>(in) + v * kLoads + l);
     float f[16], big = 0.f;
 #pragma unroll
     for (int l = 0; l < kLoads; l++) {
@@ -208,9 +215,11 @@ struct Extremes<float> {
 // stores its in-row bytes one by one.
 template <typename T, bool AZP, int CPT>
 __global__ void __launch_bounds__(1024)
-vllm_dynamic_vec_kernel(const T* __restrict__ in, int8_t* __restrict__ out,
+vllm_dynamic_vec_kernel(const T* in, int8_t* __restrict__ out,
                         float* __restrict__ scale_out, int* __restrict__ azp_out, int num_tokens,
                         int hidden) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   constexpr int EPC = 16 / sizeof(T);
   constexpr int EPW = 4 / sizeof(T);  // elements per 32-bit word
   __shared__ float2 sh[32];  // a warp's maximum and minimum
@@ -229,7 +238,7 @@ vllm_dynamic_vec_kernel(const T* __restrict__ in, int8_t* __restrict__ out,
     raw[j] = make_uint4(0, 0, 0, 0);
     if (first >= end) continue;
     if ((c0 + c) * EPC + EPC <= total) {
-      if (HQ_IN_BOUNDS(src + c, 16, in, total * sizeof(T), 403)) raw[j] = ldg_stream_u4(src + c);
+      if (HQ_IN_BOUNDS(src + c, 16, in, total * sizeof(T), 403)) raw[j] = ld_ordered_stream_u4(src + c);
     } else {  // the last chunk of the tensor may be partial: it is fetched element-wise
       T* r = reinterpret_cast<T*>(&raw[j]);
       for (int k = 0; k < EPC; k++)
@@ -358,9 +367,11 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float* sh) {
 // EPT == 0 re-reads the row.
 template <typename T, bool AZP, int EPT>
 __global__ void __launch_bounds__(kThreads)
-vllm_dynamic_kernel(const T* __restrict__ in, int8_t* __restrict__ out,
+vllm_dynamic_kernel(const T* in, int8_t* __restrict__ out,
                     float* __restrict__ scale_out, int* __restrict__ azp_out, int num_tokens,
                     int hidden) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   __shared__ float sh[kWarps];
   const int tid = threadIdx.x;
   for (int t = blockIdx.x; t < num_tokens; t += gridDim.x) {
@@ -431,10 +442,10 @@ int static_launch(int8_t* out, const void* in, size_t n, float scale, int azp, c
   const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
   const T* x = reinterpret_cast<const T*>(in);
   if (azp == 0)  // the launcher's choice, main.cu:147-152
-    vllm_static_kernel<T, false><<<grid, kThreads, 0, st>>>(x, out, n, scale, azp, vec_ok);
-  else
-    vllm_static_kernel<T, true><<<grid, kThreads, 0, st>>>(x, out, n, scale, azp, vec_ok);
-  return launch_status();
+    return cuda_status(launch_pdl(vllm_static_kernel<T, false>, dim3(grid), dim3(kThreads), 0, st, x, out,
+                                  n, scale, azp, vec_ok));
+  return cuda_status(launch_pdl(vllm_static_kernel<T, true>, dim3(grid), dim3(kThreads), 0, st, x, out, n,
+                                scale, azp, vec_ok));
 }
 
 template <typename T, bool AZP>
@@ -465,26 +476,23 @@ int dynamic_launch_ept(int8_t* out, const T* x, float* scales, int* azp, int tok
       cpt = c, threads = (int)w, best = w * c;
     }
   }
-#define HQ_GO(C)                                                                                 \
-  vllm_dynamic_vec_kernel<T, AZP, C><<<tokens, threads, 0, st>>>(x, out, scales, azp, tokens, hidden)
-  if (cpt == 1) HQ_GO(1);
-  else if (cpt == 2) HQ_GO(2);
-  else if (cpt == 3) HQ_GO(3);
-  else if (cpt == 4) HQ_GO(4);
-  else if (cpt == 5) HQ_GO(5);
-  else if (cpt == 6) HQ_GO(6);
-  else if (cpt == 7) HQ_GO(7);
-  else if (cpt == 8) HQ_GO(8);
-#undef HQ_GO
-  else if (hidden <= 8 * kThreads)
-    vllm_dynamic_kernel<T, AZP, 8><<<grid, kThreads, 0, st>>>(x, out, scales, azp, tokens, hidden);
-  else if (hidden <= 16 * kThreads)
-    vllm_dynamic_kernel<T, AZP, 16><<<grid, kThreads, 0, st>>>(x, out, scales, azp, tokens, hidden);
-  else if (hidden <= 32 * kThreads)
-    vllm_dynamic_kernel<T, AZP, 32><<<grid, kThreads, 0, st>>>(x, out, scales, azp, tokens, hidden);
-  else
-    vllm_dynamic_kernel<T, AZP, 0><<<grid, kThreads, 0, st>>>(x, out, scales, azp, tokens, hidden);
-  return launch_status();
+  auto go = [&](auto kern, unsigned blocks, int block) {
+    return cuda_status(launch_pdl(kern, dim3(blocks), dim3(block), 0, st, x, out, scales, azp, tokens, hidden));
+  };
+  switch (cpt) {
+    case 1: return go(vllm_dynamic_vec_kernel<T, AZP, 1>, tokens, threads);
+    case 2: return go(vllm_dynamic_vec_kernel<T, AZP, 2>, tokens, threads);
+    case 3: return go(vllm_dynamic_vec_kernel<T, AZP, 3>, tokens, threads);
+    case 4: return go(vllm_dynamic_vec_kernel<T, AZP, 4>, tokens, threads);
+    case 5: return go(vllm_dynamic_vec_kernel<T, AZP, 5>, tokens, threads);
+    case 6: return go(vllm_dynamic_vec_kernel<T, AZP, 6>, tokens, threads);
+    case 7: return go(vllm_dynamic_vec_kernel<T, AZP, 7>, tokens, threads);
+    case 8: return go(vllm_dynamic_vec_kernel<T, AZP, 8>, tokens, threads);
+  }
+  if (hidden <= 8 * kThreads) return go(vllm_dynamic_kernel<T, AZP, 8>, grid, kThreads);
+  if (hidden <= 16 * kThreads) return go(vllm_dynamic_kernel<T, AZP, 16>, grid, kThreads);
+  if (hidden <= 32 * kThreads) return go(vllm_dynamic_kernel<T, AZP, 32>, grid, kThreads);
+  return go(vllm_dynamic_kernel<T, AZP, 0>, grid, kThreads);
 }
 
 template <typename T>
