@@ -204,9 +204,19 @@ __device__ __forceinline__ uint2 ld_ordered_u2(const void* p) {
   asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
+__device__ __forceinline__ uint2 ld_ordered_stream_u2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint32_t ld_ordered_stream_u32(const void* p) {
   uint32_t v;
   asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_ordered_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint32_t ld_ordered_u8(const void* p) {

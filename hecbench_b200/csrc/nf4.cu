@@ -844,12 +844,13 @@ __device__ __forceinline__ void st_stream_u4(void* p, const uint4& v) {
 }
 template <bool POW2>
 __global__ void __launch_bounds__(kThreads)
-nf4_dequant_kernel(const uint8_t* __restrict__ B, const float* __restrict__ absmax,
-                   const float* __restrict__ lut16, __half* __restrict__ out, size_t nwords,
-                   int words_per_block, int shift, int low_first) {
+nf4_dequant_kernel(const uint8_t* B, const float* absmax, const float* lut16, __half* __restrict__ out,
+                   size_t nwords, int words_per_block, int shift, int low_first) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   __shared__ float lut[16 * 32];  // [code][lane]
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < 16 * 32; i += kThreads) lut[i] = lut16[i >> 5];
+  for (int i = tid; i < 16 * 32; i += kThreads) lut[i] = ld_ordered_f32(lut16 + (i >> 5));
   __syncthreads();
   const float* lut_lane = lut + lane;
   const size_t stride = (size_t)gridDim.x * kThreads;
@@ -880,10 +881,10 @@ nf4_dequant_kernel(const uint8_t* __restrict__ B, const float* __restrict__ absm
         !HQ_IN_BOUNDS(absmax + block_of(w), 4, absmax, nblocks * 4, 112) ||
         !HQ_IN_BOUNDS(reinterpret_cast<uint4*>(out) + w, 16, out, nwords * 16, 113))
       continue;
-    const uint32_t c0 = ldg_stream_u32(reinterpret_cast<const uint32_t*>(B) + w);
-    const uint32_t c1 = two ? ldg_stream_u32(reinterpret_cast<const uint32_t*>(B) + w2) : 0u;
-    const float s0 = __ldg(absmax + block_of(w));
-    const float s1 = two ? __ldg(absmax + block_of(w2)) : 0.f;
+    const uint32_t c0 = ld_ordered_stream_u32(reinterpret_cast<const uint32_t*>(B) + w);
+    const uint32_t c1 = two ? ld_ordered_stream_u32(reinterpret_cast<const uint32_t*>(B) + w2) : 0u;
+    const float s0 = ld_ordered_f32(absmax + block_of(w));
+    const float s1 = two ? ld_ordered_f32(absmax + block_of(w2)) : 0.f;
     st_stream_u4(reinterpret_cast<uint4*>(out) + w, convert(c0, s0));
     if (two) st_stream_u4(reinterpret_cast<uint4*>(out) + w2, convert(c1, s1));
   }
@@ -1299,13 +1300,9 @@ int hq_nf4_dequant_f16(const uint8_t* B, const float* absmax, const float* lut16
     while ((1 << shift) < wpb) shift++;
   }
   const int low = (flags & HQ_NF4_LOW_NIBBLE_FIRST) ? 1 : 0;
-  if (shift >= 0)
-    nf4_dequant_kernel<true><<<grid, kThreads, 0, (cudaStream_t)stream>>>(
-        B, absmax, lut16, reinterpret_cast<__half*>(out_half), nwords, wpb, shift, low);
-  else
-    nf4_dequant_kernel<false><<<grid, kThreads, 0, (cudaStream_t)stream>>>(
-        B, absmax, lut16, reinterpret_cast<__half*>(out_half), nwords, wpb, 0, low);
-  return launch_status();
+  const auto kern = shift >= 0 ? nf4_dequant_kernel<true> : nf4_dequant_kernel<false>;
+  return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), 0, (cudaStream_t)stream, B, absmax, lut16,
+                                reinterpret_cast<__half*>(out_half), nwords, wpb, std::max(shift, 0), low));
 }
 
 int hq_nf4_gemv_f16(const void* A_half, const uint8_t* B, const float* absmax, const float* lut16,

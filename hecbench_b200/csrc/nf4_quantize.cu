@@ -21,6 +21,9 @@
 // code = count + (x > midpoint): one multiply, one floor, one 64-bit
 // shared-memory read, one compare.  A level table with two midpoints in one cell
 // (levels closer than 1/32) makes the CTA count midpoints one by one instead.
+// This kernel and the dequantizer may become resident while the launch before them drains:
+// 1 Mi bf16 values quantized and read back, of a pair of calls among others, 10.2 -> 7.2 us, 32 Mi
+// 44.3 -> 40.7.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -42,8 +45,8 @@ __device__ __forceinline__ void load8(const void* base, size_t vec, size_t nvec,
     const uint4* p = reinterpret_cast<const uint4*>(base) + 2 * vec;
     uint4 a = make_uint4(0, 0, 0, 0), b = a;
     if (HQ_IN_BOUNDS(p, 32, base, nvec * 32, 801)) {
-      a = ldg_stream_u4(p);
-      b = ldg_stream_u4(p + 1);
+      a = ld_ordered_stream_u4(p);
+      b = ld_ordered_stream_u4(p + 1);
     }
     w[0] = __uint_as_float(a.x); w[1] = __uint_as_float(a.y);
     w[2] = __uint_as_float(a.z); w[3] = __uint_as_float(a.w);
@@ -52,7 +55,7 @@ __device__ __forceinline__ void load8(const void* base, size_t vec, size_t nvec,
   } else {
     const uint4* p = reinterpret_cast<const uint4*>(base) + vec;
     uint4 a = make_uint4(0, 0, 0, 0);
-    if (HQ_IN_BOUNDS(p, 16, base, nvec * 16, 802)) a = ldg_stream_u4(p);
+    if (HQ_IN_BOUNDS(p, 16, base, nvec * 16, 802)) a = ld_ordered_stream_u4(p);
     const uint32_t u[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -111,15 +114,16 @@ __device__ __forceinline__ uint32_t encode8(const float (&w)[8], float inv, cons
 // a whole block of `blocksize` weights twice
 template <int DTYPE, int LPB>
 __global__ void __launch_bounds__(kThreads)
-nf4_quantize_kernel(const void* __restrict__ W, size_t nvec, int blocksize,
-                    const float* __restrict__ lut16, int low_first, uint32_t* __restrict__ B,
+nf4_quantize_kernel(const void* W, size_t nvec, int blocksize, const float* lut16, int low_first, uint32_t* __restrict__ B,
                     float* __restrict__ absmax) {
+  pdl_launch_dependents();
+  pdl_wait();  // nothing is read or written before every earlier kernel has completed
   __shared__ __align__(16) unsigned char s_cells[kCells * kCellStride];
   __shared__ float s_mid[16];
   __shared__ float2 s_cell[kCells];
   __shared__ int s_dense;
   const int tid = threadIdx.x, lane = tid & 31;
-  if (tid < 15) s_mid[tid] = 0.5f * (__ldg(lut16 + tid) + __ldg(lut16 + tid + 1));
+  if (tid < 15) s_mid[tid] = 0.5f * (ld_ordered_f32(lut16 + tid) + ld_ordered_f32(lut16 + tid + 1));
   if (tid == 0) s_dense = 0;
   __syncthreads();
   for (int c = tid; c < kCells; c += kThreads) {
@@ -210,18 +214,17 @@ int launch(const void* W, size_t n, int blocksize, const float* lut16, int flags
   const size_t want = (nvec + kThreads - 1) / kThreads;
   // every CTA builds the table once: no more CTAs than are resident together
   const int grid = (int)std::min<size_t>(want, (size_t)sm_count() * 4);
-#define HQ_GO(LPB_)                                                                          \
-  nf4_quantize_kernel<DTYPE, LPB_><<<grid, kThreads, 0, st>>>(W, nvec, blocksize, lut16, low, b32, \
-                                                              absmax)
+  auto go = [&](auto kern) {
+    return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), 0, st, W, nvec, blocksize, lut16, low, b32,
+                                  absmax));
+  };
   switch (blocksize) {
-    case 32: HQ_GO(4); break;
-    case 64: HQ_GO(8); break;
-    case 128: HQ_GO(16); break;
-    case 256: HQ_GO(32); break;
-    default: HQ_GO(0); break;
+    case 32: return go(nf4_quantize_kernel<DTYPE, 4>);
+    case 64: return go(nf4_quantize_kernel<DTYPE, 8>);
+    case 128: return go(nf4_quantize_kernel<DTYPE, 16>);
+    case 256: return go(nf4_quantize_kernel<DTYPE, 32>);
+    default: return go(nf4_quantize_kernel<DTYPE, 0>);
   }
-#undef HQ_GO
-  return launch_status();
 }
 
 }  // namespace

@@ -1,11 +1,12 @@
-"""The activation and MXFP4 quantizers start while the launch before them drains: they read
+"""The quantizers start while the launch before them drains: they read
 nothing by loads that may move above the wait, and see what that launch wrote."""
 import pytest
 
 from test_early_start_loads import CSRC, MAY_MOVE, _blocks
 
 
-@pytest.mark.parametrize("name", ["mxfp4.cu", "vllm_quant.cu"])
+@pytest.mark.parametrize("name", ["mxfp4.cu", "vllm_quant.cu", "nf4_quantize.cu", "q3_quantize.cu",
+                                  "lutgemm_quantize.cu"])
 def test_no_load_can_pass_the_wait(name):
     blocks = _blocks((CSRC / name).read_text())
     kernels = [b for b in blocks if "__global__" in b]
@@ -15,7 +16,8 @@ def test_no_load_can_pass_the_wait(name):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("form", ["static", "dynamic", "dynamic odd", "dynamic_azp", "element-wise", "mxfp4", "qdq"])
+@pytest.mark.parametrize("form", ["static", "dynamic", "dynamic odd", "dynamic_azp", "element-wise", "mxfp4", "nf4", "q3",
+                                  "bcq"])
 @pytest.mark.parametrize("rows", [64, 3000])
 def test_input_written_by_the_launch_before(hq, dev, form, rows):
     """x is the output of a mat-vec that itself started early, and is overwritten by the next
@@ -25,13 +27,21 @@ def test_input_written_by_the_launch_before(hq, dev, form, rows):
     g = torch.Generator(device=dev).manual_seed(rows)
     mat = torch.randint(0, 256, (n, 16), generator=g, device=dev, dtype=torch.uint8)
     steps = 5
+    lut = torch.linspace(-1, 1, 16, device=dev)
     v = [torch.randn(32, generator=g, device=dev).half() for _ in range(steps)]
     buf = torch.zeros(n, dtype=torch.float16, device=dev)
     hidden = {"dynamic odd": 1023, "element-wise": 1021}.get(form, 1024)
     first = 1 if form == "element-wise" else 0               # not 16-byte aligned
 
     def call():
-        if form in ("mxfp4", "qdq"):
+        if form == "nf4":
+            codes, absmax = hq.quantize_nf4(buf, lut)
+            return codes, absmax, hq.dequantize_nf4(codes, absmax, lut, n)
+        if form == "q3":
+            return hq.quantize_q3(buf.view(rows, 1024)[:rows // 32 * 32])
+        if form == "bcq":
+            return hq.quantize_bcq(buf.view(1024, rows), 3)
+        if form == "mxfp4":
             codes, scales = hq.mxfp4_quantize(buf)
             return codes, scales, hq.mxfp4_dequantize(codes, scales, buf.dtype)
         x = buf[first:first + rows * hidden]
