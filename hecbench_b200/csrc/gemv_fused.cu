@@ -72,6 +72,7 @@ gemv_fused_kernel(const FusedParams p) {
   // Programmatic dependent launch: nothing that earlier work of the stream may
   // have produced is read, and nothing is written, before the wait.
   pdl_launch_dependents();
+  if (BITS == 4) prefetch_first_rows(p.mat, rows_mat, row_bytes, lane, warp);
   pdl_wait();
 
   // ---- RMSNorm: sum of squares over the whole vector ----

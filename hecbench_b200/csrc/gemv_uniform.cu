@@ -54,6 +54,7 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   // may be an earlier kernel's output like the input vector), and nothing is
   // written before it.
   pdl_launch_dependents();
+  if (BITS == 4) prefetch_first_rows(mat, rows, row_bytes, lane, warp);
   pdl_wait();
   // ---- prologue: inputs to shared memory (piece-major) and their sum ----
   float part = 0.f;

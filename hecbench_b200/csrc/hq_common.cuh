@@ -235,6 +235,15 @@ __device__ __forceinline__ __half ld_ordered_f16(const __half* p) {
   return __ushort_as_half(v);
 }
 
+// Asks for `bytes` bytes at p (both multiples of 16, inside one buffer) to be in L2 soon.
+// A hint that changes no memory and returns no data, so it may stand before pdl_wait():
+// L2 is where the writes of an earlier kernel arrive, a line that is written after the
+// hint is written there.  A kernel that starts early has its first weights on the way
+// while the one before it drains.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
