@@ -325,6 +325,344 @@ lutgemm_kernel(const uint32_t* bW, const __half* alpha,
   }
 }
 
+// asynchronous copies global -> shared of 16 / 8 bytes (behind the wait like any load)
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint2 lds_u2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+
+// ---- ring form: four planes in one launch, and long work per CTA --------------
+// The lookups of the register form, on 128-input tiles, with two differences.  Words,
+// alphas and bias come through shared memory by asynchronous copies, kDepth column steps of
+// a warp ahead (57 to 86 KB per SM under way instead of 29, and no registers held: four
+// planes fit one launch where the register form takes two, each with its own tables).  And
+// the CTAs are persistent: a unit is one column range of one K tile, units are numbered
+// range by range inside a tile, CTA c takes units c, c + gridDim.x, ..., and a warp's ring
+// runs on through the ends of units, so words arrive while the tables of the next tile are
+// built.  What bounds it is shared memory: the look-ups, the quads' reads of their words
+// and the tables.  us of a call among others, register form -> this: 12288 x 12288, 4 planes
+// 44.9 -> 32.6, 3 planes 28.8 -> 27.4; 4096 x 8192, 4 planes 16.1 -> 11.4; 10240 x 5120, 3 planes
+// 14.1 -> 13.3.  The register form stays where a CTA has one short unit or two planes:
+// 2052 x 2048, 2 planes 5.4 and 6.0 here, 1024 x 1024, 3 planes 5.3 and 5.7, 8192 x 4096, 2 planes
+// 8.9 and 9.6.
+constexpr int kRingThreads = 512;
+
+// Compile-time layout.  NB: planes, RPG: packed rows per alpha group inside a tile.
+// Dynamic shared memory:
+//   [padding][tables 2 x 64 KiB][rings: kWarps x kDepth stages][inputs][flags]
+// The tables start at the FIXED shared-window address kLutImm, as above.
+template <int NB, int RPG>
+struct RingLayout {
+  static constexpr int kWarps = kRingThreads / 32;
+  static constexpr int kGroups = 4 / RPG;
+  static constexpr int kLutImm = (kDynBase + kSlack + 255) / 256 * 256;
+  static constexpr int kLutBytes = 2 * 65536;
+  // a stage: one column step of one warp, [row][plane][32 columns] words, then
+  // [group][planes and bias][32 columns] halves
+  static constexpr int kWordBytes = 4 * NB * 128;
+  static constexpr int kParamBytes = kGroups * (NB + 1) * 64;
+  static constexpr int kStage = kWordBytes + kParamBytes;
+  static constexpr int kRing = kLutImm + kLutBytes;
+  static constexpr int kTail = 4 * 32 * 4 + kCounterWords * 4;
+  static constexpr int kBudget = 227 * 1024 - (kRing - kDynBase) - kTail;
+  static constexpr int kFit = kBudget / (kWarps * kStage);
+  static constexpr int kDepth = kFit > 4 ? 4 : kFit;
+  static_assert(kDepth >= 2, "a ring of two stages");
+  static constexpr int kInputs = kRing + kWarps * kDepth * kStage;
+  static constexpr int kFlags = kInputs + 4 * 32 * 4;
+  static constexpr int kSmem = kFlags + kCounterWords * 4 - kDynBase;
+};
+
+// b0, nb_total, counters and per_range as for lutgemm_kernel
+template <int NB, int RPG>
+__global__ void __launch_bounds__(kRingThreads, 1)
+lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
+               const __half* q_bias, const __half* x,
+               __half* __restrict__ out, float* __restrict__ ws, unsigned* __restrict__ counters,
+               int M, int K, int rows_per_group, int cols_per_cta, int ranges, int tiles, int nb_total,
+               int b0, int finalize, int per_range) {
+  using L = RingLayout<NB, RPG>;
+  constexpr int TR = 4, kThreads = kRingThreads;
+  constexpr int kWarps = L::kWarps, kGroups = L::kGroups, kLutImm = L::kLutImm, kDepth = L::kDepth;
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t dsm_addr = (uint32_t)__cvta_generic_to_shared(dsm);
+  // the host has checked where the dynamic region starts; never taken
+  if (dsm_addr < (uint32_t)kDynBase || dsm_addr > (uint32_t)(kDynBase + kSlack)) return;
+  unsigned char* window = dsm - dsm_addr;  // generic address of shared-window address 0
+  unsigned char* lut = window + kLutImm;
+  float* xs = reinterpret_cast<float*>(window + L::kInputs);  // the tile's inputs
+  volatile unsigned* flags = reinterpret_cast<unsigned*>(window + L::kFlags);
+  const int total_rows = K >> 5;
+  const int units = ranges * tiles;
+
+  // the next kernel of the stream may become resident while this grid drains;
+  // nothing is read or written before every earlier kernel has completed
+  pdl_launch_dependents();
+  {
+    // the words of the first steps are on their way to L2 before the wait
+    const int tile = (int)blockIdx.x / ranges, begin = ((int)blockIdx.x - tile * ranges) * cols_per_cta;
+    const int cols = min(min(M, begin + cols_per_cta) - begin, kDepth * kWarps * 32);
+    const int r = tid / NB, b = tid - r * NB;
+    if (tid < TR * NB && tile * TR + r < total_rows && cols > 0)
+      prefetch_l2(bW + ((size_t)(tile * TR + r) * nb_total + b0 + b) * M + begin, (uint32_t)cols * 4u);
+  }
+  pdl_wait();
+  // the inputs of the first tile: the tables wait for them
+  const int first_k = (int)blockIdx.x / ranges * TR * 32 + tid;
+  float x_first = 0.f;
+  if (tid < TR * 32 && first_k < K && HQ_IN_BOUNDS(x + first_k, 2, x, (size_t)K * 2, 206))
+    x_first = __half2float(ld_dependent_f16(x + first_k));
+
+  // ---- the warp's ring ----
+  // Step s of a unit is columns m_begin + (s * kWarps + warp) * 32 .. + 31.  The warp asks
+  // for its steps kDepth ahead, through the ends of units, so words arrive while the tables
+  // of the next tile are built.  Per step a lane copies up to kWordCopies runs of 16 bytes
+  // of words and kParamCopies of 8 bytes of alphas and bias.
+  constexpr int kWordCopies = (TR * NB * 8 + 31) / 32, kParamCopies = (kGroups * (NB + 1) * 8 + 31) / 32;
+  const uint32_t ring = (uint32_t)(L::kRing + warp * (kDepth * L::kStage));
+  const int seg = lane & 7;
+  // extents of the caller's buffers, used only by the index-checked build
+  const size_t bw_bytes = (size_t)total_rows * nb_total * M * 4;
+  const size_t alpha_bytes = (size_t)(total_rows / rows_per_group) * nb_total * M * 2;
+  const size_t bias_bytes = (size_t)(total_rows / rows_per_group) * M * 2;
+  (void)bw_bytes; (void)alpha_bytes; (void)bias_bytes;
+  int f_unit = blockIdx.x, f_m = 0, f_end = 0, f_row0 = 0;  // the next step to ask for
+  auto enter = [&] {  // f_unit -> its first step of this warp, skipping units without one
+    for (; f_unit < units; f_unit += gridDim.x) {
+      const int tile = f_unit / ranges, begin = (f_unit - tile * ranges) * cols_per_cta;
+      f_row0 = tile * TR;
+      f_m = begin + warp * 32;
+      f_end = min(M, begin + cols_per_cta);
+      if (f_m < f_end) return;
+    }
+  };
+  auto fetch = [&](uint32_t stage) {
+    if (f_unit < units) {
+      const int nrows = min(TR, total_rows - f_row0), m = f_m + seg * 4;
+      if (m < f_end) {
+        const uint32_t* src = bW + ((size_t)f_row0 * nb_total + b0) * M + m;
+#pragma unroll
+        for (int i = 0; i < kWordCopies; i++) {
+          const int rp = (lane >> 3) + 4 * i, r = rp / NB, b = rp - r * NB;
+          const uint32_t* at = src + (size_t)(r * nb_total + b) * M;
+          if (rp < TR * NB && r < nrows && HQ_IN_BOUNDS(at, 16, bW, bw_bytes, 201))
+            cp_async_16(stage + rp * 128 + seg * 16, at);
+        }
+        const int g0 = f_row0 / rows_per_group;
+#pragma unroll
+        for (int i = 0; i < kParamCopies; i++) {
+          const int gb = (lane >> 3) + 4 * i, gi = gb / (NB + 1), b = gb - gi * (NB + 1);
+          const uint32_t dst = stage + L::kWordBytes + gb * 64 + seg * 8;
+          if (gi < kGroups && gi * RPG < nrows) {
+            if (b < NB) {
+              const __half* at = alpha + ((size_t)(g0 + gi) * nb_total + b0 + b) * M + m;
+              if (HQ_IN_BOUNDS(at, 8, alpha, alpha_bytes, 202)) cp_async_8(dst, at);
+            } else if (q_bias != nullptr) {
+              const __half* at = q_bias + (size_t)(g0 + gi) * M + m;
+              if (HQ_IN_BOUNDS(at, 8, q_bias, bias_bytes, 203)) cp_async_8(dst, at);
+            }
+          }
+        }
+      }
+      f_m += kWarps * 32;
+      if (f_m >= f_end) {
+        f_unit += gridDim.x;
+        enter();
+      }
+    }
+    cp_async_commit();
+  };
+  enter();
+#pragma unroll
+  for (int d = 0; d < kDepth; d++) fetch(ring + d * L::kStage);
+
+  const int j = lane & 3;   // byte of the word this lane looks up
+  const int cq = lane >> 2; // column quad inside the 32-column step
+  const uint32_t hi = (uint32_t)(lane * 4);
+  const uint32_t sel = 0x7604u | ((uint32_t)j << 4);
+  uint32_t at_stage = 0;
+  int built = -1;  // tile of the tables in place
+  float ones[kGroups];
+
+  for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    const int tile = unit / ranges, m_begin = (unit - tile * ranges) * cols_per_cta;
+    const int m_end = min(M, m_begin + cols_per_cta);
+    const int row0 = tile * TR, nrows = min(TR, total_rows - row0);
+    if (tile != built) {
+      built = tile;
+      // ---- the tile's inputs (zero beyond K) ----
+      if (tid < TR * 32) {
+        const int k = row0 * 32 + tid;
+        float v = x_first;
+        if (unit != (int)blockIdx.x)
+          v = (k < K && HQ_IN_BOUNDS(x + k, 2, x, (size_t)K * 2, 206)) ? __half2float(ld_dependent_f16(x + k)) : 0.f;
+        xs[tid] = v;
+      }
+      __syncthreads();  // inputs in place, and no warp looks up in the old tables any more
+      // ---- tables: thread = (byte value, some of the rows); signed sums of 8 inputs, each
+      // stored 8 times.  Line (row pair p, byte b) at lut + p*65536 + b*256, inside
+      // [row parity][replica c][j] floats; the lanes of a warp hold consecutive lines, so
+      // they write different replicas at a time (conflict-free) ----
+      constexpr int kRowSets = kThreads / 256;      // threads per byte value
+      constexpr int kRowsEach = TR / kRowSets;      // rows per thread
+      const int bv = tid & 255, rp = tid >> 8;
+      uint32_t sgn[8];
+#pragma unroll
+      for (int t = 0; t < 8; t++) sgn[t] = ((bv >> t) & 1) ? 0u : 0x80000000u;
+#pragma unroll
+      for (int rr = 0; rr < kRowsEach; rr++) {
+        const int r = rp * kRowsEach + rr;
+        float v[4];
+#pragma unroll
+        for (int jj = 0; jj < 4; jj++) {
+          const float4 xa = *reinterpret_cast<const float4*>(xs + r * 32 + jj * 8);
+          const float4 xb = *reinterpret_cast<const float4*>(xs + r * 32 + jj * 8 + 4);
+          const float s0 = __uint_as_float(__float_as_uint(xa.x) ^ sgn[0]) +
+                           __uint_as_float(__float_as_uint(xa.y) ^ sgn[1]);
+          const float s1 = __uint_as_float(__float_as_uint(xa.z) ^ sgn[2]) +
+                           __uint_as_float(__float_as_uint(xa.w) ^ sgn[3]);
+          const float s2 = __uint_as_float(__float_as_uint(xb.x) ^ sgn[4]) +
+                           __uint_as_float(__float_as_uint(xb.y) ^ sgn[5]);
+          const float s3 = __uint_as_float(__float_as_uint(xb.z) ^ sgn[6]) +
+                           __uint_as_float(__float_as_uint(xb.w) ^ sgn[7]);
+          v[jj] = (s0 + s1) + (s2 + s3);
+        }
+        unsigned char* line = lut + (r >> 1) * 65536 + bv * 256 + (r & 1) * 128;
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+          *reinterpret_cast<float4*>(line + ((c + lane) & 7) * 16) = make_float4(v[0], v[1], v[2], v[3]);
+      }
+      __syncthreads();
+      // bias uses the all-ones entry (byte 255): sum of this lane's 8 inputs per row
+#pragma unroll
+      for (int gi = 0; gi < kGroups; gi++) {
+        float o = 0.f;
+#pragma unroll
+        for (int r = gi * RPG; r < (gi + 1) * RPG; r++)
+          o += *reinterpret_cast<const float*>(lut + (r >> 1) * 65536 + 255 * 256 + (r & 1) * 128 +
+                                               lane * 4);
+        ones[gi] = o;
+      }
+    }
+
+    // ---- lookups ----
+    // byte value b in row r: [byteperm(word, lane*4, sel) + kLutImm + (r>>1)*65536 + (r&1)*128]
+    for (int m0 = m_begin + warp * 32; m0 < m_end; m0 += kWarps * 32) {
+      cp_async_wait<kDepth - 1>();
+      __syncwarp();
+      const uint32_t stage = ring + at_stage * L::kStage;
+      const uint32_t words = stage + cq * 16, params = stage + L::kWordBytes + cq * 8;
+      const int m = m0 + cq * 4;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int gi = 0; gi < kGroups; gi++) {
+        if (gi * RPG >= nrows) break;  // rows past the end of K
+        float t[NB][4];
+#pragma unroll
+        for (int rr = 0; rr < RPG; rr++) {
+          const int r = gi * RPG + rr;
+#pragma unroll
+          for (int b = 0; b < NB; b++) {
+            const uint4 w = lds_u4(words + (r * NB + b) * 128);
+            const uint32_t w4[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const uint32_t a = __byte_perm(w4[c], hi, sel);
+              float v;
+              if (r == 0) v = lds_f32_imm<kLutImm>(a);
+              else if (r == 1) v = lds_f32_imm<kLutImm + 128>(a);
+              else if (r == 2) v = lds_f32_imm<kLutImm + 65536>(a);
+              else v = lds_f32_imm<kLutImm + 65536 + 128>(a);
+              t[b][c] = (rr == 0) ? v : t[b][c] + v;
+            }
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+          const uint2 av = lds_u2(params + (gi * (NB + 1) + b) * 64);
+          const float2 a01 = __half22float2(u32_as_half2(av.x));
+          const float2 a23 = __half22float2(u32_as_half2(av.y));
+          acc[0] = fmaf(a01.x, t[b][0], acc[0]);
+          acc[1] = fmaf(a01.y, t[b][1], acc[1]);
+          acc[2] = fmaf(a23.x, t[b][2], acc[2]);
+          acc[3] = fmaf(a23.y, t[b][3], acc[3]);
+        }
+        if (q_bias != nullptr) {
+          const uint2 av = lds_u2(params + (gi * (NB + 1) + NB) * 64);
+          const float2 b01 = __half22float2(u32_as_half2(av.x));
+          const float2 b23 = __half22float2(u32_as_half2(av.y));
+          acc[0] = fmaf(b01.x, ones[gi], acc[0]);
+          acc[1] = fmaf(b01.y, ones[gi], acc[1]);
+          acc[2] = fmaf(b23.x, ones[gi], acc[2]);
+          acc[3] = fmaf(b23.y, ones[gi], acc[3]);
+        }
+      }
+      // every lane has read the stage (the look-ups that used its words are done)
+      __syncwarp();
+      fetch(stage);
+      if (++at_stage == kDepth) at_stage = 0;
+      // combine the four byte lanes of each column quad
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
+        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
+      }
+      // every lane of the quad now holds the four column sums: lane j == 0 adds
+      // them to the scratch row with one 16-byte reduction
+      if (m < m_end && j == 0 && HQ_IN_BOUNDS(ws + m, 16, ws, (size_t)M * 4, 204))
+        red_add_v4_f32(ws + m, acc[0], acc[1], acc[2], acc[3]);
+    }
+  }
+  cp_async_wait<0>();
+
+  // ---- the last CTA of a column range converts it to fp16 and re-zeroes the scratch ----
+  if (!finalize) return;
+  __threadfence();
+  if (tid < kCounterWords) flags[tid] = 0;
+  __syncthreads();
+  const int my_units = (units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int counted = per_range ? ranges : 1;
+  for (int i = tid; i < my_units; i += kThreads) {
+    const int range = per_range ? (int)((blockIdx.x + (unsigned)i * gridDim.x) % (unsigned)ranges) : 0;
+    const unsigned total = per_range ? tiles : units;
+    if (atomicAdd(counters + range, 1u) == total - 1) flags[range] = 1;
+  }
+  __syncthreads();
+  for (int range = 0; range < counted; range++) {
+    if (!flags[range]) continue;
+    __threadfence();
+    const int lo = per_range ? range * cols_per_cta : 0, hi_m = per_range ? min(M, lo + cols_per_cta) : M;
+    for (int mm = lo + tid * 4; mm < hi_m; mm += kThreads * 4) {
+      if (!HQ_IN_BOUNDS(out + mm, 8, out, (size_t)M * 2, 205)) continue;
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(ws + mm));
+      const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(out + mm) = make_uint2(half2_as_u32(h01), half2_as_u32(h23));
+      *reinterpret_cast<float4*>(ws + mm) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (tid == 0) counters[range] = 0u;
+  }
+}
+
 // ---- bulk-copy form ---------------------------------------------------------
 // The register form above keeps one column step of packed words in flight per
 // warp, about 29 KB per SM, and waits out the HBM latency at every step.  This
@@ -373,18 +711,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
           "r"(dst), "l"(src), "r"(bytes), "r"(bar)
       : "memory");
-}
-__device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ uint2 lds_u2(uint32_t addr) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
-  return v;
 }
 
 // Shared memory: [flag 16 B][mbarriers 8 x 8 B][build scratch][padding][tables 64 KiB at
@@ -645,24 +971,44 @@ int launch_one(const LaunchArgs& a, int b0, const __half* bias, int finalize) {
                                 a.cols_per_cta, a.nb_total, b0, finalize, a.per_range));
 }
 
+template <int NB, int RPG>
+int launch_ring(const LaunchArgs& a, int b0, const __half* bias, int finalize) {
+  using L = RingLayout<NB, RPG>;
+  constexpr auto kern = lutgemm_ring_kernel<NB, RPG>;
+  cudaError_t e = ensure_dynamic_smem<kern>(L::kSmem);
+  if (e != cudaSuccess) return cuda_status(e);
+  const long long units = (long long)a.grid.x * a.grid.y;
+  const unsigned ctas = (unsigned)std::min<long long>(units, sm_count());
+  return cuda_status(launch_pdl(kern, dim3(ctas), dim3(kRingThreads), L::kSmem, a.st, a.bW, a.alpha, bias,
+                                a.x, a.out, a.ws, a.counters, a.M, a.K, a.rows_per_group, a.cols_per_cta,
+                                (int)a.grid.x, (int)a.grid.y, a.nb_total, b0, finalize, a.per_range));
+}
+
 // Bit planes are handled up to kMax at a time (what the register budget of the
-// one-step-ahead loads allows); further planes go to follow-up launches that
-// accumulate into the same scratch row.  Only the first launch adds the bias
-// term, only the last one converts the scratch row.
+// one-step-ahead loads allows, or the rings have room for); further planes go to
+// follow-up launches that accumulate into the same scratch row.  Only the first
+// launch adds the bias term, only the last one converts the scratch row.  The ring
+// form takes four planes, and three where a CTA has several units of two column
+// steps or more (times at its head).
 template <int TR, int RPG>
 int launch_planes(const LaunchArgs& a) {
-  constexpr int kMax = TR == 4 ? 3 : 4;
+  constexpr bool kFour = TR == 2 || RPG > 1;  // groups of 32 inputs: the rings hold three planes
+  const bool ring3 = TR == 4 && a.cols_per_cta >= 2 * kRingThreads &&
+                     (long long)a.grid.x * a.grid.y > sm_count();
   const int nb = a.nb_total;
-  for (int b0 = 0; b0 < nb; b0 += kMax) {
-    const int n = nb - b0 < kMax ? nb - b0 : kMax;
+  for (int b0 = 0; b0 < nb;) {
+    const int n = std::min(nb - b0, kFour ? 4 : 3);
     const int last = (b0 + n == nb) ? 1 : 0;
     const __half* bias = b0 == 0 ? a.q_bias : nullptr;
     int st;
     if (n == 1) st = launch_one<TR, 1, RPG>(a, b0, bias, last);
     else if (n == 2) st = launch_one<TR, 2, RPG>(a, b0, bias, last);
-    else if (n == 3) st = launch_one<TR, 3, RPG>(a, b0, bias, last);
-    else st = launch_one<TR, (kMax >= 4 ? 4 : 3), RPG>(a, b0, bias, last);
+    else if (TR == 2 && n == 4) st = launch_one<TR, (TR == 2 ? 4 : 3), RPG>(a, b0, bias, last);
+    else if (n == 4) st = launch_ring<(TR == 4 && RPG > 1 ? 4 : 3), RPG>(a, b0, bias, last);
+    else if (ring3) st = launch_ring<3, RPG>(a, b0, bias, last);
+    else st = launch_one<TR, 3, RPG>(a, b0, bias, last);
     if (st != HQ_OK) return st;
+    b0 += n;
   }
   return HQ_OK;
 }
