@@ -37,6 +37,7 @@
 //    rows (sum over the slices, warp-shuffle tree, one fp16 store).  With
 //    S == 1 a warp finishes its rows alone and there is no barrier.
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <mutex>
 
@@ -549,6 +550,296 @@ nf4_gemv_kernel(const GemvParams p) {
   if (packets_out) {
     // the last CTA to finish records that this gather round is complete on the
     // sending side (the packets validate themselves on the receiving side)
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned prev = atomicAdd(p.sync_words, 1u);
+      if (prev == gridDim.x - 1) {
+        p.sync_words[0] = 0u;
+        *reinterpret_cast<volatile unsigned*>(p.sync_words + 1) = epoch_in + 1u;
+      }
+    }
+  }
+}
+
+// ---- tensor form (absmax blocks of 64 weights) --------------------------------
+// The products of the looked-up half2 pairs with the inputs on mma.sync m16n8k16, which
+// takes four lookups per instruction and sums in fp32: 42 instructions per 32 lane-codes
+// instead of 94.  (A mat-vec fills one column of a tensor-core tile; the matrix rate is
+// not what is used here, the register-to-register form without a shared-memory operand is.)
+//  * A warp multiplies 16 rows by 512 inputs at a time (a super-step): lane (g, t) = (lane
+//    / 4, lane % 4) reads 16 bytes of row 2g and of row 2g + 1 per 128 inputs, the four
+//    lanes of a row 64 contiguous bytes.  The k-slots of lane t in the instruction are the
+//    inputs that its bytes stand for, in the order of the bytes, so a lookup is an
+//    A-register as it is.
+//  * Lanes t = 0, 1 hold one absmax block of 64, t = 2, 3 the next.  The columns of B keep
+//    them apart: even columns get the inputs of t = 0, 1 and zeros for the rest, odd ones
+//    the other way round; lanes of (g + t / 2) odd hold constant zeros.  After the eight
+//    instructions of 128 inputs every lane has the two block sums of its two rows, and the
+//    lane whose blocks these are scales and adds them.
+//  * The inputs lie in shared memory, 288 bytes per 128 inputs (the chunks of t = 2, 3 are
+//    moved by 32 bytes: the four addresses of a load then meet in no bank).
+//  * S warps share a tile of 16 rows, each takes every S-th super-step; G groups of S per
+//    CTA.  A lane's 128 bytes of the next super-step are requested as this one uses the
+//    registers up.
+constexpr int kMmaThreads = 512;
+constexpr int kMmaWarps = kMmaThreads / 32;
+constexpr int kMmaStepBytes = 288;  // of inputs, per 128
+__device__ __forceinline__ int mma_piece(int i) {  // offset of inputs 8i .. 8i + 7
+  return (i >> 4) * kMmaStepBytes + ((i >> 2) & 3) * 64 + ((i >> 3) & 1) * 32 + (i & 3) * 16;
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+inline size_t mma_smem_bytes(int nchunks) {
+  const int supers = (nchunks + 15) / 16;
+  return (size_t)kLutImm + kLutBytes + (size_t)supers * 4 * kMmaStepBytes + 2 * kMmaWarps * 16 * sizeof(float) +
+         (size_t)nchunks * 64;  // packet input, unpacked
+}
+
+// rows: of the matrix; p.S, p.G as above; FUSE and LL as for nf4_gemv_kernel.
+template <bool FUSE, bool LL>
+__global__ void __launch_bounds__(kMmaThreads, 1)
+nf4_gemv_mma_kernel(const GemvParams p, int rows, int tiles, int supers) {
+  __shared__ float s_sq[kMmaWarps];
+  extern __shared__ __align__(16) unsigned char dsm_raw[];
+  // [pad up to shared address kLutImm] table | inputs | partial sums [2][warp][16] | packets
+  pdl_launch_dependents();
+  if (!p.early_fetch) pdl_wait();
+  unsigned char* dsm = dsm_raw + (kLutImm - smem_u32(dsm_raw));
+  unsigned char* xs = dsm + kLutBytes;
+  float* part = reinterpret_cast<float*>(xs + (size_t)supers * 4 * kMmaStepBytes);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int S = p.S, G = p.G, grp = warp / S, q = warp - grp * S;
+  const int g = lane >> 2, t = lane & 3;
+  const int nblocks = p.nchunks / 2;
+  const int tile_step = gridDim.x * G;
+
+  // the 16 levels first, see nf4_gemv_kernel
+  constexpr int kTabTurns = 256 * 4 / kMmaThreads;
+  float lv_first[kTabTurns], lv_second[kTabTurns];
+#pragma unroll
+  for (int i = 0; i < kTabTurns; i++) {
+    const int entry = (tid + i * kMmaThreads) >> 2, hi = entry >> 4, lo = entry & 15;
+    lv_first[i] = ld_ordered_f32(p.lut16 + (p.low_first ? lo : hi));
+    lv_second[i] = ld_ordered_f32(p.lut16 + (p.low_first ? hi : lo));
+  }
+
+  // ---- this warp's super-steps: of tiles tile, tile + tile_step, ... those q, q + S, ... ----
+  int tile = blockIdx.x + gridDim.x * grp, ss = q;
+  if (grp >= G) tile = tiles;
+  uint4 w[4][2];
+  float am[4];
+  int f_tile = tile, f_ss = ss;  // the super-step that is requested next
+  const unsigned char* src = nullptr;
+  int f_chunk = 0;
+  bool f_live[2] = {false, false};
+  auto aim = [&] {
+    f_chunk = f_ss * 16 + t;
+    const int row = f_tile * 16 + 2 * g;
+    f_live[0] = f_tile < tiles && row < rows;
+    f_live[1] = f_tile < tiles && row + 1 < rows;
+    src = p.B + ((size_t)row * p.nchunks + f_chunk) * 16;
+  };
+  auto request = [&](int i) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const unsigned char* at = src + (size_t)r * p.nchunks * 16 + i * 64;
+      w[i][r] = make_uint4(0, 0, 0, 0);
+      if (f_live[r] && f_chunk + 4 * i < p.nchunks && HQ_IN_BOUNDS(at, 16, p.B, p.b_bytes, 121))
+        w[i][r] = ld_ordered_stream_u4(at);
+    }
+  };
+  auto scales = [&](float (&a)[4]) {
+    const int row = f_tile * 16 + 2 * g, block = f_ss * 8 + 2 * t;
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const float* at = p.absmax + (size_t)(row + r) * nblocks + block + e;
+        a[2 * r + e] = 0.f;
+        if (f_live[r] && block + e < nblocks && HQ_IN_BOUNDS(at, 4, p.absmax, p.absmax_bytes, 122))
+          a[2 * r + e] = ld_ordered_f32(at);
+      }
+  };
+  auto advance = [&] {
+    f_ss += S;
+    if (f_ss >= supers) { f_ss = q; f_tile += tile_step; }
+  };
+  if (p.early_fetch) {
+    aim();
+#pragma unroll
+    for (int i = 0; i < 4; i++) request(i);
+    scales(am);
+    pdl_wait();
+  }
+  const uint32_t epoch_in =
+      LL && p.sync_words != nullptr ? *reinterpret_cast<volatile unsigned*>(p.sync_words + 1) : 0u;
+  const bool packets_out = LL && p.peer_ll != nullptr, packets_in = LL && p.A_ll != nullptr;
+
+  // ---- inputs to shared memory (zeros up to a whole super-step), table ----
+  const int pieces = p.nchunks * 4;
+  const uint4* xg = reinterpret_cast<const uint4*>(p.A);
+  const uint4* gg = reinterpret_cast<const uint4*>(p.gamma);
+  const bool norm_in = FUSE && p.gamma != nullptr;
+  uint4 x0 = make_uint4(0, 0, 0, 0), g0 = x0;  // the thread's first piece
+  if (!packets_in && tid < pieces && HQ_IN_BOUNDS(xg + tid, 16, p.A, p.a_bytes, 123)) x0 = ld_dependent_u4(xg + tid);
+  if (norm_in && tid < pieces && HQ_IN_BOUNDS(gg + tid, 16, p.gamma, p.a_bytes, 124)) g0 = ld_ordered_u4(gg + tid);
+  if (!p.early_fetch) {
+    aim();
+#pragma unroll
+    for (int i = 0; i < 4; i++) request(i);
+    scales(am);
+  }
+#pragma unroll
+  for (int i = 0; i < kTabTurns; i++) {
+    const int e4 = tid + i * kMmaThreads, entry = e4 >> 2, quarter = e4 & 3;
+    const uint32_t u = half2_as_u32(__floats2half2_rn(lv_first[i], lv_second[i]));
+    const uint4 u4 = make_uint4(u, u, u, u);
+    uint4* row = reinterpret_cast<uint4*>(dsm + (size_t)entry * 256 + quarter * 32);
+    row[entry & 1] = u4;
+    row[(entry & 1) ^ 1] = u4;
+  }
+  if (packets_in) {
+    __half* flat = reinterpret_cast<__half*>(part + 2 * kMmaWarps * 16);
+    stage_packets<kMmaThreads>(flat, p.A_ll, p.a_stride, p.nchunks * 32, epoch_in, p.max_polls, p.status, tid);
+    __syncthreads();
+    xg = reinterpret_cast<const uint4*>(flat);
+  }
+  float sq = 0.f;
+  for (int i = tid; i < supers * 64; i += kMmaThreads) {
+    uint4 v = x0;
+    if (packets_in) v = i < pieces ? xg[i] : make_uint4(0, 0, 0, 0);
+    else if (i != tid) {
+      v = make_uint4(0, 0, 0, 0);
+      if (i < pieces && HQ_IN_BOUNDS(xg + i, 16, p.A, p.a_bytes, 125)) v = ld_dependent_u4(xg + i);
+    }
+    if (norm_in) {
+      const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 f = __half22float2(u32_as_half2(h[k]));
+        sq = fmaf(f.x, f.x, fmaf(f.y, f.y, sq));
+      }
+    }
+    *reinterpret_cast<uint4*>(xs + mma_piece(i)) = v;
+  }
+  if (norm_in) {
+    sq = warp_sum(sq);
+    if (lane == 0) s_sq[warp] = sq;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMmaWarps; i++) tot += s_sq[i];
+    const float norm = rsqrtf(tot / (float)(p.nchunks * 32) + p.eps);
+    for (int i = tid; i < pieces; i += kMmaThreads) {
+      uint4* at = reinterpret_cast<uint4*>(xs + mma_piece(i));
+      const uint4 v = *at;
+      uint4 gv = g0;
+      if (i != tid && HQ_IN_BOUNDS(gg + i, 16, p.gamma, p.a_bytes, 126)) gv = ld_ordered_u4(gg + i);
+      uint32_t h[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t gh[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 f = __half22float2(u32_as_half2(h[k]));
+        const float2 m = __half22float2(u32_as_half2(gh[k]));
+        h[k] = half2_as_u32(__floats2half2_rn(f.x * norm * m.x, f.y * norm * m.y));
+      }
+      *at = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+  }
+  __syncthreads();
+
+  // ---- super-steps ----
+  const uint32_t lane4 = (uint32_t)lane * 4u;
+  const bool feeds = ((g ^ (t >> 1)) & 1) == 0;  // this lane's B registers hold inputs, else zeros
+  const uint32_t x_lane = smem_u32(xs) + (uint32_t)(t * 64 + (t >> 1) * 32);
+  uint4 xv[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) xv[i] = make_uint4(0, 0, 0, 0);
+  float acc0 = 0.f, acc1 = 0.f;  // rows 2g and 2g + 1
+  int turn = 0;
+  while (tile < tiles) {
+    advance();
+    aim();
+    float am_next[4];
+    scales(am_next);
+    const uint32_t x_at = x_lane + (uint32_t)ss * (4 * kMmaStepBytes);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (feeds) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(xv[k].x), "=r"(xv[k].y), "=r"(xv[k].z), "=r"(xv[k].w)
+                       : "r"(x_at + i * kMmaStepBytes + k * 16));
+      }
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint32_t wa[4] = {w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w};
+      const uint32_t wb[4] = {w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        // byte b of the word -> (byte << 8) | lane*4: bytes {lane4.0, w.b, 0, 0}
+        const uint32_t a0 = lds_u32_imm<kLutImm>(__byte_perm(wa[k], lane4, 0x7604));
+        const uint32_t a1 = lds_u32_imm<kLutImm>(__byte_perm(wb[k], lane4, 0x7604));
+        const uint32_t a2 = lds_u32_imm<kLutImm>(__byte_perm(wa[k], lane4, 0x7614));
+        const uint32_t a3 = lds_u32_imm<kLutImm>(__byte_perm(wb[k], lane4, 0x7614));
+        mma_16816(c, a0, a1, a2, a3, xv[k].x, xv[k].y);
+        const uint32_t a4 = lds_u32_imm<kLutImm>(__byte_perm(wa[k], lane4, 0x7624));
+        const uint32_t a5 = lds_u32_imm<kLutImm>(__byte_perm(wb[k], lane4, 0x7624));
+        const uint32_t a6 = lds_u32_imm<kLutImm>(__byte_perm(wa[k], lane4, 0x7634));
+        const uint32_t a7 = lds_u32_imm<kLutImm>(__byte_perm(wb[k], lane4, 0x7634));
+        mma_16816(c, a4, a5, a6, a7, xv[k].z, xv[k].w);
+      }
+      request(i);  // the same inputs' words of the next super-step
+      if (t == i) {
+        acc0 = fmaf(c[0], am[0], fmaf(c[1], am[1], acc0));
+        acc1 = fmaf(c[2], am[2], fmaf(c[3], am[3], acc1));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) am[i] = am_next[i];
+    ss += S;
+    if (ss < supers) continue;
+
+    // ---- the warp's share of the tile is complete ----
+    acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1);
+    acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
+    acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1);
+    acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
+    float* const mine = part + ((turn & 1) * kMmaWarps + grp * S) * 16;
+    if (t == 0) *reinterpret_cast<float2*>(mine + q * 16 + 2 * g) = make_float2(acc0, acc1);
+    if (S > 1) group_barrier(1 + grp, S * 32);
+    else __syncwarp();
+    if (q == turn % S) {  // the warps of the group take turns at finishing
+      float v = 0.f;
+      for (int i = 0; i < S; i++) v += mine[i * 16 + (lane & 15)];
+      const float gate = __shfl_down_sync(0xffffffffu, v, 1);
+      const int row = tile * 16 + lane;
+      const bool live = lane < 16 && row < rows;
+      if (FUSE && p.act != 0) {
+        if (live && (lane & 1) == 0 && HQ_IN_BOUNDS(p.out + (row >> 1), 2, p.out, p.out_bytes, 127))
+          p.out[row >> 1] = __float2half_rn(v * gate_act(gate, p.act));
+      } else if (!packets_out) {
+        if (live && HQ_IN_BOUNDS(p.out + row, 2, p.out, p.out_bytes, 128)) p.out[row] = __float2half_rn(v);
+      } else if (live) {
+        const uint32_t h = __half_as_ushort(__float2half_rn(v));
+        if (p.multicast) {
+          st_packet_multicast(p.peer_ll[0] + p.gather_offset + row, h, epoch_in + 1u);
+        } else {
+          for (int r = 0; r < p.world; r++) st_packet(p.peer_ll[r] + p.gather_offset + row, h, epoch_in + 1u);
+        }
+      }
+    }
+    turn++;
+    acc0 = acc1 = 0.f;
+    ss = q;
+    tile += tile_step;
+  }
+  if (packets_out) {
+    // as in nf4_gemv_kernel
     __syncthreads();
     if (tid == 0) {
       const unsigned prev = atomicAdd(p.sync_words, 1u);
@@ -1090,6 +1381,26 @@ struct LlArgs {
 
 namespace hq {
 namespace {
+template <bool FUSE, bool LL>
+int launch_gemv_mma(GemvParams& prm, int rows, cudaStream_t st) {
+  const int supers = (prm.nchunks + 15) / 16, tiles = (rows + 15) / 16, sms = sm_count();
+  // Warps per tile: the count with the fewest rounds, a tile counting one super-step more
+  // than a warp's share of it for the sums at its end.
+  long best = LONG_MAX;
+  for (int s = 1; s <= std::min(supers, kMmaWarps); s++) {
+    const int groups = kMmaWarps / s;
+    const long rounds = (tiles + (long)sms * groups - 1) / ((long)sms * groups);
+    const long cost = rounds * ((supers + s - 1) / s + 1);
+    if (cost < best) best = cost, prm.S = s, prm.G = groups;
+  }
+  const size_t smem = mma_smem_bytes(prm.nchunks);
+  constexpr auto kern = nf4_gemv_mma_kernel<FUSE, LL>;
+  cudaError_t e = ensure_dynamic_smem<kern>(smem);
+  if (e != cudaSuccess) return cuda_status(e);
+  return cuda_status(launch_pdl(kern, dim3(std::min(sms, tiles)), dim3(kMmaThreads), smem, st, prm,
+                                rows, tiles, supers));
+}
+
 template <int C>
 int launch_gemv_bulk(GemvParams& prm, int N, cudaStream_t st) {
   const uint32_t slot_bytes =
@@ -1217,6 +1528,20 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   // 128 registers each hold C = 2 chunks of the input vector and D = 4 rows of
   // packed weights in flight per lane.
   const bool with_packets = ll.A_ll != nullptr || ll.peer_ll != nullptr;
+  // The tensor form where the lanes and warps of the other one do not come out even, or where
+  // there are few rows (its slices are 1024 inputs, two per lane; us, other form -> tensor form):
+  //   one or three slices: 28672 x 1024 9.0 -> 6.3, 4096 x 1024 2.6 -> 2.2, 28672 x 3072 16.2 -> 14.8,
+  //   2048 x 2816 3.2 -> 2.6
+  //   two, up to 64 rows per SM: 2048 x 2048 2.95 -> 2.24, 8192 x 2048 4.6 -> 4.3, 14336 x 2048
+  //   6.0 -> 6.3, 28672 x 2048 9.5 -> 10.4
+  //   four, up to 16: 1024 x 4096 2.91 -> 2.71, 2048 x 4096 3.3 -> 2.9, 4096 x 4096 4.28 -> 4.32,
+  //   28672 x 4096 14.4 -> 18.9; longer rows gain nothing (2048 x 8192 4.5 -> 4.8).
+  const long rows_per_sm = N / sm_count();
+  const bool uneven = cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
+  if (blocksize == 64 && K % 64 == 0 && uneven && !pair_packets && mma_smem_bytes(nchunks) <= 227 * 1024)
+    return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
+           : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
+                             : launch_gemv_mma<false, false>(prm, N, st);
 #define HQ_NF4_GO(C_, D_, ST_, AL_)                                                         \
   (with_packets                                                                              \
        ? (pair_packets ? launch_gemv<C_, D_, ST_, AL_, 512, true, true>(prm, units, st)      \

@@ -1,0 +1,29 @@
+"""Edges of the NF4 mat-vec's tensor form (absmax blocks of 64): rows around a tile of 16, rows
+of one absmax block up to a whole and a broken super-step of 512 inputs, one to sixteen warps
+per tile, more tiles than groups of warps, both nibble orders, early and late weights; against
+fp64 products of the stored levels."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("N,K", [(1, 64), (15, 128), (16, 512), (17, 576), (33, 1024), (513, 1088), (5000, 2816),
+                                 (2369, 4096), (31, 8256), (100, 16384), (7, 33024), (40001, 1024)])
+def test_edges(hq, dev, N, K, early):
+    """fp16 levels, exact products, fp32 sums of blocks and of their scaled sums: K * 2^-24 of the
+    sum of magnitudes, and one rounding of the result to fp16."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    x = torch.randn(K, generator=g, device=dev).half()
+    B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = (torch.rand(N * K // 64, generator=g, device=dev) + 0.5) / K ** 0.5
+    lut = torch.sort(torch.rand(16, generator=g, device=dev) * 2 - 1).values
+    for order in (hq.NF4_HIGH_NIBBLE_FIRST, hq.NF4_LOW_NIBBLE_FIRST):
+        hi, lo = (B >> 4).long(), (B & 15).long()
+        codes = torch.stack([lo, hi] if order == hq.NF4_LOW_NIBBLE_FIRST else [hi, lo], -1).view(N, K)
+        terms = lut.half().double()[codes] * x.double() * absmax.double().view(N, K // 64).repeat_interleave(64, 1)
+        want = terms.sum(1)
+        bound = want.abs() * 2.0 ** -11 + terms.abs().sum(1) * K * 2.0 ** -24 + 2.0 ** -24
+        got = hq.gemv_nf4(x, B, absmax, lut, N, K, 64, order, weights_resident=early)
+        assert bool(((got.double() - want).abs() <= bound).all())
