@@ -1536,9 +1536,12 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   //   6.0 -> 6.3, 28672 x 2048 9.5 -> 10.4
   //   four, up to 16: 1024 x 4096 2.91 -> 2.71, 2048 x 4096 3.3 -> 2.9, 4096 x 4096 4.28 -> 4.32,
   //   28672 x 4096 14.4 -> 18.9; longer rows gain nothing (2048 x 8192 4.5 -> 4.8).
+  // The fused forms always take it (RMSNorm, up / gate, SwiGLU and the plain down projection
+  // after it: 2048 - 5632 12.0 -> 10.3, 4096 - 14336 31.2 -> 30.1, 5120 - 13824 42.9 -> 35.0, 8192 -
+  // 14336 56.7 -> 54.3).
   const long rows_per_sm = N / sm_count();
-  const bool uneven = cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
-  if (blocksize == 64 && K % 64 == 0 && uneven && !pair_packets && mma_smem_bytes(nchunks) <= 227 * 1024)
+  const bool tensor = fuse != nullptr || cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
+  if (blocksize == 64 && K % 64 == 0 && tensor && !pair_packets && mma_smem_bytes(nchunks) <= 227 * 1024)
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
            : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
                              : launch_gemv_mma<false, false>(prm, N, st);
