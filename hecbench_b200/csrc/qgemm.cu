@@ -66,10 +66,13 @@
 // -> 18.6.  NF4 has the table look-ups in the chain of a block, two shared-memory
 // wavefronts per byte: 7.3 of the 10.6 million of 37 x 28672 x 8192, which keep that
 // pipe busy for 56 % of its 80 us.
+// Long layers take another division of the work, see qgemm_stream.cuh.
 // Every mbarrier wait is bounded: when the limit is hit the thread records a
 // status code, stops waiting and carries on, so the kernel always terminates
 // and frees its tensor memory; the host reads the status word.
 #include <cuda.h>
+
+#include <utility>
 
 #include "hq_common.cuh"
 
@@ -263,6 +266,14 @@ __device__ __forceinline__ void await_turn(const unsigned* counter, unsigned tur
 __device__ __forceinline__ __half* peer_slice(const QgemmParams& p, int g) {
   return p.peer_Y[g] + p.y_offset;
 }
+
+}  // namespace
+}  // namespace hq
+
+#include "qgemm_stream.cuh"
+
+namespace hq {
+namespace {
 
 // PEERS: the sharded form (tiles stored to every GPU's slice); a separate
 // instantiation so that the plain form carries none of it.
@@ -790,6 +801,11 @@ size_t qgemm_ws_bytes(int Mb, int N) {
 // 24576 in three parts 46.6 us either way, NF4 69.9 and 69.8).  Narrower layers, where
 // many short parts of a tile end together, add in any order: in turn, 64 x 4096 x 6144
 // would take 25.4 us for 12.7.
+// Whether a call gives the same bits every time: layers of at least two thirds of a tile per
+// SM, and those of few inputs.
+int plain_parts(int N, int K) { return max(1, min(2 * sm_count() / (N / kTileN), K / kBlockK / 8)); }
+bool repeatable(int N, int K) { return plain_parts(N, K) <= 2; }
+
 struct KSplit {
   int parts;
   bool ordered;
@@ -887,14 +903,17 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
     return HQ_ERR_MISALIGNED;
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
+  // the streamed form fetches twice the features and inputs at a time
+  const bool stream_form = !po.peer_Y && streamed::takes(Mb, N, K, workspace, workspace_bytes, qgemm_ws_bytes(Mb, N));
+  const int tile_n = stream_form ? streamed::kTileN : kTileN;
   CUtensorMap map_x, map_w, map_s, map_z;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
   if (st != HQ_OK) return st;
   {
-    // mat int32[K*3/32][N]: box = 128 columns x 6 rows (one block of 64 inputs)
+    // mat int32[K*3/32][N]: box = 128 columns x 6 rows (one block of 64 inputs), or 256 x 12
     const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)(K / 32 * 3)};
     const cuuint64_t strides[1] = {(cuuint64_t)N * 4};
-    const cuuint32_t box[2] = {(cuuint32_t)kTileN, 6};
+    const cuuint32_t box[2] = {(cuuint32_t)tile_n, stream_form ? 12u : 6u};
     const cuuint32_t estr[2] = {1, 1};
     if (encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int32_t*>(mat), dims, strides,
                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -902,10 +921,10 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
       return HQ_ERR_UNSUPPORTED;
   }
   for (int which = 0; which < 2; which++) {
-    // scales / zeros fp16 [K/group_size][N]: box = 128 columns x 1 group
+    // scales / zeros fp16 [K/group_size][N]: box = 128 or 256 columns x 1 group
     const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)(K / group_size)};
     const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kTileN, 1};
+    const cuuint32_t box[2] = {(cuuint32_t)tile_n, 1};
     const cuuint32_t estr[2] = {1, 1};
     if (encode(which ? &map_z : &map_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                const_cast<void*>(which ? zeros_half : scales_half), dims, strides, box, estr,
@@ -918,6 +937,8 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
   prm.peer_Y = reinterpret_cast<__half* const*>(po.peer_Y);
   prm.y_offset = po.y_offset;
   prm.world = po.world;
+  if (stream_form)
+    return streamed::launch<kFmtQ3>(map_x, map_w, map_s, map_z, prm, repeatable(N, K), stream);
   return launch_qgemm<kFmtQ3>(map_x, map_w, map_s, map_z, prm, stream);
 }
 
@@ -936,17 +957,18 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
     return HQ_ERR_MISALIGNED;
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
+  const bool stream_form = !po.peer_Y && streamed::takes(Mb, N, K, workspace, workspace_bytes, qgemm_ws_bytes(Mb, N));
   CUtensorMap map_x, map_w;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
   if (st != HQ_OK) return st;
   {
-    // B uint8[N][K/2]: box = 32 bytes (64 codes) x 128 rows
+    // B uint8[N][K/2]: box = 32 bytes (64 codes) x 128 rows, or 64 bytes x 256 with the 64-byte swizzle
     const cuuint64_t dims[2] = {(cuuint64_t)(K / 2), (cuuint64_t)N};
     const cuuint64_t strides[1] = {(cuuint64_t)(K / 2)};
-    const cuuint32_t box[2] = {32, (cuuint32_t)kTileN};
+    const cuuint32_t box[2] = {stream_form ? 64u : 32u, (cuuint32_t)(stream_form ? streamed::kTileN : kTileN)};
     const cuuint32_t estr[2] = {1, 1};
     if (encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(B), dims, strides, box,
-               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, stream_form ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HQ_ERR_UNSUPPORTED;
   }
@@ -958,6 +980,8 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
   prm.peer_Y = reinterpret_cast<__half* const*>(po.peer_Y);
   prm.y_offset = po.y_offset;
   prm.world = po.world;
+  if (stream_form)
+    return streamed::launch<kFmtNf4>(map_x, map_w, map_w, map_w, prm, repeatable(N, K), stream);
   return launch_qgemm<kFmtNf4>(map_x, map_w, map_w, map_w, prm, stream);
 }
 

@@ -483,7 +483,7 @@ int hq_mxfp4_dequantize(const uint8_t* codes, const uint8_t* scales_e8m0, void* 
  * bytes that lets the kernel split K over several CTAs when N alone gives a
  * grid that does not fill the GPU evenly; every call that ends with status 0
  * leaves it zero.  The parts meet in fp32 sums.  For N > 128 * 2 * SMs / 3 (12629
- * on 148 SMs) or K < 1536 they are added in the order of K, so a call gives the
+ * on 148 SMs) or K < 1536 they are added in a fixed order, so a call gives the
  * same bits every time; for narrower layers they are added in no fixed order.
  * Without a workspace every result is repeatable.
  * Two rules follow: (1) one workspace serves one stream - calls that may overlap on the GPU (different streams, several host threads) need a

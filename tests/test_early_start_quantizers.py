@@ -6,7 +6,7 @@ from test_early_start_loads import CSRC, MAY_MOVE, _blocks
 
 
 @pytest.mark.parametrize("name", ["mxfp4.cu", "vllm_quant.cu", "nf4_quantize.cu", "q3_quantize.cu",
-                                  "lutgemm_quantize.cu"])
+                                  "lutgemm_quantize.cu", "qgemm_stream.cuh"])
 def test_no_load_can_pass_the_wait(name):
     blocks = _blocks((CSRC / name).read_text())
     kernels = [b for b in blocks if "__global__" in b]

@@ -1,0 +1,54 @@
+"""Edges of the batched product's tiles: the last half tile of 256 features, the last half
+step of 128 inputs, token counts around multiples of 16 and the 64-token line, scale groups of
+64, one CTA per few steps and tiles cut between CTAs."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(hq, fmt, K, N, group, dev, g):
+    """call(X, **kw) and the dequantised weights [K][N] in fp64."""
+    import torch
+    if fmt == "nf4":
+        lut = torch.sort(torch.rand(16, generator=g, device=dev) * 2 - 1).values
+        B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+        absmax = torch.rand(N * K // group, generator=g, device=dev) + 0.5
+        W = hq.dequantize_nf4(B, absmax, lut, N * K, group, 0).view(N, K).t()
+        return (lambda X, **kw: hq.qgemm_nf4(X, B, absmax, lut, N, K, group, 0, **kw)), W.double()
+    mat = torch.randint(-2**31, 2**31, (K * 3 // 32, N), generator=g, device=dev).to(torch.int32)
+    scales = (torch.rand((K // group, N), generator=g, device=dev) * 0.01 + 0.001).half()
+    zeros = (scales * torch.randint(0, 8, (K // group, N), generator=g, device=dev)).half()
+    codes = hq.vecquant3_dequant(mat, torch.ones(N, device=dev), torch.zeros(N, device=dev), K * 3 // 32, N,
+                                 dtype=torch.float32)
+    up = lambda p: p.double().repeat_interleave(group, 0)
+    W = (codes.double() * up(scales) - up(zeros)).half()     # one rounding, as the fp16 fma
+    return (lambda X, **kw: hq.qgemm_q3(X, mat, scales, zeros, N, K, group, **kw)), W.double()
+
+
+@pytest.mark.parametrize("fmt", ["q3", "nf4"])
+@pytest.mark.parametrize("Mb,K,N,group", [
+    (1, 64, 128, 64), (16, 128, 128, 64), (17, 192, 384, 64), (64, 320, 256, 64), (65, 448, 640, 64),
+    (128, 1088, 128, 64), (2, 4096, 1152, 128), (37, 8192, 4224, 128), (64, 1024, 37888, 128),
+    (96, 8256, 2176, 64), (128, 2048, 38016, 128), (33, 28672, 1024, 128),
+    # the streamed form: half a step and half a tile left over, scale groups of half a step, whole and
+    # cut tiles, tokens on both sides of 64
+    (1, 8256, 14464, 64), (64, 3648, 28672, 64), (65, 16448, 7296, 64), (128, 1088, 104704, 64),
+    (16, 28672, 4096, 128), (100, 1024, 120064, 128)])
+def test_edges(hq, dev, fmt, Mb, K, N, group):
+    """Within 2^-11 of the result (one fp16 rounding) plus what fp32 sums of K products may
+    lose, K * 2^-24 of the sum of their magnitudes; the scratch is left zero, without
+    scratch the same bound holds."""
+    import torch
+    from hecbench_b200 import api
+    g = torch.Generator(device=dev).manual_seed(Mb + K + N)
+    call, W = _operands(hq, fmt, K, N, group, dev, g)
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    want = X.double() @ W
+    bound = want.abs() * 2.0 ** -11 + (X.double().abs() @ W.abs()) * K * 2.0 ** -24 + 2.0 ** -24
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    for split in (True, True, False):
+        got = call(X, status=status, split_k=split)
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0, "a bounded in-kernel wait ran out"
+        assert bool(((got.double() - want).abs() <= bound).all())
+    assert all(int(torch.count_nonzero(w)) == 0 for w in api._qgemm_ws.values())
