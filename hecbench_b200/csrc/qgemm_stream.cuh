@@ -26,12 +26,15 @@
 //    way, and waiting warps sleep in try_wait instead of polling;
 //  * 224 tiles of 128 features left 72 of 148 SMs half empty.
 // us of a call among others, the other form -> this one, 3-bit (NF4): 64 x 8192 x 28672 56.3 ->
-// 46.8 (89.6 -> 69.9), 128 x 8192 x 28672 82.9 -> 60.8 (116.5 -> 81.7), 37 x 28672 x 8192 51.3 -> 45 (80.7
-// -> 67.5), 64 x 28672 x 28672 159.7 -> 134.2 (252 -> 195), 32 x 8192 x 14336 31.9 -> 28.6 (48.6 ->
-// 41.5), 64 x 4096 x 28672 30.6 -> 30.7 (47.9 -> 44.2).  Below 24 steps per SM the ends of the ranges
+// 46.2 (89.6 -> 68.7), 128 x 8192 x 28672 82.6 -> 60.4 (116.6 -> 77.6), 37 x 28672 x 8192 51.3 -> 45 (80.6
+// -> 66.8), 64 x 28672 x 28672 158.7 -> 131.2 (252 -> 191), 32 x 8192 x 14336 31.9 -> 28.6 (48.6 ->
+// 40.7), 64 x 4096 x 28672 30.5 -> 30.4 (47.9 -> 43.6).  Below 24 steps per SM the ends of the ranges
 // (some 3 us for each cut tile) outweigh the rest: 64 x 8192 x 8192, 14 steps, 20.5 and 23.2 (30.1 and
 // 31.6), 64 x 4096 x 6144 12.1 and 17.1.  Unpacking 3-bit pairs by byte permutes and magic numbers
 // instead of the table takes more slots: 51.6 at 64 x 8192 x 28672 (half of the pairs: 48.1).
+// Taken back: reading a tile's accumulators one step into the next, and settling the parts of
+// a cut tile warp by warp without a barrier of the CTA, are shorter at the ends of ranges but
+// cost the inner loop its registers (96 of 96, spills): 3-bit 64 x 8192 x 28672 55.6 and 49.5.
 #ifndef HQ_QGEMM_STREAM_CUH_
 #define HQ_QGEMM_STREAM_CUH_
 namespace hq {
@@ -81,6 +84,7 @@ struct Params {
   int tiles, steps;     // 256-feature tiles, 128-input steps of a tile
   int ordered;          // the parts of a tile add to the scratch in a fixed order
   int one_group;        // 3-bit: both halves of a step lie in one scale group
+  int am_shift;         // NF4: log2 of the 64-input blocks per absmax value, or -1
   // NF4 only (group_size is the absmax block size there)
   const float* absmax;
   const float* lut16;
@@ -311,8 +315,8 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       [[maybe_unused]] const float* am_row = nullptr;
       [[maybe_unused]] auto absmax_at = [&](int k) {
         const int kb = 2 * k + h;
-        return n < p.N && kb * kBlockK < p.K ? ld_ordered_f32(am_row + (kb * kBlockK) / p.group_size)
-                                             : 0.f;
+        if (n >= p.N || kb * kBlockK >= p.K) return 0.f;
+        return ld_ordered_f32(am_row + (p.am_shift >= 0 ? kb >> p.am_shift : kb * kBlockK / p.group_size));
       };
       [[maybe_unused]] float am_next = 0.f;
       if constexpr (FMT == kFmtNf4) {
@@ -620,6 +624,9 @@ int launch(const CUtensorMap& map_x, const CUtensorMap& map_w, const CUtensorMap
   prm.absmax = q.absmax;
   prm.lut16 = q.lut16;
   prm.low_first = q.low_first;
+  prm.am_shift = -1;
+  for (int i = 0; i < 25; i++)
+    if (q.group_size == kBlockK << i) prm.am_shift = i;
   return q.Mb > 64 ? launch_shape<FMT, true>(map_x, map_w, map_s, map_z, prm, stream)
                    : launch_shape<FMT, false>(map_x, map_w, map_s, map_z, prm, stream);
 }
