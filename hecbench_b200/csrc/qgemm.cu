@@ -809,6 +809,7 @@ bool repeatable(int N, int K) { return plain_parts(N, K) <= 2; }
 struct KSplit {
   int parts;
   bool ordered;
+  double cost;
 };
 // The sharded form never takes more parts than the plain choice: split, the last CTA
 // of a tile stores it to every GPU in 8-byte pieces instead of 256-byte rows, a cost
@@ -827,14 +828,41 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
   double limit = 0.95 * cost(best);
   for (int k = 1; k <= (sharded ? min(most, plain) : most); k++)
     if (cost(k) < limit) { best = k; limit = cost(k); }
-  return {best, plain <= 2 && best > 2};
+  return {best, plain <= 2 && best > 2, cost(best)};
+}
+
+// Whether a call takes the streamed form: where tiles may be cut (a scratch, one GPU: the
+// sharded form stores whole tiles to every GPU and has not been timed in parts) and a
+// model of both expects 3 % less.  us, from 140 layers of 9 to 40 steps per SM, 2 to 128
+// tokens, both formats, least squares of relative errors (2 to 6 % off): the form with
+// parts by its cost in blocks, the streamed one by its steps per SM, both by tokens.
+// Over those layers it takes 0.90 of the time of the form with parts alone (the better of the two
+// each time 0.90, streaming from 24 steps per SM on 0.94), 2 % more at worst.
+bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t workspace_bytes) {
+  const int sms = sm_count();
+  const int tiles = (N + streamed::kTileN - 1) / streamed::kTileN;
+  const double units = (double)tiles * ((K + 2 * kBlockK - 1) / (2 * kBlockK));
+  if (workspace == nullptr || workspace_bytes < qgemm_ws_bytes(Mb, N) || !aligned16(workspace) ||
+      units < 4.0 * sms || tiles < 8 || reserved_smem_per_block() != (int)streamed::kBase)
+    return false;
+  struct Model { double parts[3], stream[3]; };
+  static const Model models[2][2] = {  // [format][more than 64 tokens]
+      {{{0.7, 0.408, 1.9}, {8.0, 0.68, 6.4}}, {{-1.8, 0.28, 3.8}, {4.9, 0.70, 9.2}}},
+      {{{0.3, 0.59, 2.5}, {10.9, 0.93, 6.4}}, {{0.0, 0.376, 3.5}, {8.7, 0.94, 8.4}}}};
+  const Model& m = models[fmt == kFmtNf4][Mb > 64];
+  const double cost = choose_ksplit(N / kTileN, K / kBlockK, Mb > 64, false, sms).cost, t = Mb / 64.0;
+  // ordered sums of three or more parts of a tile that end together (90 x 7040 x 12800, 3-bit:
+  // 36.4 where 31 are expected without, 35.0 in parts); below eight tiles a tile has some 20
+  const double turns = tiles < sms / 2 && repeatable(N, K) ? 4.0 : 0.0;
+  return m.stream[0] + m.stream[1] * (units / sms) + m.stream[2] * t + turns <
+         0.97 * (m.parts[0] + m.parts[1] * cost + m.parts[2] * t);
 }
 
 QgemmParams make_params(void* Y_half, bool sharded, int Mb, int N, int K, int group_size,
                         void* workspace, size_t workspace_bytes, int* status_word) {
   QgemmParams prm;
   const int tiles = N / kTileN;
-  KSplit split = {1, false};  // K is split only with a workspace
+  KSplit split = {1, false, 0.0};  // K is split only with a workspace
   if (workspace != nullptr && workspace_bytes >= qgemm_ws_bytes(Mb, N) && aligned16(workspace))
     split = choose_ksplit(tiles, K / kBlockK, Mb > 64, sharded, sm_count());
   prm.Y = reinterpret_cast<__half*>(Y_half);
@@ -904,7 +932,7 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
   // the streamed form fetches twice the features and inputs at a time
-  const bool stream_form = !po.peer_Y && streamed::takes(Mb, N, K, workspace, workspace_bytes, qgemm_ws_bytes(Mb, N));
+  const bool stream_form = !po.peer_Y && takes_stream(kFmtQ3, Mb, N, K, workspace, workspace_bytes);
   const int tile_n = stream_form ? streamed::kTileN : kTileN;
   CUtensorMap map_x, map_w, map_s, map_z;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
@@ -957,7 +985,7 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
     return HQ_ERR_MISALIGNED;
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
-  const bool stream_form = !po.peer_Y && streamed::takes(Mb, N, K, workspace, workspace_bytes, qgemm_ws_bytes(Mb, N));
+  const bool stream_form = !po.peer_Y && takes_stream(kFmtNf4, Mb, N, K, workspace, workspace_bytes);
   CUtensorMap map_x, map_w;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
   if (st != HQ_OK) return st;

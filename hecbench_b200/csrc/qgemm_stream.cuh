@@ -1,5 +1,6 @@
-// The streamed form of the batched product (formats, rules and helpers: qgemm.cu): long layers,
-// from 24 steps of 128 inputs x 256 features per SM on.
+// The streamed form of the batched product (formats, helpers and the rule that chooses it:
+// qgemm.cu), for long layers: some 24 steps of 128 inputs x 256 features per SM up to 64
+// tokens, 13 beyond, fewer for NF4.
 //
 // One CTA of 608 threads per SM takes a contiguous range of (tile, step) units, so that
 // every SM has the same work whatever the number of tiles; a tile is 256 output features
@@ -28,7 +29,7 @@
 // us of a call among others, the other form -> this one, 3-bit (NF4): 64 x 8192 x 28672 56.3 ->
 // 46.2 (89.6 -> 68.7), 128 x 8192 x 28672 82.6 -> 60.4 (116.6 -> 77.6), 37 x 28672 x 8192 51.3 -> 45 (80.6
 // -> 66.8), 64 x 28672 x 28672 158.7 -> 131.2 (252 -> 191), 32 x 8192 x 14336 31.9 -> 28.6 (48.6 ->
-// 40.7), 64 x 4096 x 28672 30.5 -> 30.4 (47.9 -> 43.6).  Below 24 steps per SM the ends of the ranges
+// 40.7), 64 x 4096 x 28672 30.5 -> 30.4 (47.9 -> 43.6).  On short layers the ends of the ranges
 // (some 3 us for each cut tile) outweigh the rest: 64 x 8192 x 8192, 14 steps, 20.5 and 23.2 (30.1 and
 // 31.6), 64 x 4096 x 6144 12.1 and 17.1.  Unpacking 3-bit pairs by byte permutes and magic numbers
 // instead of the table takes more slots: 51.6 at 64 x 8192 x 28672 (half of the pairs: 48.1).
@@ -583,14 +584,6 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
                  : "memory");
   }
-}
-
-// From 24 steps per SM on, where tiles may be cut (a scratch, one GPU: the sharded form
-// stores whole tiles to every GPU and has not been timed in parts).
-bool takes(int Mb, int N, int K, const void* workspace, size_t workspace_bytes, size_t need) {
-  const long long units = (long long)((N + kTileN - 1) / kTileN) * ((K + 2 * kBlockK - 1) / (2 * kBlockK));
-  return units >= 24LL * sm_count() && workspace != nullptr && workspace_bytes >= need &&
-         aligned16(workspace) && reserved_smem_per_block() == (int)kBase;
 }
 
 template <int FMT, bool WIDE>
