@@ -241,7 +241,7 @@ struct QgemmParams {
   unsigned* counters;
   int* status;
   int Mb, N, K, group_size, tokens_padded, ksplit;
-  int ordered;          // the parts of a tile add to the scratch in the order of K
+  int ordered;          // the parts of a tile add to the scratch in a fixed order (that of K)
   // NF4 only (group_size is the absmax block size there)
   const float* absmax;
   const float* lut16;

@@ -15,7 +15,8 @@
 //   warp 18     X by TMA into the stages, 64 inputs x all tokens per half.
 //
 // What bounds it: issue slots and the half-rate integer and fp16 pipes of the unpack warps
-// (350 warp instructions per warp and step, 128 of them the unpacking itself).  Of
+// (257 instructions per warp and step for 3-bit, 318 for NF4; 128 and 160 are the
+// unpacking itself).  Of
 // what the other form spent:
 //  * tcgen05.mma takes N / 2 cycles on the tensor pipe, but issuing one took 64 (a commit 95)
 //    where its addresses come from registers, 26 (15) where they are constants: the CTA
