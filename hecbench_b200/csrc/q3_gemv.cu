@@ -16,9 +16,9 @@
 //    memory) gives q*x directly from AND + FMA, no shift, no int->float;
 //  * the affine part is factored: sum (s*q - z)*x = s*sum(q*x) - z*sum(x);
 //  * a warp's packed rows are requested one group ahead, the first ones before the inputs are
-//    staged and the next column block's before the sums of this one meet (fp32 inputs 28672 x
-//    4096 22.4 -> 20.5 us with the zeroing of the sums, 1024 x 4096 5.7 -> 4.1 to 5.0, 32768 x
-//    8192 38.4 -> 35.1; fp16 8192 x 8192 13.2 -> 12.3, 49152 x 12288 54.6 either way);
+//    staged, those of a short next column block before the sums of this one meet (fp32 inputs
+//    28672 x 4096 22.4 -> 20.5 us with the zeroing of the sums, 1024 x 4096 5.7 -> 4.1 to 5.0, 32768
+//    x 8192 38.4 -> 35.1; fp16 8192 x 8192 13.0 -> 12.3, 49152 x 12288 54.7 -> 53.4);
 //  * K is split over the 8 warps of a CTA and over gridDim.y; partial sums are
 //    combined in shared memory and added to mul with one atomicAdd per column
 //    per CTA (the reference API accumulates into mul).
@@ -44,7 +44,7 @@ __device__ __forceinline__ int f16_window_start(int w) {
 
 // MULTI: a CTA takes several column blocks one after the other (a separate
 // instantiation: the single-block form keeps its code).
-template <bool F16IN, bool MULTI>
+template <bool F16IN, bool MULTI, bool LONG>
 __global__ void __launch_bounds__(kThreads)
 q3_gemv_kernel(const void* vec_, const int32_t* mat,
                float* mul, const float* scales,
@@ -73,6 +73,11 @@ q3_gemv_kernel(const void* vec_, const int32_t* mat,
   // group ahead through the column blocks, the first before the inputs are staged.
   uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0, n2 = n0;
   const int ncb = MULTI ? colblocks_per_cta : 1;
+  // Across column blocks only where a warp has up to four groups in each (16384 x 2048, one
+  // group: 9.8 -> 8.4 us; 28672 x 8192, three or four: 28.4 -> 27.1); with longer slices the first
+  // request of a block waits for its start (49152 x 12288, eight: 54.9 asked ahead, 53.4 not).
+  // LONG: a slice of more than five groups per warp, an instantiation without that code.
+  const bool ahead = groups_per_cta <= 4 * kWarps;
   auto request = [&](int cb, int gi) {
     const int col0 = (blockIdx.x * ncb + cb) * kColsPerCta + lane * 4;
     if (col0 < width && gi < ng) {
@@ -141,10 +146,11 @@ q3_gemv_kernel(const void* vec_, const int32_t* mat,
     // ---- main loop: this warp takes groups warp, warp+8, ... of the CTA slice ----
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     float sumx = 0.f;
+    if (MULTI && (LONG || !ahead) && cb > 0) request(cb, warp);
     for (int gi = warp; gi < ng; gi += kWarps) {
       const uint4 u0 = n0, u1 = n1, u2 = n2;
       if (gi + kWarps < ng) request(cb, gi + kWarps);
-      else if (MULTI && cb + 1 < ncb) request(cb + 1, warp);
+      else if (MULTI && !LONG && ahead && cb + 1 < ncb) request(cb + 1, warp);
       sumx += gsum[gi];
       const uint32_t w0s[4] = {u0.x, u0.y, u0.z, u0.w};
       const uint32_t w1s[4] = {u1.x, u1.y, u1.z, u1.w};
@@ -272,6 +278,11 @@ q3_dequant_kernel(const int32_t* __restrict__ mat, const float* __restrict__ sca
   }
 }
 
+template <auto Kern>
+struct Form {
+  static constexpr auto value = Kern;
+};
+
 template <bool F16IN>
 int q3_gemv_launch(const void* vec, const int32_t* mat, float* mul, const float* scales,
                    const float* zeros, int height, int width, hq_stream_t stream) {
@@ -315,22 +326,22 @@ int q3_gemv_launch(const void* vec, const int32_t* mat, float* mul, const float*
   size_t smem = (size_t)gpc * xp_words * 4 + (size_t)((gpc + 3) & ~3) * 4 +
                 (size_t)kWarps * kColsPerCta * 4 + 16;
   dim3 grid(colblocks, ksplit);
-  if (cbs > 1) {
-    constexpr auto kern = q3_gemv_kernel<F16IN, true>;
+  auto go = [&](auto form) {
+    constexpr auto kern = decltype(form)::value;
     if (smem > 48 * 1024) {
       cudaError_t e = ensure_dynamic_smem<kern>(smem);
       if (e != cudaSuccess) return cuda_status(e);
     }
-    return cuda_status(launch_pdl(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, vec, mat,
-                                  mul, scales, zeros, groups, width, gpc, cbs));
+    return cuda_status(launch_pdl(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, vec, mat, mul,
+                                  scales, zeros, groups, width, gpc, cbs));
+  };
+  if (cbs == 1) return go(Form<q3_gemv_kernel<F16IN, false, false>>());
+  // fp32 inputs always take one block
+  if constexpr (F16IN) {
+    if (gpc > 5 * kWarps) return go(Form<q3_gemv_kernel<true, true, true>>());
+    return go(Form<q3_gemv_kernel<true, true, false>>());
   }
-  constexpr auto kern = q3_gemv_kernel<F16IN, false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = ensure_dynamic_smem<kern>(smem);
-    if (e != cudaSuccess) return cuda_status(e);
-  }
-  return cuda_status(launch_pdl(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, vec, mat,
-                                mul, scales, zeros, groups, width, gpc, 1));
+  return HQ_ERR_UNSUPPORTED;  // not reached
 }
 
 template <bool F16OUT>
