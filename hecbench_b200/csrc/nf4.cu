@@ -593,17 +593,20 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-inline size_t mma_smem_bytes(int nchunks) {
+// dynamic shared memory (the kernel has no other); packets: the input comes as packets and is
+// unpacked there first
+constexpr int kMaxChunks = 2048;  // of a row: K <= 65536
+constexpr size_t mma_smem_bytes(int nchunks, bool packets) {
   const int supers = (nchunks + 15) / 16;
   return (size_t)kLutImm + kLutBytes + (size_t)supers * 4 * kMmaStepBytes + 2 * kMmaWarps * 16 * sizeof(float) +
-         (size_t)nchunks * 64;  // packet input, unpacked
+         (packets ? (size_t)nchunks * 64 : 0);
 }
+static_assert(mma_smem_bytes(kMaxChunks, false) <= 227 * 1024, "every row without packets fits");
 
 // rows: of the matrix; p.S, p.G as above; FUSE and LL as for nf4_gemv_kernel.
 template <bool FUSE, bool LL>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 nf4_gemv_mma_kernel(const GemvParams p, int rows, int tiles, int supers) {
-  __shared__ float s_sq[kMmaWarps];
   extern __shared__ __align__(16) unsigned char dsm_raw[];
   // [pad up to shared address kLutImm] table | inputs | partial sums [2][warp][16] | packets
   pdl_launch_dependents();
@@ -728,11 +731,11 @@ nf4_gemv_mma_kernel(const GemvParams p, int rows, int tiles, int supers) {
   }
   if (norm_in) {
     sq = warp_sum(sq);
-    if (lane == 0) s_sq[warp] = sq;
+    if (lane == 0) part[warp] = sq;  // (the partial sums come behind the last barrier below)
     __syncthreads();
     float tot = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMmaWarps; i++) tot += s_sq[i];
+    for (int i = 0; i < kMmaWarps; i++) tot += part[i];
     const float norm = rsqrtf(tot / (float)(p.nchunks * 32) + p.eps);
     for (int i = tid; i < pieces; i += kMmaThreads) {
       uint4* at = reinterpret_cast<uint4*>(xs + mma_piece(i));
@@ -1393,7 +1396,7 @@ int launch_gemv_mma(GemvParams& prm, int rows, cudaStream_t st) {
     const long cost = rounds * ((supers + s - 1) / s + 1);
     if (cost < best) best = cost, prm.S = s, prm.G = groups;
   }
-  const size_t smem = mma_smem_bytes(prm.nchunks);
+  const size_t smem = mma_smem_bytes(prm.nchunks, prm.A_ll != nullptr);
   constexpr auto kern = nf4_gemv_mma_kernel<FUSE, LL>;
   cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
@@ -1441,7 +1444,7 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   if (reserved_smem_per_block() > kLutImm) return HQ_ERR_UNSUPPORTED;
   const int nchunks = K / 32;
   const int cols = (nchunks + 31) / 32;  // 1024-input slices per row
-  if (cols > 64) return HQ_ERR_TOO_LARGE;  // K > 65536
+  if (nchunks > kMaxChunks) return HQ_ERR_TOO_LARGE;
   const int cpb = blocksize / 32;
   int shift = -1;
   if ((cpb & (cpb - 1)) == 0) {
@@ -1541,7 +1544,8 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   // 14336 56.7 -> 54.3).
   const long rows_per_sm = N / sm_count();
   const bool tensor = fuse != nullptr || cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
-  if (blocksize == 64 && K % 64 == 0 && tensor && !pair_packets && mma_smem_bytes(nchunks) <= 227 * 1024)
+  if (blocksize == 64 && K % 64 == 0 && tensor && !pair_packets &&
+      mma_smem_bytes(nchunks, ll.A_ll != nullptr) <= 227 * 1024)
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
            : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
                              : launch_gemv_mma<false, false>(prm, N, st);

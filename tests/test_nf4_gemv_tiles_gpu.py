@@ -27,3 +27,29 @@ def test_edges(hq, dev, N, K, early):
         bound = want.abs() * 2.0 ** -11 + terms.abs().sum(1) * K * 2.0 ** -24 + 2.0 ** -24
         got = hq.gemv_nf4(x, B, absmax, lut, N, K, 64, order, weights_resident=early)
         assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("K", [38144, 38208, 65536])
+def test_longest_fused_rows(hq, dev, K):
+    """RMSNorm, value / gate pairs and SwiGLU on the longest rows, against fp64 of the scaled inputs
+    rounded to fp16.  Those roundings may fall the other way where fp32 and fp64 norms differ: 2^-11 of
+    the sum of magnitudes more; both bounds pass through the product with the activation, whose slope is below 1.1."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(K)
+    rows = 34
+    x = torch.randn(K, generator=g, device=dev).half()
+    gamma = (torch.rand(K, generator=g, device=dev) + 0.5).half()
+    B = torch.randint(0, 256, (rows, K // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = (torch.rand(rows * K // 64, generator=g, device=dev) + 0.5) / K ** 0.5
+    lut = torch.sort(torch.rand(16, generator=g, device=dev) * 2 - 1).values
+    codes = torch.stack([(B >> 4).long(), (B & 15).long()], -1).view(rows, K)
+    xd = x.double()
+    xn = (xd * torch.rsqrt((xd * xd).mean() + 1e-5) * gamma.double()).half().double()
+    terms = lut.half().double()[codes] * xn * absmax.double().view(rows, K // 64).repeat_interleave(64, 1)
+    sums, off = terms.sum(1), terms.abs().sum(1) * (K * 2.0 ** -24 + 2.0 ** -11)
+    value, gate = sums[0::2], sums[1::2]
+    want = value * torch.nn.functional.silu(gate)
+    bound = want.abs() * 2.0 ** -10 + off[0::2] * gate.abs() + off[1::2] * 1.1 * value.abs() + 1.1 * off[0::2] * off[1::2]
+    got = hq.gemv_fused("nf4", x, B, rows // 2, gamma=gamma, eps=1e-5, act=hq.ACT_SWIGLU, absmax=absmax, lut16=lut,
+                        blocksize=64)
+    assert bool(((got.double() - want).abs() <= bound).all())
