@@ -452,6 +452,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         if (w_slot >= kWordAhead) { w_slot -= kWordAhead; w_parity ^= 1u; }
         // the A tile of this stage must have been released by the tensor core
         if (a_use != 0 && !mbar_wait(empty0 + 8 * a_stage, (a_use - 1u) & 1u, ok)) ok = false;
+        __syncwarp();  // .aligned instructions want the warp as a whole: lanes may leave a wait one by one
         tc_fence_after();  // orders the stores after the tensor core's reads of the stage
         tmem_store_32(a_lane + a_stage * (uint32_t)kAColumns, o);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -506,6 +507,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         w_slot += 2;
         if (w_slot >= kWordAhead) { w_slot -= kWordAhead; w_parity ^= 1u; }
         if (a_use != 0 && !mbar_wait(empty0 + 8 * a_stage, (a_use - 1u) & 1u, ok)) ok = false;
+        __syncwarp();  // .aligned instructions want the warp as a whole: lanes may leave a wait one by one
         tc_fence_after();  // orders the stores after the tensor core's reads of the stage
         tmem_store_32(a_lane + a_stage * (uint32_t)kAColumns, o);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -606,6 +608,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   if (warp < 8) {
     // ------------------------------ epilogue ------------------------------
     if (!mbar_wait(accum_bar, 0, ok)) ok = false;
+    __syncwarp();
     tc_fence_after();
     const int n = n0 + (warp & 3) * 32 + lane;  // TMEM lane = D row = output feature
     const uint32_t taddr = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);

@@ -387,6 +387,7 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         __syncwarp();
         if (lane == 0) mbar_arrive(slot_done);  // the words were consumed, so their loads have returned
         if (left > 0) take_words(words_ready);
+        __syncwarp();  // .aligned instructions want the warp as a whole: lanes may leave a wait one by one
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
@@ -398,9 +399,10 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const bool whole = k0 == 0 && k1 == p.steps;
       if (!mbar_wait(done, segment & 1u, ok)) ok = false;
       segment++;
+      __syncwarp();
       tc_fence_after();
       const uint32_t taddr = lanes + (uint32_t)(s * S::kTokens);
-      const bool live = n < p.N;
+      const bool live = tile * kTileN + s * 128 < p.N;  // all or none of a warp: N is a multiple of 128
       // the groups of half 0 take the even 16-token chunks, those of half 1 the odd ones
       for (int j0 = h * 16; j0 < p.tokens_padded; j0 += 32) {
         uint32_t v[16];
