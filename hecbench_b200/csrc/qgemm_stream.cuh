@@ -118,7 +118,8 @@ __device__ __forceinline__ void tmem_store(uint32_t taddr, const uint32_t (&v)[8
                : "memory");
 }
 
-// whether the phase with the given parity is over, without waiting
+// whether the phase with the given parity is over, without waiting: this lane's answer, the
+// caller brings the warp together
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
@@ -276,7 +277,10 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t nw[8];
     [[maybe_unused]] const uint32_t par_at = 12 * 1024 + (uint32_t)((p.one_group ? 0 : h * 512) + col * 2);
     auto take_words = [&](bool ready) {
-      if (!ready && !mbar_wait(wfull + 8 * w.at, w.parity, ok)) ok = false;
+      if (!ready) {
+        if (!mbar_wait(wfull + 8 * w.at, w.parity, ok)) ok = false;
+        __syncwarp();
+      }
       const uint32_t slot = w_ring + w.at * S::kWordBytes;
       if constexpr (FMT == kFmtQ3) {
         const uint32_t src = slot + (uint32_t)(h * 6 * 1024 + col * 4), par = slot + par_at;
@@ -330,7 +334,7 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const bool stage_free = mbar_test(empty + 8 * a.at, a.parity ^ 1u);
         const uint32_t slot_done = wempty + 8 * w.at;
         w.next();
-        const bool words_ready = --left > 0 && mbar_test(wfull + 8 * w.at, w.parity);
+        const bool words_ready = --left > 0 && mbar_over(wfull + 8 * w.at, w.parity);
         // the A stage must have been released by the tensor core
         if (!stage_free && !mbar_wait(empty + 8 * a.at, a.parity ^ 1u, ok)) ok = false;
         __syncwarp();
@@ -385,9 +389,8 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(slot_done);  // the words were consumed, so their loads have returned
+        mbar_arrive_lane0(slot_done, lane);  // the words were consumed, so their loads have returned
         if (left > 0) take_words(words_ready);
-        __syncwarp();  // .aligned instructions want the warp as a whole: lanes may leave a wait one by one
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
@@ -402,7 +405,7 @@ qgemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       __syncwarp();
       tc_fence_after();
       const uint32_t taddr = lanes + (uint32_t)(s * S::kTokens);
-      const bool live = tile * kTileN + s * 128 < p.N;  // all or none of a warp: N is a multiple of 128
+      const bool live = n < p.N;  // all or none of a warp: N is a multiple of 128
       // the groups of half 0 take the even 16-token chunks, those of half 1 the odd ones
       for (int j0 = h * 16; j0 < p.tokens_padded; j0 += 32) {
         uint32_t v[16];
