@@ -1384,24 +1384,69 @@ struct LlArgs {
 
 namespace hq {
 namespace {
+// Division of the tensor form's work over a GPU of `sms` SMs: S warps per tile, G tiles at a time
+// per CTA.  The S with the fewest rounds, a tile counting one super-step more than a warp's
+// share of it for the sums at its end.
+struct MmaSplit {
+  int supers, tiles, S, G;
+  long rounds;
+};
+MmaSplit mma_split(int rows, int nchunks, int sms) {
+  MmaSplit m = {(nchunks + 15) / 16, (rows + 15) / 16, 1, kMmaWarps, 0};
+  long best = LONG_MAX;
+  for (int s = 1; s <= std::min(m.supers, kMmaWarps); s++) {
+    const int groups = kMmaWarps / s;
+    const long rounds = (m.tiles + (long)sms * groups - 1) / ((long)sms * groups);
+    const long cost = rounds * ((m.supers + s - 1) / s + 1);
+    if (cost < best) best = cost, m.S = s, m.G = groups, m.rounds = rounds;
+  }
+  return m;
+}
+
+// Whether a fused call (RMSNorm and / or a gated activation) with absmax blocks of 64 takes the
+// tensor form.  us, row form -> tensor form, weights resident:
+//  * rows of up to 4096 inputs always, RMSNorm with SwiGLU or without (28672 x 4096 21.8 -> 20.1,
+//    1024 x 4096 4.8 -> 3.4, 2048 x 2048 5.1 -> 2.9); from 3073 inputs on and without the early fetch, which
+//    would cover its longer start, up to one tile per SM (2368 x 4096 5.5 -> 4.8, without norm 3072 rows
+//    1.16 of the time);
+//  * up to 32768 where a model of both expects less.  A tile of 16 rows is a CTA's: few rows or a second
+//    round for a few leave SMs idle (512 x 16384 5.2 -> 7.5, 2560 x 28672 18.3 -> 20.9), and the
+//    row form has idle warps where its slices of 2048 inputs do not divide 16 (4096 x 11008 13.7 -> 10.8,
+//    8192 x 20480 0.66 of the time; 14336 x 8192 0.91).  Fitted to 966 layers of 64 to 28672 rows, norm, activation
+//    and early fetch on and off (4 % off): over them it takes 0.925 of the row form's time, the better form
+//    each time 0.922, the tensor form always 1.02;
+//  * up to 57344, where the row form has half its rows in flight, from K / 45 rows on (1024 x 40960 25.3 -> 17.2,
+//    512 x 40960 16.5 -> 16.9, 1024 x 57344 0.87 to 0.98 of the time, 512 1.3 to 1.55); beyond never (65536: 2368
+//    rows 51.7 -> 34.5, but 2560 46.7 -> 58.3).
+bool fused_takes_tensor(int rows, int nchunks, bool norm, bool act, bool resident) {
+  const int sms = sm_count(), cols = (nchunks + 31) / 32;
+  if (cols <= 4) return cols < 4 || resident || rows <= 16 * sms;
+  if (cols > 32) return cols <= 56 && rows * 45ll >= nchunks * 32ll;
+  const MmaSplit m = mma_split(rows, nchunks, sms);
+  const double tile_rounds = (double)m.rounds * ((m.supers + m.S - 1) / m.S);
+  const double busiest = (double)std::min<long>(m.G, (m.tiles + sms - 1) / sms) * m.supers * m.rounds / kMmaWarps;
+  const double all = (double)m.tiles * m.supers / (16.0 * sms);
+  const double tensor = resident ? (norm ? 2.42 : 1.49) + 0.72 * tile_rounds + 0.05 * m.supers + 0.86 * busiest + 0.94 * all
+                                 : (norm ? 3.73 : 2.79) + 0.45 * tile_rounds + 0.05 * m.supers + 1.21 * busiest + all;
+  const int units = act ? rows / 2 : rows, at_once = sms * (16 / ((cols + 1) / 2));
+  const double turns = (double)((units + at_once - 1) / at_once) * (act ? 2 : 1), share = (double)rows * cols / (32.0 * sms);
+  const double by_rows = act ? (norm ? (resident ? 3.33 : 4.02) : (resident ? 1.89 : 2.61)) + 0.61 * turns + 0.02 * cols + 0.15 * share
+                             : (resident ? 3.51 : 4.20) + 0.57 * turns + 0.02 * cols + 0.16 * share;
+  return tensor < by_rows;
+}
+
 template <bool FUSE, bool LL>
 int launch_gemv_mma(GemvParams& prm, int rows, cudaStream_t st) {
-  const int supers = (prm.nchunks + 15) / 16, tiles = (rows + 15) / 16, sms = sm_count();
-  // Warps per tile: the count with the fewest rounds, a tile counting one super-step more
-  // than a warp's share of it for the sums at its end.
-  long best = LONG_MAX;
-  for (int s = 1; s <= std::min(supers, kMmaWarps); s++) {
-    const int groups = kMmaWarps / s;
-    const long rounds = (tiles + (long)sms * groups - 1) / ((long)sms * groups);
-    const long cost = rounds * ((supers + s - 1) / s + 1);
-    if (cost < best) best = cost, prm.S = s, prm.G = groups;
-  }
+  const int sms = sm_count();
+  const MmaSplit m = mma_split(rows, prm.nchunks, sms);
+  prm.S = m.S;
+  prm.G = m.G;
   const size_t smem = mma_smem_bytes(prm.nchunks, prm.A_ll != nullptr);
   constexpr auto kern = nf4_gemv_mma_kernel<FUSE, LL>;
   cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
-  return cuda_status(launch_pdl(kern, dim3(std::min(sms, tiles)), dim3(kMmaThreads), smem, st, prm,
-                                rows, tiles, supers));
+  return cuda_status(launch_pdl(kern, dim3(std::min(sms, m.tiles)), dim3(kMmaThreads), smem, st, prm,
+                                rows, m.tiles, m.supers));
 }
 
 template <int C>
@@ -1480,6 +1525,7 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   prm.gamma = nullptr;
   prm.eps = 0.f;
   prm.act = HQ_ACT_NONE;
+  bool bare = false;  // a fused call of the row form without normalisation and activation
   int units = N;  // what a group of warps walks: rows, or value / gate pairs
   if (fuse != nullptr) {
     if (fuse->act != HQ_ACT_NONE && fuse->act != HQ_ACT_SWIGLU && fuse->act != HQ_ACT_GEGLU)
@@ -1493,6 +1539,15 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
     prm.gamma = reinterpret_cast<const __half*>(fuse->gamma);
     prm.eps = fuse->eps;
     prm.act = fuse->act;
+    // Neither: the plain mat-vec in its own forms (weights resident, 28672 x 4096 19.8 -> 14.6 us, 512 x
+    // 16384 3.8 -> 3.5).  Without the early fetch the row form with this option compiled in is the faster
+    // one from 4.5 to 21 Mi weights (1024 x 16384 5.4 us, plain 6.3; 3072 x 4096 4.65 and 5.35; 2048 x 16384
+    // 8.4 and 8.2, 512 x 8192 3.97 and 3.84); the reason has not been found.
+    if (fuse->gamma == nullptr && fuse->act == HQ_ACT_NONE) {
+      const double weights = (double)N * K;
+      bare = !prm.early_fetch && K > 3072 && weights > 4.5e6 && weights < 21e6;
+      if (!bare) fuse = nullptr;
+    }
   }
   // Packet output, opt-in (environment HQ_LL_PAIRS=1): walk the rows in adjacent
   // pairs and send both results in one 16-byte store per GPU - half as many
@@ -1539,11 +1594,9 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   //   6.0 -> 6.3, 28672 x 2048 9.5 -> 10.4
   //   four, up to 16: 1024 x 4096 2.91 -> 2.71, 2048 x 4096 3.3 -> 2.9, 4096 x 4096 4.28 -> 4.32,
   //   28672 x 4096 14.4 -> 18.9; longer rows gain nothing (2048 x 8192 4.5 -> 4.8).
-  // The fused forms always take it (RMSNorm, up / gate, SwiGLU and the plain down projection
-  // after it: 2048 - 5632 12.0 -> 10.3, 4096 - 14336 31.2 -> 30.1, 5120 - 13824 42.9 -> 35.0, 8192 -
-  // 14336 56.7 -> 54.3).
   const long rows_per_sm = N / sm_count();
-  const bool tensor = fuse != nullptr || cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
+  const bool tensor = fuse != nullptr ? !bare && fused_takes_tensor(N, nchunks, fuse->gamma != nullptr, fuse->act != HQ_ACT_NONE, prm.early_fetch != 0)
+                                      : cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
   if (blocksize == 64 && K % 64 == 0 && tensor && !pair_packets &&
       mma_smem_bytes(nchunks, ll.A_ll != nullptr) <= 227 * 1024)
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)

@@ -65,7 +65,9 @@ def test_fused_against_oracle(hq, oracle, dev, fmt, rows_out, n, act, norm):
     (777, 8192, 64, 2),      # run-time number of warps per row
     (96, 11008, 64, 1),      # ragged last slice (11008 = 10 * 1024 + 768)
     (64, 2080, 96, 1),       # blocks that straddle rows (not a power of two)
-    (40, 40960, 64, 0)])     # four chunks per lane
+    (40, 40960, 64, 0),      # four chunks per lane
+    # the row form's aligned instantiations, which blocks of 64 reach for few long rows alone
+    (1024, 4096, 128, 1), (777, 8192, 128, 2), (96, 11008, 256, 1)])
 def test_fused_nf4_kernel_forms(hq, oracle, dev, rows_out, n, bs, act):
     """Every form of the NF4 kernel (chunks per lane, warps per row, aligned or
     straddling absmax blocks) with the RMSNorm and the row pairing switched on,
@@ -83,6 +85,41 @@ def test_fused_nf4_kernel_forms(hq, oracle, dev, rows_out, n, bs, act):
         ref = oracle.gemv_fused_f64("nf4", mat, x, gamma, 1e-5, rows_out, act, absmax=absmax,
                                     lut16=lut, blocksize=bs, low_first=order)
         assert oracle.rel_err(y.cpu().numpy().astype(np.float64), ref) < TOL_F16
+
+
+@pytest.mark.parametrize("rows_mat,n,act,norm,resident,form", [
+    (1024, 16384, 0, True, True, "rows"), (1024, 16384, 1, True, True, "rows"), (2560, 28672, 1, True, False, "rows"),
+    (512, 40960, 1, True, True, "rows"), (2048, 40960, 1, True, True, "tensor"), (28672, 4096, 1, True, True, "tensor"),
+    (6144, 4096, 0, True, True, "tensor"), (14336, 8192, 1, True, True, "tensor"), (4096, 11008, 0, True, False, "tensor"),
+    (4096, 4096, 1, False, False, "rows"), (1024, 4096, 1, False, False, "tensor"),
+    (2048, 65536, 1, True, True, "rows"), (2048, 8192, 0, False, False, "rows"), (28672, 4096, 0, False, False, "plain rows"),
+    (28672, 4096, 0, False, True, "plain rows"), (512, 16384, 0, False, True, "plain rows"), (1024, 4096, 0, False, True, "plain tensor")])
+def test_fused_nf4_form_by_rule(hq, oracle, dev, rows_mat, n, act, norm, resident, form):
+    """Fused calls run the form that is the faster one there: few or unevenly many tiles of long rows
+    go to the row form, and without normalisation and activation the plain mat-vec's kernels run.
+    A stride of the results against the oracle."""
+    import torch
+    from launches import launched
+    g = torch.Generator(device=dev).manual_seed(rows_mat + n)
+    x = (torch.randn(n, generator=g, device=dev) * 3).half()
+    gamma = (torch.rand(n, generator=g, device=dev) + 0.5).half() if norm else None
+    mat = torch.randint(0, 256, (rows_mat, n // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = (torch.rand((rows_mat, n // 64), generator=g, device=dev) + 0.5) / n ** 0.5
+    lut = torch.linspace(-1, 1, 16, device=dev)
+    rows_out = rows_mat // 2 if act else rows_mat
+    y = []
+    call = lambda: y.append(hq.gemv_fused("nf4", x, mat, rows_out, gamma=gamma, eps=1e-5, act=act, absmax=absmax.view(-1),
+                                          lut16=lut, blocksize=64, weights_resident=resident))
+    ((name, _),) = launched(call)
+    assert ("nf4_gemv_mma_kernel" in name) == form.endswith("tensor"), name
+    # the template argument before the last: FUSE
+    assert name.split("EEEv")[0].split("ELb")[-2][-1] == ("0" if form.startswith("plain") else "1"), name
+    pick = torch.arange(0, rows_out, max(1, rows_out // 16), device=dev)
+    mrows = torch.stack([2 * pick, 2 * pick + 1], 1).view(-1) if act else pick
+    ref = oracle.gemv_fused_f64("nf4", mat[mrows].cpu().numpy(), x.cpu().numpy(), None if gamma is None else gamma.cpu().numpy(),
+                                1e-5, len(pick), act, absmax=absmax[mrows].reshape(-1).cpu().numpy(), lut16=lut.cpu().numpy(),
+                                blocksize=64)
+    assert oracle.rel_err(y[0][pick].cpu().numpy().astype(np.float64), ref) < TOL_F16
 
 
 def test_fused_equals_separate_kernels_nf4(hq, oracle, dev):
