@@ -1408,7 +1408,8 @@ MmaSplit mma_split(int rows, int nchunks, int sms) {
 //  * rows of up to 4096 inputs always, RMSNorm with SwiGLU or without (28672 x 4096 21.8 -> 20.1,
 //    1024 x 4096 4.8 -> 3.4, 2048 x 2048 5.1 -> 2.9); from 3073 inputs on and without the early fetch, which
 //    would cover its longer start, up to one tile per SM (2368 x 4096 5.5 -> 4.8, without norm 3072 rows
-//    1.16 of the time);
+//    1.16 of the time).  Up to 8192 with RMSNorm and the early fetch, whose start is the shorter one in this
+//    form (64 x 6144 4.74 -> 4.23, 8192 x 8192 14.5 -> 13.2; 2560 x 6144, the worst, 6.2 -> 6.5);
 //  * up to 32768 where a model of both expects less.  A tile of 16 rows is a CTA's: few rows or a second
 //    round for a few leave SMs idle (512 x 16384 5.2 -> 7.5, 2560 x 28672 18.3 -> 20.9), and the
 //    row form has idle warps where its slices of 2048 inputs do not divide 16 (4096 x 11008 13.7 -> 10.8,
@@ -1421,6 +1422,7 @@ MmaSplit mma_split(int rows, int nchunks, int sms) {
 bool fused_takes_tensor(int rows, int nchunks, bool norm, bool act, bool resident) {
   const int sms = sm_count(), cols = (nchunks + 31) / 32;
   if (cols <= 4) return cols < 4 || resident || rows <= 16 * sms;
+  if (cols <= 8 && norm && resident) return true;
   if (cols > 32) return cols <= 56 && rows * 45ll >= nchunks * 32ll;
   const MmaSplit m = mma_split(rows, nchunks, sms);
   const double tile_rounds = (double)m.rounds * ((m.supers + m.S - 1) / m.S);
