@@ -53,3 +53,35 @@ def test_longest_fused_rows(hq, dev, K):
     got = hq.gemv_fused("nf4", x, B, rows // 2, gamma=gamma, eps=1e-5, act=hq.ACT_SWIGLU, absmax=absmax, lut16=lut,
                         blocksize=64)
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("level", [0, 3, 15])
+@pytest.mark.parametrize("N,K", [(33, 1024), (40, 576), (100, 2816), (70, 4096)])
+def test_infinite_level(hq, dev, N, K, level):
+    """A level that no fp16 number holds: rows without its code keep their value, the others become
+    infinite with the sign of the product, or NaN where two signs meet, as the sum of the products has it."""
+    import torch
+    from launches import launched
+    g = torch.Generator(device=dev).manual_seed(N + K + level)
+    x = torch.randn(K, generator=g, device=dev).half()
+    codes = torch.randint(0, 15, (N, K), generator=g, device=dev)
+    codes += codes >= level                                            # every code but `level`
+    once = torch.arange(0, N, 3, device=dev)                           # one such code in every third row,
+    codes[once, torch.randint(0, K, (len(once),), generator=g, device=dev)] = level
+    codes[0, [1, 40]] = level                                          # and two of one block in the first
+    x[1], x[40] = 1.0, -1.0
+    B = (codes[:, 0::2] << 4 | codes[:, 1::2]).to(torch.uint8)
+    absmax = (torch.rand(N * K // 64, generator=g, device=dev) + 0.5) / K ** 0.5
+    lut = torch.linspace(-1, 1, 16, device=dev)
+    lut[level] = 1e30 if level else -float("inf")
+    terms = lut.half().double()[codes] * x.double() * absmax.double().view(N, K // 64).repeat_interleave(64, 1)
+    want = terms.sum(1)
+    got = []
+    ((name, _),) = launched(lambda: got.append(hq.gemv_nf4(x, B, absmax, lut, N, K, 64)))
+    assert "nf4_gemv_mma_kernel" in name
+    got = got[0].double()
+    finite = want.isfinite()
+    assert bool(want[0].isnan()) and bool(want.isinf().any()) and bool(finite.any())
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[want.isinf()], want[want.isinf()])
+    bound = want.abs() * 2.0 ** -11 + terms.abs().sum(1) * K * 2.0 ** -24 + 2.0 ** -24
+    assert bool(((got - want).abs() <= bound)[finite].all())
