@@ -1,6 +1,6 @@
 """Edges of the LUT-GEMM mat-vec's units: column counts around a warp's 32 and a range's 256, K
-tiles past the end of K, alpha groups below a tile, four planes in one launch, several units
-per CTA and more column ranges than completion counters."""
+tiles past the end of K, alpha groups below a tile, four planes in one launch, more column
+ranges than completion counters, and several units per CTA with ragged last ranges and tiles."""
 import numpy as np
 import pytest
 
@@ -30,3 +30,22 @@ def test_edges(hq, oracle, dev, M, K, nb, gs, bias):
         got = out.cpu().numpy().astype(np.float64)
         assert np.linalg.norm(got - ref) <= 1e-3 * np.linalg.norm(ref)
     assert torch.count_nonzero(w.workspace()) == 0
+
+
+@pytest.mark.parametrize("M,K,nb,gs,bias", [
+    (6148, 9632, 3, 32, True), (6148, 9664, 4, 64, True), (3076, 20544, 4, 64, False), (8196, 9664, 3, 64, False)])
+def test_several_units_per_cta(hq, oracle, dev, M, K, nb, gs, bias):
+    """228 to 322 units on the CTAs of the ring form, one per SM of 148: a last column range of four columns
+    more than a warp's, one to two rows of four in the last tile."""
+    import torch
+    from launches import launched
+    x, bW, alpha, qb = synth.lutgemm_case(M, K, nb, gs, seed=M + K + nb, bias=bias)
+    w = hq.nQWeight_fp16()
+    w.parsing(bW, alpha.astype(np.float32), K, M, nb, False, K // gs,
+              None if qb is None else qb.astype(np.float32), device=dev)
+    out = torch.empty(M, dtype=torch.float16, device=dev)
+    dx = to_dev(x.view(np.uint16), dev).view(torch.float16)
+    ((name, grid),) = launched(lambda: hq.matmul(out, dx, w))
+    assert f"lutgemm_ring_kernelILi{nb}E" in name
+    assert grid == torch.cuda.get_device_properties(dev).multi_processor_count
+    test_edges(hq, oracle, dev, M, K, nb, gs, bias)

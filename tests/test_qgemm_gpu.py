@@ -133,6 +133,20 @@ def test_qgemm_parts_of_k_repeat(hq, dev, fmt, Mb, K, N):
         assert torch.equal(y, first)
 
 
+@pytest.mark.parametrize("fmt,Mb,K,N", [("q3", 64, 8960, 14976), ("q3", 2, 8960, 14976), ("nf4", 64, 8960, 15104)])
+def test_qgemm_ordered_parts_of_two_ctas(hq, dev, fmt, Mb, K, N):
+    """The few wide layers that stay in more than two parts with one tile per CTA, where the parts add in
+    the order of K: the same bits from every call as well."""
+    import torch
+    from launches import launched
+    from test_qgemm_tiles_gpu import _operands
+    call, _ = _operands(hq, fmt, K, N, 128, dev, torch.Generator(device=dev).manual_seed(K))
+    X = torch.zeros((Mb, K), dtype=torch.float16, device=dev)
+    ((name, grid),) = launched(lambda: call(X))
+    assert "12qgemm_kernel" in name and grid > 2 * (N // 128)
+    test_qgemm_parts_of_k_repeat(hq, dev, fmt, Mb, K, N)
+
+
 LLAMA3_70B_MLP = [(8192, 28672), (28672, 8192)]  # (K, N): up/gate and down projections
 
 

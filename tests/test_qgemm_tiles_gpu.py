@@ -30,8 +30,8 @@ def _operands(hq, fmt, K, N, group, dev, g):
     (1, 64, 128, 64), (16, 128, 128, 64), (17, 192, 384, 64), (64, 320, 256, 64), (65, 448, 640, 64),
     (128, 1088, 128, 64), (2, 4096, 1152, 128), (37, 8192, 4224, 128), (64, 1024, 37888, 128),
     (96, 8256, 2176, 64), (128, 2048, 38016, 128), (33, 28672, 1024, 128),
-    # the streamed form: half a step and half a tile left over, scale groups of half a step, whole and
-    # cut tiles, tokens on both sides of 64
+    # long layers on both sides of the line to the streamed form: half a step and half a tile left over,
+    # scale groups of half a step, whole and cut tiles, tokens on both sides of 64
     (1, 8256, 14464, 64), (64, 3648, 28672, 64), (65, 16448, 7296, 64), (128, 1088, 104704, 64),
     (16, 28672, 4096, 128), (100, 1024, 120064, 128)])
 def test_edges(hq, dev, fmt, Mb, K, N, group):
@@ -52,3 +52,20 @@ def test_edges(hq, dev, fmt, Mb, K, N, group):
         assert int(status.item()) == 0, "a bounded in-kernel wait ran out"
         assert bool(((got.double() - want).abs() <= bound).all())
     assert all(int(torch.count_nonzero(w)) == 0 for w in api._qgemm_ws.values())
+
+
+@pytest.mark.parametrize("fmt", ["q3", "nf4"])
+@pytest.mark.parametrize("Mb,K,N,group", [
+    (1, 8256, 14464, 64), (64, 5184, 38016, 64), (65, 16448, 7296, 64), (128, 1088, 104704, 64),
+    (64, 28736, 6528, 64), (16, 28672, 8064, 128), (100, 1024, 120064, 128)])
+def test_streamed_edges(hq, dev, fmt, Mb, K, N, group):
+    """The same bounds where the streamed form runs (one CTA per SM of 148): a half step and a half tile
+    left over, 1 to 128 tokens, whole tiles, cut ones in a fixed order and, on narrow layers, in none."""
+    import torch
+    from launches import launched
+    g = torch.Generator(device=dev).manual_seed(Mb + K + N)
+    call, _ = _operands(hq, fmt, K, N, group, dev, g)
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    ((name, grid),) = launched(lambda: call(X))
+    assert "qgemm_stream_kernel" in name and grid == torch.cuda.get_device_properties(dev).multi_processor_count
+    test_edges(hq, dev, fmt, Mb, K, N, group)
