@@ -501,7 +501,7 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
   const uint32_t hi = (uint32_t)(lane * 4);
   const uint32_t sel = 0x7604u | ((uint32_t)j << 4);
   uint32_t at_stage = 0;
-  int built = -1;  // tile of the tables in place
+  int built = -1;  // tile of the tables in place (kept only with more ranges than CTAs: millions of columns)
   float ones[kGroups];
 
   for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
@@ -984,12 +984,13 @@ int launch_ring(const LaunchArgs& a, int b0, const __half* bias, int finalize) {
                                 (int)a.grid.x, (int)a.grid.y, a.nb_total, b0, finalize, a.per_range));
 }
 
-// Bit planes are handled up to kMax at a time (what the register budget of the
-// one-step-ahead loads allows, or the rings have room for); further planes go to
-// follow-up launches that accumulate into the same scratch row.  Only the first
-// launch adds the bias term, only the last one converts the scratch row.  The ring
-// form takes four planes, and three where a CTA has several units of two column
-// steps or more (times at its head).
+// Planes go in launches of up to four (three with alpha groups of 32 inputs, whose parameters leave
+// the rings no room for a fourth) that accumulate into the same scratch row.  Only the first
+// launch adds the bias term, only the last one converts the scratch row.  On tiles of 128
+// inputs the ring form takes four planes, and three where a CTA has several units of two column
+// steps or more (times at its head); the register form takes the rest.  Five to eight planes as 4 + 1
+// to 4 + 4 take 0.75 to 1.00 of what 3 + 2 to 3 + 3 + 2 took (4096 x 4096, 7 planes 17.8 -> 13.8 us; 12288 x
+// 12288, 8 planes 74.4 -> 60.9), five planes of 4096 x 12288 1.02 (25.7 -> 26.1).
 template <int TR, int RPG>
 int launch_planes(const LaunchArgs& a) {
   constexpr bool kFour = TR == 2 || RPG > 1;  // groups of 32 inputs: the rings hold three planes

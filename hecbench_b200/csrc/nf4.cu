@@ -578,6 +578,8 @@ nf4_gemv_kernel(const GemvParams p) {
 //    lane whose blocks these are scales and adds them.
 //  * The inputs lie in shared memory, 288 bytes per 128 inputs (the chunks of t = 2, 3 are
 //    moved by 32 bytes: the four addresses of a load then meet in no bank).
+//  * Packets: 16 lanes hold the results of 16 rows, so a store to one GPU is 128 contiguous bytes, where
+//    the row form's lanes store one row's 8 bytes to every GPU; not timed on several GPUs.
 //  * S warps share a tile of 16 rows, each takes every S-th super-step; G groups of S per
 //    CTA.  A lane's 128 bytes of the next super-step are requested as this one uses the
 //    registers up.

@@ -16,9 +16,9 @@
 //    memory) gives q*x directly from AND + FMA, no shift, no int->float;
 //  * the affine part is factored: sum (s*q - z)*x = s*sum(q*x) - z*sum(x);
 //  * a warp's packed rows are requested one group ahead, the first ones before the inputs are
-//    staged, those of a short next column block before the sums of this one meet (fp32 inputs
-//    28672 x 4096 22.4 -> 20.5 us with the zeroing of the sums, 1024 x 4096 5.7 -> 4.1 to 5.0, 32768
-//    x 8192 38.4 -> 35.1; fp16 8192 x 8192 13.0 -> 12.3, 49152 x 12288 54.7 -> 53.4);
+//    staged, those of a short next column block before the sums of this one meet (device time of
+//    calls among others, with the zeroing of the sums: fp32 inputs 28672 x 4096 22.4 -> 20.5 us,
+//    32768 x 8192 38.4 -> 35.1; fp16 8192 x 8192 13.0 -> 12.3, 49152 x 12288 54.7 -> 53.4);
 //  * K is split over the 8 warps of a CTA and over gridDim.y; partial sums are
 //    combined in shared memory and added to mul with one atomicAdd per column
 //    per CTA (the reference API accumulates into mul).

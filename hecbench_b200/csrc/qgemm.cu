@@ -810,6 +810,16 @@ size_t qgemm_ws_bytes(int Mb, int N) {
   return ((size_t)Mb * N * 4 + 255) / 256 * 256 + ((size_t)(N / kTileN + 1) * 4 + 255) / 256 * 256;
 }
 
+// Whether a call gives the same bits every time: layers of at least two thirds of a tile per
+// SM, and those of few inputs.
+int plain_parts(int N, int K) { return max(1, min(2 * sm_count() / (N / kTileN), K / kBlockK / 8)); }
+bool repeatable(int N, int K) { return plain_parts(N, K) <= 2; }
+
+struct KSplit {
+  int parts;
+  bool ordered;
+  double cost;
+};
 // Number of parts K is cut into, for `tiles` tiles of nkb blocks.  The plain choice
 // makes up to two CTAs per SM (beyond 64 tokens, where one takes the SM, that is up to
 // two waves); another one replaces it where this model, in blocks of a CTA that
@@ -819,7 +829,8 @@ size_t qgemm_ws_bytes(int Mb, int N) {
 //  * every wave after the first costs 9 blocks (beyond 64 tokens, where one CTA
 //    takes the SM, 16) for its start, a split 10 (14) + 0.25 per part for the fp32
 //    reduction.
-// Measured against every count from one to six, both formats, 4 to 128 tokens, 16
+// Measured for this form alone (the streamed one now takes most long layers, these examples among
+// them) against every count from one to six, both formats, 4 to 128 tokens, 16
 // layers of K 2048 to 28672: never slower than the plain choice, within 5 % of the
 // best.  us, plain -> model, 3-bit (NF4):
 //   64 x 8192 x 20480, 1 -> 3 parts: 55.0 -> 45.9 (87.5 -> 69.2); 4 tokens: 52.9 -> 41.7
@@ -832,16 +843,6 @@ size_t qgemm_ws_bytes(int Mb, int N) {
 // 24576 in three parts 46.6 us either way, NF4 69.9 and 69.8).  Narrower layers, where
 // many short parts of a tile end together, add in any order: in turn, 64 x 4096 x 6144
 // would take 25.4 us for 12.7.
-// Whether a call gives the same bits every time: layers of at least two thirds of a tile per
-// SM, and those of few inputs.
-int plain_parts(int N, int K) { return max(1, min(2 * sm_count() / (N / kTileN), K / kBlockK / 8)); }
-bool repeatable(int N, int K) { return plain_parts(N, K) <= 2; }
-
-struct KSplit {
-  int parts;
-  bool ordered;
-  double cost;
-};
 // The sharded form never takes more parts than the plain choice: split, the last CTA
 // of a tile stores it to every GPU in 8-byte pieces instead of 256-byte rows, a cost
 // that the model does not know (no timing on several GPUs).

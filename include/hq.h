@@ -112,7 +112,10 @@ int hq_nf4_dequant_f16(const uint8_t* B, const float* absmax, const float* lut16
 /* NF4 4-bit GEMV (no counterpart in the reference tree):
  * out[n] = half_rn(sum_k A[k] * lut16[code[n][k]] * absmax[(n*K+k)/blocksize]),
  * B is [N][K/2] bytes row-major; K % 32 == 0, blocksize a multiple of 32 that
- * divides K. */
+ * divides K.  A call gives the same bits every time.  How a row's sum is divided, and
+ * whether products of a block of 64 are summed in fp16 or in fp32, is chosen by N, K and
+ * blocksize (fused calls: by the flags, gamma and act too), so a row may differ in its last
+ * bits between a layer and a slice of it. */
 int hq_nf4_gemv_f16(const void* A_half, const uint8_t* B, const float* absmax,
                     const float* lut16, void* out_half, int N, int K, int blocksize,
                     int flags, hq_stream_t stream);
