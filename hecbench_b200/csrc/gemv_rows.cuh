@@ -25,10 +25,12 @@ inline size_t smem_request(size_t need, int grid) {
 }
 
 // 4-bit rows of up to 4 KiB: the rows a warp starts with are on their way to L2 before the
-// wait for the kernel before and the staging of the inputs.  4096 x 4096 4.79 -> 4.18 us,
-// 28672 x 4096 16.9 -> 15.7, 8192 x 8192 11.9 -> 11.6, the two products of an MLP block 2048 -
-// 5632 14.8 -> 12.9.  Twice as many bytes per SM delay the inputs that wait behind them:
-// int4 4096 x 11008 10.13 -> 10.27, int8 8192 x 8192 14.4 -> 17.4.
+// wait for the kernel before and the staging of the inputs.  us of a call among others:
+// 4096 x 4096 4.8 -> 4.2, 28672 x 4096 17.0 -> 16.0, 8192 x 8192 12.0 -> 11.9, the two products of an
+// MLP block 2048 - 5632 14.8 -> 12.9; few short rows gain a little too (512 x 1024 2.57 -> 2.49).
+// Longer rows gain nothing (4096 x 11008 10.13 -> 10.27), and 8-bit rows of the same lengths
+// lose: 512 x 1024 2.65 -> 3.01, 4096 x 1024 2.69 -> 3.36, 1024 x 4096 4.67 -> 5.40, 28672 x 4096 21.97 -> 25.5
+// (8192 x 2048 alone 5.90 -> 5.05; 8192 x 8192 14.4 -> 17.4).
 __device__ __forceinline__ void prefetch_first_rows(const unsigned char* mat, int rows, size_t row_bytes,
                                                     int lane, int warp) {
   const long long row = ((long long)blockIdx.x * kWarps + warp) * kRows + lane;

@@ -76,7 +76,9 @@ q3_gemv_kernel(const void* vec_, const int32_t* mat,
   // Across column blocks only where a warp has up to four groups in each (16384 x 2048, one
   // group: 9.8 -> 8.4 us; 28672 x 8192, three or four: 28.4 -> 27.1); with longer slices the first
   // request of a block waits for its start (49152 x 12288, eight: 54.9 asked ahead, 53.4 not).
-  // LONG: a slice of more than five groups per warp, an instantiation without that code.
+  // LONG: a slice of more than five groups per warp, an instantiation without that code.  One line at
+  // four groups for both gains slices of 33 to 40 groups 1 to 2 % (28672 x 12800 37.1 -> 36.3 us) and costs
+  // the shorter ones as much, whose code it changes (28672 x 8192 27.2 -> 27.8, 16384 x 2048 8.47 -> 8.62).
   const bool ahead = groups_per_cta <= 4 * kWarps;
   auto request = [&](int cb, int gi) {
     const int col0 = (blockIdx.x * ncb + cb) * kColsPerCta + lane * 4;

@@ -1,8 +1,9 @@
-"""Which kernels a call launches, read from a stream capture of it (nothing runs then)."""
+"""Which of the library's kernels a call launches, read from a stream capture of it (nothing runs then)."""
 
 
 def launched(call):
-    """[(mangled name, grid blocks)] of the kernels of call(), in no fixed order."""
+    """[(mangled name, grid blocks)] of the kernels of call(), in no fixed order; a fill of fresh
+    scratch is not among them."""
     import torch
     from cuda.bindings import driver
 
@@ -24,5 +25,6 @@ def launched(call):
             continue
         (p,) = done(driver.cuGraphKernelNodeGetParams(node))
         (name,) = done(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))
-        found.append((name.decode(), p.gridDimX * p.gridDimY * p.gridDimZ))
+        if name.startswith(b"_ZN2hq"):
+            found.append((name.decode(), p.gridDimX * p.gridDimY * p.gridDimZ))
     return found
