@@ -15,7 +15,7 @@
 //   warp 18     X by TMA into the stages, 64 inputs x all tokens per half.
 //
 // What bounds it: issue slots and the half-rate integer and fp16 pipes of the unpack warps
-// (257 instructions per warp and step for 3-bit, 318 for NF4; 128 and 160 are the
+// (261 instructions per warp and step for 3-bit, 319 for NF4; 128 and 160 are the
 // unpacking itself).  Of
 // what the other form spent:
 //  * tcgen05.mma takes N / 2 cycles on the tensor pipe, but issuing one took 64 (a commit 95)
@@ -27,7 +27,8 @@
 //    step's barriers before their arithmetic and read its words while their stores are under
 //    way, and waiting warps sleep in try_wait instead of polling;
 //  * 224 tiles of 128 features left 72 of 148 SMs half empty.
-// us of a call among others, the other form -> this one, 3-bit (NF4): 64 x 8192 x 28672 56.3 ->
+// us of a call among some hundreds at 1965 MHz (over a second the power cap takes the clock to 1702
+// MHz: 3-bit 64 x 8192 x 28672 51.7, NF4 37 x 28672 x 8192 66.2), the other form -> this one, 3-bit (NF4): 64 x 8192 x 28672 56.3 ->
 // 46.2 (89.6 -> 68.7), 128 x 8192 x 28672 82.6 -> 60.4 (116.6 -> 77.6), 37 x 28672 x 8192 51.3 -> 45 (80.6
 // -> 66.8), 64 x 28672 x 28672 158.7 -> 131.2 (252 -> 191), 32 x 8192 x 14336 31.9 -> 28.6 (48.6 ->
 // 40.7), 64 x 4096 x 28672 30.5 -> 30.4 (47.9 -> 43.6).  On short layers the ends of the ranges
