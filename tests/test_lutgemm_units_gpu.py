@@ -36,7 +36,7 @@ def test_edges(hq, oracle, dev, M, K, nb, gs, bias):
     (6148, 9632, 3, 32, True), (6148, 9664, 4, 64, True), (3076, 20544, 4, 64, False), (8196, 9664, 3, 64, False)])
 def test_several_units_per_cta(hq, oracle, dev, M, K, nb, gs, bias):
     """228 to 322 units on the CTAs of the ring form, one per SM of 148: a last column range of four columns
-    more than a warp's, one to two rows of four in the last tile."""
+    more than whole warps, one to two rows of four in the last tile."""
     import torch
     from launches import launched
     x, bW, alpha, qb = synth.lutgemm_case(M, K, nb, gs, seed=M + K + nb, bias=bias)
