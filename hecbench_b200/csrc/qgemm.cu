@@ -865,12 +865,12 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
 
 // Whether a call takes the streamed form: where tiles may be cut (a scratch, one GPU: the
 // sharded form stores whole tiles to every GPU and has not been timed in parts) and a
-// model of both expects 3 % less.  us, from 140 layers of 9 to 40 steps per SM, 2 to 128
-// tokens, both formats, least squares of relative errors (2 to 6 % off): the form with
-// parts by its cost in blocks, the streamed one by its steps per SM, both by tokens.
-// Over those layers it takes 0.90 of the time of the form with parts alone (the better of the two
-// each time 0.90, streaming from 24 steps per SM on 0.94), 2 % more at worst.
-bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t workspace_bytes) {
+// model of both expects 3 % less.  us, from 72 layers of 6 to 48 steps per SM and 8, 37, 64 and 100
+// tokens for each format, least squares of relative errors (1 to 4 % off; the last row: 140 layers of 9
+// to 40 steps): the form with parts by its cost in blocks, the streamed one by its steps per
+// SM, both by tokens.  Over those layers the choice takes 0.90 (3-bit) and 0.84 (NF4) of the time of
+// the form with parts alone, 0.5 % more than the better of the two each time.
+bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t workspace_bytes, bool tma_only) {
   const int sms = sm_count();
   const int tiles = (N + streamed::kTileN - 1) / streamed::kTileN;
   const double units = (double)tiles * ((K + 2 * kBlockK - 1) / (2 * kBlockK));
@@ -878,16 +878,21 @@ bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t w
       units < 4.0 * sms || tiles < 8 || reserved_smem_per_block() != (int)streamed::kBase)
     return false;
   struct Model { double parts[3], stream[3]; };
-  static const Model models[2][2] = {  // [format][more than 64 tokens]
-      {{{0.7, 0.408, 1.9}, {8.0, 0.68, 6.4}}, {{-1.8, 0.28, 3.8}, {4.9, 0.70, 9.2}}},
+  static const Model models[3][2] = {  // [format; NF4 whose absmax the unpack warps load][more than 64 tokens]
+      {{{0.7, 0.408, 1.9}, {7.7, 0.52, 7.4}}, {{-1.8, 0.28, 3.8}, {5.3, 0.68, 8.3}}},
+      {{{0.3, 0.59, 2.5}, {10.3, 0.73, 6.6}}, {{0.0, 0.376, 3.5}, {5.8, 0.905, 9.1}}},
       {{{0.3, 0.59, 2.5}, {10.9, 0.93, 6.4}}, {{0.0, 0.376, 3.5}, {8.7, 0.94, 8.4}}}};
-  const Model& m = models[fmt == kFmtNf4][Mb > 64];
-  const double cost = choose_ksplit(N / kTileN, K / kBlockK, Mb > 64, false, sms).cost, t = Mb / 64.0;
+  const Model& m = models[fmt == kFmtQ3 ? 0 : tma_only ? 1 : 2][Mb > 64];
+  const KSplit split = choose_ksplit(N / kTileN, K / kBlockK, Mb > 64, false, sms);
+  const double t = Mb / 64.0;
   // ordered sums of three or more parts of a tile that end together (90 x 7040 x 12800, 3-bit:
   // 36.4 where 31 are expected without, 35.0 in parts); below eight tiles a tile has some 20
-  const double turns = tiles < sms / 2 && repeatable(N, K) ? 4.0 : 0.0;
+  // The few that three or more parts in turn take as well (N 12672 to 15872, K from 8960 on) stay in
+  // parts until the streamed form is 13 us ahead: their sums keep the order they had (up to K 11000
+  // or so, 2 % of layers; 64 x 8960 x 14976 36.3 us, 32.6 streamed; NF4 48.7, 39.6).
+  const double turns = tiles < sms / 2 && repeatable(N, K) ? (split.ordered ? 13.5 : 4.0) : 0.0;
   return m.stream[0] + m.stream[1] * (units / sms) + m.stream[2] * t + turns <
-         0.97 * (m.parts[0] + m.parts[1] * cost + m.parts[2] * t);
+         0.97 * (m.parts[0] + m.parts[1] * split.cost + m.parts[2] * t);
 }
 
 QgemmParams make_params(void* Y_half, bool sharded, int Mb, int N, int K, int group_size,
@@ -964,7 +969,7 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
   // the streamed form fetches twice the features and inputs at a time
-  const bool stream_form = !po.peer_Y && takes_stream(kFmtQ3, Mb, N, K, workspace, workspace_bytes);
+  const bool stream_form = !po.peer_Y && takes_stream(kFmtQ3, Mb, N, K, workspace, workspace_bytes, true);
   const int tile_n = stream_form ? streamed::kTileN : kTileN;
   CUtensorMap map_x, map_w, map_s, map_z;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
@@ -998,7 +1003,7 @@ static int qgemm_q3_impl(const void* X_half, const int32_t* mat, const void* sca
   prm.y_offset = po.y_offset;
   prm.world = po.world;
   if (stream_form)
-    return streamed::launch<kFmtQ3>(map_x, map_w, map_s, map_z, prm, repeatable(N, K), stream);
+    return streamed::launch<kFmtQ3>(map_x, map_w, map_s, map_z, prm, repeatable(N, K), false, stream);
   return launch_qgemm<kFmtQ3>(map_x, map_w, map_s, map_z, prm, stream);
 }
 
@@ -1017,7 +1022,9 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
     return HQ_ERR_MISALIGNED;
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return HQ_ERR_UNSUPPORTED;
-  const bool stream_form = !po.peer_Y && takes_stream(kFmtNf4, Mb, N, K, workspace, workspace_bytes);
+  // absmax by TMA (streamed form): blocks of 64 inputs, pairs of rows that begin on 16 bytes
+  const bool am_tma = blocksize == kBlockK && K % (2 * kBlockK) == 0 && aligned16(absmax);
+  const bool stream_form = !po.peer_Y && takes_stream(kFmtNf4, Mb, N, K, workspace, workspace_bytes, am_tma);
   CUtensorMap map_x, map_w;
   int st = encode_x_map(encode, &map_x, X_half, Mb, K);
   if (st != HQ_OK) return st;
@@ -1032,6 +1039,18 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return HQ_ERR_UNSUPPORTED;
   }
+  CUtensorMap map_s = map_w;
+  if (stream_form && am_tma) {
+    // absmax fp32 [N / 2][2 K / 64], two rows as one: box = four values (two steps) x 128
+    const cuuint64_t dims[2] = {(cuuint64_t)(2 * (K / kBlockK)), (cuuint64_t)(N / 2)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(2 * (K / kBlockK)) * 4};
+    const cuuint32_t box[2] = {4, (cuuint32_t)streamed::kTileN / 2};
+    const cuuint32_t estr[2] = {1, 1};
+    if (encode(&map_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(absmax), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return HQ_ERR_UNSUPPORTED;
+  }
   QgemmParams prm = make_params(Y_half, po.peer_Y != nullptr, Mb, N, K, blocksize, workspace,
                                 workspace_bytes, status_word);
   prm.absmax = absmax;
@@ -1041,7 +1060,7 @@ static int qgemm_nf4_impl(const void* X_half, const uint8_t* B, const float* abs
   prm.y_offset = po.y_offset;
   prm.world = po.world;
   if (stream_form)
-    return streamed::launch<kFmtNf4>(map_x, map_w, map_w, map_w, prm, repeatable(N, K), stream);
+    return streamed::launch<kFmtNf4>(map_x, map_w, map_s, map_w, prm, repeatable(N, K), am_tma, stream);
   return launch_qgemm<kFmtNf4>(map_x, map_w, map_w, map_w, prm, stream);
 }
 

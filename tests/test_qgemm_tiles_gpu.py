@@ -69,3 +69,27 @@ def test_streamed_edges(hq, dev, fmt, Mb, K, N, group):
     ((name, grid),) = launched(lambda: call(X))
     assert "qgemm_stream_kernel" in name and grid == torch.cuda.get_device_properties(dev).multi_processor_count
     test_edges(hq, dev, fmt, Mb, K, N, group)
+
+
+@pytest.mark.parametrize("Mb,K,N", [(64, 8320, 14464), (100, 8320, 14464), (37, 8448, 14464), (128, 8448, 7296),
+                                    (3, 28800, 8064), (65, 28800, 8064)])
+def test_streamed_absmax(hq, dev, Mb, K, N):
+    """NF4 in blocks of 64 inputs: absmax rows that begin on 16 bytes and rows of which every other one
+    begins in the middle of 16 (K = 128 modulo 256); the same values from an address that the
+    copy unit cannot take give the same bits (fixed order of the sums)."""
+    import torch
+    from launches import launched
+    test_edges(hq, dev, "nf4", Mb, K, N, 64)
+    g = torch.Generator(device=dev).manual_seed(Mb + K + N)
+    lut = torch.sort(torch.rand(16, generator=g, device=dev) * 2 - 1).values
+    B = torch.randint(0, 256, (N, K // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = torch.rand(N * K // 64, generator=g, device=dev) + 0.5
+    shifted = torch.cat([absmax[:1], absmax])[1:]
+    X = torch.randn((Mb, K), generator=g, device=dev).half()
+    a = hq.qgemm_nf4(X, B, absmax, lut, N, K, 64, 0)
+    out = []
+    ((name, _),) = launched(lambda: out.append(hq.qgemm_nf4(X, B, shifted, lut, N, K, 64, 0)))
+    if "qgemm_stream_kernel" in name and N > 14000:
+        assert torch.equal(a, out[0])
+    else:
+        assert float((a - out[0]).double().norm() / a.double().norm()) < 2.0 ** -11
