@@ -350,20 +350,81 @@ __device__ __forceinline__ uint2 lds_u2(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float lds_f16(uint32_t addr) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return __half2float(__ushort_as_half(v));
+}
+
+// byte permute with the sign-replicating selectors, which __byte_perm masks out
+__device__ __forceinline__ uint32_t permute(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+
+// Look-up addresses of a lane.  Lane (c, q) of a warp owns column 4c + q of its 32 and looks up all four
+// bytes of its words, byte (t + q) % 4 in turn t: in every turn the 32 lanes read 32 different
+// (replica c, byte lane) cells of a table line, that is, 32 different banks.  The address - byte value in
+// bits 8 to 15, the cell's offset in bits 0 to 7 - is one byte permute: the offsets of the four turns are the
+// bytes of `cells` (below 128, so their sign is the zero of the upper bytes).
+struct Lookup {
+  uint32_t cells, sel[4];
+  __device__ __forceinline__ explicit Lookup(int lane) {
+    cells = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const uint32_t byte = (uint32_t)(t + lane) & 3u;
+      cells |= ((uint32_t)(lane >> 2) * 16u + byte * 4u) << (8 * t);
+      sel[t] = 0xcc00u | (byte << 4) | (uint32_t)(4 + t);
+    }
+  }
+  // the four entries of a word of packed row ROW, added to `sum`
+  template <int IMM, int ROW>
+  __device__ __forceinline__ float add(uint32_t word, float sum) const {
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      sum += lds_f32_imm<IMM + (ROW >> 1) * 65536 + (ROW & 1) * 128>(permute(word, cells, sel[t]));
+    return sum;
+  }
+  template <int IMM>
+  __device__ __forceinline__ float add(int row, uint32_t word, float sum) const {  // row: known when unrolled
+    return row == 0   ? add<IMM, 0>(word, sum)
+           : row == 1 ? add<IMM, 1>(word, sum)
+           : row == 2 ? add<IMM, 2>(word, sum)
+                      : add<IMM, 3>(word, sum);
+  }
+};
+// sum of a packed row's 32 inputs, from the table's all-ones entries
+__device__ __forceinline__ float row_sum(const unsigned char* lut, int row, int lane) {
+  const float4 v = *reinterpret_cast<const float4*>(lut + (row >> 1) * 65536 + 255 * 256 + (row & 1) * 128 + (lane >> 2) * 16);
+  return (v.x + v.y) + (v.z + v.w);
+}
+__device__ __forceinline__ void red_add_f32(float* addr, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
+}
+
 // ---- ring form: four planes in one launch, and long work per CTA --------------
-// The lookups of the register form, on 128-input tiles, with two differences.  Words,
-// alphas and bias come through shared memory by asynchronous copies, kDepth column steps of
-// a warp ahead (57 to 86 KB per SM under way instead of 29, and no registers held: four
-// planes fit one launch where the register form takes two, each with its own tables).  And
-// the CTAs are persistent: a unit is one column range of one K tile, units are numbered
-// range by range inside a tile, CTA c takes units c, c + gridDim.x, ..., and a warp's ring
-// runs on through the ends of units, so words arrive while the tables of the next tile are
-// built.  What bounds it is shared memory: the look-ups, the quads' reads of their words
-// and the tables.  us of a call among others, register form -> this: 12288 x 12288, 4 planes
-// 44.9 -> 32.6, 3 planes 28.8 -> 27.4; 4096 x 8192, 4 planes 16.1 -> 11.4; 10240 x 5120, 3 planes
-// 14.1 -> 13.3.  The register form stays where a CTA has one short unit or two planes:
-// 2052 x 2048, 2 planes 5.4 and 6.0 here, 1024 x 1024, 3 planes 5.3 and 5.7, 8192 x 4096, 2 planes
-// 8.9 and 9.6.
+// 128-input tiles and the tables of the register form.  Words, alphas and bias come through shared
+// memory by asynchronous copies, kDepth column steps of a warp ahead (57 to 86 KB per SM under
+// way instead of 29, and no registers held: four planes fit one launch where the register form
+// takes two, each with its own tables).  The CTAs are persistent: a unit is one column range of one
+// K tile, units are numbered range by range inside a tile, CTA c takes units c, c + gridDim.x, ...,
+// and a warp's ring runs on through the ends of units, so words arrive while the tables of the
+// next tile are built.  A lane owns one column and looks up all four bytes of its words (Lookup
+// below): in the register form's division, one byte of four columns, a word goes to four lanes, and the
+// reads of the words took as many shared-memory wavefronts as the look-ups (4.1 M at 12288 x 12288, 3
+// planes, 60 % of the time); a lane's own column also needs no sum over lanes and a quarter of the
+// products with the scales.  us of a call among others, quads -> own columns: 12288 x 12288, 3 planes 27.5 -> 23.8, 4 planes
+// 32.7 -> 27.7; 4096 x 12288, 4 planes 17.9 -> 15.3; 4096 x 4096, 4 planes 8.4 -> 8.0.  What bounds it is shared
+// memory still: the look-ups, and the tables of a tile (eight copies of 1024 sums for each column range).
+// Words from global memory straight into registers do not take this division: a lane's 4-byte loads
+// are too short for HBM's latency (12288 x 12288, 1 plane 19.2 -> 24.8, 2 planes with groups of 64 26.0 -> 31.9).
 constexpr int kRingThreads = 512;
 
 // Compile-time layout.  NB: planes, RPG: packed rows per alpha group inside a tile.
@@ -496,10 +557,7 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
 #pragma unroll
   for (int d = 0; d < kDepth; d++) fetch(ring + d * L::kStage);
 
-  const int j = lane & 3;   // byte of the word this lane looks up
-  const int cq = lane >> 2; // column quad inside the 32-column step
-  const uint32_t hi = (uint32_t)(lane * 4);
-  const uint32_t sel = 0x7604u | ((uint32_t)j << 4);
+  const Lookup at(lane);
   uint32_t at_stage = 0;
   int built = -1;  // tile of the tables in place (kept only with more ranges than CTAs: millions of columns)
   float ones[kGroups];
@@ -553,84 +611,44 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
           *reinterpret_cast<float4*>(line + ((c + lane) & 7) * 16) = make_float4(v[0], v[1], v[2], v[3]);
       }
       __syncthreads();
-      // bias uses the all-ones entry (byte 255): sum of this lane's 8 inputs per row
+      // for the bias: sum of the group's inputs
 #pragma unroll
       for (int gi = 0; gi < kGroups; gi++) {
         float o = 0.f;
 #pragma unroll
-        for (int r = gi * RPG; r < (gi + 1) * RPG; r++)
-          o += *reinterpret_cast<const float*>(lut + (r >> 1) * 65536 + 255 * 256 + (r & 1) * 128 +
-                                               lane * 4);
+        for (int r = gi * RPG; r < (gi + 1) * RPG; r++) o += row_sum(lut, r, lane);
         ones[gi] = o;
       }
     }
 
     // ---- lookups ----
-    // byte value b in row r: [byteperm(word, lane*4, sel) + kLutImm + (r>>1)*65536 + (r&1)*128]
     for (int m0 = m_begin + warp * 32; m0 < m_end; m0 += kWarps * 32) {
       cp_async_wait<kDepth - 1>();
       __syncwarp();
       const uint32_t stage = ring + at_stage * L::kStage;
-      const uint32_t words = stage + cq * 16, params = stage + L::kWordBytes + cq * 8;
-      const int m = m0 + cq * 4;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint32_t words = stage + lane * 4, params = stage + L::kWordBytes + lane * 2;
+      const int m = m0 + lane;
+      float acc = 0.f;
 #pragma unroll
       for (int gi = 0; gi < kGroups; gi++) {
         if (gi * RPG >= nrows) break;  // rows past the end of K
-        float t[NB][4];
+        float t[NB];
 #pragma unroll
-        for (int rr = 0; rr < RPG; rr++) {
-          const int r = gi * RPG + rr;
+        for (int b = 0; b < NB; b++) t[b] = 0.f;
 #pragma unroll
-          for (int b = 0; b < NB; b++) {
-            const uint4 w = lds_u4(words + (r * NB + b) * 128);
-            const uint32_t w4[4] = {w.x, w.y, w.z, w.w};
+        for (int r = gi * RPG; r < (gi + 1) * RPG; r++) {
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-              const uint32_t a = __byte_perm(w4[c], hi, sel);
-              float v;
-              if (r == 0) v = lds_f32_imm<kLutImm>(a);
-              else if (r == 1) v = lds_f32_imm<kLutImm + 128>(a);
-              else if (r == 2) v = lds_f32_imm<kLutImm + 65536>(a);
-              else v = lds_f32_imm<kLutImm + 65536 + 128>(a);
-              t[b][c] = (rr == 0) ? v : t[b][c] + v;
-            }
-          }
+          for (int b = 0; b < NB; b++) t[b] = at.add<kLutImm>(r, lds_u32(words + (r * NB + b) * 128), t[b]);
         }
 #pragma unroll
-        for (int b = 0; b < NB; b++) {
-          const uint2 av = lds_u2(params + (gi * (NB + 1) + b) * 64);
-          const float2 a01 = __half22float2(u32_as_half2(av.x));
-          const float2 a23 = __half22float2(u32_as_half2(av.y));
-          acc[0] = fmaf(a01.x, t[b][0], acc[0]);
-          acc[1] = fmaf(a01.y, t[b][1], acc[1]);
-          acc[2] = fmaf(a23.x, t[b][2], acc[2]);
-          acc[3] = fmaf(a23.y, t[b][3], acc[3]);
-        }
-        if (q_bias != nullptr) {
-          const uint2 av = lds_u2(params + (gi * (NB + 1) + NB) * 64);
-          const float2 b01 = __half22float2(u32_as_half2(av.x));
-          const float2 b23 = __half22float2(u32_as_half2(av.y));
-          acc[0] = fmaf(b01.x, ones[gi], acc[0]);
-          acc[1] = fmaf(b01.y, ones[gi], acc[1]);
-          acc[2] = fmaf(b23.x, ones[gi], acc[2]);
-          acc[3] = fmaf(b23.y, ones[gi], acc[3]);
-        }
+        for (int b = 0; b < NB; b++) acc = fmaf(lds_f16(params + (gi * (NB + 1) + b) * 64), t[b], acc);
+        if (q_bias != nullptr) acc = fmaf(lds_f16(params + (gi * (NB + 1) + NB) * 64), ones[gi], acc);
       }
       // every lane has read the stage (the look-ups that used its words are done)
       __syncwarp();
       fetch(stage);
       if (++at_stage == kDepth) at_stage = 0;
-      // combine the four byte lanes of each column quad
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
-        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
-      }
-      // every lane of the quad now holds the four column sums: lane j == 0 adds
-      // them to the scratch row with one 16-byte reduction
-      if (m < m_end && j == 0 && HQ_IN_BOUNDS(ws + m, 16, ws, (size_t)M * 4, 204))
-        red_add_v4_f32(ws + m, acc[0], acc[1], acc[2], acc[3]);
+      if (m < m_end && HQ_IN_BOUNDS(ws + m, 4, ws, (size_t)M * 4, 204)) red_add_f32(ws + m, acc);
     }
   }
   cp_async_wait<0>();
@@ -987,27 +1005,48 @@ int launch_ring(const LaunchArgs& a, int b0, const __half* bias, int finalize) {
 // Planes go in launches of up to four (three with alpha groups of 32 inputs, whose parameters leave
 // the rings no room for a fourth) that accumulate into the same scratch row.  Only the first
 // launch adds the bias term, only the last one converts the scratch row.  On tiles of 128
-// inputs the ring form takes four planes, and three where a CTA has several units of two column
-// steps or more (times at its head); the register form takes the rest.  Five to eight planes as 4 + 1
-// to 4 + 4 take 0.75 to 1.00 of what 3 + 2 to 3 + 3 + 2 took (4096 x 4096, 7 planes 17.8 -> 13.8 us; 12288 x
-// 12288, 8 planes 74.4 -> 60.9), five planes of 4096 x 12288 1.02 (25.7 -> 26.1).
+// inputs the ring form takes four planes, and fewer where a warp has some column steps (takes_ring);
+// the register form takes the rest.  Five to eight planes as 4 + 1 to 4 + 4 take 0.75 to 1.00 of what 3 + 2
+// to 3 + 3 + 2 took when both were in the quads' division.
 template <int TR, int RPG>
 int launch_planes(const LaunchArgs& a) {
   constexpr bool kFour = TR == 2 || RPG > 1;  // groups of 32 inputs: the rings hold three planes
-  const bool ring3 = TR == 4 && a.cols_per_cta >= 2 * kRingThreads &&
-                     (long long)a.grid.x * a.grid.y > sm_count();
+  // The rings take over where a warp has some column steps: us, register form -> rings, at steps per warp
+  // 3 planes: 1.3 (12288 x 1024) 7.3 -> 7.6, 1.7 (4096 x 4096) 7.8 -> 7.4, 3.5 (8192 x 4096) 10.4 -> 9.6;
+  // 2 planes: 2.6 (12288 x 2048) 7.9 -> 8.2, 3.5 8.9 -> 8.85, 15.6 (12288 x 12288) 23.3 -> 21.3; with groups of
+  // 64, 3.5 9.6 -> 9.9, 6.9 (8192 x 8192) 14.1 -> 14.0, 15.6 26.0 -> 24.4;
+  // 1 plane: 3.9 (3072 x 12288) 8.9 -> 9.4, 5.2 (4096 x 12288) 10.6 -> 10.3, 15.6 19.2 -> 18.2.
+  // Groups of 32 inputs: as before, three planes in long units.
+  const double steps = (double)a.M * a.grid.y / ((double)kRingThreads * sm_count());
+  auto takes_ring = [&](int n) {
+    if (TR != 4) return false;
+    if (RPG == 1) return n == 3 && a.cols_per_cta >= 2 * kRingThreads && (long long)a.grid.x * a.grid.y > sm_count();
+    return n == 4 || steps >= (n == 3 ? 1.5 : n == 1 ? 5.0 : RPG == 4 ? 3.3 : 6.0);
+  };
   const int nb = a.nb_total;
   for (int b0 = 0; b0 < nb;) {
     const int n = std::min(nb - b0, kFour ? 4 : 3);
     const int last = (b0 + n == nb) ? 1 : 0;
     const __half* bias = b0 == 0 ? a.q_bias : nullptr;
     int st;
-    if (n == 1) st = launch_one<TR, 1, RPG>(a, b0, bias, last);
-    else if (n == 2) st = launch_one<TR, 2, RPG>(a, b0, bias, last);
-    else if (TR == 2 && n == 4) st = launch_one<TR, (TR == 2 ? 4 : 3), RPG>(a, b0, bias, last);
-    else if (n == 4) st = launch_ring<(TR == 4 && RPG > 1 ? 4 : 3), RPG>(a, b0, bias, last);
-    else if (ring3) st = launch_ring<3, RPG>(a, b0, bias, last);
-    else st = launch_one<TR, 3, RPG>(a, b0, bias, last);
+    if (takes_ring(n)) {
+      if constexpr (TR == 4 && RPG > 1) {
+        st = n == 1   ? launch_ring<1, RPG>(a, b0, bias, last)
+             : n == 2 ? launch_ring<2, RPG>(a, b0, bias, last)
+             : n == 3 ? launch_ring<3, RPG>(a, b0, bias, last)
+                      : launch_ring<4, RPG>(a, b0, bias, last);
+      } else {
+        st = launch_ring<3, RPG>(a, b0, bias, last);
+      }
+    } else if (n == 1) {
+      st = launch_one<TR, 1, RPG>(a, b0, bias, last);
+    } else if (n == 2) {
+      st = launch_one<TR, 2, RPG>(a, b0, bias, last);
+    } else if (TR == 2 && n == 4) {
+      st = launch_one<TR, (TR == 2 ? 4 : 3), RPG>(a, b0, bias, last);
+    } else {
+      st = launch_one<TR, 3, RPG>(a, b0, bias, last);
+    }
     if (st != HQ_OK) return st;
     b0 += n;
   }

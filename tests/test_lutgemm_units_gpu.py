@@ -49,3 +49,23 @@ def test_several_units_per_cta(hq, oracle, dev, M, K, nb, gs, bias):
     assert f"lutgemm_ring_kernelILi{nb}E" in name
     assert grid == torch.cuda.get_device_properties(dev).multi_processor_count
     test_edges(hq, oracle, dev, M, K, nb, gs, bias)
+
+
+@pytest.mark.parametrize("M,K,nb,gs,bias", [
+    (6148, 9664, 1, 64, True), (6148, 9664, 2, 64, False), (8196, 9728, 1, 128, True), (8196, 9728, 2, 128, True),
+    (4100, 4096, 3, 128, False), (4100, 4096, 7, 64, True)])
+def test_fewer_planes_in_rings(hq, oracle, dev, M, K, nb, gs, bias):
+    """One to three planes where the ring form takes them, alone or after four: lanes of a column of their
+    own, a last column range that ends inside a warp, two rows of four in the last tile."""
+    import torch
+    from launches import launched
+    x, bW, alpha, qb = synth.lutgemm_case(M, K, nb, gs, seed=M + K + nb, bias=bias)
+    w = hq.nQWeight_fp16()
+    w.parsing(bW, alpha.astype(np.float32), K, M, nb, False, K // gs,
+              None if qb is None else qb.astype(np.float32), device=dev)
+    out = torch.empty(M, dtype=torch.float16, device=dev)
+    dx = to_dev(x.view(np.uint16), dev).view(torch.float16)
+    names = [name for name, _ in launched(lambda: hq.matmul(out, dx, w))]
+    planes = [4] * (nb // 4) + [nb % 4]
+    assert len(names) == len(planes) and all(f"lutgemm_ring_kernelILi{n}E" in k for n, k in zip(planes, names))
+    test_edges(hq, oracle, dev, M, K, nb, gs, bias)
