@@ -42,6 +42,7 @@ struct FusedParams {
   __half* out;
   float eps, scale, zero_point;
   int rows_out, n, act;
+  Share share;
 };
 
 // sum over the CTA (all threads get the result); buf holds kWarps floats
@@ -72,7 +73,7 @@ gemv_fused_kernel(const FusedParams p) {
   // Programmatic dependent launch: nothing that earlier work of the stream may
   // have produced is read, and nothing is written, before the wait.
   pdl_launch_dependents();
-  if (BITS == 4) prefetch_first_rows(p.mat, rows_mat, row_bytes, lane, warp);
+  if (BITS == 4) prefetch_first_rows(p.mat, rows_mat, row_bytes, p.share, lane, warp);
   pdl_wait();
 
   // ---- RMSNorm: sum of squares over the whole vector ----
@@ -125,7 +126,7 @@ gemv_fused_kernel(const FusedParams p) {
   constexpr int kPerRow = kInFlight / kRows;
   const size_t mat_bytes = (size_t)rows_mat * row_bytes;
   (void)mat_bytes;
-  for (long long row0 = ((long long)blockIdx.x * kWarps + warp) * kRows; row0 < rows_mat;
+  for (long long row0 = first_row(p.share, warp); row0 < rows_mat;
        row0 += (long long)warps_total * kRows) {
     const unsigned char* src = p.mat + (size_t)row0 * row_bytes;
     float acc[kRows];
@@ -188,7 +189,8 @@ int launch(FusedParams prm, hq_stream_t stream) {
   // beyond 113 KiB only one CTA fits an SM
   if ((size_t)prm.n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;
   const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
-  const int grid = std::min(2 * sm_count(), (rows_mat + kWarps * kRows - 1) / (kWarps * kRows));
+  prm.share = share_rows(rows_mat, (size_t)prm.n * BITS / 8);
+  const int grid = prm.share.ctas;
   const size_t smem = smem_request((size_t)prm.n * 2, grid);
   constexpr auto kern = gemv_fused_kernel<BITS>;
   const cudaError_t e = ensure_dynamic_smem<kern>(smem);

@@ -40,7 +40,7 @@ using namespace rows;
 template <int BITS>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
-                    __half* __restrict__ res, int rows, int n, float scale, float zero_point) {
+                    __half* __restrict__ res, int rows, int n, float scale, float zero_point, const Share share) {
   extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
   __shared__ float s_part[kWarps];
   __half* xs = reinterpret_cast<__half*>(dsm_raw);
@@ -54,7 +54,7 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   // may be an earlier kernel's output like the input vector), and nothing is
   // written before it.
   pdl_launch_dependents();
-  if (BITS == 4) prefetch_first_rows(mat, rows, row_bytes, lane, warp);
+  if (BITS == 4) prefetch_first_rows(mat, rows, row_bytes, share, lane, warp);
   pdl_wait();
   // ---- prologue: inputs to shared memory (piece-major) and their sum ----
   float part = 0.f;
@@ -81,7 +81,7 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   constexpr int kPerRow = kInFlight / kRows;  // loads per row and batch
   const size_t mat_bytes = (size_t)rows * row_bytes;
   (void)mat_bytes;
-  for (long long row0 = ((long long)blockIdx.x * kWarps + warp) * kRows; row0 < rows;
+  for (long long row0 = first_row(share, warp); row0 < rows;
        row0 += (long long)warps_total * kRows) {
     const unsigned char* src = mat + (size_t)row0 * row_bytes;
     float acc[kRows];
@@ -129,7 +129,8 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   if (rows <= 0 || n <= 0 || n % (128 / BITS) != 0) return HQ_ERR_BAD_SHAPE;
   if (!aligned16(mat) || !aligned16(vec_half)) return HQ_ERR_MISALIGNED;
   if ((size_t)n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
-  const int grid = std::min(2 * sm_count(), (rows + kWarps * kRows - 1) / (kWarps * kRows));
+  const Share share = share_rows(rows, (size_t)n * BITS / 8);
+  const int grid = share.ctas;
   const size_t smem = smem_request((size_t)n * 2, grid);
   constexpr auto kern = gemv_uniform_kernel<BITS>;
   const cudaError_t e = ensure_dynamic_smem<kern>(smem);
@@ -140,7 +141,7 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream,
                                 reinterpret_cast<const unsigned char*>(mat),
                                 reinterpret_cast<const __half*>(vec_half),
-                                reinterpret_cast<__half*>(res_half), rows, n, s, z));
+                                reinterpret_cast<__half*>(res_half), rows, n, s, z, share));
 }
 
 }  // namespace

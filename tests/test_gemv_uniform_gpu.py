@@ -134,3 +134,25 @@ def test_gemv_uniform_against_reference_kernel(hq, oracle, dev, bits):
     assert ea < TOL_F16 and eb < TOL_F16
     assert oracle.rel_err(b.cpu().numpy().astype(np.float64),
                           a.cpu().numpy().astype(np.float64)) < TOL_F16
+
+
+# one to a few pairs of rows; both sides of the lines between one and two CTAs per SM, blocks of 16 pairs and
+# pairs one by one, and a last round a quarter full (148 SMs: 126, 148, 252 and 296 blocks; 4736 pairs a round)
+@pytest.mark.parametrize("rows", [1, 2, 3, 33, 295, 296, 4000, 4031, 4033, 4736, 4739, 8051, 8053, 9473, 11839, 11843])
+@pytest.mark.parametrize("bits,n", [(8, 48), (4, 2112)])
+def test_every_row_once(hq, dev, rows, bits, n):
+    """Each row's product, fp16 of fp32 sums of fp16 partial sums (rows of small integers and inputs of
+    small halves: every sum is exact), where nothing but the division of the rows can go wrong."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(rows + n)
+    x = torch.randint(-1, 2, (n,), generator=g, device=dev).half()
+    if bits == 8:
+        w = torch.randint(-2, 3, (rows, n), generator=g, device=dev)
+        out = hq.gemv_int8_quantized(w.to(torch.int8), x, 1.0, 1.0)
+        want = (w.double() - 1.0) @ x.double()
+    else:
+        b = torch.randint(0, 256, (rows, n // 2), generator=g, device=dev)
+        w = torch.stack([b & 15, b >> 4], dim=2).reshape(rows, n)
+        out = hq.gemv_int4_quantized(b.to(torch.uint8), x, 1.0, 8.0)
+        want = (w.double() - 8.0) @ x.double()
+    assert torch.equal(out.double(), want.half().double())
