@@ -30,6 +30,30 @@ constexpr int kWarps2x8 = 8;
 inline int rows_per_warp_for(int prob_m, int warps) {
   return prob_m / (warps * 4) >= 2 * sm_count() ? 4 : 2;
 }
+// How runs of rows_per_warp rows are divided: run warp * per_warp + CTA * per_cta goes to a warp.  Dealt one
+// by one over as many CTAs for every SM (per_cta = 1) the SMs have the same number of rows: the
+// gathers are bound by each SM's L1, and in blocks of a run for each warp the fullest SM has 32 rows of a 4096-row
+// layer where 27.7 are even, and a 1024-row layer is on 64 SMs.  us of a call among others, blocks -> dealt:
+// 1x16 300 x 4096 8.2 -> 3.7, 1024 x 8192 12.3 -> 6.9, 4096 x 4096 11.0 -> 10.0, 8192 x 4096 20.6 -> 18.4,
+// 14336 x 4096 36.9 -> 30.8; 2x8 4096 x 4096 8.4 -> 6.6, 3000 x 2048 6.7 -> 4.5, 11008 x 4096 15.5 -> 14.5.  Blocks
+// stay where they are nearly even (2x8 2368 x 4096 7.2, dealt 7.6), and where the CTAs per SM would leave
+// a slot free for an uneven start of the next launch (1x16, three of four: 6144 x 4096 16.0 and 17.3) or not fit
+// at once (2x8, more than three: 14336 x 4096 24.0 and 25.8).
+struct Runs {
+  int ctas, per_warp, per_cta;
+};
+inline Runs divide_rows(int prob_m, int warps, int rows_per_warp, unsigned dealt_counts) {
+  const int sms = sm_count(), per_cta = warps * rows_per_warp;
+  const int blocks = prob_m / per_cta + (prob_m % per_cta != 0), each = (blocks + sms - 1) / sms;
+  // dealt_counts: bit k stands for k CTAs per SM
+  if (each > 4 || !(dealt_counts >> each & 1u) || blocks >= 0.95 * each * sms) return {blocks, 1, warps};
+  const int ctas = std::min(prob_m / rows_per_warp + (prob_m % rows_per_warp != 0), each * sms);
+  return {ctas, ctas, 1};
+}
+constexpr unsigned kDealt1x16 = 1u << 1 | 1u << 2 | 1u << 4, kDealt2x8 = 1u << 1 | 1u << 2 | 1u << 3;
+__device__ __forceinline__ int first_row(const Runs& r, int warp, int rows_per_warp) {
+  return (warp * r.per_warp + (int)blockIdx.x * r.per_cta) * rows_per_warp;
+}
 constexpr int kPad = 9;  // input slots per 8 groups (one pad slot: conflict-free 128-bit reads)
 
 __device__ __forceinline__ float dot8_ref_order(const uint4& a, const uint4& b) {
@@ -76,12 +100,12 @@ template <int VPL, int RPW>
 __global__ void __launch_bounds__(kWarps1x16 * 32)
 aqlm_1x16_kernel(const uint4* codes, const uint4* x,
                  __half* __restrict__ out, const uint4* codebook, int prob_m,
-                 int prob_k, int4 cb_sizes, int cb_stride, const __half* scales) {
+                 int prob_k, int4 cb_sizes, int cb_stride, const __half* scales, const Runs runs) {
   extern __shared__ __align__(16) uint4 sh_x[];  // padded inputs: slot 9*(g/8) + g%8
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int groups = prob_k >> 3;    // 16-byte input groups
   const int vec_per_row = prob_k >> 6;
-  const int row_begin = (blockIdx.x * kWarps1x16 + warp) * RPW;
+  const int row_begin = first_row(runs, warp, RPW);
   // the next kernel of the stream may become resident while this grid drains;
   // nothing is read or written before every earlier kernel has completed (codes,
   // codebook and scales may be their output: ordered loads below)
@@ -145,6 +169,8 @@ aqlm_1x16_kernel(const uint4* codes, const uint4* x,
   }
 }
 
+// DEALT: the division with per_cta = 1 (as launch parameters it took 2 to 8 % of a small layer's time)
+template <bool DEALT>
 __global__ void __launch_bounds__(kWarps2x8 * 32)
 aqlm_2x8_kernel(const uint4* codes, const uint4* x,
                 __half* __restrict__ out, const uint4* codebooks, int prob_m,
@@ -176,7 +202,7 @@ aqlm_2x8_kernel(const uint4* codes, const uint4* x,
 
   const uint4* cb0 = cbs + (lane & 7);
   const uint4* cb1 = cbs + 256 * 8 + (lane & 7);
-  const int row_begin = (blockIdx.x * kWarps2x8 + warp) * rows_per_warp;
+  const int row_begin = (DEALT ? warp * (int)gridDim.x + (int)blockIdx.x : (int)blockIdx.x * kWarps2x8 + warp) * rows_per_warp;
   for (int rr = 0; rr < rows_per_warp; rr++) {
     const int m = row_begin + rr;
     if (m >= prob_m) break;
@@ -211,6 +237,11 @@ aqlm_2x8_kernel(const uint4* codes, const uint4* x,
   }
 }
 
+template <auto Kern>
+struct Form {
+  static constexpr auto value = Kern;
+};
+
 }  // namespace
 }  // namespace hq
 
@@ -229,8 +260,8 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
   const int groups = prob_k / 8;
   const size_t smem = (size_t)kPad * ((groups + 7) / 8) * 16;
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps1x16);
-  const int rows_per_cta = kWarps1x16 * rows_per_warp;
-  const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
+  const Runs runs = divide_rows(prob_m, kWarps1x16, rows_per_warp, kDealt1x16);
+  const int grid = runs.ctas;
   // A grid that fills the SMs starts while the one before it drains (4096 x 4096
   // back to back: 12.4 -> 11.0 us; in a replayed graph 10.7 -> 10.6, and 2368 x 4096,
   // 148 CTAs, 6.6 -> 6.4).  A smaller one does not: the CTAs of an early start are not
@@ -252,9 +283,9 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
     const auto sc = reinterpret_cast<const __half*>(scales_half);                            \
     if (grid >= sm_count())                                                                  \
       return cuda_status(launch_pdl(kern, dim3(grid), dim3(kWarps1x16 * 32), smem, st, c, x, o, \
-                                    cb, prob_m, prob_k, sizes, cb_stride_int4, sc));         \
+                                    cb, prob_m, prob_k, sizes, cb_stride_int4, sc, runs));   \
     kern<<<grid, kWarps1x16 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sizes,            \
-                                              cb_stride_int4, sc);                           \
+                                              cb_stride_int4, sc, runs);                     \
   }
 #define HQ_AQLM_ROWS(VPL)                                \
   if (rows_per_warp == 4) HQ_AQLM_LAUNCH(VPL, 4)         \
@@ -279,10 +310,9 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const int groups = prob_k / 8;
   const size_t smem = (size_t)2 * 256 * 8 * 16 + (size_t)kPad * ((groups + 7) / 8) * 16;
   if (smem > 220 * 1024) return HQ_ERR_TOO_LARGE;
-  constexpr auto kern2x8 = aqlm_2x8_kernel;
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps2x8);
-  const int rows_per_cta = kWarps2x8 * rows_per_warp;
-  const int grid = (prob_m + rows_per_cta - 1) / rows_per_cta;
+  const Runs runs = divide_rows(prob_m, kWarps2x8, rows_per_warp, kDealt2x8);
+  const int grid = runs.ctas;
   const auto c = reinterpret_cast<const uint4*>(codes);
   const auto x = reinterpret_cast<const uint4*>(x_half);
   const auto o = reinterpret_cast<__half*>(out_half);
@@ -298,13 +328,17 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const int per_sm = (grid + sm_count() - 1) / sm_count();
   const size_t share = (size_t)228 * 1024 / (per_sm + 1);  // 1 KiB of it is reserved per CTA
   const size_t request = std::max(smem, share > 1024 ? share - 1024 + 16 : 0);
-  cudaError_t e = ensure_dynamic_smem<kern2x8>(request);
-  if (e != cudaSuccess) return cuda_status(e);
-  if (grid >= 2 * sm_count())
-    return cuda_status(launch_pdl(kern2x8, dim3(grid), dim3(kWarps2x8 * 32), request, st, c, x, o, cb,
-                                  prob_m, prob_k, sc, rows_per_warp));
-  kern2x8<<<grid, kWarps2x8 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sc, rows_per_warp);
-  return launch_status();
+  auto go = [&](auto form) {
+    constexpr auto kern = decltype(form)::value;
+    const cudaError_t e = ensure_dynamic_smem<kern>(request);
+    if (e != cudaSuccess) return cuda_status(e);
+    if (grid >= 2 * sm_count())
+      return cuda_status(launch_pdl(kern, dim3(grid), dim3(kWarps2x8 * 32), request, st, c, x, o, cb, prob_m,
+                                    prob_k, sc, rows_per_warp));
+    kern<<<grid, kWarps2x8 * 32, smem, st>>>(c, x, o, cb, prob_m, prob_k, sc, rows_per_warp);
+    return launch_status();
+  };
+  return runs.per_cta == 1 ? go(Form<aqlm_2x8_kernel<true>>()) : go(Form<aqlm_2x8_kernel<false>>());
 }
 
 }  // extern "C"
