@@ -14,9 +14,9 @@
 //               scales and zeros, NF4 256 rows x 64 bytes and their absmax values);
 //   warp 18     X by TMA into the stages, 64 inputs x all tokens per half.
 //
-// What bounds it.  3-bit, up to 64 tokens: issue slots of the unpack warps, about 2650 instructions a
-// step, 1630 of them the unpacking (a byte permute, a look-up, an fp16 fma per pair), and the
-// ends of the ranges (15 of 41 us at 64 x 8192 x 28672).  NF4: the shared-memory pipe, two wavefronts
+// What bounds it.  3-bit, up to 64 tokens: issue slots, 3360 instructions a step with all
+// roles and the ends (4175 before the two changes below), 1630 of them the unpacking (a byte
+// permute, a look-up, an fp16 fma per pair), and the ends of the ranges (15 of 41 us at 64 x 8192 x 28672).  NF4: the shared-memory pipe, two wavefronts
 // for every look-up of a byte, 1024 of a step's 1430 cycles.  Beyond 64 tokens: the two stages that
 // tensor memory leaves.
 //  * A table row is a byte and a lane's copy, one byte permute, for both formats: four 3-bit pairs lie in
