@@ -887,10 +887,15 @@ bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t w
   const double t = Mb / 64.0;
   // ordered sums of three or more parts of a tile that end together (90 x 7040 x 12800, 3-bit:
   // 36.4 where 31 are expected without, 35.0 in parts); below eight tiles a tile has some 20
-  // The few that three or more parts in turn take as well (N 12672 to 15872, K from 8960 on) stay in
-  // parts until the streamed form is 13 us ahead: their sums keep the order they had (up to K 11000
-  // or so, 2 % of layers; 64 x 8960 x 14976 36.3 us, 32.6 streamed; NF4 48.7, 39.6).
-  const double turns = tiles < sms / 2 && repeatable(N, K) ? (split.ordered ? 13.5 : 4.0) : 0.0;
+  double turns = tiles < sms / 2 && repeatable(N, K) ? 4.0 : 0.0;
+  // 3-bit layers, up to 64 tokens, that the other form takes in three or more ordered parts: the line
+  // between the forms stands where it stood when a step of the streamed form took 0.68 us, not 0.52.  What
+  // it leaves in parts (N 12672 to 15104, K 8960 to 21760, a twentieth of these layers at 64 tokens, none at
+  // 2) would gain by streaming (64 x 8960 x 14976 36.9 us, streamed 32.9; 2 tokens 32.9 and 24.4), but next
+  // to no other call on one GPU reaches those ordered parts.  Further away the streamed form is always the
+  // faster one: 64 x 15744 x 12800 42.0 us, in parts 52.9; 16 x 9472 x 12800 25.4 and 33.5; NF4 64 x 9472 x
+  // 12800 39.6 and 50.4; 128 x 12544 x 12928 50.8 and 63.7.
+  if (split.ordered && turns > 0 && fmt == kFmtQ3 && Mb <= 64) turns += 0.3 + 0.16 * (units / sms) - t;
   return m.stream[0] + m.stream[1] * (units / sms) + m.stream[2] * t + turns <
          0.97 * (m.parts[0] + m.parts[1] * split.cost + m.parts[2] * t);
 }
