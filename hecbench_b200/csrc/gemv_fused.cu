@@ -42,7 +42,6 @@ struct FusedParams {
   __half* out;
   float eps, scale, zero_point;
   int rows_out, n, act;
-  Share share;
 };
 
 // sum over the CTA (all threads get the result); buf holds kWarps floats
@@ -57,7 +56,7 @@ __device__ __forceinline__ float block_sum(float v, float* buf, int lane, int wa
   return t;
 }
 
-template <int BITS>
+template <int BITS, bool DEALT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_fused_kernel(const FusedParams p) {
   extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
@@ -73,7 +72,7 @@ gemv_fused_kernel(const FusedParams p) {
   // Programmatic dependent launch: nothing that earlier work of the stream may
   // have produced is read, and nothing is written, before the wait.
   pdl_launch_dependents();
-  if (BITS == 4) prefetch_first_rows(p.mat, rows_mat, row_bytes, p.share, lane, warp);
+  if (BITS == 4) prefetch_first_rows<DEALT>(p.mat, rows_mat, row_bytes, lane, warp);
   pdl_wait();
 
   // ---- RMSNorm: sum of squares over the whole vector ----
@@ -126,7 +125,7 @@ gemv_fused_kernel(const FusedParams p) {
   constexpr int kPerRow = kInFlight / kRows;
   const size_t mat_bytes = (size_t)rows_mat * row_bytes;
   (void)mat_bytes;
-  for (long long row0 = first_row(p.share, warp); row0 < rows_mat;
+  for (long long row0 = first_row<DEALT>(warp); row0 < rows_mat;
        row0 += (long long)warps_total * kRows) {
     const unsigned char* src = p.mat + (size_t)row0 * row_bytes;
     float acc[kRows];
@@ -179,7 +178,7 @@ gemv_fused_kernel(const FusedParams p) {
 }
 
 template <int BITS>
-int launch(FusedParams prm, hq_stream_t stream) {
+int launch(const FusedParams& prm, hq_stream_t stream) {
   if (!prm.mat || !prm.x || !prm.out) return HQ_ERR_NULL_POINTER;
   if (prm.rows_out <= 0 || prm.n <= 0 || prm.n % (128 / BITS) != 0) return HQ_ERR_BAD_SHAPE;
   if (prm.act != HQ_ACT_NONE && prm.act != HQ_ACT_SWIGLU && prm.act != HQ_ACT_GEGLU)
@@ -189,14 +188,16 @@ int launch(FusedParams prm, hq_stream_t stream) {
   // beyond 113 KiB only one CTA fits an SM
   if ((size_t)prm.n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;
   const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
-  prm.share = share_rows(rows_mat, (size_t)prm.n * BITS / 8);
-  const int grid = prm.share.ctas;
+  const Share share = share_rows(rows_mat, (size_t)prm.n * BITS / 8);
+  const int grid = share.ctas;
   const size_t smem = smem_request((size_t)prm.n * 2, grid);
-  constexpr auto kern = gemv_fused_kernel<BITS>;
-  const cudaError_t e = ensure_dynamic_smem<kern>(smem);
-  if (e != cudaSuccess) return cuda_status(e);
-  return cuda_status(
-      launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream, prm));
+  auto go = [&](auto dealt) {
+    constexpr auto kern = gemv_fused_kernel<BITS, decltype(dealt)::value>;
+    const cudaError_t e = ensure_dynamic_smem<kern>(smem);
+    if (e != cudaSuccess) return cuda_status(e);
+    return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream, prm));
+  };
+  return share.dealt ? go(std::true_type()) : go(std::false_type());
 }
 
 FusedParams base_params(const void* mat, const void* x_half, const void* gamma_half, float eps,

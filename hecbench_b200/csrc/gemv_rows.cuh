@@ -4,6 +4,7 @@
 #ifndef HQ_GEMV_ROWS_CUH_
 #define HQ_GEMV_ROWS_CUH_
 #include <algorithm>
+#include <type_traits>
 
 #include "hq_common.cuh"
 
@@ -26,19 +27,22 @@ inline size_t smem_request(size_t need, int grid) {
   return grid <= sm_count() && need < kOverHalf ? kOverHalf : need;
 }
 
-// How the row pairs are divided: pair warp * per_warp + CTA * per_cta goes to a warp first, then every
-// ctas * kWarps-th.  Dealt one by one (per_cta = 1), every SM has the same number; in blocks of 16, one for
-// each warp, 4096 pairs leave 108 of 148 SMs with 32 and 40 with 16 where 28 are even, and 512 pairs use
-// 32 SMs.  us of a call among others, blocks -> one by one, int4 (int8): 1024 x 4096 3.9 -> 2.8 (4.8 -> 3.6),
+// How the row pairs are divided: in blocks of 16, pair CTA * 16 + warp goes to a warp first; dealt one by one,
+// pair warp * CTAs + CTA; then every CTAs * 16-th.  Dealt, every SM has the same number; in blocks, 4096
+// pairs leave 108 of 148 SMs with 32 and 40 with 16 where 28 are even, and 512 pairs use 32 SMs.  us of a
+// call among others, blocks -> one by one, int4 (int8): 1024 x 4096 3.9 -> 2.8 (4.8 -> 3.6),
 // 1024 x 16384 11.2 -> 7.7 (15.6 -> 13.2), 2368 x 4096 4.1 -> 3.3 (5.6 -> 5.0), 5120 x 5120 8.0 -> 6.7 (9.8 -> 8.5),
 // 8192 x 8192 12.0 -> 11.8 (14.7 -> 14.5), 14336 x 4096 11.3 -> 10.0 (14.5 -> 13.0).  Blocks are kept
 //  * where they fill the SMs with one CTA each (4096 x 4096 4.30, one by one 4.37), or with two and rows of
 //    up to 1 KiB (8192 x 2048 int4 4.33 and 4.45): the rows of a CTA follow one another;
 //  * where the last of several rounds is less than a quarter full: it falls to a few CTAs and the next
 //    launch starts on the other SMs (10000 x 8192 int4 14.7, one by one 15.8; 49152 x 2048 16.0 and 16.6).
-// A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1).
+// A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and so
+// does a division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9
+// for 12.9): each is a kernel of its own.
 struct Share {
-  int ctas, per_warp, per_cta;
+  int ctas;
+  bool dealt;
 };
 inline Share share_rows(int rows, size_t row_bytes) {
   const int pairs = rows / kRows + (rows % kRows != 0), sms = sm_count();
@@ -47,11 +51,12 @@ inline Share share_rows(int rows, size_t row_bytes) {
   const bool in_blocks = blocks <= sms       ? blocks >= 0.85 * sms
                          : blocks <= 2 * sms ? blocks >= 1.7 * sms && row_bytes <= 1024
                                              : pairs % round < round / 4;
-  if (in_blocks) return {std::min(blocks, 2 * sms), 1, kWarps};
-  return {ctas, ctas, 1};
+  if (in_blocks) return {std::min(blocks, 2 * sms), false};
+  return {ctas, true};
 }
-__device__ __forceinline__ long long first_row(const Share& s, int warp) {
-  return ((long long)warp * s.per_warp + (long long)blockIdx.x * s.per_cta) * kRows;
+template <bool DEALT>
+__device__ __forceinline__ long long first_row(int warp) {
+  return (DEALT ? (long long)warp * gridDim.x + blockIdx.x : (long long)blockIdx.x * kWarps + warp) * kRows;
 }
 
 // 4-bit rows of up to 4 KiB: the rows a warp starts with are on their way to L2 before the
@@ -61,9 +66,10 @@ __device__ __forceinline__ long long first_row(const Share& s, int warp) {
 // Longer rows gain nothing (4096 x 11008 10.13 -> 10.27), and 8-bit rows of the same lengths
 // lose: 512 x 1024 2.65 -> 3.01, 4096 x 1024 2.69 -> 3.36, 1024 x 4096 4.67 -> 5.40, 28672 x 4096 21.97 -> 25.5
 // (8192 x 2048 alone 5.90 -> 5.05; 8192 x 8192 14.4 -> 17.4).
+template <bool DEALT>
 __device__ __forceinline__ void prefetch_first_rows(const unsigned char* mat, int rows, size_t row_bytes,
-                                                    const Share& share, int lane, int warp) {
-  const long long row = first_row(share, warp) + lane;
+                                                    int lane, int warp) {
+  const long long row = first_row<DEALT>(warp) + lane;
   if (row_bytes <= 4096 && lane < kRows && row < rows)
     prefetch_l2(mat + (size_t)row * row_bytes, (uint32_t)row_bytes);
 }

@@ -37,10 +37,10 @@ namespace {
 using namespace rows;
 
 // n: inputs per row; row_bytes = n * BITS / 8 (a multiple of 16).
-template <int BITS>
+template <int BITS, bool DEALT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
-                    __half* __restrict__ res, int rows, int n, float scale, float zero_point, const Share share) {
+                    __half* __restrict__ res, int rows, int n, float scale, float zero_point) {
   extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
   __shared__ float s_part[kWarps];
   __half* xs = reinterpret_cast<__half*>(dsm_raw);
@@ -54,7 +54,7 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   // may be an earlier kernel's output like the input vector), and nothing is
   // written before it.
   pdl_launch_dependents();
-  if (BITS == 4) prefetch_first_rows(mat, rows, row_bytes, share, lane, warp);
+  if (BITS == 4) prefetch_first_rows<DEALT>(mat, rows, row_bytes, lane, warp);
   pdl_wait();
   // ---- prologue: inputs to shared memory (piece-major) and their sum ----
   float part = 0.f;
@@ -81,7 +81,7 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   constexpr int kPerRow = kInFlight / kRows;  // loads per row and batch
   const size_t mat_bytes = (size_t)rows * row_bytes;
   (void)mat_bytes;
-  for (long long row0 = first_row(share, warp); row0 < rows;
+  for (long long row0 = first_row<DEALT>(warp); row0 < rows;
        row0 += (long long)warps_total * kRows) {
     const unsigned char* src = mat + (size_t)row0 * row_bytes;
     float acc[kRows];
@@ -132,16 +132,19 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   const Share share = share_rows(rows, (size_t)n * BITS / 8);
   const int grid = share.ctas;
   const size_t smem = smem_request((size_t)n * 2, grid);
-  constexpr auto kern = gemv_uniform_kernel<BITS>;
-  const cudaError_t e = ensure_dynamic_smem<kern>(smem);
-  if (e != cudaSuccess) return cuda_status(e);
   // the launcher of the reference rounds both parameters to fp16 (gemv.cu:21-22)
   const float s = __half2float(__float2half_rn(scale));
   const float z = __half2float(__float2half_rn(zero_point));
-  return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream,
-                                reinterpret_cast<const unsigned char*>(mat),
-                                reinterpret_cast<const __half*>(vec_half),
-                                reinterpret_cast<__half*>(res_half), rows, n, s, z, share));
+  auto go = [&](auto dealt) {
+    constexpr auto kern = gemv_uniform_kernel<BITS, decltype(dealt)::value>;
+    const cudaError_t e = ensure_dynamic_smem<kern>(smem);
+    if (e != cudaSuccess) return cuda_status(e);
+    return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream,
+                                  reinterpret_cast<const unsigned char*>(mat),
+                                  reinterpret_cast<const __half*>(vec_half),
+                                  reinterpret_cast<__half*>(res_half), rows, n, s, z));
+  };
+  return share.dealt ? go(std::true_type()) : go(std::false_type());
 }
 
 }  // namespace

@@ -156,3 +156,21 @@ def test_every_row_once(hq, dev, rows, bits, n):
         out = hq.gemv_int4_quantized(b.to(torch.uint8), x, 1.0, 8.0)
         want = (w.double() - 8.0) @ x.double()
     assert torch.equal(out.double(), want.half().double())
+
+
+@pytest.mark.parametrize("bits", [16, 8, 4])
+@pytest.mark.parametrize("rows,n,dealt", [(1024, 512, 1), (4736, 1024, 0)])
+def test_a_kernel_for_each_division(hq, dev, bits, rows, n, dealt):
+    """Blocks of pairs and pairs one by one are kernels of their own, plain and fused (as a parameter the
+    division costs the 4-bit loops 3 to 7 %)."""
+    import torch
+    from launches import launched
+    mat = torch.zeros((rows, n * bits // 8), dtype=torch.uint8, device=dev)
+    w = {16: mat.view(torch.float16), 8: mat.view(torch.int8), 4: mat}[bits]
+    x = torch.ones(n, dtype=torch.float16, device=dev)
+    plain = {16: lambda: hq.gemv_fp16(w, x), 8: lambda: hq.gemv_int8_quantized(w, x, 1.0, 0.0),
+             4: lambda: hq.gemv_int4_quantized(w, x, 1.0, 0.0)}[bits]
+    fused = lambda: hq.gemv_fused({16: "f16", 8: "int8", 4: "int4"}[bits], x, w, rows // 2, gamma=x, act=hq.ACT_SWIGLU)
+    for call, kernel in ((plain, "gemv_uniform_kernel"), (fused, "gemv_fused_kernel")):
+        ((name, _),) = launched(call)
+        assert f"{kernel}ILi{bits}ELb{dealt}E" in name
