@@ -39,7 +39,8 @@ inline size_t smem_request(size_t need, int grid) {
 //    launch starts on the other SMs (10000 x 8192 int4 14.7, one by one 15.8; 49152 x 2048 16.0 and 16.6).
 // A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and so
 // does a division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9
-// for 12.9): each is a kernel of its own.
+// for 12.9): each is a kernel of its own.  The plain 8-bit kernel alone is the faster one with parameters (28672 x
+// 2048 12.64 us, 12.9 without, 10000 x 1024 4.66 and 4.78; pairs one by one the same).
 struct Share {
   int ctas;
   bool dealt;

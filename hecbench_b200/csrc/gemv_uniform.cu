@@ -36,11 +36,13 @@ namespace {
 
 using namespace rows;
 
-// n: inputs per row; row_bytes = n * BITS / 8 (a multiple of 16).
+// n: inputs per row; row_bytes = n * BITS / 8 (a multiple of 16).  DEALT: the division of the rows; 8 bits take
+// it from per_warp and per_cta (gemv_rows.cuh).
 template <int BITS, bool DEALT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
-                    __half* __restrict__ res, int rows, int n, float scale, float zero_point) {
+                    __half* __restrict__ res, int rows, int n, float scale, float zero_point, int per_warp,
+                    int per_cta) {
   extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
   __shared__ float s_part[kWarps];
   __half* xs = reinterpret_cast<__half*>(dsm_raw);
@@ -81,8 +83,9 @@ gemv_uniform_kernel(const unsigned char* mat, const __half* vec,
   constexpr int kPerRow = kInFlight / kRows;  // loads per row and batch
   const size_t mat_bytes = (size_t)rows * row_bytes;
   (void)mat_bytes;
-  for (long long row0 = first_row<DEALT>(warp); row0 < rows;
-       row0 += (long long)warps_total * kRows) {
+  const long long first = BITS == 8 ? ((long long)warp * per_warp + (long long)blockIdx.x * per_cta) * kRows
+                                    : first_row<DEALT>(warp);
+  for (long long row0 = first; row0 < rows; row0 += (long long)warps_total * kRows) {
     const unsigned char* src = mat + (size_t)row0 * row_bytes;
     float acc[kRows];
 #pragma unroll
@@ -142,9 +145,10 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
     return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream,
                                   reinterpret_cast<const unsigned char*>(mat),
                                   reinterpret_cast<const __half*>(vec_half),
-                                  reinterpret_cast<__half*>(res_half), rows, n, s, z));
+                                  reinterpret_cast<__half*>(res_half), rows, n, s, z, share.dealt ? grid : 1,
+                                  share.dealt ? 1 : kWarps));
   };
-  return share.dealt ? go(std::true_type()) : go(std::false_type());
+  return share.dealt && BITS != 8 ? go(std::bool_constant<BITS != 8>()) : go(std::false_type());
 }
 
 }  // namespace
