@@ -188,7 +188,7 @@ int launch(const FusedParams& prm, hq_stream_t stream) {
   // beyond 113 KiB only one CTA fits an SM
   if ((size_t)prm.n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;
   const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
-  const Share share = share_rows(rows_mat, (size_t)prm.n * BITS / 8);
+  const Share share = share_rows(rows_mat, (size_t)prm.n * BITS / 8, BITS, false);
   const int grid = share.ctas;
   const size_t smem = smem_request((size_t)prm.n * 2, grid);
   auto go = [&](auto dealt) {

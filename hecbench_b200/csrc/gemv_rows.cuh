@@ -33,10 +33,17 @@ inline size_t smem_request(size_t need, int grid) {
 // call among others, blocks -> one by one, int4 (int8): 1024 x 4096 3.9 -> 2.8 (4.8 -> 3.6),
 // 1024 x 16384 11.2 -> 7.7 (15.6 -> 13.2), 2368 x 4096 4.1 -> 3.3 (5.6 -> 5.0), 5120 x 5120 8.0 -> 6.7 (9.8 -> 8.5),
 // 8192 x 8192 12.0 -> 11.8 (14.7 -> 14.5), 14336 x 4096 11.3 -> 10.0 (14.5 -> 13.0).  Blocks are kept
-//  * where they fill the SMs with one CTA each (4096 x 4096 4.30, one by one 4.37), or with two and rows of
-//    up to 1 KiB (8192 x 2048 int4 4.33 and 4.45): the rows of a CTA follow one another;
+//  * where they fill the SMs with one CTA each (int4 4096 x 4096 4.30, one by one 4.37), or with two and
+//    4-bit rows of up to 3 KiB (8192 x 2048 4.33 and 4.45, 9000 x 4096 6.33 and 6.62, 9000 x 6144 10.64 and
+//    10.75), 8-bit ones of 2 (9000 x 2048 6.7 and 6.85; 8192 x 3072 8.01 and 7.84) or fp16 ones of 1 (2 KiB: one
+//    by one 1 % less): the rows of a CTA follow one another;
 //  * where the last of several rounds is less than a quarter full: it falls to a few CTAs and the next
 //    launch starts on the other SMs (10000 x 8192 int4 14.7, one by one 15.8; 49152 x 2048 16.0 and 16.6).
+//    From the fourth round on 4-bit rows do that up to half full, when one CTA of each SM has a pair per warp
+//    more (32000 x 4096 17.1 and 17.6, 41000 x 2048 13.4 and 14.3); rows of up to 512 bytes from the fifth
+//    (32000 x 1024 gains 3 %, 41000 x 1024 loses 6; up to 1 KiB 33000 x 2048 gains 3), 8-bit and fp16 rows never (41000 x 2048 gain 3 and 2 %).
+//    In the third round a third full is still few for plain 4-bit rows whose batches of 2 KiB are whole or
+//    nearly so (22016 x 4096 12.8 and 13.4, x 8192 23.6 and 24.8; x 2048 9.7 and 9.2, x 6144 22.2 and 20.0).
 // A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and so
 // does a division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9
 // for 12.9): each is a kernel of its own.  The plain 8-bit kernel alone is the faster one with parameters (28672 x
@@ -45,13 +52,20 @@ struct Share {
   int ctas;
   bool dealt;
 };
-inline Share share_rows(int rows, size_t row_bytes) {
+inline Share share_rows(int rows, size_t row_bytes, int bits, bool plain) {
   const int pairs = rows / kRows + (rows % kRows != 0), sms = sm_count();
   const int blocks = pairs / kWarps + (pairs % kWarps != 0);  // CTAs of a pair per warp
   const int ctas = blocks <= sms ? std::min(pairs, sms) : 2 * sms, round = ctas * kWarps;
+  const int rounds = pairs / round;  // whole ones
+  const bool whole_batches = row_bytes <= 4096 && (row_bytes + 256) % 2048 <= 256;
+  double few = 0.25;
+  if (bits == 4 && rounds >= 4) few = 0.5;
+  if (bits == 4 && rounds == 3 && row_bytes > 512) few = row_bytes > 1024 ? 0.5 : 0.42;
+  if (bits == 4 && rounds == 2 && plain && whole_batches) few = 0.34;
+  const size_t short_rows = bits == 4 ? 3072 : bits == 8 ? 2048 : 1024;
   const bool in_blocks = blocks <= sms       ? blocks >= 0.85 * sms
-                         : blocks <= 2 * sms ? blocks >= 1.7 * sms && row_bytes <= 1024
-                                             : pairs % round < round / 4;
+                         : blocks <= 2 * sms ? blocks >= 1.65 * sms && row_bytes <= short_rows
+                                             : pairs % round < few * round;
   if (in_blocks) return {std::min(blocks, 2 * sms), false};
   return {ctas, true};
 }

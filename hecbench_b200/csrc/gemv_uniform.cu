@@ -132,7 +132,7 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   if (rows <= 0 || n <= 0 || n % (128 / BITS) != 0) return HQ_ERR_BAD_SHAPE;
   if (!aligned16(mat) || !aligned16(vec_half)) return HQ_ERR_MISALIGNED;
   if ((size_t)n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
-  const Share share = share_rows(rows, (size_t)n * BITS / 8);
+  const Share share = share_rows(rows, (size_t)n * BITS / 8, BITS, true);
   const int grid = share.ctas;
   const size_t smem = smem_request((size_t)n * 2, grid);
   // the launcher of the reference rounds both parameters to fp16 (gemv.cu:21-22)

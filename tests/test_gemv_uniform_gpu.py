@@ -174,3 +174,19 @@ def test_a_kernel_for_each_division(hq, dev, bits, rows, n, dealt):
     for call, kernel in ((plain, "gemv_uniform_kernel"), (fused, "gemv_fused_kernel")):
         ((name, _),) = launched(call)
         assert f"{kernel}ILi{bits}ELb{0 if (bits, call) == (8, plain) else dealt}E" in name
+
+
+@pytest.mark.parametrize("bits,rows,n,dealt", [
+    (4, 9000, 4096, 0), (4, 8000, 6144, 0), (8, 9000, 2048, 0), (8, 9000, 3072, 1), (4, 7500, 4096, 1),  # two CTAs per SM
+    (4, 32000, 2048, 0), (4, 41000, 4096, 0), (4, 41000, 512, 0), (4, 32000, 512, 1), (4, 35000, 2048, 1),  # a last round
+    (4, 22016, 4096, 0), (4, 22016, 2048, 1), (8, 41000, 512, 1), (4, 12800, 2048, 1)])
+def test_division_by_rule(hq, dev, bits, rows, n, dealt):
+    """Rows in blocks where pairs one by one are 2 to 8 % slower (148 SMs), one by one where they gain."""
+    import torch
+    from launches import launched
+    w = torch.zeros((rows, n * bits // 8), dtype=torch.uint8, device=dev).view(torch.int8 if bits == 8 else torch.uint8)
+    x = torch.ones(n, dtype=torch.float16, device=dev)
+    call = (lambda: hq.gemv_fused("int8", x, w, rows, gamma=x)) if bits == 8 else \
+        (lambda: hq.gemv_int4_quantized(w, x, 1.0, 0.0))
+    ((name, _),) = launched(call)
+    assert f"ILi{bits}ELb{dealt}E" in name
