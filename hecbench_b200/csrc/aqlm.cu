@@ -38,15 +38,22 @@ inline int rows_per_warp_for(int prob_m, int warps) {
 // 14336 x 4096 36.9 -> 30.8; 2x8 4096 x 4096 8.4 -> 6.6, 3000 x 2048 6.7 -> 4.5, 11008 x 4096 15.5 -> 14.5.  Blocks
 // stay where they are nearly even (2x8 2368 x 4096 7.2, dealt 7.6), and where the CTAs per SM would leave
 // a slot free for an uneven start of the next launch (1x16, three of four: 6144 x 4096 16.0 and 17.3) or not fit
-// at once (2x8, more than three: 14336 x 4096 24.0 and 25.8).
+// at once (2x8, more than three: 14336 x 4096 24.0 and 25.8).  fit: how many a 2x8 SM holds, three up to
+// 4992 inputs and two beyond.  Where more are dealt each of them stages the codebooks again, for a last
+// round that blocks may leave nearly empty: 4737 x 8192 14.2 us, dealt 20.8, 9473 x 5056 18.2 and 29.0, 6144 x
+// 6144 17.4 and 17.3.  Only long rows pay for that, from a tenth of a round on (11008 x 8192 38.2, dealt
+// 36.5, 6144 x 14336 35.5 and 34.4; rows of a CTA x inputs from some 150000 on, 5504 x 6144 15.7 and 16.4).
+// 1x16, which stages nothing but its inputs, gains dealt whatever fits (14240 x 8192, one per SM, 72.6 -> 60.8).
 struct Runs {
   int ctas, per_warp, per_cta;
 };
-inline Runs divide_rows(int prob_m, int warps, int rows_per_warp, unsigned dealt_counts) {
+inline Runs divide_rows(int prob_m, int warps, int rows_per_warp, unsigned dealt_counts, int fit = 4,
+                        bool long_rows = true) {
   const int sms = sm_count(), per_cta = warps * rows_per_warp;
   const int blocks = prob_m / per_cta + (prob_m % per_cta != 0), each = (blocks + sms - 1) / sms;
   // dealt_counts: bit k stands for k CTAs per SM
   if (each > 4 || !(dealt_counts >> each & 1u) || blocks >= 0.95 * each * sms) return {blocks, 1, warps};
+  if (each > fit && (!long_rows || blocks < (each - 0.9) * sms)) return {blocks, 1, warps};
   const int ctas = std::min(prob_m / rows_per_warp + (prob_m % rows_per_warp != 0), each * sms);
   return {ctas, ctas, 1};
 }
@@ -311,7 +318,9 @@ int hq_aqlm_2x8_matvec(const void* codes, const void* x_half, void* out_half, co
   const size_t smem = (size_t)2 * 256 * 8 * 16 + (size_t)kPad * ((groups + 7) / 8) * 16;
   if (smem > 220 * 1024) return HQ_ERR_TOO_LARGE;
   const int rows_per_warp = rows_per_warp_for(prob_m, kWarps2x8);
-  const Runs runs = divide_rows(prob_m, kWarps2x8, rows_per_warp, kDealt2x8);
+  const int fit = (int)((size_t)228 * 1024 / (smem + 1024));  // CTAs that an SM holds, 1 KiB of each reserved
+  const bool long_rows = (long long)kWarps2x8 * rows_per_warp * prob_k >= 150000;
+  const Runs runs = divide_rows(prob_m, kWarps2x8, rows_per_warp, kDealt2x8, fit, long_rows);
   const int grid = runs.ctas;
   const auto c = reinterpret_cast<const uint4*>(codes);
   const auto x = reinterpret_cast<const uint4*>(x_half);

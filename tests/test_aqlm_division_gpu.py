@@ -39,3 +39,20 @@ def test_2x8_rows(hq, oracle, dev, m):
     want = oracle.aqlm_2x8_f64(codes, x, cbs, m, k, scales)
     got = out.cpu().numpy().astype(np.float64)
     assert np.linalg.norm(got[:m] - want) <= 2.0 ** -9 * np.linalg.norm(want) and (got[m:] == 7.0).all()
+
+
+@pytest.mark.parametrize("m,k,dealt", [
+    (4737, 8192, 0), (9473, 5056, 0), (5504, 6144, 0), (9728, 11008, 0), (11008, 5056, 1), (6144, 14336, 1),
+    (4737, 4992, 1), (9473, 4096, 1)])
+def test_2x8_deals_what_fits(hq, dev, m, k, dealt):
+    """More CTAs than an SM holds (two beyond 4992 inputs) only for long rows and more than a tenth of a
+    last round: each stages the codebooks again, up to 1.6 times the time (148 SMs)."""
+    import torch
+    from launches import launched
+    codes = torch.zeros((m, k // 8, 2), dtype=torch.uint8, device=dev)
+    x, cbs = (torch.ones(s, dtype=torch.float16, device=dev) for s in (k, (2, 256, 8)))
+    out, scales = (torch.ones(m, dtype=torch.float16, device=dev) for _ in range(2))
+    ((name, grid),) = launched(lambda: hq.code2x8_matvec(codes, x, out, cbs, m, k, scales))
+    rows = 32 if m // 32 >= 296 else 16
+    assert f"aqlm_2x8_kernelILb{dealt}E" in name and grid == (444 if dealt else -(-m // rows))
+    assert bool((out == 2 * k).all())
