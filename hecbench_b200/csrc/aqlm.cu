@@ -44,20 +44,25 @@ inline int rows_per_warp_for(int prob_m, int warps) {
 // 6144 17.4 and 17.3.  Only long rows pay for that, from a tenth of a round on (11008 x 8192 38.2, dealt
 // 36.5, 6144 x 14336 35.5 and 34.4; rows of a CTA x inputs from some 150000 on, 5504 x 6144 15.7 and 16.4).
 // 1x16, which stages nothing but its inputs, gains dealt whatever fits (14240 x 8192, one per SM, 72.6 -> 60.8).
+// Lines: by CTAs per SM, one to four, how full blocks must be to stay (0: always).  2x8, blocks and dealt: 2048 x
+// 4096 (0.86 of one) 7.2 and 7.2, 2240 x 4096 (0.95) 7.2 and 7.7; 4480 x 4096 (0.95 of two) 8.3 and 7.0; 6300 x 4096
+// (0.89 of three) 9.03 and 8.87, 6656 x 4096 (0.94) 9.05 and 9.2, 13312 x 4096 (0.94) 15.6 and 15.9; where three
+// do not fit 13400 x 8192 (0.94) 38.8 and 38.2.
+using Lines = double[4];
+constexpr Lines kDealt1x16 = {0.95, 0.95, 0, 0.95}, kDealt2x8 = {0.88, 0.95, 0.91, 0};
 struct Runs {
   int ctas, per_warp, per_cta;
 };
-inline Runs divide_rows(int prob_m, int warps, int rows_per_warp, unsigned dealt_counts, int fit = 4,
+inline Runs divide_rows(int prob_m, int warps, int rows_per_warp, const Lines& dealt_below, int fit = 4,
                         bool long_rows = true) {
   const int sms = sm_count(), per_cta = warps * rows_per_warp;
   const int blocks = prob_m / per_cta + (prob_m % per_cta != 0), each = (blocks + sms - 1) / sms;
-  // dealt_counts: bit k stands for k CTAs per SM
-  if (each > 4 || !(dealt_counts >> each & 1u) || blocks >= 0.95 * each * sms) return {blocks, 1, warps};
+  if (each > 4 || dealt_below[each - 1] == 0) return {blocks, 1, warps};
+  if (blocks >= (each > fit ? 0.95 : dealt_below[each - 1]) * each * sms) return {blocks, 1, warps};
   if (each > fit && (!long_rows || blocks < (each - 0.9) * sms)) return {blocks, 1, warps};
   const int ctas = std::min(prob_m / rows_per_warp + (prob_m % rows_per_warp != 0), each * sms);
   return {ctas, ctas, 1};
 }
-constexpr unsigned kDealt1x16 = 1u << 1 | 1u << 2 | 1u << 4, kDealt2x8 = 1u << 1 | 1u << 2 | 1u << 3;
 __device__ __forceinline__ int first_row(const Runs& r, int warp, int rows_per_warp) {
   return (warp * r.per_warp + (int)blockIdx.x * r.per_cta) * rows_per_warp;
 }

@@ -43,10 +43,13 @@ def test_2x8_rows(hq, oracle, dev, m):
 
 @pytest.mark.parametrize("m,k,dealt", [
     (4737, 8192, 0), (9473, 5056, 0), (5504, 6144, 0), (9728, 11008, 0), (11008, 5056, 1), (6144, 14336, 1),
-    (4737, 4992, 1), (9473, 4096, 1)])
+    (4737, 4992, 1), (9473, 4096, 1),
+    # nearly even blocks stay
+    (2240, 4096, 0), (6656, 4096, 0), (13312, 4096, 0), (12288, 4096, 1), (13400, 8192, 1)])
 def test_2x8_deals_what_fits(hq, dev, m, k, dealt):
     """More CTAs than an SM holds (two beyond 4992 inputs) only for long rows and more than a tenth of a
-    last round: each stages the codebooks again, up to 1.6 times the time (148 SMs)."""
+    last round: each stages the codebooks again, up to 1.6 times the time (148 SMs).  Blocks that are
+    nearly even stay."""
     import torch
     from launches import launched
     codes = torch.zeros((m, k // 8, 2), dtype=torch.uint8, device=dev)
