@@ -190,3 +190,48 @@ def test_division_by_rule(hq, dev, bits, rows, n, dealt):
         (lambda: hq.gemv_int4_quantized(w, x, 1.0, 0.0))
     ((name, _),) = launched(call)
     assert f"ILi{bits}ELb{dealt}E" in name
+
+
+def _small_case(bits, rows, n, dev):
+    """Integer weights and inputs whose sums are exact in every order: weights for the kernels, their values less
+    the zero point in fp64, inputs."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(rows + n)
+    x = torch.randint(-1, 2, (n,), generator=g, device=dev).half()
+    if bits == 4:
+        b = torch.randint(0, 256, (rows, n // 2), generator=g, device=dev).to(torch.uint8)
+        return b, torch.stack([b & 15, b >> 4], dim=2).reshape(rows, n).double() - 8.0, x
+    w = torch.randint(-2, 3, (rows, n), generator=g, device=dev)
+    return (w.half(), w.double(), x) if bits == 16 else (w.to(torch.int8), w.double() - 1.0, x)
+
+
+ROWS_OVER_LINES = [1, 2, 3, 33, 296, 4000, 4033, 4736, 7999, 8053, 9473, 11839, 11843, 21500, 30783, 32003]
+
+
+@pytest.mark.parametrize("rows", ROWS_OVER_LINES)
+def test_every_f16_row_once(hq, dev, rows):
+    """fp16 rows, where nothing but their division can go wrong (every sum is exact)."""
+    import torch
+    mat, w, x = _small_case(16, rows, 264, dev)
+    assert torch.equal(hq.gemv_fp16(mat, x).double(), w @ x.double())
+
+
+@pytest.mark.parametrize("rows_out", [(r + 1) // 2 for r in ROWS_OVER_LINES])
+@pytest.mark.parametrize("bits,n", [(16, 264), (8, 48), (4, 2112)])
+def test_every_fused_pair_once(hq, dev, bits, n, rows_out):
+    """Value / gate pairs over the same lines.  v and g are exact; the gate is fp32 (2^-20 for its exponential,
+    quotient and products), the result rounded to fp16 once, to 2^-25 where it is subnormal."""
+    import torch
+    mat, w, x = _small_case(bits, 2 * rows_out, n, dev)
+    zero = {16: 0.0, 8: 1.0, 4: 8.0}[bits]
+    kw = {} if bits == 16 else dict(scale=1.0, zero_point=zero)
+    fmt = {16: "f16", 8: "int8", 4: "int4"}[bits]
+    y = w @ x.double()
+    v, gate = y[0::2], y[1::2]
+    want = v * gate / (1 + torch.exp(-gate))
+    got = hq.gemv_fused(fmt, x, mat, rows_out, act=hq.ACT_SWIGLU, **kw).double()
+    finite = want.abs() < 65504
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -11 + 2.0 ** -20) + 2.0 ** -25)[finite].all())
+    assert bool((got.abs() >= 65504)[~finite].all())
+    plain = hq.gemv_fused(fmt, x, mat, 2 * rows_out, **kw)
+    assert torch.equal(plain.double(), y.half().double())
