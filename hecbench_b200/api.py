@@ -516,7 +516,8 @@ def qgemm_nf4(X, B, absmax, lut16, N: int, K: int, blocksize: int = 64, nibble_o
     """Y[Mb][N] = X[Mb][K] @ W with W[k][n] the NF4 weight that dequantize_nf4
     gives for element n*K + k of B (uint8[N*K/2], absmax per `blocksize`
     elements); same conventions as gemv_nf4, same workspace, status and `peers`
-    rules as qgemm_q3 (no counterpart in the reference tree)."""
+    rules as qgemm_q3 (no counterpart in the reference tree).  Fastest with blocks of
+    64, K a multiple of 128 and absmax on 16 bytes, as a fresh tensor is (hq.h)."""
     lib = load_library()
     host = lib.host
     Mb = X.shape[0]

@@ -507,7 +507,11 @@ int hq_qgemm_q3_f16(const void* X_half, const int32_t* mat, const void* scales_h
  * W[k][n] = half(lut16[code] * absmax[(n*K + k) / blocksize]) exactly as
  * hq_nf4_dequant_f16 produces it.  No counterpart in the reference tree.
  * 1 <= Mb <= 128, N % 128 == 0, blocksize % 64 == 0, K % blocksize == 0.
- * workspace and status_word as for hq_qgemm_q3_f16. */
+ * workspace and status_word as for hq_qgemm_q3_f16.  Blocks of 64 with K % 128
+ * == 0 and absmax on 16 bytes are the fast ones (long layers take 0.7 to 0.95
+ * of the time of larger blocks, or of an absmax that begins elsewhere).  absmax is aligned to
+ * 4 bytes; whether it begins on 16 may choose another kernel, so the same bits
+ * from every call hold for either kind of address by itself. */
 int hq_qgemm_nf4_f16(const void* X_half, const uint8_t* B, const float* absmax, const float* lut16,
                      void* Y_half, int Mb, int N, int K, int blocksize, int flags, void* workspace,
                      size_t workspace_bytes, int* status_word, hq_stream_t stream);
