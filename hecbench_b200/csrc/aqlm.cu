@@ -278,7 +278,8 @@ int hq_aqlm_1x16_matvec(const void* codes, const void* x_half, void* out_half, c
   // back to back: 12.4 -> 11.0 us; in a replayed graph 10.7 -> 10.6, and 2368 x 4096,
   // 148 CTAs, 6.6 -> 6.4).  A smaller one does not: the CTAs of an early start are not
   // spread over all SMs, and the gathers are bound by each SM's L1 (1024 x 8192 in 64 CTAs: 13.2
-  // us, 18.9 with the early start; 2048 x 4096 in 128, in a graph, 6.6 and 10.0).
+  // us, 18.9 with the early start; 2048 x 4096 in 128, in a graph, 6.6 and 10.0).  Dealt over 148 it does: 1024
+  // x 8192 6.9, in a graph 6.5 (in blocks 11.0), 2048 x 4096 6.6, in a graph 6.3 (7.0).
   const int4 sizes = make_int4(cb_sizes[0], cb_sizes[1], cb_sizes[2], cb_sizes[3]);
   cudaStream_t st = (cudaStream_t)stream;
 #define HQ_AQLM_LAUNCH(VPL, RPW)                                                             \

@@ -409,15 +409,15 @@ __device__ __forceinline__ void red_add_f32(float* addr, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
 }
 
-// ---- ring form: four planes in one launch, and long work per CTA --------------
+// ---- ring form: one to four planes in one launch, long work per CTA -----------
 // 128-input tiles and the tables of the register form.  Words, alphas and bias come through shared
-// memory by asynchronous copies, kDepth column steps of a warp ahead (57 to 86 KB per SM under
-// way instead of 29, and no registers held: four planes fit one launch where the register form
-// takes two, each with its own tables).  The CTAs are persistent: a unit is one column range of one
+// memory by asynchronous copies, kDepth column steps of a warp ahead (76 to 98 KB per SM under way,
+// with one plane 41 to 49, instead of 29, and no registers held: four planes fit one launch where the
+// register form takes two, each with its own tables).  The CTAs are persistent: a unit is one column range of one
 // K tile, units are numbered range by range inside a tile, CTA c takes units c, c + gridDim.x, ...,
 // and a warp's ring runs on through the ends of units, so words arrive while the tables of the
 // next tile are built.  A lane owns one column and looks up all four bytes of its words (Lookup
-// below): in the register form's division, one byte of four columns, a word goes to four lanes, and the
+// above): in the register form's division, one byte of four columns, a word goes to four lanes, and the
 // reads of the words took as many shared-memory wavefronts as the look-ups (4.1 M at 12288 x 12288, 3
 // planes, 60 % of the time); a lane's own column also needs no sum over lanes and a quarter of the
 // products with the scales.  us of a call among others, quads -> own columns: 12288 x 12288, 3 planes 27.5 -> 23.8, 4 planes

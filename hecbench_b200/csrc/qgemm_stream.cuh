@@ -29,6 +29,10 @@
 //  * NF4's absmax values, 4 bytes from each of 32 rows per warp and half step, were 32 wavefronts
 //    of the load pipe; the TMA unit brings them with the words (57.8 -> 48.7; 100 x 28672 x 8192 72.6 ->
 //    64.7).
+// The tables and slots take 217 to 230 KB of shared memory (172 and 180 before): no neighbour in the stream
+// becomes resident beside this kernel any more.  In chains the gain is larger than that: 64 tokens int8-quantized,
+// then x 8192 x 28672, 3-bit 50.8 -> 47.8 us (the quantizer's share 4.6 -> 5.8; in a graph 52.3 -> 48.3), NF4 74.4 ->
+// 59.5; followed by an int4 mat-vec of 4096 x 4096 51.3 -> 47.9 and 76.6 -> 59.6.
 // Of what the other form spent:
 //  * tcgen05.mma takes N / 2 cycles on the tensor pipe, but issuing one took 64 (a commit 95)
 //    where its addresses come from registers, 26 (15) where they are constants: the CTA
