@@ -873,7 +873,8 @@ KSplit choose_ksplit(int tiles, int nkb, bool wide, bool sharded, int sms) {
 bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t workspace_bytes, bool tma_only) {
   const int sms = sm_count();
   const int tiles = (N + streamed::kTileN - 1) / streamed::kTileN;
-  const double units = (double)tiles * ((K + 2 * kBlockK - 1) / (2 * kBlockK));
+  const int steps = (K + 2 * kBlockK - 1) / (2 * kBlockK);
+  const double units = (double)tiles * steps;
   if (workspace == nullptr || workspace_bytes < qgemm_ws_bytes(Mb, N) || !aligned16(workspace) ||
       units < 4.0 * sms || tiles < 8 || reserved_smem_per_block() != (int)streamed::kBase)
     return false;
@@ -896,7 +897,14 @@ bool takes_stream(int fmt, int Mb, int N, int K, const void* workspace, size_t w
   // faster one: 64 x 15744 x 12800 42.0 us, in parts 52.9; 16 x 9472 x 12800 25.4 and 33.5; NF4 64 x 9472 x
   // 12800 39.6 and 50.4; 128 x 12544 x 12928 50.8 and 63.7.
   if (split.ordered && turns > 0 && fmt == kFmtQ3 && Mb <= 64) turns += 0.3 + 0.16 * (units / sms) - t;
-  return m.stream[0] + m.stream[1] * (units / sms) + m.stream[2] * t + turns <
+  // Short layers, whose tiles end often: a us (NF4 two) for each tile of an SM, unless none is cut.  Of 630
+  // layers of K 1024 to 12288 the only ones that the fit above took to the slower form (us, in parts, streamed):
+  // 3-bit 8 x 1024 x 52224 15.8, 17.2, 37 x 1536 x 50432 22.2, 23.9, 128 x 2176 x 19968 28.1, 30.0; NF4 64 x 1536 x
+  // 50432 30.4, 31.9.  With whole tiles 100 x 1024 x 75776 36.8, 23.8.
+  double ends = 0.0;
+  if (tiles % sms != 0 && steps < (Mb <= 64 ? 13 : fmt == kFmtQ3 ? 18 : 0))
+    ends = (fmt == kFmtQ3 ? 1.0 : 2.0) * tiles / sms;
+  return m.stream[0] + m.stream[1] * (units / sms) + m.stream[2] * t + turns + ends <
          0.97 * (m.parts[0] + m.parts[1] * split.cost + m.parts[2] * t);
 }
 
