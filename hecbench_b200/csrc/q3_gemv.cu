@@ -4,247 +4,348 @@
 // for output column c and K-group r (32 inputs) rows 3r..3r+2 of mat[:,c] form a
 // 96-bit little-endian stream, code j at bits 3j..3j+2.
 //
-// Design.  HBM-bound on the packed words, but at 12 bytes per 32 weights the
-// instruction issue rate is the second wall, so the unpack costs one logic op
-// per weight (fp32 path) or per two weights (fp16 path):
-//  * a thread owns four adjacent columns and reads one 16-byte vector per
-//    packed row, so a warp reads 512 contiguous bytes of each row;
-//  * a 3-bit field left in place inside a zero word IS a denormal number:
-//    (w & (7 << p)) read as fp32 is q * 2^(p-149); read as a half in either
-//    half of the word it is q * 2^(p-24).  Multiplying by an input that was
-//    pre-scaled by the matching power of two (done once per CTA in shared
-//    memory) gives q*x directly from AND + FMA, no shift, no int->float;
-//  * the affine part is factored: sum (s*q - z)*x = s*sum(q*x) - z*sum(x);
-//  * a warp's packed rows are requested one group ahead, the first ones before the inputs are
-//    staged, those of a short next column block before the sums of this one meet (device time of
-//    calls among others, with the zeroing of the sums: fp32 inputs 28672 x 4096 22.4 -> 20.5 us,
-//    32768 x 8192 38.4 -> 35.1; fp16 8192 x 8192 13.0 -> 12.3, 49152 x 12288 54.7 -> 53.4);
-//  * K is split over the 8 warps of a CTA and over gridDim.y; partial sums are
-//    combined in shared memory and added to mul with one atomicAdd per column
-//    per CTA (the reference API accumulates into mul).
+// Design.
+//  * The products run on mma.sync m16n8k16 in bf16.  A 3-bit field left in place in the low eight bits
+//    of a half of a word is the bf16 number q * 2^(p - 133) (the exponents 0 and 1 have one spacing), so
+//    two weights of an A register cost one logic operation; a group's 16 pairs lie in three words
+//    as they are and six windows of them (kPair).  Inputs are pre-scaled by the matching powers of two.
+//  * An input is split into bf16 pieces by truncation, two for fp16, three for fp32, which hold it
+//    exactly; piece i is column i of B, so both input types cost the same and every product is exact.
+//    fp32 inputs are scaled by the largest exponent of their 128 (a quad of groups).
+//  * The affine part is factored: sum (s*q - z)*x = s*sum(q*x) - z*sum(x).
+//  * A warp owns 32 columns and takes four groups (a quad) at a time: lane (g, t) multiplies
+//    columns 4g .. 4g + 3 of group t.  NB warps side by side, W / NB in turn along K.
+//  * One CTA per SM takes an equal range of (block of 32 NB columns, quads) steps; sums go to mul
+//    (the reference API accumulates into it) once per range and block, one atomicAdd per column.
+//  * Words come by cp.async, two quads ahead per warp, eight lanes to a 128-byte line: with a quarter-warp
+//    over four lines a read of 226 MB took 57 us, with whole lines 35 (the copy rate).
+//
+// What bounds it: the logic pipe (two cycles an operation, 22 of them for 32 weights), 56 %, and HBM.
+// us in replayed graphs, sums of fp16 products in registers, a group ahead (before) -> this
+// form, fp16 (fp32) inputs: 49152 x 12288 50.3 -> 41.1 (72.7 -> 42.8), 28672 x 8192 24.5 -> 18.7 (30.3 -> 19.3), 8192 x
+// 8192 9.8 -> 7.4 (11.3 -> 7.6), 4096 x 4096 3.8 -> 3.3 (4.3 -> 3.3), 1024 x 4096 3.3 -> 2.5 (2.9 -> 2.5); 180
+// layers 0.81, worst 1.1 (7268 x 1600, fp32, 3.4 -> 3.6).
+// Error against fp64 sums: 5e-4 to 1.1e-3 -> 1e-7 to 2.5e-7 (fp32 inputs 1e-7 to 5.7e-7 -> 1e-7 to 2.1e-7).
+// Taken back: windows by multiplications on the other pipe (49152 x 12288 45.1 -> 54.6).
+#include <type_traits>
+#include <utility>
+
 #include "hq_common.cuh"
 
 namespace hq {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = 8;
-constexpr int kColsPerCta = 128;  // 32 lanes x 4 columns
-constexpr int kF16Words = 20;     // 18 half2 input pairs per group + 2 pad (16-byte rows)
+constexpr int kDepth = 3;                // quads of packed words per warp: one in use, the others on the way
+constexpr int kSlot = 3 * 32 * 16;       // bytes of a warp's words of a quad
+constexpr int kColsPerWarp = 32;
+constexpr int kSliceQuads = 128;
 
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
-// Window starts (in codes) of the six 32-bit windows of the fp16 path.  Window a
-// holds codes a..a+2 at bits 1,4,7 of its low half and codes a+5..a+7 at bits
-// 0,3,6 of its high half.
-__device__ __forceinline__ int f16_window_start(int w) {
-  return w == 0 ? 0 : w == 1 ? 3 : w == 2 ? 11 : w == 3 ? 14 : w == 4 ? 22 : 25;
+constexpr int kPairs = 16;
+struct Pair { int shift, lo, hi; };  // window's first bit in the group's stream; codes in its low and high half
+constexpr Pair kPair[kPairs] = {{0, 0, 6},    {0, 1, 7},    {6, 2, 8},    {6, 3, 9},    {12, 4, 10},  {12, 5, 11},
+                                {32, 12, 17}, {37, 13, 18}, {37, 14, 19}, {43, 15, 20}, {43, 16, 21}, {64, 22, 27},
+                                {64, 23, 28}, {70, 24, 29}, {70, 25, 30}, {73, 26, 31}};
+// bit positions of a pair's fields in the halves of its window
+__host__ __device__ constexpr int field_lo(int j) { return 3 * kPair[j].lo - kPair[j].shift; }
+__host__ __device__ constexpr int field_hi(int j) { return 3 * kPair[j].hi - kPair[j].shift - 16; }
+constexpr bool pairs_cover() {
+  unsigned seen = 0;
+  for (int j = 0; j < kPairs; j++) {
+    if (field_lo(j) < 0 || field_lo(j) > 5 || field_hi(j) < 0 || field_hi(j) > 5) return false;
+    seen |= 1u << kPair[j].lo | 1u << kPair[j].hi;
+  }
+  return seen == 0xffffffffu;
+}
+static_assert(pairs_cover(), "every code once, its field in the low eight bits of a half");
+
+template <int V>
+using Int = std::integral_constant<int, V>;
+// codes and bit positions of pair j
+template <int... J>
+__device__ __forceinline__ void find_pair(int j, int& lo, int& hi, int& plo, int& phi,
+                                          std::integer_sequence<int, J...>) {
+  ((lo = j == J ? Int<kPair[J].lo>::value : lo, hi = j == J ? Int<kPair[J].hi>::value : hi,
+    plo = j == J ? Int<field_lo(J)>::value : plo, phi = j == J ? Int<field_hi(J)>::value : phi),
+   ...);
 }
 
-// MULTI: a CTA takes several column blocks one after the other (a separate
-// instantiation: the single-block form keeps its code).
-template <bool F16IN, bool MULTI, bool LONG>
-__global__ void __launch_bounds__(kThreads)
-q3_gemv_kernel(const void* vec_, const int32_t* mat,
-               float* mul, const float* scales,
-               const float* zeros, int groups, int width, int groups_per_cta,
-               int colblocks_per_cta) {
-  // the next kernel of the stream may become resident while this grid runs;
-  // nothing is read or written before every earlier kernel has completed
-  pdl_launch_dependents();
-  pdl_wait();
+template <int SHIFT>
+__device__ __forceinline__ uint32_t window(const uint32_t (&w)[3]) {
+  if constexpr (SHIFT % 32 == 0) return w[SHIFT / 32];
+  else if constexpr (SHIFT / 32 == 2) return w[2] >> (SHIFT % 32);
+  else return __funnelshift_r(w[SHIFT / 32], w[SHIFT / 32 + 1], SHIFT % 32);
+}
+template <int J>
+__device__ __forceinline__ uint32_t pair_of(const uint32_t (&w)[3]) {
+  return window<kPair[J].shift>(w) & (7u << field_lo(J) | 7u << (16 + field_hi(J)));
+}
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                         uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// sums of two columns' words (u: row of this lane, v: that row + 8) over the lane's group
+template <int... J>
+__device__ __forceinline__ void multiply(float (&d)[4], const uint32_t (&u)[3], const uint32_t (&v)[3],
+                                         const uint32_t (&x)[kPairs], std::integer_sequence<int, J...>) {
+  (mma_bf16(d, pair_of<2 * J>(u), pair_of<2 * J>(v), pair_of<2 * J + 1>(u), pair_of<2 * J + 1>(v), x[2 * J],
+            x[2 * J + 1]),
+   ...);
+}
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void copy_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 lds_u4(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(at)
+               : "memory");
+  return v;
+}
+
+template <bool F16IN>
+constexpr int kPieces = F16IN ? 2 : 3;
+// shared bytes of a quad's inputs
+template <bool F16IN>
+constexpr int kQuadBytes = kPairs * 4 * kPieces<F16IN> * 4;
+
+struct Shape {
+  int width, groups;  // columns; 32 inputs each
+  int slice_quads;    // quads of a slice of K (blockIdx.y)
+  int blocks, steps;  // blocks of 32 NB columns; steps of W / NB quads in each
+  int share, over;    // steps of a CTA; the first `over` CTAs take one more
+  int staged;         // steps whose inputs the fullest CTA holds
+};
+
+template <bool F16IN, int W, int NB>
+__global__ void __launch_bounds__(W * 32, 1)
+q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* scales, const float* zeros,
+               const Shape p) {
+  constexpr int KW = W / NB, P = kPieces<F16IN>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const int g0 = blockIdx.y * groups_per_cta;
-  const int ng = min(groups_per_cta, groups - g0);
+  // [ring W x kDepth slots][inputs staged x KW quads][their sums and scales, float2]
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int g = lane >> 2, t = lane & 3;
+  const int kw = warp / NB, cw = warp % NB;
+  const int q_lo = blockIdx.y * p.slice_quads;
+  const int g_hi = min(p.groups, (q_lo + p.slice_quads) * 4);
+  const int u0 = (int)blockIdx.x * p.share + min((int)blockIdx.x, p.over);
+  const int u1 = u0 + p.share + ((int)blockIdx.x < p.over ? 1 : 0);
+  const int staged = min(u1 - u0, p.steps);
+  const int b0 = u0 / p.steps, k0 = u0 - b0 * p.steps;
+  // eight lanes copy a line of a row (ct: group, cg: 16-byte piece); pieces of the four groups are turned
+  // against one another, so that the lanes (g, t) of a quarter-warp read different banks
+  const int ct = lane >> 3, cg = lane & 7;
+  const uint32_t ring = smem_at(smem_raw) + (uint32_t)(warp * kDepth * kSlot);
+  const uint32_t ring_in = ring + (uint32_t)((ct * 8 + ((cg + 2 * ct) & 7)) * 16);
+  const uint32_t ring_out = ring + (uint32_t)((t * 8 + ((g + 2 * t) & 7)) * 16);
+  unsigned char* const table = smem_raw + W * kDepth * kSlot;
+  float2* const sums = reinterpret_cast<float2*>(table + (size_t)p.staged * KW * kQuadBytes<F16IN>);
 
-  // shared layout: [xp table][gsum ng floats][red kWarps*128 floats][misc 4 floats]
-  const int xp_words = F16IN ? kF16Words : 32;
-  uint32_t* xp = reinterpret_cast<uint32_t*>(smem_raw);
-  float* gsum = reinterpret_cast<float*>(xp + (size_t)groups_per_cta * xp_words);
-  float* red = gsum + ((groups_per_cta + 3) & ~3);
-  float* misc = red + kWarps * kColsPerCta;
+  // this lane's pair of a group when inputs are staged
+  const int j = lane & 15;
+  int lo = 0, hi = 0, plo = 0, phi = 0;
+  find_pair(j, lo, hi, plo, phi, std::make_integer_sequence<int, kPairs>());
 
-  __shared__ float s_sumx[kWarps];
-  // The three packed rows of this warp's next group, four columns per lane.  Requested one
-  // group ahead through the column blocks, the first before the inputs are staged.
-  uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0, n2 = n0;
-  const int ncb = MULTI ? colblocks_per_cta : 1;
-  // Across column blocks only where a warp has up to four groups in each (16384 x 2048, one
-  // group: 9.8 -> 8.4 us; 28672 x 8192, three or four: 28.4 -> 27.1); with longer slices the first
-  // request of a block waits for its start (49152 x 12288, eight: 54.9 asked ahead, 53.4 not).
-  // LONG: a slice of more than five groups per warp, an instantiation without that code.  One line at
-  // four groups for both gains slices of 33 to 40 groups 1 to 2 % (28672 x 12800 37.1 -> 36.3 us) and costs
-  // the shorter ones as much, whose code it changes (28672 x 8192 27.2 -> 27.8, 16384 x 2048 8.47 -> 8.62).
-  const bool ahead = groups_per_cta <= 4 * kWarps;
-  auto request = [&](int cb, int gi) {
-    const int col0 = (blockIdx.x * ncb + cb) * kColsPerCta + lane * 4;
-    if (col0 < width && gi < ng) {
-      const int32_t* p = mat + (size_t)(g0 + gi) * 3 * width + col0;
-      n0 = ld_ordered_stream_u4(p);
-      n1 = ld_ordered_stream_u4(p + width);
-      n2 = ld_ordered_stream_u4(p + 2 * (size_t)width);
-    }
-  };
-  // ---- prologue: per-CTA scaling exponent, pre-scaled inputs, group sums ----
-  const float* xf = reinterpret_cast<const float*>(vec_);
-  const __half* xh = reinterpret_cast<const __half*>(vec_);
-  auto load_x = [&](int k) -> float {
-    return F16IN ? __half2float(ld_dependent_f16(xh + (size_t)g0 * 32 + k))
-                 : ld_dependent_f32(xf + (size_t)g0 * 32 + k);
-  };
-  // (the inputs first: they would queue behind the packed rows)
-  float amax = tid < ng * 32 ? fabsf(load_x(tid)) : 0.f;
-  request(0, warp);
-  for (int i = tid + kThreads; i < ng * 32; i += kThreads) amax = fmaxf(amax, fabsf(load_x(i)));
-  amax = warp_max(amax);
-  if (lane == 0) red[warp] = amax;
-  __syncthreads();
-  if (tid == 0) {
-    float m = red[0];
-    for (int w = 1; w < kWarps; w++) m = fmaxf(m, red[w]);
-    misc[0] = m;
-  }
-  __syncthreads();
-  amax = misc[0];
-  int e = ((__float_as_int(amax) >> 23) & 0xff) - 126;  // amax < 2^e
-  if (F16IN) e = max(-24, min(e, 17));
-  else e = max(-20, min(e, 100));
-
-  for (int gi = warp; gi < ng; gi += kWarps) {
-    float x = load_x(gi * 32 + lane);
-    float s = warp_sum(x);
-    if (lane == 0) gsum[gi] = s;
-    if (!F16IN) {
-      // field position of code j inside its fp32 window is 3*(j%7)
-      xp[gi * 32 + lane] = __float_as_uint(x * pow2f(100 - e - 3 * (lane % 7)));
-    } else {
-      // all lanes take part in the shuffles; lanes 0..17 own one input pair each
-      const int t = min(lane, 17);
-      const int w = t / 3, i = t - 3 * w;
-      const int a = f16_window_start(w);
-      const bool skip_lo = (i == 2) && (w == 1 || w == 3 || w == 5);
-      const bool skip_hi = (i == 2) && (w == 5);
-      const float xlo = __shfl_sync(0xffffffffu, x, a + i);
-      const float xhi = __shfl_sync(0xffffffffu, x, min(a + 5 + i, 31));
-      const __half hlo =
-          skip_lo ? __float2half(0.f) : __float2half(xlo * pow2f(15 - e - (1 + 3 * i)));
-      const __half hhi = skip_hi ? __float2half(0.f) : __float2half(xhi * pow2f(15 - e - 3 * i));
-      if (lane < 18) xp[gi * kF16Words + lane] = half2_as_u32(__halves2half2(hlo, hhi));
-      else if (lane < 20) xp[gi * kF16Words + lane] = 0u;
+  pdl_launch_dependents();
+  // The lines of the first steps on their way to L2 while the kernel before drains, where a CTA has three
+  // steps or more (8192 x 8192 8.2 -> 7.4 us, 12288 x 16384 17.5 -> 16.3; one step, 1184 x 6976, 2.6 -> 3.0).
+  if (u1 - u0 > 2) {
+#pragma unroll
+    for (int d = 0; d < kDepth - 1; d++) {
+      const int row = (q_lo + (k0 + d) * KW) * 12 + tid, col = b0 * NB * kColsPerWarp;
+      if (k0 + d < p.steps && tid < 12 * KW && row < g_hi * 3)
+        prefetch_l2(mat + (size_t)row * p.width + col, (uint32_t)min(NB * kColsPerWarp, p.width - col) * 4u);
     }
   }
-  __syncthreads();
+  pdl_wait();
 
-  // The staged inputs serve colblocks_per_cta blocks of 128 columns one after the
-  // other: the staging is about a third of a block's main loop, so a CTA that
-  // takes several blocks of a shorter K slice spends less of its time on it.
-  for (int cb = 0; cb < ncb; cb++) {
-    const int colblock = blockIdx.x * ncb + cb;
-    if (colblock * kColsPerCta >= width) break;
-    // ---- main loop: this warp takes groups warp, warp+8, ... of the CTA slice ----
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float sumx = 0.f;
-    if (MULTI && (LONG || !ahead) && cb > 0) request(cb, warp);
-    for (int gi = warp; gi < ng; gi += kWarps) {
-      const uint4 u0 = n0, u1 = n1, u2 = n2;
-      if (gi + kWarps < ng) request(cb, gi + kWarps);
-      else if (MULTI && !LONG && ahead && cb + 1 < ncb) request(cb + 1, warp);
-      sumx += gsum[gi];
-      const uint32_t w0s[4] = {u0.x, u0.y, u0.z, u0.w};
-      const uint32_t w1s[4] = {u1.x, u1.y, u1.z, u1.w};
-      const uint32_t w2s[4] = {u2.x, u2.y, u2.z, u2.w};
+  // ---- packed words: this lane's four columns of three rows, kDepth - 1 quads ahead ----
+  // (rows past the slice and columns past the width are not copied: what the slot held is multiplied
+  // by inputs of zero, or its sums go nowhere)
+  int pk = k0, pb = b0, left = u1 - u0;
+  const size_t row = (size_t)p.width, next = 12 * KW * row;
+  int rows_left;  // groups of the slice from this lane's on
+  const int32_t* src;
+  auto aim = [&] {
+    const int group = (q_lo + pk * KW + kw) * 4 + ct, col = (pb * NB + cw) * kColsPerWarp + cg * 4;
+    src = mat + (size_t)group * 3 * row + col;
+    rows_left = col < p.width ? g_hi - group : 0;
+  };
+  aim();
+  auto request = [&](int slot) {
+    if (left > 0) {
+      left--;
+      const uint32_t dst = ring_in + slot * kSlot;
+      if (rows_left > 0) {
+        copy_16(dst, src);
+        copy_16(dst + 512, src + row);
+        copy_16(dst + 1024, src + 2 * row);
+      }
+      src += next;
+      rows_left -= 4 * KW;
+      if (++pk == p.steps) { pk = 0; pb++; aim(); }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
 
+  // scale and zero of this lane's column in the block, and in the next one: asked for a block ahead, a
+  // range of two or three steps would wait for them as long as for its words
+  int block = b0;
+  float2 par = make_float2(0.f, 0.f), par_next = par;
+  auto parameters = [&](int of) {
+    const int col = (of * NB + cw) * kColsPerWarp + lane;
+    if (col >= p.width) return make_float2(0.f, 0.f);
+    const float s = ld_ordered_f32(scales + col);
+    return make_float2(s, ld_ordered_f32(zeros + col));
+  };
+  auto first_parameters = [&] {
+    par = parameters(b0);
+    if ((b0 + 1) * p.steps < u1) par_next = parameters(b0 + 1);
+  };
+
+  // ---- inputs: a warp stages a quad at a time ----
+  {
+    bool asked = false;
+    for (int i = warp; i < staged * KW; i += W) {
+      int st = k0 + i / KW;
+      if (st >= p.steps) st -= p.steps;
+      const int group = (q_lo + st * KW + i % KW) * 4;
+      using In = typename std::conditional<F16IN, __half, float>::type;
+      In raw[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        raw[r] = (In)0.f;
+        if (group + r < g_hi) {
+          const In* at = reinterpret_cast<const In*>(vec) + (size_t)(group + r) * 32 + lane;
+          if constexpr (F16IN) raw[r] = ld_dependent_f16(at);
+          else raw[r] = ld_dependent_f32(at);
+        }
+      }
+      if (!asked) {  // the inputs first: they would queue behind the packed words
+        asked = true;
+#pragma unroll
+        for (int d = 0; d < kDepth - 1; d++) request(d);
+        first_parameters();
+      }
+      const float x[4] = {(float)raw[0], (float)raw[1], (float)raw[2], (float)raw[3]};
+      const float sum = warp_sum((x[0] + x[1]) + (x[2] + x[3]));
+      int e = 0;
       if (!F16IN) {
-        float x[32];
-        const float4* xv = reinterpret_cast<const float4*>(xp + gi * 32);
-  #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          float4 t = xv[q];
-          x[4 * q] = t.x; x[4 * q + 1] = t.y; x[4 * q + 2] = t.z; x[4 * q + 3] = t.w;
-        }
-  #pragma unroll
-        for (int c = 0; c < 4; c++) {
-          uint32_t win[5];
-          win[0] = w0s[c];
-          win[1] = __funnelshift_r(w0s[c], w1s[c], 21);
-          win[2] = __funnelshift_r(w1s[c], w2s[c], 10);
-          win[3] = __funnelshift_r(w1s[c], w2s[c], 31);
-          win[4] = w2s[c] >> 20;
-          float a = acc[c];
-  #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int w = j / 7, i = j % 7;
-            a = fmaf(__uint_as_float(win[w] & (7u << (3 * i))), x[j], a);
-          }
-          acc[c] = a;
-        }
-      } else {
-        uint32_t x2[kF16Words];
-        const uint4* xv = reinterpret_cast<const uint4*>(xp + gi * kF16Words);
-  #pragma unroll
-        for (int q = 0; q < 5; q++) {
-          uint4 t = xv[q];
-          x2[4 * q] = t.x; x2[4 * q + 1] = t.y; x2[4 * q + 2] = t.z; x2[4 * q + 3] = t.w;
-        }
-  #pragma unroll
-        for (int c = 0; c < 4; c++) {
-          uint32_t win[6];
-          win[0] = w0s[c] << 1;
-          win[1] = __funnelshift_r(w0s[c], w1s[c], 8);
-          win[2] = w1s[c];
-          win[3] = __funnelshift_r(w1s[c], w2s[c], 9);
-          win[4] = w2s[c] >> 1;
-          win[5] = w2s[c] >> 10;
-          __half2 a2 = __float2half2_rn(0.f);
-  #pragma unroll
-          for (int w = 0; w < 6; w++) {
-  #pragma unroll
-            for (int i = 0; i < 3; i++) {
-              const uint32_t m = (7u << (1 + 3 * i)) | (7u << (16 + 3 * i));
-              a2 = __hfma2(u32_as_half2(win[w] & m), u32_as_half2(x2[3 * w + i]), a2);
-            }
-          }
-          acc[c] += __low2float(a2) + __high2float(a2);
+        uint32_t m = 0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) m = max(m, __float_as_uint(x[r]) & 0x7fffffffu);
+        e = max(0, (int)(__reduce_max_sync(0xffffffffu, m) >> 23) - 126);  // all of them below 2^e
+      }
+      if (lane == 0) sums[i] = make_float2(sum, F16IN ? 1.f : pow2f(e - 13));
+      const int top = F16IN ? 110 : 126 - e;
+      const float slo = pow2f(top - plo), shi = pow2f(top - phi);
+      unsigned char* const quad = table + (size_t)i * kQuadBytes<F16IN> + (j & 3) * 4;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        float a = __shfl_sync(0xffffffffu, x[2 * h], lo), b = __shfl_sync(0xffffffffu, x[2 * h], hi);
+        const float a1 = __shfl_sync(0xffffffffu, x[2 * h + 1], lo), b1 = __shfl_sync(0xffffffffu, x[2 * h + 1], hi);
+        if (lane >= 16) { a = a1; b = b1; }
+        const int r = 2 * h + (lane >> 4);
+        a *= slo; b *= shi;
+#pragma unroll
+        for (int q = 0; q < P; q++) {
+          uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+          *reinterpret_cast<uint32_t*>(quad + (((j >> 2) * 4 + r) * P + q) * 16) = __byte_perm(ua, ub, 0x7632);
+          // an infinity has no rest
+          a = isinf(a) ? 0.f : a - __uint_as_float(ua & 0xffff0000u);
+          b = isinf(b) ? 0.f : b - __uint_as_float(ub & 0xffff0000u);
         }
       }
     }
+    if (!asked) {
+      for (int d = 0; d < kDepth - 1; d++) request(d);
+      first_parameters();
+    }
+  }
+  __syncthreads();
 
-    // ---- epilogue: combine the 8 warps, apply scale/zero, accumulate into mul ----
-  #pragma unroll
-    for (int c = 0; c < 4; c++) red[warp * kColsPerCta + lane * 4 + c] = acc[c];
-    __syncthreads();
-    if (lane == 0) s_sumx[warp] = sumx;
-    __syncthreads();
-    if (tid < kColsPerCta) {
-      const int col = colblock * kColsPerCta + tid;
-      if (col < width) {
-        float q = 0.f, sx = 0.f;
-  #pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-          q += red[w * kColsPerCta + tid];
-          sx += s_sumx[w];
-        }
-        // undo the input pre-scaling: fp32 path 2^(49+e), fp16 path 2^(9+e)
-        q = F16IN ? q * pow2f(9 + e) : (q * pow2f(49)) * pow2f(e);
-        // (no __restrict__: the parameters may alias mul for all the compiler knows, so
-        // these are ordinary loads behind the wait)
-        float sc, nz;
-        if (F16IN) {
-          // the reference rounds both parameters to fp16 (kernels.h:121-122)
-          sc = __half2float(__float2half_rn(scales[col]));
-          nz = __half2float(__float2half_rn(-zeros[col]));
-        } else {
-          sc = scales[col];
-          nz = -zeros[col];
-        }
-        atomicAdd(&mul[col], fmaf(sc, q, nz * sx));
+  // ---- products ----
+  const uint32_t xtab = smem_at(table) + (uint32_t)(kw * kQuadBytes<F16IN> + (t * P + min(g, P - 1)) * 16);
+  const float2* const ktab = sums + kw;
+  float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f}, sumx = 0.f;
+  int k = k0;
+  uint32_t xat = xtab;
+  const uint32_t xend = xtab + (uint32_t)(staged * KW * kQuadBytes<F16IN>);
+  const float2* sat = ktab;
+  for (int u = u0; u < u1;) {
+#pragma unroll
+    for (int slot = 0; slot < kDepth; slot++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 2) : "memory");
+      __syncwarp();
+      const uint4 w0 = lds_u4(ring_out + slot * kSlot), w1 = lds_u4(ring_out + slot * kSlot + 512),
+                  w2 = lds_u4(ring_out + slot * kSlot + 1024);
+      uint32_t x[kPairs];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint4 v = lds_u4(xat + (uint32_t)(q * 64 * P));
+        x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
       }
+      const float2 sf = *sat;
+      xat += KW * kQuadBytes<F16IN>;
+      sat += KW;
+      if (xat == xend) { xat = xtab; sat = ktab; }
+      request((slot + kDepth - 1) % kDepth);
+      const uint32_t c0[3] = {w0.x, w1.x, w2.x}, c1[3] = {w0.y, w1.y, w2.y}, c2[3] = {w0.z, w1.z, w2.z},
+                     c3[3] = {w0.w, w1.w, w2.w};
+      if constexpr (F16IN) {
+        multiply(acc0, c0, c1, x, std::make_integer_sequence<int, kPairs / 2>());
+        multiply(acc1, c2, c3, x, std::make_integer_sequence<int, kPairs / 2>());
+      } else {
+        float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+        multiply(d0, c0, c1, x, std::make_integer_sequence<int, kPairs / 2>());
+        multiply(d1, c2, c3, x, std::make_integer_sequence<int, kPairs / 2>());
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          acc0[i] = fmaf(d0[i], sf.y, acc0[i]);
+          acc1[i] = fmaf(d1[i], sf.y, acc1[i]);
+        }
+      }
+      sumx += sf.x;
+      const bool end = ++k == p.steps;
+      if (end || u + 1 == u1) {
+        // the pieces of the inputs are columns 0 .. P - 1 of the sums: lanes t = 0 and, of the third, t = 1
+        const bool first = t == 0, any = P == 3 ? t < 2 : first;
+        float s[4] = {(any ? acc0[0] : 0.f) + (first ? acc0[1] : 0.f), (any ? acc0[2] : 0.f) + (first ? acc0[3] : 0.f),
+                      (any ? acc1[0] : 0.f) + (first ? acc1[1] : 0.f), (any ? acc1[2] : 0.f) + (first ? acc1[3] : 0.f)};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
+          s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
+        }
+        // lane = column of the warp
+        float q = t == 0 ? s[0] : t == 1 ? s[1] : t == 2 ? s[2] : s[3];
+        q *= F16IN ? pow2f(23) : pow2f(20);
+        const int col = (block * NB + cw) * kColsPerWarp + lane;
+        // (fp16 inputs: the reference rounds both parameters to fp16, kernels.h:121-122)
+        const float sc = F16IN ? __half2float(__float2half_rn(par.x)) : par.x;
+        const float nz = F16IN ? __half2float(__float2half_rn(-par.y)) : -par.y;
+        if (col < p.width) atomicAdd(&mul[col], fmaf(sc, q, nz * sumx));
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc0[i] = acc1[i] = 0.f;
+        sumx = 0.f;
+        if (end) { k = 0; block++; }
+        if (end && u + 1 < u1) {
+          par = par_next;
+          if ((block + 1) * p.steps < u1) par_next = parameters(block + 1);
+        }
+      }
+      if (++u >= u1) break;
     }
-    if (MULTI) __syncthreads();  // `red` and the warp sums are reused by the next column block
   }
 }
 
@@ -280,10 +381,24 @@ q3_dequant_kernel(const int32_t* __restrict__ mat, const float* __restrict__ sca
   }
 }
 
-template <auto Kern>
-struct Form {
-  static constexpr auto value = Kern;
-};
+template <bool F16IN, int W, int NB>
+int q3_gemv_go(const void* vec, const int32_t* mat, float* mul, const float* scales, const float* zeros,
+               Shape p, int slices, hq_stream_t stream) {
+  constexpr int KW = W / NB;
+  p.blocks = (p.width + NB * kColsPerWarp - 1) / (NB * kColsPerWarp);
+  p.steps = (p.slice_quads + KW - 1) / KW;
+  const long long total = (long long)p.blocks * p.steps;
+  const int grid = (int)min(total, (long long)max(1, sm_count() / slices));
+  p.share = (int)(total / grid);
+  p.over = (int)(total % grid);
+  p.staged = min(p.steps, p.share + (p.over ? 1 : 0));
+  const size_t smem = (size_t)W * kDepth * kSlot + (size_t)p.staged * KW * (kQuadBytes<F16IN> + sizeof(float2));
+  constexpr auto kern = q3_gemv_kernel<F16IN, W, NB>;
+  cudaError_t e = ensure_dynamic_smem<kern>(smem);
+  if (e != cudaSuccess) return cuda_status(e);
+  return cuda_status(launch_pdl(kern, dim3(grid, slices), dim3(W * 32), smem, (cudaStream_t)stream, vec, mat, mul,
+                                scales, zeros, p));
+}
 
 template <bool F16IN>
 int q3_gemv_launch(const void* vec, const int32_t* mat, float* mul, const float* scales,
@@ -292,58 +407,46 @@ int q3_gemv_launch(const void* vec, const int32_t* mat, float* mul, const float*
   if (height <= 0 || width <= 0 || height % 3 != 0 || width % 4 != 0) return HQ_ERR_BAD_SHAPE;
   if (!aligned16(mat)) return HQ_ERR_MISALIGNED;
   if (!aligned4(vec) || !aligned4(mul)) return HQ_ERR_MISALIGNED;
-  const int groups = height / 3;
-  const int colblocks_total = (width + kColsPerCta - 1) / kColsPerCta;
-  // Grid = (column blocks / CB) x (K split).  A slice holds at most 256 groups
-  // (8192 inputs: the pre-scaled inputs fit shared memory) and at least one
-  // group per warp.  Cost model per CTA, in group iterations of one column block:
-  // 6 fixed + g * (CB + 0.34) - staging a group's inputs costs about a third of
-  // using them for one block - times the number of waves the grid needs on the
-  // resident CTA slots (a grid of 2.1 waves runs as long as one of 3).
-  const int sms = sm_count();
-  const int slots = sms * (F16IN ? 4 : 3);  // resident CTAs at 59 / 74 registers per thread
-  const int k_lo = max(1, (groups + 255) / 256);
-  int ksplit = k_lo, cbs = 1;
-  double best = 1e30;
-  // (fp32 inputs: staging is cheap there and several blocks per CTA measured slower)
-  for (int cb = 1; cb <= (F16IN ? 4 : 1); cb *= 2) {
-    const int colblocks = (colblocks_total + cb - 1) / cb;
-    const int k_hi =
-        max(k_lo, min((groups + kWarps - 1) / kWarps, (16 * sms + colblocks - 1) / colblocks));
-    for (int k = k_lo; k <= k_hi; k++) {
-      const int g = (groups + k - 1) / k;
-      const int kk = (groups + g - 1) / g;
-      const long ctas = (long)colblocks * kk;
-      const long waves = (ctas + slots - 1) / slots;
-      // a grid that leaves most slots of its last wave empty pays with idle SMs
-      const double fill = (double)ctas / (double)(waves * slots);
-      const double cost = (double)waves * (6.0 + g * (cb + 0.34)) / (fill > 0.5 ? 1.0 : 2.0 * fill);
-      if (cost < best - 1e-9) { best = cost; ksplit = kk; cbs = cb; }
-    }
-  }
-  const int colblocks = (colblocks_total + cbs - 1) / cbs;
-  int gpc = (groups + ksplit - 1) / ksplit;
-  ksplit = (groups + gpc - 1) / gpc;
-  const int xp_words = F16IN ? kF16Words : 32;
-  size_t smem = (size_t)gpc * xp_words * 4 + (size_t)((gpc + 3) & ~3) * 4 +
-                (size_t)kWarps * kColsPerCta * 4 + 16;
-  dim3 grid(colblocks, ksplit);
-  auto go = [&](auto form) {
-    constexpr auto kern = decltype(form)::value;
-    if (smem > 48 * 1024) {
-      cudaError_t e = ensure_dynamic_smem<kern>(smem);
-      if (e != cudaSuccess) return cuda_status(e);
-    }
-    return cuda_status(launch_pdl(kern, grid, dim3(kThreads), smem, (cudaStream_t)stream, vec, mat, mul,
-                                  scales, zeros, groups, width, gpc, cbs));
+  Shape p;
+  p.width = width;
+  p.groups = height / 3;
+  // a CTA holds the inputs of a slice, 16384 of them at most (96 KB, fp32)
+  const int quads = (p.groups + 3) / 4;
+  const int slices = (quads + kSliceQuads - 1) / kSliceQuads;
+  p.slice_quads = (quads + slices - 1) / slices;
+  const int slots = max(1, sm_count() / slices);
+  // Steps of the CTA that has most of them, W warps, NB side by side.  The widest block (whole
+  // lines of DRAM pages, one set of inputs) unless a narrower one leaves less of its last block empty: 4100 columns
+  // of 33 quads are 3 steps with 16 warps side by side and 2 with 8.
+  auto longest = [&](int w, int nb) {
+    const long long blocks = (width + nb * kColsPerWarp - 1) / (nb * kColsPerWarp);
+    const long long steps = (p.slice_quads + w / nb - 1) / (w / nb);
+    return (blocks * steps + slots - 1) / slots;
   };
-  if (cbs == 1) return go(Form<q3_gemv_kernel<F16IN, false, false>>());
-  // fp32 inputs always take one block
-  if constexpr (F16IN) {
-    if (gpc > 5 * kWarps) return go(Form<q3_gemv_kernel<true, true, true>>());
-    return go(Form<q3_gemv_kernel<true, true, false>>());
+  auto narrow = [&](int w) {  // log2 of W / NB
+    int n = 0;
+    for (int i = 1; i <= 2; i++)
+      if (longest(w, w >> i) < longest(w, w >> n)) n = i;
+    return n;
+  };
+  // 20 warps hide more of what a step waits for and take the same time for a warp's share of it: us in
+  // graphs, 16 and 20 warps, at 20 l20 / 16 l16 of 0.62 (8804 x 1280) 3.5 and 2.9, 0.83 (5116 x 4288) 4.6 and 4.4, 0.95
+  // (26236 x 7232) 17.1 and 16.3, 1 (36388 x 16128) 43.4 and 41.1, 1.04 (10012 x 5248) 7.6 and 7.9, 1.25 (11124 x
+  // 1664) 4.1 and 4.6.
+  const int n16 = narrow(16), n20 = narrow(20);
+  const long long l16 = longest(16, 16 >> n16), l20 = longest(20, 20 >> n20);
+  const bool wide = 20 * l20 <= 16 * l16;
+  // Layers of up to half a step for every SM start sooner with 8 warps (512 x 1024, graphs, 2.5 -> 2.0 us).
+  const long long u8 = (long long)((width + 255) / 256) * p.slice_quads;
+  if (2 * u8 <= slots) return q3_gemv_go<F16IN, 8, 8>(vec, mat, mul, scales, zeros, p, slices, stream);
+  switch (wide ? 3 + n20 : n16) {
+    case 0: return q3_gemv_go<F16IN, 16, 16>(vec, mat, mul, scales, zeros, p, slices, stream);
+    case 1: return q3_gemv_go<F16IN, 16, 8>(vec, mat, mul, scales, zeros, p, slices, stream);
+    case 2: return q3_gemv_go<F16IN, 16, 4>(vec, mat, mul, scales, zeros, p, slices, stream);
+    case 3: return q3_gemv_go<F16IN, 20, 20>(vec, mat, mul, scales, zeros, p, slices, stream);
+    case 4: return q3_gemv_go<F16IN, 20, 10>(vec, mat, mul, scales, zeros, p, slices, stream);
+    default: return q3_gemv_go<F16IN, 20, 5>(vec, mat, mul, scales, zeros, p, slices, stream);
   }
-  return HQ_ERR_UNSUPPORTED;  // not reached
 }
 
 template <bool F16OUT>

@@ -1,0 +1,72 @@
+"""The 3-bit mat-vec's division into blocks of columns and steps along K: ranges that begin inside a
+block, a last block, a last quad of groups and a last slice of K that are not full, 8, 16 and 20
+warps side by side or in turn; inputs of every exponent, and an infinity."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# N, K, at 148 SMs: 8 warps; 16 warps, one step; 20 warps (11008: ranges of four steps); 16 warps, eight
+# side by side (4100 columns of 33 quads); two slices of K, the second of them shorter
+SIZES = [(4, 32), (260, 160), (512, 1024), (3200, 3040), (8804, 1280), (5116, 4288), (11008, 4096), (4100, 4160),
+         (516, 16416), (1028, 33024)]
+
+
+def _layer(hq, dev, N, K):
+    import torch
+    g = torch.Generator(device=dev).manual_seed(N * 7 + K)
+    mat = torch.randint(-2**31, 2**31, (K * 3 // 32, N), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    scales = torch.rand(N, generator=g, device=dev) * 0.01 + 0.001
+    zeros = scales * torch.randint(0, 8, (N,), generator=g, device=dev)
+    codes = hq.vecquant3_dequant(mat, torch.ones(N, device=dev), torch.zeros(N, device=dev), K * 3 // 32, N)
+    return g, mat, scales, zeros, codes.double()
+
+
+@pytest.mark.parametrize("half", [True, False])
+@pytest.mark.parametrize("N,K", SIZES)
+def test_divisions(hq, dev, N, K, half):
+    """Products are exact, so what differs from fp64 is the order of fp32 sums: K * 2^-24 of the sum of
+    the products' magnitudes at most, whatever the inputs' exponents (here 2^-8 to 2^8)."""
+    import torch
+    g, mat, scales, zeros, codes = _layer(hq, dev, N, K)
+    x = torch.randn(K, generator=g, device=dev) * torch.exp2(torch.randint(-8, 9, (K,), generator=g, device=dev).float())
+    x = x.half() if half else x
+    call = hq.vecquant3matmul_faster if half else hq.vecquant3matmul
+    s, z = (scales.half().double(), zeros.half().double()) if half else (scales.double(), zeros.double())
+    start = torch.randn(N, generator=g, device=dev)
+    out = start.clone()
+    call(x, mat, out, scales, zeros, K * 3 // 32, N)
+    want = start.double() + s * (x.double() @ codes) - z * x.double().sum()
+    size = s * (x.double().abs() @ codes) + z * x.double().abs().sum()
+    assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24 + want.abs() * 2.0 ** -22 + 2.0 ** -22).all())
+
+
+@pytest.mark.parametrize("exponent", [-110, -60, -1, 0, 60, 110])
+def test_fp32_inputs_of_any_exponent(hq, dev, exponent):
+    """Inputs are split exactly and scaled by their largest exponent: the bound above holds for tiny and huge
+    ones, also beside ones of another size (every 256 inputs 2^-20 of the others)."""
+    import torch
+    N, K = 516, 2048
+    g, mat, scales, zeros, codes = _layer(hq, dev, N, K)
+    x = torch.randn(K, generator=g, device=dev) * 2.0 ** exponent
+    x[256:512] *= 2.0 ** -20
+    out = torch.zeros(N, device=dev)
+    hq.vecquant3matmul(x, mat, out, scales, zeros, K * 3 // 32, N)
+    want = scales.double() * (x.double() @ codes) - zeros.double() * x.double().sum()
+    size = scales.double() * (x.double().abs() @ codes) + zeros.double() * x.double().abs().sum()
+    assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24).all())
+
+
+@pytest.mark.parametrize("half", [True, False])
+def test_an_infinite_input(hq, dev, half):
+    """An infinity times a code above zero is one, with the sign of the input (zeros below zero: what the
+    sum of inputs adds has that sign too); times zero it is no number."""
+    import torch
+    N, K = 132, 96
+    g, mat, scales, zeros, codes = _layer(hq, dev, N, K)
+    x = torch.randn(K, generator=g, device=dev)
+    x[37] = float("-inf")
+    x = x.half() if half else x
+    out = torch.zeros(N, device=dev)
+    (hq.vecquant3matmul_faster if half else hq.vecquant3matmul)(x, mat, out, scales, -scales, K * 3 // 32, N)
+    above = codes[37] > 0
+    assert bool((out[above] == float("-inf")).all()) and bool(out[~above].isnan().all())
