@@ -22,11 +22,13 @@
 //
 // What bounds it: the logic pipe (two cycles an operation, 22 of them for 32 weights), 56 %, and HBM.
 // us in replayed graphs, sums of fp16 products in registers, a group ahead (before) -> this
-// form, fp16 (fp32) inputs: 49152 x 12288 50.3 -> 41.1 (72.7 -> 42.8), 28672 x 8192 24.5 -> 18.7 (30.3 -> 19.3), 8192 x
-// 8192 9.8 -> 7.4 (11.3 -> 7.6), 4096 x 4096 3.8 -> 3.3 (4.3 -> 3.3), 1024 x 4096 3.3 -> 2.5 (2.9 -> 2.5); 180
-// layers 0.81, worst 1.1 (7268 x 1600, fp32, 3.4 -> 3.6).
+// form, fp16 (fp32) inputs: 49152 x 12288 50.3 -> 40.9 (72.7 -> 41.9), 28672 x 8192 24.5 -> 18.3 (30.3 -> 18.7), 8192 x
+// 8192 9.8 -> 7.4 (11.3 -> 7.6), 4096 x 4096 3.8 -> 3.2 (4.3 -> 3.2), 1024 x 4096 3.3 -> 2.4 (2.9 -> 2.4), 512 x
+// 1024 2.4 -> 1.8 (2.1 -> 1.8); 300 layers of 512 to 49152 columns, 1024 to 16384 inputs 0.78, worst 1.07 (768 x 9408).
 // Error against fp64 sums: 5e-4 to 1.1e-3 -> 1e-7 to 2.5e-7 (fp32 inputs 1e-7 to 5.7e-7 -> 1e-7 to 2.1e-7).
 // Taken back: windows by multiplications on the other pipe (49152 x 12288 45.1 -> 54.6).
+#include <limits.h>
+
 #include <type_traits>
 #include <utility>
 
@@ -61,16 +63,16 @@ constexpr bool pairs_cover() {
 }
 static_assert(pairs_cover(), "every code once, its field in the low eight bits of a half");
 
-template <int V>
-using Int = std::integral_constant<int, V>;
-// codes and bit positions of pair j
-template <int... J>
-__device__ __forceinline__ void find_pair(int j, int& lo, int& hi, int& plo, int& phi,
-                                          std::integer_sequence<int, J...>) {
-  ((lo = j == J ? Int<kPair[J].lo>::value : lo, hi = j == J ? Int<kPair[J].hi>::value : hi,
-    plo = j == J ? Int<field_lo(J)>::value : plo, phi = j == J ? Int<field_hi(J)>::value : phi),
-   ...);
+// The same for a pair that is known at run time only: codes by their three runs, positions from
+// nibbles.
+__device__ __forceinline__ int code_lo(int j) { return j + (j >= 6 ? 6 : 0) + (j >= 11 ? 5 : 0); }
+__device__ __forceinline__ int code_hi(int j) { return j + 6 + (j >= 6 ? 5 : 0) + (j >= 11 ? 5 : 0); }
+constexpr uint64_t fields(bool high) {
+  uint64_t v = 0;
+  for (int j = 0; j < kPairs; j++) v |= (uint64_t)(high ? field_hi(j) : field_lo(j)) << (4 * j);
+  return v;
 }
+constexpr uint64_t kFieldsLo = fields(false), kFieldsHi = fields(true);
 
 template <int SHIFT>
 __device__ __forceinline__ uint32_t window(const uint32_t (&w)[3]) {
@@ -151,11 +153,6 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
   unsigned char* const table = smem_raw + W * kDepth * kSlot;
   float2* const sums = reinterpret_cast<float2*>(table + (size_t)p.staged * KW * kQuadBytes<F16IN>);
 
-  // this lane's pair of a group when inputs are staged
-  const int j = lane & 15;
-  int lo = 0, hi = 0, plo = 0, phi = 0;
-  find_pair(j, lo, hi, plo, phi, std::make_integer_sequence<int, kPairs>());
-
   pdl_launch_dependents();
   // The lines of the first steps on their way to L2 while the kernel before drains, where a CTA has three
   // steps or more (8192 x 8192 8.2 -> 7.4 us, 12288 x 16384 17.5 -> 16.3; one step, 1184 x 6976, 2.6 -> 3.0).
@@ -172,29 +169,31 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
   // ---- packed words: this lane's four columns of three rows, kDepth - 1 quads ahead ----
   // (rows past the slice and columns past the width are not copied: what the slot held is multiplied
   // by inputs of zero, or its sums go nowhere)
-  int pk = k0, pb = b0, left = u1 - u0;
   const size_t row = (size_t)p.width, next = 12 * KW * row;
+  int pk = k0, pb = b0, left = u1 - u0;  // of the next request
+  int run = 0;    // requests until the block or the range ends
   int rows_left;  // groups of the slice from this lane's on
   const int32_t* src;
   auto aim = [&] {
     const int group = (q_lo + pk * KW + kw) * 4 + ct, col = (pb * NB + cw) * kColsPerWarp + cg * 4;
     src = mat + (size_t)group * 3 * row + col;
-    rows_left = col < p.width ? g_hi - group : 0;
+    rows_left = col < p.width && left > 0 ? g_hi - group : 0;
+    run = left > 0 ? min(p.steps - pk, left) : INT_MAX;
+    left -= run;
+    pk = 0;
+    pb++;
   };
   aim();
   auto request = [&](int slot) {
-    if (left > 0) {
-      left--;
-      const uint32_t dst = ring_in + slot * kSlot;
-      if (rows_left > 0) {
-        copy_16(dst, src);
-        copy_16(dst + 512, src + row);
-        copy_16(dst + 1024, src + 2 * row);
-      }
-      src += next;
-      rows_left -= 4 * KW;
-      if (++pk == p.steps) { pk = 0; pb++; aim(); }
+    const uint32_t dst = ring_in + slot * kSlot;
+    if (rows_left > 0) {
+      copy_16(dst, src);
+      copy_16(dst + 512, src + row);
+      copy_16(dst + 1024, src + 2 * row);
     }
+    src += next;
+    rows_left -= 4 * KW;
+    if (--run == 0) aim();
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
@@ -208,36 +207,43 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
     const float s = ld_ordered_f32(scales + col);
     return make_float2(s, ld_ordered_f32(zeros + col));
   };
-  auto first_parameters = [&] {
-    par = parameters(b0);
-    if ((b0 + 1) * p.steps < u1) par_next = parameters(b0 + 1);
-  };
 
   // ---- inputs: a warp stages a quad at a time ----
   {
-    bool asked = false;
-    for (int i = warp; i < staged * KW; i += W) {
+    // lane: pair j of the groups r0 and r0 + 2
+    using In = typename std::conditional<F16IN, __half, float>::type;
+    const int j = lane & 15, r0 = lane >> 4;
+    const int plo = (int)(kFieldsLo >> (4 * j)) & 15, phi = (int)(kFieldsHi >> (4 * j)) & 15;
+    const In* const mine_lo = reinterpret_cast<const In*>(vec) + code_lo(j);
+    const In* const mine_hi = reinterpret_cast<const In*>(vec) + code_hi(j);
+    In raw[4];
+    auto load = [&](int i) {
       int st = k0 + i / KW;
       if (st >= p.steps) st -= p.steps;
-      const int group = (q_lo + st * KW + i % KW) * 4;
-      using In = typename std::conditional<F16IN, __half, float>::type;
-      In raw[4];
+      const int group = (q_lo + st * KW + i % KW) * 4 + r0;
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        raw[r] = (In)0.f;
-        if (group + r < g_hi) {
-          const In* at = reinterpret_cast<const In*>(vec) + (size_t)(group + r) * 32 + lane;
-          if constexpr (F16IN) raw[r] = ld_dependent_f16(at);
-          else raw[r] = ld_dependent_f32(at);
+      for (int h = 0; h < 2; h++) {
+        raw[2 * h] = raw[2 * h + 1] = (In)0.f;
+        if (i < staged * KW && group + 2 * h < g_hi) {
+          const size_t at = (size_t)(group + 2 * h) * 32;
+          if constexpr (F16IN) {
+            raw[2 * h] = ld_dependent_f16(mine_lo + at);
+            raw[2 * h + 1] = ld_dependent_f16(mine_hi + at);
+          } else {
+            raw[2 * h] = ld_dependent_f32(mine_lo + at);
+            raw[2 * h + 1] = ld_dependent_f32(mine_hi + at);
+          }
         }
       }
-      if (!asked) {  // the inputs first: they would queue behind the packed words
-        asked = true;
+    };
+    load(warp);  // the inputs first: they would queue behind the packed words
 #pragma unroll
-        for (int d = 0; d < kDepth - 1; d++) request(d);
-        first_parameters();
-      }
+    for (int d = 0; d < kDepth - 1; d++) request(d);
+    par = parameters(b0);
+    if ((b0 + 1) * p.steps < u1) par_next = parameters(b0 + 1);
+    for (int i = warp; i < staged * KW; i += W) {
       const float x[4] = {(float)raw[0], (float)raw[1], (float)raw[2], (float)raw[3]};
+      load(i + W);
       const float sum = warp_sum((x[0] + x[1]) + (x[2] + x[3]));
       int e = 0;
       if (!F16IN) {
@@ -252,11 +258,8 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
       unsigned char* const quad = table + (size_t)i * kQuadBytes<F16IN> + (j & 3) * 4;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        float a = __shfl_sync(0xffffffffu, x[2 * h], lo), b = __shfl_sync(0xffffffffu, x[2 * h], hi);
-        const float a1 = __shfl_sync(0xffffffffu, x[2 * h + 1], lo), b1 = __shfl_sync(0xffffffffu, x[2 * h + 1], hi);
-        if (lane >= 16) { a = a1; b = b1; }
-        const int r = 2 * h + (lane >> 4);
-        a *= slo; b *= shi;
+        float a = x[2 * h] * slo, b = x[2 * h + 1] * shi;
+        const int r = 2 * h + r0;
 #pragma unroll
         for (int q = 0; q < P; q++) {
           uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
@@ -267,22 +270,21 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
         }
       }
     }
-    if (!asked) {
-      for (int d = 0; d < kDepth - 1; d++) request(d);
-      first_parameters();
-    }
   }
   __syncthreads();
 
   // ---- products ----
   const uint32_t xtab = smem_at(table) + (uint32_t)(kw * kQuadBytes<F16IN> + (t * P + min(g, P - 1)) * 16);
   const float2* const ktab = sums + kw;
-  float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f}, sumx = 0.f;
-  int k = k0;
+  float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
+  float sumx = 0.f;
+  // a segment: steps of one block whose inputs lie in a row; u, k, at: where it begins
+  int u = u0, k = k0, at = 0, seg = 0, todo = 0;
   uint32_t xat = xtab;
-  const uint32_t xend = xtab + (uint32_t)(staged * KW * kQuadBytes<F16IN>);
   const float2* sat = ktab;
-  for (int u = u0; u < u1;) {
+  auto segment = [&] { seg = todo = min(min(p.steps - k, u1 - u), staged - at); };
+  segment();
+  for (;;) {
 #pragma unroll
     for (int slot = 0; slot < kDepth; slot++) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 2) : "memory");
@@ -298,7 +300,6 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
       const float2 sf = *sat;
       xat += KW * kQuadBytes<F16IN>;
       sat += KW;
-      if (xat == xend) { xat = xtab; sat = ktab; }
       request((slot + kDepth - 1) % kDepth);
       const uint32_t c0[3] = {w0.x, w1.x, w2.x}, c1[3] = {w0.y, w1.y, w2.y}, c2[3] = {w0.z, w1.z, w2.z},
                      c3[3] = {w0.w, w1.w, w2.w};
@@ -316,35 +317,45 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
         }
       }
       sumx += sf.x;
-      const bool end = ++k == p.steps;
-      if (end || u + 1 == u1) {
-        // the pieces of the inputs are columns 0 .. P - 1 of the sums: lanes t = 0 and, of the third, t = 1
-        const bool first = t == 0, any = P == 3 ? t < 2 : first;
-        float s[4] = {(any ? acc0[0] : 0.f) + (first ? acc0[1] : 0.f), (any ? acc0[2] : 0.f) + (first ? acc0[3] : 0.f),
-                      (any ? acc1[0] : 0.f) + (first ? acc1[1] : 0.f), (any ? acc1[2] : 0.f) + (first ? acc1[3] : 0.f)};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
-          s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
+      if (--todo == 0) {
+        u += seg;
+        k += seg;
+        at += seg;
+        if (at == staged) {
+          at = 0;
+          xat = xtab;
+          sat = ktab;
         }
-        // lane = column of the warp
-        float q = t == 0 ? s[0] : t == 1 ? s[1] : t == 2 ? s[2] : s[3];
-        q *= F16IN ? pow2f(23) : pow2f(20);
-        const int col = (block * NB + cw) * kColsPerWarp + lane;
-        // (fp16 inputs: the reference rounds both parameters to fp16, kernels.h:121-122)
-        const float sc = F16IN ? __half2float(__float2half_rn(par.x)) : par.x;
-        const float nz = F16IN ? __half2float(__float2half_rn(-par.y)) : -par.y;
-        if (col < p.width) atomicAdd(&mul[col], fmaf(sc, q, nz * sumx));
+        if (k == p.steps || u == u1) {
+          // the pieces of the inputs are columns 0 .. P - 1 of the sums: lanes t = 0 and, of the third, t = 1
+          const bool first = t == 0, any = P == 3 ? t < 2 : first;
+          float s[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc0[i] = acc1[i] = 0.f;
-        sumx = 0.f;
-        if (end) { k = 0; block++; }
-        if (end && u + 1 < u1) {
+          for (int i = 0; i < 4; i++) {
+            const float a = i < 2 ? acc0[2 * i] : acc1[2 * i - 4], b = i < 2 ? acc0[2 * i + 1] : acc1[2 * i - 3];
+            s[i] = (any ? a : 0.f) + (first ? b : 0.f);
+            s[i] += __shfl_xor_sync(0xffffffffu, s[i], 1);
+            s[i] += __shfl_xor_sync(0xffffffffu, s[i], 2);
+          }
+          // lane = column of the warp
+          float q = t == 0 ? s[0] : t == 1 ? s[1] : t == 2 ? s[2] : s[3];
+          q *= F16IN ? pow2f(23) : pow2f(20);
+          const int col = (block * NB + cw) * kColsPerWarp + lane;
+          // (fp16 inputs: the reference rounds both parameters to fp16, kernels.h:121-122)
+          const float sc = F16IN ? __half2float(__float2half_rn(par.x)) : par.x;
+          const float nz = F16IN ? __half2float(__float2half_rn(-par.y)) : -par.y;
+          if (col < p.width) atomicAdd(&mul[col], fmaf(sc, q, nz * sumx));
+#pragma unroll
+          for (int i = 0; i < 4; i++) acc0[i] = acc1[i] = 0.f;
+          sumx = 0.f;
+          if (u == u1) return;
+          k = 0;
+          block++;
           par = par_next;
           if ((block + 1) * p.steps < u1) par_next = parameters(block + 1);
         }
+        segment();
       }
-      if (++u >= u1) break;
     }
   }
 }
