@@ -9,10 +9,9 @@
 // Semantics (the host references of the stand-alone benchmarks):
 //  * RMSNorm (rmsnorm-cuda/reference.h:4-25): xn[k] = x[k] * rsqrt(mean(x^2) +
 //    eps) * gamma[k]; skipped when gamma is null.  Computed in fp32, rounded to
-//    fp16 once (the products of the mat-vec are fp16 pairs).
+//    fp16 once.
 //  * mat-vec: as hq_gemv_f16 / hq_gemv_int8_f16 / hq_gemv_int4_f16 (same
-//    layouts, same scale / zero point rules), fp32 accumulation over 32- or
-//    64-weight partial sums.
+//    layouts, same scale / zero point rules), exact products, fp32 sums.
 //  * gated activation: with act != 0 the matrix has 2 * rows_out rows, row 2m the
 //    value row and row 2m + 1 the gate row of output m (the x / gate order of
 //    geglu-cuda/reference.h:8-16, per output feature), and
@@ -21,11 +20,10 @@
 //    in fp32, rounded to fp16 once.  With act == 0 the kernel is the plain
 //    mat-vec (plus the RMSNorm) and writes rows_out results.
 //
-// Design: the row-streaming form of gemv_uniform.cu (two 512-thread CTAs per SM,
+// Design: the row-streaming form of gemv_uniform.cu (gemv_rows.cuh; two 512-thread CTAs per SM,
 // a warp owns a PAIR of adjacent rows - here exactly a value / gate pair -, the
-// input vector piece-major in shared memory, eight 128-bit streaming loads per
-// lane in flight).  The prologue reads the input vector twice from L1/L2 (sum of
-// squares, then scale and stage).
+// input vector in shared memory).  The prologue reads the input vector there twice (sum of
+// squares, then scale and round).
 #include <algorithm>
 
 #include "gemv_rows.cuh"
@@ -44,10 +42,9 @@ struct FusedParams {
   int rows_out, n, act;
 };
 
-// sum over the CTA (all threads get the result); buf holds kWarps floats
+// sum over the CTA (all threads get the result); buf holds kWarps floats and is used once
 __device__ __forceinline__ float block_sum(float v, float* buf, int lane, int warp) {
   v = warp_sum(v);
-  __syncthreads();  // buf may still be read from an earlier use
   if (lane == 0) buf[warp] = v;
   __syncthreads();
   float t = 0.f;
@@ -56,17 +53,15 @@ __device__ __forceinline__ float block_sum(float v, float* buf, int lane, int wa
   return t;
 }
 
-template <int BITS, bool DEALT>
+template <int BITS, bool DEALT, bool RING>
 __global__ void __launch_bounds__(kThreads, 2)
 gemv_fused_kernel(const FusedParams p) {
-  extern __shared__ __align__(16) unsigned char dsm_raw[];  // the inputs
-  __shared__ float s_part[kWarps];
-  __half* xs = reinterpret_cast<__half*>(dsm_raw);
+  extern __shared__ __align__(16) unsigned char dsm_raw[];  // [ring] inputs
+  __shared__ float s_squares[kWarps], s_part[kWarps];
+  __half* xs = reinterpret_cast<__half*>(dsm_raw + (RING ? kRing : 0));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int kPieces = BITS == 16 ? 1 : 16 / BITS;  // 16-byte pieces of inputs per chunk
   const int n = p.n;
   const size_t row_bytes = (size_t)n * BITS / 8;
-  const int chunks = (int)(row_bytes / 16);
   const int rows_mat = p.act ? 2 * p.rows_out : p.rows_out;
 
   // Programmatic dependent launch: nothing that earlier work of the stream may
@@ -74,16 +69,25 @@ gemv_fused_kernel(const FusedParams p) {
   pdl_launch_dependents();
   if (BITS == 4) prefetch_first_rows<DEALT>(p.mat, rows_mat, row_bytes, lane, warp);
   pdl_wait();
+  PairStream<BITS, RING> stream(p.mat, first_row<DEALT>(warp), (int)gridDim.x * kWarps * kRows, rows_mat, n,
+                                dsm_raw + warp * (kDepth * kSlot), lane, 504);
+  const Inputs<BITS, RING> inputs = {p.x, xs, n, tid, 501};
+  inputs.ask();
+  auto gamma = [&](int i) {
+    const uint4* at = reinterpret_cast<const uint4*>(p.gamma) + i;
+    return p.gamma != nullptr && i < n / 8 && HQ_IN_BOUNDS(at, 16, p.gamma, (size_t)n * 2, 503) ? ld_ordered_u4(at)
+                                                                                                : make_uint4(0, 0, 0, 0);
+  };
+  const uint4 first_gamma = gamma(tid);
+  stream.begin();
+  inputs.arrived();
 
   // ---- RMSNorm: sum of squares over the whole vector ----
-  const uint4* xg = reinterpret_cast<const uint4*>(p.x);
-  const uint4* gg = reinterpret_cast<const uint4*>(p.gamma);
   float norm = 1.f;
   if (p.gamma != nullptr) {
     float sq = 0.f;
     for (int i = tid; i < n / 8; i += kThreads) {
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (HQ_IN_BOUNDS(xg + i, 16, p.x, (size_t)n * 2, 501)) v = ld_dependent_u4(xg + i);
+      const uint4 v = inputs.in(i);
       const uint32_t h[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int k = 0; k < 4; k++) {
@@ -91,17 +95,15 @@ gemv_fused_kernel(const FusedParams p) {
         sq = fmaf(f.x, f.x, fmaf(f.y, f.y, sq));
       }
     }
-    sq = block_sum(sq, s_part, lane, warp);
+    sq = block_sum(sq, s_squares, lane, warp);
     norm = rsqrtf(sq / (float)n + p.eps);
   }
-  // ---- scale, round to fp16, stage piece-major; sum of the staged inputs ----
+  // ---- scale, round to fp16; sum of the inputs ----
   float part = 0.f;
   for (int i = tid; i < n / 8; i += kThreads) {
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (HQ_IN_BOUNDS(xg + i, 16, p.x, (size_t)n * 2, 502)) v = ld_dependent_u4(xg + i);
+    uint4 v = inputs.in(i);
     if (p.gamma != nullptr) {
-      uint4 g = make_uint4(0, 0, 0, 0);
-      if (HQ_IN_BOUNDS(gg + i, 16, p.gamma, (size_t)n * 2, 503)) g = ld_ordered_u4(gg + i);
+      const uint4 g = i == tid ? first_gamma : gamma(i);
       uint32_t h[4] = {v.x, v.y, v.z, v.w};
       const uint32_t gh[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
@@ -112,69 +114,25 @@ gemv_fused_kernel(const FusedParams p) {
       }
       v = make_uint4(h[0], h[1], h[2], h[3]);
     }
-    // 16-byte piece q of chunk c goes to [q][c] (int4: in the order of its conversion)
-    reinterpret_cast<uint4*>(xs)[(i % kPieces) * chunks + i / kPieces] = BITS == 4 ? pair_inputs(v) : v;
-    const float2 f0 = __half22float2(u32_as_half2(v.x)), f1 = __half22float2(u32_as_half2(v.y)),
-                 f2 = __half22float2(u32_as_half2(v.z)), f3 = __half22float2(u32_as_half2(v.w));
-    part += ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+    inputs.out(i, v, part);
   }
-  const float sumx = block_sum(part, s_part, lane, warp);  // also: table and inputs complete
+  const float sumx = block_sum(part, s_part, lane, warp);  // also: inputs complete
 
   // ---- row pairs of this warp ----
-  const int warps_total = gridDim.x * kWarps;
-  constexpr int kPerRow = kInFlight / kRows;
-  const size_t mat_bytes = (size_t)rows_mat * row_bytes;
-  (void)mat_bytes;
-  for (long long row0 = first_row<DEALT>(warp); row0 < rows_mat;
-       row0 += (long long)warps_total * kRows) {
-    const unsigned char* src = p.mat + (size_t)row0 * row_bytes;
-    float acc[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; r++) acc[r] = 0.f;
-    for (int c0 = lane; c0 < chunks; c0 += 32 * kPerRow) {
-      uint4 w[kPerRow][kRows];
-#pragma unroll
-      for (int u = 0; u < kPerRow; u++) {
-        const int c = c0 + 32 * u;
-#pragma unroll
-        for (int r = 0; r < kRows; r++) {
-          const unsigned char* at = src + (size_t)r * row_bytes + (size_t)c * 16;
-          w[u][r] = make_uint4(0, 0, 0, 0);  // a row past the end contributes zeros
-          if (c < chunks && row0 + r < rows_mat && HQ_IN_BOUNDS(at, 16, p.mat, mat_bytes, 504))
-            w[u][r] = ld_ordered_stream_u4(at);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kPerRow; u++) {
-        const int c = c0 + 32 * u;
-        if (c < chunks) {
-          float part2[kRows];
-          chunk_dot<BITS, kRows>(w[u], reinterpret_cast<const uint4*>(xs) + c, chunks, part2);
-#pragma unroll
-          for (int r = 0; r < kRows; r++)
-            acc[r] += part2[r];
-        }
-      }
+  stream.run_rows(xs, [&](uint32_t row0, float total) {
+    const float v = BITS == 16 ? total : p.scale * (total - p.zero_point * sumx);
+    if (p.act) {
+      const float gate = __shfl_down_sync(0xffffffffu, v, 4);
+      const uint32_t m = row0 >> 1;  // row0 is even: the value row; row0 + 1 the gate row
+      if (lane == 0 && HQ_IN_BOUNDS(p.out + m, 2, p.out, (size_t)p.rows_out * 2, 506))
+        p.out[m] = __float2half_rn(v * gate_act(gate, p.act));
+    } else {
+      const uint32_t row = row0 + (lane >> 2);
+      if ((lane == 0 || (lane == 4 && row < (uint32_t)rows_mat)) &&
+          HQ_IN_BOUNDS(p.out + row, 2, p.out, (size_t)p.rows_out * 2, 507))
+        p.out[row] = __float2half_rn(v);
     }
-    float val[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; r++) {
-      const float total = warp_sum(acc[r]);
-      val[r] = BITS == 16 ? total : p.scale * (total - p.zero_point * sumx);
-    }
-    if (lane == 0) {
-      if (p.act) {
-        const long long m = row0 >> 1;  // row0 is even: the value row; row0 + 1 the gate row
-        if (HQ_IN_BOUNDS(p.out + m, 2, p.out, (size_t)p.rows_out * 2, 506))
-          p.out[m] = __float2half_rn(val[0] * gate_act(val[1], p.act));
-      } else {
-#pragma unroll
-        for (int r = 0; r < kRows; r++)
-          if (row0 + r < rows_mat && HQ_IN_BOUNDS(p.out + row0 + r, 2, p.out, (size_t)p.rows_out * 2, 507))
-            p.out[row0 + r] = __float2half_rn(val[r]);
-      }
-    }
-  }
+  });
 }
 
 template <int BITS>
@@ -190,14 +148,16 @@ int launch(const FusedParams& prm, hq_stream_t stream) {
   const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
   const Share share = share_rows(rows_mat, (size_t)prm.n * BITS / 8, BITS, false);
   const int grid = share.ctas;
-  const size_t smem = smem_request((size_t)prm.n * 2, grid);
-  auto go = [&](auto dealt) {
-    constexpr auto kern = gemv_fused_kernel<BITS, decltype(dealt)::value>;
+  const bool ring = takes_ring(rows_mat, input_steps<BITS>(prm.n), BITS, input_bytes<BITS>(prm.n), grid);
+  const size_t smem = smem_request((ring ? kRing : 0) + input_bytes<BITS>(prm.n), grid);
+  auto go = [&](auto dealt, auto by_ring) {
+    constexpr auto kern = gemv_fused_kernel<BITS, decltype(dealt)::value, decltype(by_ring)::value>;
     const cudaError_t e = ensure_dynamic_smem<kern>(smem);
     if (e != cudaSuccess) return cuda_status(e);
     return cuda_status(launch_pdl(kern, dim3(grid), dim3(kThreads), smem, (cudaStream_t)stream, prm));
   };
-  return share.dealt ? go(std::true_type()) : go(std::false_type());
+  auto by_ring = [&](auto dealt) { return ring ? go(dealt, std::true_type()) : go(dealt, std::false_type()); };
+  return share.dealt ? by_ring(std::true_type()) : by_ring(std::false_type());
 }
 
 FusedParams base_params(const void* mat, const void* x_half, const void* gamma_half, float eps,
