@@ -76,6 +76,19 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// A chunk's codes and absmax into the registers that hold a stage, if `there`.  The operands are read and
+// written: a load behind a branch is another value than the one it replaces, and where the compiler copied it
+// into place at the loop's end the warp waited for the row it had just asked for (fused 28672 x 4096 21.4 -> 16.3 us, plain 28672 x
+// 8192 27.2 -> 25.8).
+__device__ __forceinline__ void load_in_place(uint4& codes, float& absmax, const void* at, const float* scale, bool there) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %7, 0;\n"
+      " @p ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%5];\n"
+      " @p ld.global.f32 %4, [%6];\n}\n"
+      : "+r"(codes.x), "+r"(codes.y), "+r"(codes.z), "+r"(codes.w), "+f"(absmax)
+      : "l"(at), "l"(scale), "r"((uint32_t)there));
+}
+
 // sum of the 32 products of one 16-byte chunk against 16 half2 inputs
 __device__ __forceinline__ float chunk_dot(const uint4& codes, const uint4 (&xp)[4],
                                            uint32_t lane4) {
@@ -230,7 +243,7 @@ __device__ __forceinline__ void stage_packets(__half* xs, const uint2* ll, long 
 }
 
 // C = chunks (32 codes) per lane per row; D = rows in flight per lane; S warps
-// share a row (ST > 0: compile time, ST == 0: run time), G groups per CTA;
+// share a row (ST > 0: compile time, ST == 0: run time, two or more), G groups per CTA;
 // ALIGNED: every row
 // starts on an absmax block boundary and blocks are a power of two, so the
 // absmax pointer of a lane advances by a constant.  Nothing is divided on the
@@ -241,7 +254,7 @@ __device__ __forceinline__ void stage_packets(__half* xs, const uint2* ll, long 
 // geglu-cuda/reference.h:8-16), see GemvParams; plain fp16 input and output only.
 // LL: packet input and / or packet output (hq_nf4_gemv_f16_ll); the plain
 // instantiations carry none of that code.
-template <int C, int D, int ST, bool ALIGNED, int THREADS, bool FUSE, bool LL>
+template <int C, int D, int ST, bool ALIGNED, int THREADS, bool IN_PLACE, bool FUSE, bool LL>
 __global__ void __launch_bounds__(THREADS, 1)
 nf4_gemv_kernel(const GemvParams p) {
   constexpr int W = THREADS / 32;
@@ -258,6 +271,7 @@ nf4_gemv_kernel(const GemvParams p) {
   if (!p.early_fetch) pdl_wait();
   unsigned char* dsm = dsm_raw + (kLutImm - smem_u32(dsm_raw));
   const int S = ST > 0 ? ST : p.S;
+  const bool kShared = C == 4 ? S > 1 : ST != 1;  // (known to the compiler but for C = 4, which gains nothing)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = warp / S, q = warp - g * S;
   const int G = p.G;
@@ -309,8 +323,11 @@ nf4_gemv_kernel(const GemvParams p) {
       const float* a = ap[i];                                                                   \
       if (!ALIGNED)                                                                             \
         a = p.absmax + (p.cpb_shift >= 0 ? (ci[i] >> p.cpb_shift) : (ci[i] / (uint32_t)p.cpb)); \
-      if (live[i] && HQ_IN_BOUNDS(wp[i], 16, p.B, p.b_bytes, 101) &&                            \
-          HQ_IN_BOUNDS(a, 4, p.absmax, p.absmax_bytes, 102)) {                                  \
+      const bool there = live[i] && HQ_IN_BOUNDS(wp[i], 16, p.B, p.b_bytes, 101) &&             \
+                         HQ_IN_BOUNDS(a, 4, p.absmax, p.absmax_bytes, 102);                     \
+      if (IN_PLACE) {                                                                           \
+        load_in_place(cw[STAGE][i], cs[STAGE][i], wp[i], a, there);                             \
+      } else if (there) {                                                                       \
         cw[STAGE][i] = ld_ordered_stream_u4(wp[i]);                                             \
         cs[STAGE][i] = ld_ordered_f32(a);                                                       \
       }                                                                                         \
@@ -500,7 +517,7 @@ nf4_gemv_kernel(const GemvParams p) {
 #pragma unroll
         for (int i = 0; i < C; i++) acc = fmaf(chunk_dot(cw[d][i], xr[i], lane4), cs[d][i], acc);
         if (j0 + d + D < my_rows) HQ_NF4_LOAD(d)
-        if (S > 1) {
+        if (kShared) {
           part_r[(d * S + q) * 32] = acc;
         } else if (paired) {
           const float total = warp_sum(acc);
@@ -516,7 +533,7 @@ nf4_gemv_kernel(const GemvParams p) {
         }
       }
     }
-    if (S > 1 && paired) {
+    if (kShared && paired) {
       group_barrier(1 + g, S * 32);
       for (int pr = q; 2 * pr < rows_in_round; pr += S) {
         float v = 0.f, gt = 0.f;
@@ -528,7 +545,7 @@ nf4_gemv_kernel(const GemvParams p) {
       }
       n_out += (long long)(D / 2) * row_stride;
       parity ^= 1;
-    } else if (S > 1) {
+    } else if (kShared) {
       group_barrier(1 + g, S * 32);
       for (int d = q; d < rows_in_round; d += S) {
         float v = 0.f;
@@ -1380,7 +1397,7 @@ namespace hq {
 namespace {
 
 // N: rows of the matrix, or (FUSE with a gated activation) pairs of rows
-template <int C, int D, int ST, bool AL, int THREADS, bool FUSE, bool LL>
+template <int C, int D, int ST, bool AL, int THREADS, bool IN_PLACE, bool FUSE, bool LL>
 int launch_gemv(GemvParams& prm, int N, cudaStream_t st) {
   constexpr int W = THREADS / 32;
   const int S = prm.S;
@@ -1407,7 +1424,7 @@ int launch_gemv(GemvParams& prm, int N, cudaStream_t st) {
   if (prm.A_ll != nullptr || (FUSE && prm.gamma != nullptr))
     smem += (size_t)prm.nchunks * 32 * sizeof(__half);
   if (smem > 227 * 1024) return HQ_ERR_TOO_LARGE;
-  constexpr auto kern = nf4_gemv_kernel<C, D, ST, AL, THREADS, FUSE, LL>;
+  constexpr auto kern = nf4_gemv_kernel<C, D, ST, AL, THREADS, IN_PLACE, FUSE, LL>;
   cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
   return cuda_status(launch_pdl(kern, dim3(grid), dim3(THREADS), smem, st, prm));
@@ -1650,16 +1667,36 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
            : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
                              : launch_gemv_mma<false, false>(prm, N, st);
-#define HQ_NF4_GO(C_, D_, ST_, AL_)                                                         \
-  (with_packets                                                                              \
-       ? (pair_packets ? launch_gemv<C_, D_, ST_, AL_, 512, true, true>(prm, units, st)      \
-                       : launch_gemv<C_, D_, ST_, AL_, 512, false, true>(prm, units, st))    \
-       : (fuse != nullptr ? launch_gemv<C_, D_, ST_, AL_, 512, true, false>(prm, units, st)  \
-                          : launch_gemv<C_, D_, ST_, AL_, 512, false, false>(prm, units, st)))
+  // Without the early fetch plain calls, and fused ones of up to 40 Mi weights, keep the loads behind a branch,
+  // whose wait for the input is shorter: plain 4096 x 4096 5.7 us, in place 6.5, 28672 x 4096 16.0 and 16.7; RMSNorm 4096 x
+  // 4096 6.1 and 8.0, 6144 x 4096 7.9 and 9.1, but 8192 x 8192 14.5 and 13.1, 28672 x 4096 21.6 and 18.4.  Packets too.
+  const bool in_place = prm.early_fetch || (fuse != nullptr && (double)N * K > 40e6);
+#define HQ_NF4_GO(C_, D_, ST_, AL_)                                                               \
+  (with_packets                                                                                    \
+       ? (pair_packets ? launch_gemv<C_, D_, ST_, AL_, 512, false, true, true>(prm, units, st)     \
+                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, true>(prm, units, st))   \
+   : fuse != nullptr   ? (in_place ? launch_gemv<C_, D_, ST_, AL_, 512, true, true, false>(prm, units, st)    \
+                                   : launch_gemv<C_, D_, ST_, AL_, 512, false, true, false>(prm, units, st)) \
+   : in_place          ? launch_gemv<C_, D_, ST_, AL_, 512, true, false, false>(prm, units, st)    \
+                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, false>(prm, units, st))
   if (aligned && cols == 4) { prm.S = 2; return HQ_NF4_GO(2, 4, 2, true); }
   int C = cols <= 1 ? 1 : (cols <= 32 ? 2 : 4);
   prm.S = (cols + C - 1) / C;
   if (C == 1) return aligned ? HQ_NF4_GO(1, 4, 1, true) : HQ_NF4_GO(1, 4, 1, false);
+  if (C == 2 && prm.S == 1) return aligned ? HQ_NF4_GO(2, 4, 1, true) : HQ_NF4_GO(2, 4, 1, false);
+  // Fused rows of 4097 to 16384 inputs: the count of warps at compile time, else the loop waits for its
+  // loads (see load_in_place; SwiGLU with RMSNorm 28672 x 8192 39.6 -> 27.9 us, 4096 x 14336 14.3 -> 10.9).
+  if (C == 2 && aligned && fuse != nullptr && !with_packets && in_place) {
+    switch (prm.S) {
+      case 3: return launch_gemv<2, 4, 3, true, 512, true, true, false>(prm, units, st);
+      case 4: return launch_gemv<2, 4, 4, true, 512, true, true, false>(prm, units, st);
+      case 5: return launch_gemv<2, 4, 5, true, 512, true, true, false>(prm, units, st);
+      case 6: return launch_gemv<2, 4, 6, true, 512, true, true, false>(prm, units, st);
+      case 7: return launch_gemv<2, 4, 7, true, 512, true, true, false>(prm, units, st);
+      case 8: return launch_gemv<2, 4, 8, true, 512, true, true, false>(prm, units, st);
+      default: break;
+    }
+  }
   if (C == 2) return aligned ? HQ_NF4_GO(2, 4, 0, true) : HQ_NF4_GO(2, 4, 0, false);
   return aligned ? HQ_NF4_GO(4, 2, 0, true) : HQ_NF4_GO(4, 2, 0, false);
 #undef HQ_NF4_GO
