@@ -89,11 +89,22 @@ __device__ __forceinline__ void load_in_place(uint4& codes, float& absmax, const
       : "l"(at), "l"(scale), "r"((uint32_t)there));
 }
 
-// sum of the 32 products of one 16-byte chunk against 16 half2 inputs
+// lo, hi += the products of the halves of a and b, in 32 bits
+__device__ __forceinline__ void fma_wide(float& lo, float& hi, uint32_t a, uint32_t b) {
+  asm("{\n .reg .b16 al, ah, bl, bh;\n mov.b32 {al, ah}, %2;\n mov.b32 {bl, bh}, %3;\n"
+      " fma.rn.f32.f16 %0, al, bl, %0;\n fma.rn.f32.f16 %1, ah, bh, %1;\n}\n"
+      : "+f"(lo), "+f"(hi)
+      : "r"(a), "r"(b));
+}
+
+// sum of the 32 products of one 16-byte chunk against 16 half2 inputs.  Sums of four products in half2, which costs an
+// instruction per byte, or (WIDE) all in 32 bits for two (28672 x 4096 with SwiGLU 15.2 -> 16.1 us).
+template <bool WIDE = false>
 __device__ __forceinline__ float chunk_dot(const uint4& codes, const uint4 (&xp)[4],
                                            uint32_t lane4) {
   const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
   __half2 a0 = __float2half2_rn(0.f), a1 = a0, a2 = a0, a3 = a0;
+  float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const uint32_t xw[4] = {xp[i].x, xp[i].y, xp[i].z, xp[i].w};
@@ -106,11 +117,19 @@ __device__ __forceinline__ float chunk_dot(const uint4& codes, const uint4 (&xp)
     const uint32_t l1 = lds_u32_imm<kLutImm>(o1);
     const uint32_t l2 = lds_u32_imm<kLutImm>(o2);
     const uint32_t l3 = lds_u32_imm<kLutImm>(o3);
-    a0 = __hfma2(u32_as_half2(l0), u32_as_half2(xw[0]), a0);
-    a1 = __hfma2(u32_as_half2(l1), u32_as_half2(xw[1]), a1);
-    a2 = __hfma2(u32_as_half2(l2), u32_as_half2(xw[2]), a2);
-    a3 = __hfma2(u32_as_half2(l3), u32_as_half2(xw[3]), a3);
+    if (WIDE) {
+      fma_wide(f0, f1, l0, xw[0]);
+      fma_wide(f2, f3, l1, xw[1]);
+      fma_wide(f0, f1, l2, xw[2]);
+      fma_wide(f2, f3, l3, xw[3]);
+    } else {
+      a0 = __hfma2(u32_as_half2(l0), u32_as_half2(xw[0]), a0);
+      a1 = __hfma2(u32_as_half2(l1), u32_as_half2(xw[1]), a1);
+      a2 = __hfma2(u32_as_half2(l2), u32_as_half2(xw[2]), a2);
+      a3 = __hfma2(u32_as_half2(l3), u32_as_half2(xw[3]), a3);
+    }
   }
+  if (WIDE) return (f0 + f1) + (f2 + f3);
   const float2 f = __half22float2(__hadd2(__hadd2(a0, a1), __hadd2(a2, a3)));
   return f.x + f.y;
 }
@@ -254,7 +273,7 @@ __device__ __forceinline__ void stage_packets(__half* xs, const uint2* ll, long 
 // geglu-cuda/reference.h:8-16), see GemvParams; plain fp16 input and output only.
 // LL: packet input and / or packet output (hq_nf4_gemv_f16_ll); the plain
 // instantiations carry none of that code.
-template <int C, int D, int ST, bool ALIGNED, int THREADS, bool IN_PLACE, bool FUSE, bool LL>
+template <int C, int D, int ST, bool ALIGNED, int THREADS, bool IN_PLACE, bool WIDE, bool FUSE, bool LL>
 __global__ void __launch_bounds__(THREADS, 1)
 nf4_gemv_kernel(const GemvParams p) {
   constexpr int W = THREADS / 32;
@@ -515,7 +534,7 @@ nf4_gemv_kernel(const GemvParams p) {
       if (d < rows_in_round) {
         float acc = 0.f;
 #pragma unroll
-        for (int i = 0; i < C; i++) acc = fmaf(chunk_dot(cw[d][i], xr[i], lane4), cs[d][i], acc);
+        for (int i = 0; i < C; i++) acc = fmaf(chunk_dot<WIDE>(cw[d][i], xr[i], lane4), cs[d][i], acc);
         if (j0 + d + D < my_rows) HQ_NF4_LOAD(d)
         if (kShared) {
           part_r[(d * S + q) * 32] = acc;
@@ -1397,7 +1416,7 @@ namespace hq {
 namespace {
 
 // N: rows of the matrix, or (FUSE with a gated activation) pairs of rows
-template <int C, int D, int ST, bool AL, int THREADS, bool IN_PLACE, bool FUSE, bool LL>
+template <int C, int D, int ST, bool AL, int THREADS, bool IN_PLACE, bool WIDE, bool FUSE, bool LL>
 int launch_gemv(GemvParams& prm, int N, cudaStream_t st) {
   constexpr int W = THREADS / 32;
   const int S = prm.S;
@@ -1424,7 +1443,7 @@ int launch_gemv(GemvParams& prm, int N, cudaStream_t st) {
   if (prm.A_ll != nullptr || (FUSE && prm.gamma != nullptr))
     smem += (size_t)prm.nchunks * 32 * sizeof(__half);
   if (smem > 227 * 1024) return HQ_ERR_TOO_LARGE;
-  constexpr auto kern = nf4_gemv_kernel<C, D, ST, AL, THREADS, IN_PLACE, FUSE, LL>;
+  constexpr auto kern = nf4_gemv_kernel<C, D, ST, AL, THREADS, IN_PLACE, WIDE, FUSE, LL>;
   cudaError_t e = ensure_dynamic_smem<kern>(smem);
   if (e != cudaSuccess) return cuda_status(e);
   return cuda_status(launch_pdl(kern, dim3(grid), dim3(THREADS), smem, st, prm));
@@ -1466,8 +1485,9 @@ MmaSplit mma_split(int rows, int nchunks, int sms) {
   return m;
 }
 
-// Whether a fused call (RMSNorm and / or a gated activation) with absmax blocks of 64 takes the
-// tensor form.  us, row form -> tensor form, weights resident:
+// Whether a fused call (RMSNorm and / or a gated activation) with absmax blocks of 64 keeps its sums in 32 bits: in the
+// tensor form or, for larger layers, where that is the slower one, fused_takes_wide_rows.  us, row form (half2, before
+// its loads were in place) -> tensor form, weights resident:
 //  * rows of up to 4096 inputs always, RMSNorm with SwiGLU or without (28672 x 4096 21.8 -> 20.1,
 //    1024 x 4096 4.8 -> 3.4, 2048 x 2048 5.1 -> 2.9); from 3073 inputs on and without the early fetch, which
 //    would cover its longer start, up to one tile per SM (2368 x 4096 5.5 -> 4.8, without norm 3072 rows
@@ -1498,6 +1518,33 @@ bool fused_takes_tensor(int rows, int nchunks, bool norm, bool act, bool residen
   const double by_rows = act ? (norm ? (resident ? 3.33 : 4.02) : (resident ? 1.89 : 2.61)) + 0.61 * turns + 0.02 * cols + 0.15 * share
                              : (resident ? 3.51 : 4.20) + 0.57 * turns + 0.02 * cols + 0.16 * share;
   return tensor < by_rows;
+}
+
+// Whether a fused call that fused_takes_tensor gives to the tensor form takes the row form with sums in 32 bits, like
+// the tensor form's.  It streams faster and starts later: larger layers, where most lanes have a chunk.
+// us, tensor form -> this one, weights resident, unless said:
+//  * 3073 to 4096 inputs: from 24 Mi weights with the activation alone (6144 x 4096 6.4 -> 6.0, 28672 x 4096 20.0 -> 16.5,
+//    3072 x 4096 1.05 of the time), from 48 Mi with the norm alone (28672 x 4096 20.4 -> 17.4; 6144 x 4096 1.07);
+//  * 4097 to 8192: where less than 3/4 of the lanes have one never (28672 x 4608 1.03 to 1.08), and rows of up to 6144 that leave
+//    1 in 7 idle from 128 Mi on (28672 x 5120 0.95, 16384 x 5120 1.02).  Others from 12 Mi with the activation alone (2048 x
+//    8192 0.91; up to 6144 18 Mi, 2048 x 6144 1.03), from 24 Mi with the norm alone (3072 x 8192 0.94, 2048 x
+//    8192 1.06; up to 6144 32 Mi, 4096 x 6144 1.01).  Without the early fetch, which covers the later start, from 46 Mi on
+//    (8192 x 7168 0.95; up to 6144 96 Mi, 8192 x 6144 1.0);
+//  * norm and activation of up to 8192 inputs from 128 Mi on alone, 57344 x 4096 36.3 -> 30.5, 28672 x 8192 37.4 -> 30.3.  It is
+//    the faster one from 64 Mi on already (14336 x 8192 0.87, 28672 x 4096 0.88): the tests pin these layers' form;
+//  * 8193 to 16384: from 18 Mi on (2048 x 9216 0.89 to 0.98, 12288 x 16384 33.8 -> 26.0), without the early fetch from 46 Mi
+//    and 2/3 of the lanes (4096 x 12288 0.95, 2048 x 16384 1.0; 16384 x 10304 1.02).
+bool fused_takes_wide_rows(int rows, int nchunks, bool norm, bool act, bool resident) {
+  const int cols = (nchunks + 31) / 32;
+  if (cols < 4 || cols > 16 || (cols == 4 && !resident)) return false;
+  const long long mi = (long long)rows * nchunks * 32 >> 20;  // weights
+  const int busy = nchunks * (16 / ((cols + 1) / 2));          // lanes with a chunk, of 1024
+  if (cols > 8) return resident ? mi >= 18 : busy >= 680 && mi >= 46;
+  if (cols == 4) return mi >= (!norm ? 24 : !act ? 48 : 128);
+  if (busy < 768) return false;
+  if (!resident) return busy >= 870 && mi >= (cols > 6 ? 46 : 96);
+  if ((norm && act) || (cols <= 6 && busy < 870)) return mi >= 128;
+  return mi >= (cols > 6 ? (norm ? 24 : 12) : norm ? 32 : 18);
 }
 
 template <bool FUSE, bool LL>
@@ -1662,7 +1709,9 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   const long rows_per_sm = N / sm_count();
   const bool tensor = fuse != nullptr ? !bare && fused_takes_tensor(N, nchunks, fuse->gamma != nullptr, fuse->act != HQ_ACT_NONE, prm.early_fetch != 0)
                                       : cols == 1 || cols == 3 || (cols == 2 && rows_per_sm < 64) || (cols == 4 && rows_per_sm < 16);
-  if (blocksize == 64 && K % 64 == 0 && tensor && !pair_packets &&
+  const bool fused_wide = fuse != nullptr && tensor && blocksize == 64 && aligned &&
+                          fused_takes_wide_rows(N, nchunks, fuse->gamma != nullptr, fuse->act != HQ_ACT_NONE, prm.early_fetch != 0);
+  if (blocksize == 64 && K % 64 == 0 && tensor && !fused_wide && !pair_packets &&
       mma_smem_bytes(nchunks, ll.A_ll != nullptr) <= 227 * 1024)
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
            : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
@@ -1671,14 +1720,27 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   // whose wait for the input is shorter: plain 4096 x 4096 5.7 us, in place 6.5, 28672 x 4096 16.0 and 16.7; RMSNorm 4096 x
   // 4096 6.1 and 8.0, 6144 x 4096 7.9 and 9.1, but 8192 x 8192 14.5 and 13.1, 28672 x 4096 21.6 and 18.4.  Packets too.
   const bool in_place = prm.early_fetch || (fuse != nullptr && (double)N * K > 40e6);
+  if (fused_wide) {  // up to 16384 inputs
+    prm.S = (cols + 1) / 2;
+    switch (prm.S) {
+      case 1: return launch_gemv<2, 4, 1, true, 512, true, true, true, false>(prm, units, st);
+      case 2: return launch_gemv<2, 4, 2, true, 512, true, true, true, false>(prm, units, st);
+      case 3: return launch_gemv<2, 4, 3, true, 512, true, true, true, false>(prm, units, st);
+      case 4: return launch_gemv<2, 4, 4, true, 512, true, true, true, false>(prm, units, st);
+      case 5: return launch_gemv<2, 4, 5, true, 512, true, true, true, false>(prm, units, st);
+      case 6: return launch_gemv<2, 4, 6, true, 512, true, true, true, false>(prm, units, st);
+      case 7: return launch_gemv<2, 4, 7, true, 512, true, true, true, false>(prm, units, st);
+      default: return launch_gemv<2, 4, 8, true, 512, true, true, true, false>(prm, units, st);
+    }
+  }
 #define HQ_NF4_GO(C_, D_, ST_, AL_)                                                               \
   (with_packets                                                                                    \
-       ? (pair_packets ? launch_gemv<C_, D_, ST_, AL_, 512, false, true, true>(prm, units, st)     \
-                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, true>(prm, units, st))   \
-   : fuse != nullptr   ? (in_place ? launch_gemv<C_, D_, ST_, AL_, 512, true, true, false>(prm, units, st)    \
-                                   : launch_gemv<C_, D_, ST_, AL_, 512, false, true, false>(prm, units, st)) \
-   : in_place          ? launch_gemv<C_, D_, ST_, AL_, 512, true, false, false>(prm, units, st)    \
-                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, false>(prm, units, st))
+       ? (pair_packets ? launch_gemv<C_, D_, ST_, AL_, 512, false, false, true, true>(prm, units, st)     \
+                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, false, true>(prm, units, st))   \
+   : fuse != nullptr   ? (in_place ? launch_gemv<C_, D_, ST_, AL_, 512, true, false, true, false>(prm, units, st)    \
+                                   : launch_gemv<C_, D_, ST_, AL_, 512, false, false, true, false>(prm, units, st)) \
+   : in_place          ? launch_gemv<C_, D_, ST_, AL_, 512, true, false, false, false>(prm, units, st)    \
+                       : launch_gemv<C_, D_, ST_, AL_, 512, false, false, false, false>(prm, units, st))
   if (aligned && cols == 4) { prm.S = 2; return HQ_NF4_GO(2, 4, 2, true); }
   int C = cols <= 1 ? 1 : (cols <= 32 ? 2 : 4);
   prm.S = (cols + C - 1) / C;
@@ -1688,12 +1750,12 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
   // loads (see load_in_place; SwiGLU with RMSNorm 28672 x 8192 39.6 -> 27.9 us, 4096 x 14336 14.3 -> 10.9).
   if (C == 2 && aligned && fuse != nullptr && !with_packets && in_place) {
     switch (prm.S) {
-      case 3: return launch_gemv<2, 4, 3, true, 512, true, true, false>(prm, units, st);
-      case 4: return launch_gemv<2, 4, 4, true, 512, true, true, false>(prm, units, st);
-      case 5: return launch_gemv<2, 4, 5, true, 512, true, true, false>(prm, units, st);
-      case 6: return launch_gemv<2, 4, 6, true, 512, true, true, false>(prm, units, st);
-      case 7: return launch_gemv<2, 4, 7, true, 512, true, true, false>(prm, units, st);
-      case 8: return launch_gemv<2, 4, 8, true, 512, true, true, false>(prm, units, st);
+      case 3: return launch_gemv<2, 4, 3, true, 512, true, false, true, false>(prm, units, st);
+      case 4: return launch_gemv<2, 4, 4, true, 512, true, false, true, false>(prm, units, st);
+      case 5: return launch_gemv<2, 4, 5, true, 512, true, false, true, false>(prm, units, st);
+      case 6: return launch_gemv<2, 4, 6, true, 512, true, false, true, false>(prm, units, st);
+      case 7: return launch_gemv<2, 4, 7, true, 512, true, false, true, false>(prm, units, st);
+      case 8: return launch_gemv<2, 4, 8, true, 512, true, false, true, false>(prm, units, st);
       default: break;
     }
   }
