@@ -488,11 +488,13 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
       prefetch_l2(bW + ((size_t)(tile * TR + r) * nb_total + b0 + b) * M + begin, (uint32_t)cols * 4u);
   }
   pdl_wait();
-  // the inputs of the first tile: the tables wait for them
-  const int first_k = (int)blockIdx.x / ranges * TR * 32 + tid;
-  float x_first = 0.f;
-  if (tid < TR * 32 && first_k < K && HQ_IN_BOUNDS(x + first_k, 2, x, (size_t)K * 2, 206))
-    x_first = __half2float(ld_dependent_f16(x + first_k));
+  // the inputs of the first tile, which the tables wait for; later each unit's one unit ahead
+  auto input_of = [&](int unit) {  // zero beyond K
+    const int k = unit / ranges * (TR * 32) + tid;
+    return tid < TR * 32 && unit < units && k < K && HQ_IN_BOUNDS(x + k, 2, x, (size_t)K * 2, 206) ? ld_dependent_f16(x + k)
+                                                                                                  : __ushort_as_half(0);
+  };
+  __half x_next = input_of(blockIdx.x);
 
   // ---- the warp's ring ----
   // Step s of a unit is columns m_begin + (s * kWarps + warp) * 32 .. + 31.  The warp asks
@@ -568,14 +570,7 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
     const int row0 = tile * TR, nrows = min(TR, total_rows - row0);
     if (tile != built) {
       built = tile;
-      // ---- the tile's inputs (zero beyond K) ----
-      if (tid < TR * 32) {
-        const int k = row0 * 32 + tid;
-        float v = x_first;
-        if (unit != (int)blockIdx.x)
-          v = (k < K && HQ_IN_BOUNDS(x + k, 2, x, (size_t)K * 2, 206)) ? __half2float(ld_dependent_f16(x + k)) : 0.f;
-        xs[tid] = v;
-      }
+      if (tid < TR * 32) xs[tid] = __half2float(x_next);
       __syncthreads();  // inputs in place, and no warp looks up in the old tables any more
       // ---- tables: thread = (byte value, some of the rows); signed sums of 8 inputs, each
       // stored 8 times.  Line (row pair p, byte b) at lut + p*65536 + b*256, inside
@@ -620,6 +615,7 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
         ones[gi] = o;
       }
     }
+    x_next = input_of(unit + gridDim.x);
 
     // ---- lookups ----
     for (int m0 = m_begin + warp * 32; m0 < m_end; m0 += kWarps * 32) {
