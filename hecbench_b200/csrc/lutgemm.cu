@@ -509,46 +509,56 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
   const size_t alpha_bytes = (size_t)(total_rows / rows_per_group) * nb_total * M * 2;
   const size_t bias_bytes = (size_t)(total_rows / rows_per_group) * M * 2;
   (void)bw_bytes; (void)alpha_bytes; (void)bias_bytes;
-  int f_unit = blockIdx.x, f_m = 0, f_end = 0, f_row0 = 0;  // the next step to ask for
+  // The lane's addresses are worked out once a unit (per step, with a division by the group's rows and
+  // 64-bit products, they were 100 of the 370 instructions a step of three planes took).
+  int f_unit = blockIdx.x, f_m = 0, f_end = 0;  // the next step to ask for: column of the lane's pieces, range's end
+  const uint32_t* words_at[kWordCopies];
+  const __half* params_at[kParamCopies];
+  unsigned live = 0;  // copies that the unit has
   auto enter = [&] {  // f_unit -> its first step of this warp, skipping units without one
     for (; f_unit < units; f_unit += gridDim.x) {
       const int tile = f_unit / ranges, begin = (f_unit - tile * ranges) * cols_per_cta;
-      f_row0 = tile * TR;
-      f_m = begin + warp * 32;
       f_end = min(M, begin + cols_per_cta);
-      if (f_m < f_end) return;
+      if (begin + warp * 32 >= f_end) continue;
+      const int row0 = tile * TR, nrows = min(TR, total_rows - row0), g0 = row0 / rows_per_group;
+      f_m = begin + warp * 32 + seg * 4;
+      live = 0;
+#pragma unroll
+      for (int i = 0; i < kWordCopies; i++) {
+        const int rp = (lane >> 3) + 4 * i, r = rp / NB, b = rp - r * NB;
+        words_at[i] = bW + ((size_t)(row0 + r) * nb_total + b0 + b) * M + f_m;
+        if (rp < TR * NB && r < nrows) live |= 1u << i;
+      }
+#pragma unroll
+      for (int i = 0; i < kParamCopies; i++) {
+        const int gb = (lane >> 3) + 4 * i, gi = gb / (NB + 1), b = gb - gi * (NB + 1);
+        params_at[i] = b < NB ? alpha + ((size_t)(g0 + gi) * nb_total + b0 + b) * M + f_m : q_bias + (size_t)(g0 + gi) * M + f_m;
+        if (gi < kGroups && gi * RPG < nrows && (b < NB || q_bias != nullptr)) live |= 256u << i;
+      }
+      return;
     }
   };
+  const uint32_t words_to = (lane >> 3) * 128 + seg * 16, params_to = L::kWordBytes + (lane >> 3) * 64 + seg * 8;
   auto fetch = [&](uint32_t stage) {
     if (f_unit < units) {
-      const int nrows = min(TR, total_rows - f_row0), m = f_m + seg * 4;
-      if (m < f_end) {
-        const uint32_t* src = bW + ((size_t)f_row0 * nb_total + b0) * M + m;
+      const bool inside = f_m < f_end;
 #pragma unroll
-        for (int i = 0; i < kWordCopies; i++) {
-          const int rp = (lane >> 3) + 4 * i, r = rp / NB, b = rp - r * NB;
-          const uint32_t* at = src + (size_t)(r * nb_total + b) * M;
-          if (rp < TR * NB && r < nrows && HQ_IN_BOUNDS(at, 16, bW, bw_bytes, 201))
-            cp_async_16(stage + rp * 128 + seg * 16, at);
-        }
-        const int g0 = f_row0 / rows_per_group;
+      for (int i = 0; i < kWordCopies; i++) {
+        if (inside && (live >> i & 1) && HQ_IN_BOUNDS(words_at[i], 16, bW, bw_bytes, 201))
+          cp_async_16(stage + words_to + i * 512, words_at[i]);
+        words_at[i] += kWarps * 32;
+      }
 #pragma unroll
-        for (int i = 0; i < kParamCopies; i++) {
-          const int gb = (lane >> 3) + 4 * i, gi = gb / (NB + 1), b = gb - gi * (NB + 1);
-          const uint32_t dst = stage + L::kWordBytes + gb * 64 + seg * 8;
-          if (gi < kGroups && gi * RPG < nrows) {
-            if (b < NB) {
-              const __half* at = alpha + ((size_t)(g0 + gi) * nb_total + b0 + b) * M + m;
-              if (HQ_IN_BOUNDS(at, 8, alpha, alpha_bytes, 202)) cp_async_8(dst, at);
-            } else if (q_bias != nullptr) {
-              const __half* at = q_bias + (size_t)(g0 + gi) * M + m;
-              if (HQ_IN_BOUNDS(at, 8, q_bias, bias_bytes, 203)) cp_async_8(dst, at);
-            }
-          }
-        }
+      for (int i = 0; i < kParamCopies; i++) {
+        const bool scale = ((lane >> 3) + 4 * i) % (NB + 1) < NB;
+        (void)scale;
+        if (inside && (live >> (8 + i) & 1) &&
+            HQ_IN_BOUNDS(params_at[i], 8, scale ? alpha : q_bias, scale ? alpha_bytes : bias_bytes, scale ? 202 : 203))
+          cp_async_8(stage + params_to + i * 256, params_at[i]);
+        params_at[i] += kWarps * 32;
       }
       f_m += kWarps * 32;
-      if (f_m >= f_end) {
+      if (f_m - seg * 4 >= f_end) {
         f_unit += gridDim.x;
         enter();
       }
