@@ -421,8 +421,11 @@ __device__ __forceinline__ void red_add_f32(float* addr, float v) {
 // reads of the words took as many shared-memory wavefronts as the look-ups (4.1 M at 12288 x 12288, 3
 // planes, 60 % of the time); a lane's own column also needs no sum over lanes and a quarter of the
 // products with the scales.  us of a call among others, quads -> own columns: 12288 x 12288, 3 planes 27.5 -> 23.8, 4 planes
-// 32.7 -> 27.7; 4096 x 12288, 4 planes 17.9 -> 15.3; 4096 x 4096, 4 planes 8.4 -> 8.0.  What bounds it is shared
-// memory still: the look-ups, and the tables of a tile (eight copies of 1024 sums for each column range).
+// 32.7 -> 27.7; with the copies' addresses per unit and the inputs a unit ahead 20.4 and 25.4.  What bounds it: the
+// end (3.5 us: fence, counters, conversion of a range by one CTA), the look-ups (5 us of issue and shared memory), the
+// tables of a tile (eight copies of 1024 sums for each column range); without words and look-ups 12288 x 12288 still took
+// 15.5 of 24.5 us before the addresses were moved.  On mma.sync instead of look-ups (bits in place as bytes, inputs as
+// digits of 4 bits) 29.7 us: the s8 form takes 15 cycles per scheduler for 16 x 32 weights, the e4m3 form 24.
 // Words from global memory straight into registers do not take this division: a lane's 4-byte loads
 // are too short for HBM's latency (12288 x 12288, 1 plane 19.2 -> 24.8, 2 planes with groups of 64 26.0 -> 31.9).
 constexpr int kRingThreads = 512;
@@ -1018,16 +1021,18 @@ template <int TR, int RPG>
 int launch_planes(const LaunchArgs& a) {
   constexpr bool kFour = TR == 2 || RPG > 1;  // groups of 32 inputs: the rings hold three planes
   // The rings take over where a warp has some column steps: us, register form -> rings, at steps per warp
-  // 3 planes: 1.3 (12288 x 1024) 7.3 -> 7.6, 1.7 (4096 x 4096) 7.8 -> 7.4, 3.5 (8192 x 4096) 10.4 -> 9.6;
-  // 2 planes: 2.6 (12288 x 2048) 7.9 -> 8.2, 3.5 8.9 -> 8.85, 15.6 (12288 x 12288) 23.3 -> 21.3; with groups of
-  // 64, 3.5 9.6 -> 9.9, 6.9 (8192 x 8192) 14.1 -> 14.0, 15.6 26.0 -> 24.4;
-  // 1 plane: 3.9 (3072 x 12288) 8.9 -> 9.4, 5.2 (4096 x 12288) 10.6 -> 10.3, 15.6 19.2 -> 18.2.
+  // 3 planes: 1.3 (12288 x 1024) 7.2 -> 7.5, 1.5 (6400 x 2304) 7.8 -> 7.4, 1.7 (4096 x 4096) 7.9 -> 7.4, 3.5 (8192 x 4096)
+  // 10.6 -> 8.9;
+  // 2 planes: 1.7 7.0 -> 7.2, 2.6 (12288 x 2048) 7.9 -> 7.8, 2.7 (5120 x 5120) 8.5 -> 7.7, with groups of 64 9.4 -> 8.1, 5.2
+  // (4096 x 12288) 12.9 -> 10.4;
+  // 1 plane: 2.7 6.8 -> 7.0, 3.5 7.1 -> 7.3, 3.9 (3072 x 12288) 8.7 -> 8.2, 5.2 10.2 -> 8.9; with groups of 64, 2.6 7.1 -> 7.2,
+  // 2.7 7.5 -> 7.0, 5.2 11.5 -> 9.3.
   // Groups of 32 inputs: as before, three planes in long units.
   const double steps = (double)a.M * a.grid.y / ((double)kRingThreads * sm_count());
   auto takes_ring = [&](int n) {
     if (TR != 4) return false;
     if (RPG == 1) return n == 3 && a.cols_per_cta >= 2 * kRingThreads && (long long)a.grid.x * a.grid.y > sm_count();
-    return n == 4 || steps >= (n == 3 ? 1.5 : n == 1 ? 5.0 : RPG == 4 ? 3.3 : 6.0);
+    return n == 4 || steps >= (n == 3 ? 1.5 : n == 1 && RPG == 4 ? 3.6 : 2.65);
   };
   const int nb = a.nb_total;
   for (int b0 = 0; b0 < nb;) {
