@@ -55,13 +55,14 @@ inline size_t smem_request(size_t need, int grid) {
 //    From the fourth round on 4-bit rows do that up to half full, when one CTA of each SM has a pair per warp
 //    more (32000 x 4096 17.1 and 17.6, 41000 x 2048 13.4 and 14.3); rows of up to 512 bytes from the fifth
 //    (32000 x 1024 gains 3 %, 41000 x 1024 loses 6; up to 1 KiB 33000 x 2048 gains 3), 8-bit and fp16 rows never
-// (41000 x 2048 gain 3 and 2 %).    In the third round a third full is still few for plain 4-bit rows whose batches
-// of 2 KiB are whole or    nearly so (22016 x 4096 12.8 and 13.4, x 8192 23.6 and 24.8; x 2048 9.7 and 9.2, x 6144
-// 22.2 and 20.0). A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and
-// so does a division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9 for
-// 12.9): each is a kernel of its own.  (Figures of this comment: fp16 multiply-adds, loads into registers.)  The
-// plain 8-bit kernel alone is the faster one with parameters (28672 x 2048 12.64 us, 12.9 without, 10000 x 1024 4.66
-// and 4.78; pairs one by one the same).
+//    (41000 x 2048 gain 3 and 2 %).  In the third round a third full is still few for plain 4-bit rows whose
+//    batches of 2 KiB are whole or nearly so (22016 x 4096 12.8 and 13.4, x 8192 23.6 and 24.8; x 2048 9.7 and
+//    9.2, x 6144 22.2 and 20.0).
+// A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and so does a
+// division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9 for
+// 12.9): each is a kernel of its own.  The plain 8-bit kernel alone is the faster one with parameters (28672 x
+// 2048 12.64 us, 12.9 without, 10000 x 1024 4.66 and 4.78; pairs one by one the same).  (Figures of this
+// comment: fp16 multiply-adds, loads into registers.)
 struct Share {
   int ctas;
   bool dealt;
