@@ -679,12 +679,23 @@ lutgemm_ring_kernel(const uint32_t* bW, const __half* alpha,
     if (!flags[range]) continue;
     __threadfence();
     const int lo = per_range ? range * cols_per_cta : 0, hi_m = per_range ? min(M, lo + cols_per_cta) : M;
-    for (int mm = lo + tid * 4; mm < hi_m; mm += kThreads * 4) {
-      if (!HQ_IN_BOUNDS(out + mm, 8, out, (size_t)M * 2, 205)) continue;
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(ws + mm));
-      const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
-      *reinterpret_cast<uint2*>(out + mm) = make_uint2(half2_as_u32(h01), half2_as_u32(h23));
-      *reinterpret_cast<float4*>(ws + mm) = make_float4(0.f, 0.f, 0.f, 0.f);
+    // all of a thread's sums of 4096 columns are asked for before the first is used
+    constexpr int kAtOnce = 2;
+    for (int m0 = lo + tid * 4; m0 < hi_m; m0 += kAtOnce * kThreads * 4) {
+      float4 v[kAtOnce];
+#pragma unroll
+      for (int i = 0; i < kAtOnce; i++) {
+        const int mm = m0 + i * kThreads * 4;
+        if (mm < hi_m && HQ_IN_BOUNDS(ws + mm, 16, ws, (size_t)M * 4, 204)) v[i] = __ldcg(reinterpret_cast<const float4*>(ws + mm));
+      }
+#pragma unroll
+      for (int i = 0; i < kAtOnce; i++) {
+        const int mm = m0 + i * kThreads * 4;
+        if (mm >= hi_m || !HQ_IN_BOUNDS(out + mm, 8, out, (size_t)M * 2, 205)) continue;
+        const __half2 h01 = __floats2half2_rn(v[i].x, v[i].y), h23 = __floats2half2_rn(v[i].z, v[i].w);
+        *reinterpret_cast<uint2*>(out + mm) = make_uint2(half2_as_u32(h01), half2_as_u32(h23));
+        *reinterpret_cast<float4*>(ws + mm) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
     if (tid == 0) counters[range] = 0u;
   }
