@@ -421,8 +421,8 @@ __device__ __forceinline__ void red_add_f32(float* addr, float v) {
 // reads of the words took as many shared-memory wavefronts as the look-ups (4.1 M at 12288 x 12288, 3
 // planes, 60 % of the time); a lane's own column also needs no sum over lanes and a quarter of the
 // products with the scales.  us of a call among others, quads -> own columns: 12288 x 12288, 3 planes 27.5 -> 23.8, 4 planes
-// 32.7 -> 27.7; with the copies' addresses per unit and the inputs a unit ahead 20.4 and 25.4.  What bounds it: the
-// end (3.5 us: fence, counters, conversion of a range by one CTA), the look-ups (5 us of issue and shared memory), the
+// 32.7 -> 27.7; with the copies' addresses per unit and the inputs a unit ahead 20.2 and 25.2.  What bounds it: the
+// end (3 us: fence, counters, conversion of a range by one CTA), the look-ups (5 us of issue and shared memory), the
 // tables of a tile (eight copies of 1024 sums for each column range); without words and look-ups 12288 x 12288 still took
 // 15.5 of 24.5 us before the addresses were moved.  On mma.sync instead of look-ups (bits in place as bytes, inputs as
 // digits of 4 bits) 29.7 us: the s8 form takes 15 cycles per scheduler for 16 x 32 weights, the e4m3 form 24.
