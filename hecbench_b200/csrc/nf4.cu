@@ -97,6 +97,16 @@ __device__ __forceinline__ void fma_wide(float& lo, float& hi, uint32_t a, uint3
       : "r"(a), "r"(b));
 }
 
+// acc += a chunk's sum times its absmax, if the lane has the chunk: beyond a row's end codes and inputs are zero, and
+// a level 0 that no fp16 number holds times zero is no number.  Predicated: 0.2 % over 590 layers; a select after
+// the sum too, up to 3 % of single ones; zeros to look up beside the table took loops their registers (8192 x 8192
+// 9.6 -> 11.9 us).
+__device__ __forceinline__ void add_chunk(float& acc, float sum, float absmax, bool there) {
+  asm("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p fma.rn.f32 %0, %1, %2, %0;\n}\n"
+      : "+f"(acc)
+      : "f"(sum), "f"(absmax), "r"((uint32_t)there));
+}
+
 // sum of the 32 products of one 16-byte chunk against 16 half2 inputs.  Sums of four products in half2, which costs an
 // instruction per byte, or (WIDE) all in 32 bits for two (28672 x 4096 with SwiGLU 15.2 -> 16.1 us).
 template <bool WIDE = false>
@@ -534,7 +544,7 @@ nf4_gemv_kernel(const GemvParams p) {
       if (d < rows_in_round) {
         float acc = 0.f;
 #pragma unroll
-        for (int i = 0; i < C; i++) acc = fmaf(chunk_dot<WIDE>(cw[d][i], xr[i], lane4), cs[d][i], acc);
+        for (int i = 0; i < C; i++) add_chunk(acc, chunk_dot<WIDE>(cw[d][i], xr[i], lane4), cs[d][i], live[i]);
         if (j0 + d + D < my_rows) HQ_NF4_LOAD(d)
         if (kShared) {
           part_r[(d * S + q) * 32] = acc;

@@ -85,3 +85,37 @@ def test_wide_rows_hold_sums_beyond_fp16(hq, dev, rows, n, act):
         v = v[0::2] * v[1::2] * torch.sigmoid(v[1::2])
     tol = 2.0**-11 + (2.2 * n * 2.0**-24 + 2.0**-20 if act else n * 2.0**-24 + 2.0**-11)
     assert bool(((y[:len(v)].double() - v).abs() <= tol * v).all())
+
+
+@pytest.mark.parametrize("rows,n,norm,act,resident,bs", [
+    # 32-bit sums
+    (14339, 3520, 1, 0, True, 64), (3586, 5632, 0, 1, True, 64), (2050, 6208, 0, 1, True, 64), (2290, 8256, 1, 1, True, 64),
+    (4097, 12352, 1, 0, False, 64),
+    # half2: fused, plain, loads behind a branch, rows that begin inside an absmax block, four chunks per lane
+    (1021, 10304, 1, 0, True, 64), (333, 4160, 0, 0, True, 64), (333, 4160, 0, 0, False, 64), (333, 1376, 0, 0, True, 128),
+    (37, 33792, 0, 0, True, 64)])
+def test_infinite_level_beside_idle_lanes(hq, dev, rows, n, norm, act, resident, bs):
+    """Level 0 is one that no fp16 number holds, and lanes beyond the row's end hold its code: rows without
+    it have the value that a finite level 0 gives, bit for bit; one such code makes its row infinite."""
+    import torch
+    g = torch.Generator(device=dev).manual_seed(rows + n)
+    x = torch.randn(n, generator=g, device=dev).half()
+    codes = torch.randint(1, 16, (rows, n), generator=g, device=dev)
+    codes[::3, 5] = 0
+    mat = (codes[:, 0::2] << 4 | codes[:, 1::2]).to(torch.uint8)
+    absmax = (torch.rand(-(-rows * n // bs), generator=g, device=dev) + 0.5) / n ** 0.5
+    gamma = (torch.rand(n, generator=g, device=dev) + 0.5).half() if norm else None
+    got = []
+    for level in (-1.0, -1e30):
+        lut = torch.linspace(-1, 1, 16, device=dev)
+        lut[0] = level
+        got.append(hq.gemv_fused("nf4", x, mat, rows // 2, gamma=gamma, act=act, absmax=absmax, lut16=lut, weights_resident=resident)
+                   if act else
+                   hq.gemv_fused("nf4", x, mat, rows, gamma=gamma, absmax=absmax, lut16=lut, weights_resident=resident)
+                   if norm else hq.gemv_nf4(x, mat, absmax, lut, rows, n, bs, weights_resident=resident))
+    hit = (codes == 0).any(1)
+    if act:
+        hit = hit.view(-1, 2).any(1)
+    assert torch.equal(got[1][~hit], got[0][~hit]) and bool(got[0].isfinite().all())
+    if not act:
+        assert bool((got[1][hit] == (float("-inf") if x[5] > 0 else float("inf"))).all())
