@@ -466,10 +466,11 @@ nf4_gemv_kernel(const GemvParams p) {
     cp_async_wait_all();
   }
   __syncthreads();
-  if (FUSE && p.gamma != nullptr) {
+  if (FUSE && p.gamma != nullptr && g < G) {  // (warps left over by S = 3, 5, 6, 7 have no rows)
     // the S warps of a group hold the whole vector between them
     float tot = 0.f;
-    for (int t = 0; t < S; t++) tot += s_sq[g * S + t];
+    for (int t = 0; t < S; t++)
+      tot += HQ_IN_BOUNDS(s_sq + g * S + t, 4, s_sq, sizeof(s_sq), 107) ? s_sq[g * S + t] : 0.f;
     const float norm = rsqrtf(tot / (float)(p.nchunks * 32) + p.eps);
 #pragma unroll
     for (int i = 0; i < C; i++) {
@@ -1726,7 +1727,7 @@ static int nf4_gemv_impl(const void* A_half, const uint8_t* B, const float* absm
     return with_packets      ? launch_gemv_mma<false, true>(prm, N, st)
            : fuse != nullptr ? launch_gemv_mma<true, false>(prm, N, st)
                              : launch_gemv_mma<false, false>(prm, N, st);
-  // Without the early fetch plain calls, and fused ones of up to 40 Mi weights, keep the loads behind a branch,
+  // Without the early fetch plain calls, and fused ones of up to 40 million weights, keep the loads behind a branch,
   // whose wait for the input is shorter: plain 4096 x 4096 5.7 us, in place 6.5, 28672 x 4096 16.0 and 16.7; RMSNorm 4096 x
   // 4096 6.1 and 8.0, 6144 x 4096 7.9 and 9.1, but 8192 x 8192 14.5 and 13.1, 28672 x 4096 21.6 and 18.4.  Packets too.
   const bool in_place = prm.early_fetch || (fuse != nullptr && (double)N * K > 40e6);

@@ -85,3 +85,27 @@ def test_kquantize_and_vllm_quant_checked(hq, oracle, dev, checked):
     hq.dynamic_scaled_int8_quant(q, x, x.shape[1], x.shape[0], sc, None)
     assert np.array_equal(q.cpu().numpy(), gv["dyn_float16"])
     assert _violations(checked)[0] == 0
+
+
+@pytest.mark.parametrize("rows,n,act", [(14339, 3520, 0), (5803, 6144, 0), (1021, 10240, 0), (2051, 10304, 0), (1531, 12352, 0),
+                                        (1022, 16384, 1)])
+def test_fused_nf4_rows_checked(hq, dev, checked, rows, n, act):
+    """RMSNorm in the row form, 2, 3, 5, 6, 7 and 8 warps per row: 3, 5, 6 and 7 leave some of sixteen over."""
+    import torch
+    from launches import launched
+    g = torch.Generator(device=dev).manual_seed(rows + n)
+    x = torch.randn(n, generator=g, device=dev).half()
+    gamma = (torch.rand(n, generator=g, device=dev) + 0.5).half()
+    mat = torch.randint(0, 256, (rows, n // 2), generator=g, device=dev, dtype=torch.uint8)
+    absmax = (torch.rand((rows, n // 64), generator=g, device=dev) + 0.5) / n ** 0.5
+    lut = torch.arange(-8, 8, device=dev).float() / 8
+    y = []
+    ((name, _),) = launched(lambda: y.append(hq.gemv_fused(
+        "nf4", x, mat, rows // 2 if act else rows, gamma=gamma, act=act, absmax=absmax.view(-1), lut16=lut, weights_resident=True)))
+    assert "nf4_gemv_kernel" in name
+    w = lut[torch.stack([mat.long() >> 4, mat.long() & 15], 2)].view(rows, n).double() * absmax.double().repeat_interleave(64, 1)
+    v = w @ (x.double() * torch.rsqrt((x.double() ** 2).mean() + 1e-5) * gamma.double())
+    if act:
+        v = v[0::2] * v[1::2] * torch.sigmoid(v[1::2])
+    assert float((y[0].double() - v).norm() / v.norm()) < TOL_F16
+    assert _violations(checked)[0] == 0, _violations(checked)
