@@ -84,6 +84,12 @@ inline Share share_rows(int rows, size_t row_bytes, int bits, bool plain) {
   if (in_blocks) return {std::min(blocks, 2 * sms), false};
   return {ctas, true};
 }
+// Shared memory that a launch of the ring takes besides its inputs, the kernels' static arrays among it; CTAs that fit
+// an SM (228 KiB, one of them reserved per CTA).
+inline bool ring_fits(size_t input_bytes, int ctas_per_sm) {
+  const size_t need = kRing + input_bytes + 128;
+  return need <= 227 * 1024 && ctas_per_sm * (need + 1024) <= 228 * 1024;
+}
 // Whether the rows come through the ring or into registers, eight loads per lane at a time: where it fits, from
 // two rounds of pairs on (its requests run on across the ends of rows), 8-bit ones from the first whole round, and
 // for rows of more than four steps, 4-bit ones of more than eight where a CTA has an SM for itself (few warps: a
@@ -92,10 +98,21 @@ inline Share share_rows(int rows, size_t row_bytes, int bits, bool plain) {
 // x 8192 10.2 -> 9.8, 4096 x 14336 10.0 -> 8.2; int8: 7268 x 1600 4.8 -> 5.4, 11124 x 1664 7.9 -> 7.3, 16000 x 2048
 // 8.1 -> 8.3, 41000 x 2048 16.7 -> 16.1, 4096 x 4096 6.3 -> 4.9, 1024 x 16384 14.7 -> 8.5; fp16: 9000 x 1024 4.9 ->
 // 5.8, 1024 x 4096 6.1 -> 4.1.
-inline bool takes_ring(int rows, int steps, int bits, size_t input_bytes, int ctas) {
-  const int pairs = rows / kRows + (rows % kRows != 0), rounds = pairs / kWarps / ctas;  // whole ones
-  const bool alone = bits == 4 && ctas <= sm_count();
-  return kRing + input_bytes <= 227 * 1024 - 128 && (rounds >= (bits == 8 ? 1 : 2) || steps > (alone ? 8 : 4));
+// Where one CTA of the ring fits an SM and two of the registers' form do, a CTA per SM takes the ring, pairs dealt one by one
+// (two per SM and the ring would be two waves): int4 8192 x 28672 25.8 -> 21.3, two waves 25.3, with RMSNorm and SwiGLU
+// 29.6, 24.4 and 29.1; int8 39.1, 38.6 and 39.5, 41.7, 40.7 and 44.5.  8 and 16 bits with up to 1.4 or 1.5 pairs per warp, whose
+// second turn is nearly empty, keep two CTAs and the registers (int8 5120 x 27648 26.7 and 30.7, fp16 5072 x 33536 55.8 and 71).
+inline bool takes_ring(int rows, int steps, int bits, size_t input_bytes, Share* share) {
+  if (!ring_fits(input_bytes, 1)) return false;
+  const int pairs = rows / kRows + (rows % kRows != 0), sms = sm_count();
+  if (pairs > sms * kWarps && !ring_fits(input_bytes, 2)) {
+    if (bits != 4 && pairs < (bits == 8 ? 1.4 : 1.5) * sms * kWarps) return false;
+    *share = {sms, true};
+    return true;
+  }
+  const int rounds = pairs / kWarps / share->ctas;  // whole ones
+  const bool alone = bits == 4 && share->ctas <= sms;
+  return rounds >= (bits == 8 ? 1 : 2) || steps > (alone ? 8 : 4);
 }
 template <bool DEALT>
 __device__ __forceinline__ long long first_row(int warp) {

@@ -85,9 +85,9 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   if (rows <= 0 || n <= 0 || n % (128 / BITS) != 0) return HQ_ERR_BAD_SHAPE;
   if (!aligned16(mat) || !aligned16(vec_half)) return HQ_ERR_MISALIGNED;
   if ((size_t)n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
-  const Share share = share_rows(rows, (size_t)n * BITS / 8, BITS, true);
+  Share share = share_rows(rows, (size_t)n * BITS / 8, BITS, true);
+  const bool ring = takes_ring(rows, input_steps<BITS>(n), BITS, input_bytes<BITS>(n), &share);
   const int grid = share.ctas;
-  const bool ring = takes_ring(rows, input_steps<BITS>(n), BITS, input_bytes<BITS>(n), grid);
   const size_t smem = smem_request((ring ? kRing : 0) + input_bytes<BITS>(n), grid);
   // the launcher of the reference rounds both parameters to fp16 (gemv.cu:21-22)
   const float s = __half2float(__float2half_rn(scale));

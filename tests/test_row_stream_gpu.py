@@ -52,6 +52,26 @@ def test_rows_by_ring_and_registers(hq, dev, bits, rows, steps, more, ring):
         assert ("Lb1EE" if form else "Lb0EE") in name
 
 
+# the longest inputs beside which two rings fit an SM and the shortest beside which one does; rows just beyond a pair per
+# warp, and the fewest of 8 and 16 bits that one CTA per SM takes by ring
+@pytest.mark.parametrize("bits,n,per_warp,one", [(4, 24576, 1.0, None), (4, 24608, 1.0, True), (4, 57344, 2.0, True),
+                                                 (8, 24592, 1.0, False), (8, 24592, 1.4, True), (16, 25096, 1.0, False),
+                                                 (16, 25096, 1.5, True)])
+def test_one_ring_per_sm(hq, dev, bits, n, per_warp, one):
+    """Where the ring leaves an SM room for one CTA, as many are launched as there are SMs, or two of the register form."""
+    import torch
+    from launches import launched
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    rows = 2 * int(per_warp * 16 * sms + 1)
+    mat, w, x = _layer(bits, rows, n, dev)
+    want = w @ x.double()
+    finite = want.abs() < 65504
+    for call in _calls(hq, bits, mat, x, rows):
+        assert torch.equal(call().double()[finite], want.half().double()[finite])
+        ((name, blocks),) = launched(call)
+        assert ("Lb1EE" in name) == (one is not False) and blocks == (sms if one else 2 * sms)
+
+
 @pytest.mark.parametrize("bits,n", [(16, 60032), (8, 90112), (4, 115712)])
 def test_rows_too_long_for_the_ring(hq, dev, bits, n):
     """Inputs that leave the ring no room come from registers, up to the longest vector that the calls take."""
