@@ -61,8 +61,9 @@ inline size_t smem_request(size_t need, int grid) {
 // A share of consecutive pairs per CTA took registers that the loops need (8 bits 1.05 to 1.1), and so does a
 // division that comes as a parameter (int4 in blocks, 4736 x 8192 7.2 us for 7.0, 22016 x 4096 13.9 for
 // 12.9): each is a kernel of its own.  The plain 8-bit kernel alone is the faster one with parameters (28672 x
-// 2048 12.64 us, 12.9 without, 10000 x 1024 4.66 and 4.78; pairs one by one the same).  (Figures of this
-// comment: fp16 multiply-adds, loads into registers.)
+// 2048 12.64 us, 12.9 without, 10000 x 1024 4.66 and 4.78; pairs one by one the same).
+// (Figures of this comment: fp16 multiply-adds, loads into registers.  With the present forms, 1650 layers in graphs: these
+// lines take 0.2 to 0.3 % more than the better division of each layer, always one by one 0.2 to 0.5, always blocks 8 to 10.)
 struct Share {
   int ctas;
   bool dealt;
@@ -132,6 +133,17 @@ __device__ __forceinline__ void prefetch_first_rows(const unsigned char* mat, in
   const long long row = first_row<DEALT>(warp) + lane;
   if (row_bytes <= 4096 && lane < kRows && row < rows)
     prefetch_l2(mat + (size_t)row * row_bytes, (uint32_t)row_bytes);
+}
+
+// 16 bytes into the registers of v, if `there`.  Behind a branch the value is another than the one it replaces, and
+// the compiler waited for loads of a turn before it asked for the next (8 bits 1.03 -> 0.86 of the time of fp16
+// multiply-adds over 530 layers).
+__device__ __forceinline__ void load_in_place(uint4& v, const void* at, bool there) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n"
+      " @p ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n}\n"
+      : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+      : "l"(at), "r"((uint32_t)there));
 }
 
 // 16 bytes from global to shared memory; zeros where there are none
@@ -321,7 +333,8 @@ __device__ __forceinline__ void chunk_mma(const uint4 (&w)[kRows], const uint4* 
 // run_rows() multiplies and calls finish(row0, total), see PairSums::total.
 // RING: 512 bytes of each row at a time come by cp.async, up to four such pieces ahead, across the ends of
 // the rows and from before the inputs are staged; every lane reads what it copied itself.  Else eight 16-byte
-// loads per lane and turn.
+// loads per lane and turn, or (fp16, few registers besides them) each piece's next loads behind its product (fused rows
+// 1.05 -> 0.92 of the time of fp16 multiply-adds over 190 layers; plain ones 0.93 -> 0.92; 4 and 8 bits spill).
 template <int BITS, bool RING>
 struct PairStream {
   const unsigned char* mat;
@@ -400,26 +413,40 @@ struct PairStream {
       }
     } else {
       constexpr int kPerRow = 4;
+      constexpr bool kTurns = BITS == 16;
       for (; row0 < rows; row0 += stride) {
         const unsigned char* src = mat + (size_t)row0 * row_bytes;
         PairSums<BITS> sums;
         sums.clear();
-        for (int s0 = 0; s0 < steps; s0 += kPerRow) {
-          uint4 w[kPerRow][kRows];
+        uint4 w[kPerRow][kRows];
+        auto load = [&](int u, int s) {
+          const int c = s * 32 + lane;
 #pragma unroll
-          for (int u = 0; u < kPerRow; u++) {
-            const int c = (s0 + u) * 32 + lane;
-#pragma unroll
-            for (int r = 0; r < kRows; r++) {
-              const unsigned char* at = src + (size_t)r * row_bytes + (size_t)c * 16;
-              w[u][r] = make_uint4(0, 0, 0, 0);  // a row past the end contributes zeros
-              if (c < chunks && row0 + r < rows && in_matrix(at)) w[u][r] = ld_ordered_stream_u4(at);
+          for (int r = 0; r < kRows; r++) {
+            const unsigned char* at = src + (size_t)r * row_bytes + (size_t)c * 16;
+            const bool there = c < chunks && row0 + r < rows && in_matrix(at);
+            w[u][r] = make_uint4(0, 0, 0, 0);  // a row past the end contributes zeros
+            if constexpr (BITS == 4) {
+              if (there) w[u][r] = ld_ordered_stream_u4(at);
+            } else {
+              load_in_place(w[u][r], at, there);
             }
+          }
+        };
+        if (kTurns) {
+#pragma unroll
+          for (int u = 0; u < kPerRow; u++) load(u, u);
+        }
+        for (int s0 = 0; s0 < steps; s0 += kPerRow) {
+          if (!kTurns) {
+#pragma unroll
+            for (int u = 0; u < kPerRow; u++) load(u, s0 + u);
           }
 #pragma unroll
           for (int u = 0; u < kPerRow; u++) {
             if (s0 + u >= steps) break;
             chunk_mma<BITS, RING>(w[u], x0 + (s0 + u) * (kStepBytes<BITS> / 16), first, sums);
+            if (kTurns && s0 + u + kPerRow < steps) load(u, s0 + u + kPerRow);
           }
         }
         finish(row0, sums.total(lane));
