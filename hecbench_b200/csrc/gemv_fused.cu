@@ -147,7 +147,7 @@ int launch(const FusedParams& prm, hq_stream_t stream) {
   if ((size_t)prm.n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;
   const int rows_mat = prm.act ? 2 * prm.rows_out : prm.rows_out;
   Share share = share_rows(rows_mat, (size_t)prm.n * BITS / 8, BITS, false);
-  const bool ring = takes_ring(rows_mat, input_steps<BITS>(prm.n), BITS, input_bytes<BITS>(prm.n), &share);
+  const bool ring = takes_ring(rows_mat, input_steps<BITS>(prm.n), BITS, input_bytes<BITS>(prm.n), false, &share);
   const int grid = share.ctas;
   const size_t smem = smem_request((ring ? kRing : 0) + input_bytes<BITS>(prm.n), grid);
   auto go = [&](auto dealt, auto by_ring) {

@@ -6,11 +6,10 @@
 // What bounds it: HBM, and for 4 bits the logic pipe (five operations of two cycles for eight weights).  us in
 // graphs, fp16 multiply-adds with eight loads per lane -> this form (with RMSNorm and SwiGLU): int4 8192 x 8192 11.9
 // -> 9.8 (13.5 -> 11.0), 28672 x 4096 15.6 -> 13.3 (16.8 -> 14.9), 4096 x 14336 11.8 -> 8.2 (12.9 -> 9.7), 4096 x
-// 4096 4.0 -> 3.3 (4.7 -> 4.1); int8 8192 x 8192 14.4 -> 13.4 (15.7 -> 13.3), 28672 x 4096 21.6 -> 21.0 (22.9 ->
-// 20.1), 4096 x 14336 15.2 -> 11.7 (17.3 -> 13.2), 1024 x 16384 12.9 -> 8.5; fp16 8192 x 8192 22.6 -> 22.5 (24.1 ->
-// 25.0), 4096 x 4096 8.7 -> 7.3.  Over 280 layers of 512 to 49152 rows and 1024 to 16384 inputs 0.86, worst 1.11
-// (fp16 10962 x 1600 8.3 -> 9.1).  Sums of 32 to 64 products were rounded to fp16; now products are exact and sums
-// fp32.
+// 4096 4.5 -> 3.9 (5.2 -> 4.7); int8 8192 x 8192 14.3 -> 13.8 (15.7 -> 13.3), 28672 x 4096 21.6 -> 21.2 (22.8 ->
+// 19.9), 4096 x 14336 15.2 -> 11.7 (17.3 -> 13.2), 1024 x 16384 13.0 -> 8.4; fp16 8192 x 8192 22.5 -> 22.8 (24.0 ->
+// 23.9), 4096 x 4096 8.5 -> 7.3, 10962 x 1600 8.4 -> 8.1.  Sums of 32 to 64 products were rounded to fp16; now products
+// are exact and sums fp32.
 #ifndef HQ_GEMV_ROWS_CUH_
 #define HQ_GEMV_ROWS_CUH_
 #include <limits.h>
@@ -91,29 +90,49 @@ inline bool ring_fits(size_t input_bytes, int ctas_per_sm) {
   const size_t need = kRing + input_bytes + 128;
   return need <= 227 * 1024 && ctas_per_sm * (need + 1024) <= 228 * 1024;
 }
-// Whether the rows come through the ring or into registers, eight loads per lane at a time: where it fits, from
-// two rounds of pairs on (its requests run on across the ends of rows), 8-bit ones from the first whole round, and
-// for rows of more than four steps, 4-bit ones of more than eight where a CTA has an SM for itself (few warps: a
-// step of the ring waits for its own copies and products).  us in graphs, registers -> ring, int4: 4096 x 4096 3.3
-// -> 4.2, 4096 x 8192 5.6 -> 6.2, 16000 x 2048 5.5 -> 6.3, 22016 x 4096 12.2 -> 10.3, 49152 x 1024 9.8 -> 7.9, 8192
-// x 8192 10.2 -> 9.8, 4096 x 14336 10.0 -> 8.2; int8: 7268 x 1600 4.8 -> 5.4, 11124 x 1664 7.9 -> 7.3, 16000 x 2048
-// 8.1 -> 8.3, 41000 x 2048 16.7 -> 16.1, 4096 x 4096 6.3 -> 4.9, 1024 x 16384 14.7 -> 8.5; fp16: 9000 x 1024 4.9 ->
-// 5.8, 1024 x 4096 6.1 -> 4.1.
-// Where one CTA of the ring fits an SM and two of the registers' form do, a CTA per SM takes the ring, pairs dealt one by one
-// (two per SM and the ring would be two waves): int4 8192 x 28672 25.8 -> 21.3, two waves 25.3, with RMSNorm and SwiGLU
-// 29.6, 24.4 and 29.1; int8 39.1, 38.6 and 39.5, 41.7, 40.7 and 44.5.  8 and 16 bits with up to 1.4 or 1.5 pairs per warp, whose
-// second turn is nearly empty, keep two CTAs and the registers (int8 5120 x 27648 26.7 and 30.7, fp16 5072 x 33536 55.8 and 71).
-inline bool takes_ring(int rows, int steps, int bits, size_t input_bytes, Share* share) {
+// Whether the rows come through the ring or into registers, eight loads per lane at a time.  us in graphs, weights from
+// HBM, registers -> ring, "fused" with RMSNorm and SwiGLU:
+//  * where one CTA of the ring fits an SM and two of the registers' form do, a CTA per SM takes the ring, pairs dealt one by one
+//    (two per SM and the ring would be two waves): int4 8192 x 28672 25.8 -> 21.3, two waves 25.3, fused 29.6, 24.4 and 29.1;
+//    int8 39.1, 38.6 and 39.5, fused 41.7, 40.7 and 44.5.  8 and 16 bits with up to 1.4 or 1.5 pairs per warp, whose second
+//    turn is nearly empty, keep two CTAs and the registers (int8 5120 x 27648 26.7 and 30.7, fp16 5072 x 33536 55.8 and 71);
+//  * with one CTA per SM the ring, whose first weights are asked for before the inputs are staged: int4 1024 x 4096 3.0 -> 2.6,
+//    fused 1024 x 2048 3.4 -> 2.7, int8 768 x 1152 2.42 -> 2.35, 1024 x 16384 9.8 -> 8.4, fp16 1024 x 4096 5.2 -> 4.5.
+//    Not plain int4 rows of one or two steps in up to four pairs per SM (1030 x 1024 1.86 -> 2.00), nor those of three and four in
+//    blocks (4096 x 4096 3.87 -> 4.10).  Up to 1.1 pairs per SM, too few for lines of their own, the lines
+//    of before: rows of more than four steps, 4 bits of eight (the ring would take 0.84 to 0.91 of the time over 250 layers of
+//    32 to 600 rows, 1.03 at most);
+//  * with two, 4 bits: rows of more than four steps, or two whole rounds of pairs (its requests run on across the ends of
+//    rows; 49152 x 1024 9.8 -> 8.2, 22016 x 4096 12.3 -> 10.6, 8192 x 2048 3.75 -> 4.3, 16000 x 2048 5.6 -> 5.9);
+//  * 8 bits: rows of more than four steps (28672 x 4096 fused 21.3 -> 19.9), or some whole rounds (15142 x 512 fused 5.1 ->
+//    4.5, 49152 x 1024 11.35 -> 10.8; 16000 x 2048 7.6 -> 8.0, 41000 x 2048 15.3 -> 16.4);
+//  * 16 bits: the registers where rounds are many or the last one is full, their loads following one another as closely
+//    (10962 x 1600 8.1 -> 9.2, 28672 x 4096 fused 38.0 -> 39.9, 8192 x 8192 fused 23.7 -> 25.3; 12288 x 4096 17.9 -> 17.2, fused
+//    12288 x 2176 11.8 -> 10.9, 22528 x 1280 11.1 -> 10.7, 9000 x 1024 4.94 -> 4.60).
+// Over 1345 layers of 512 to 57344 rows and 1024 to 57344 inputs 0.82 of the time of the fp16 multiply-adds, worst 1.03 (fp16
+// 9396 x 8064 24.2 -> 25.0).
+inline bool takes_ring(int rows, int steps, int bits, size_t input_bytes, bool plain, Share* share) {
   if (!ring_fits(input_bytes, 1)) return false;
   const int pairs = rows / kRows + (rows % kRows != 0), sms = sm_count();
-  if (pairs > sms * kWarps && !ring_fits(input_bytes, 2)) {
+  const bool two = pairs > sms * kWarps;  // CTAs per SM
+  if (two && !ring_fits(input_bytes, 2)) {
     if (bits != 4 && pairs < (bits == 8 ? 1.4 : 1.5) * sms * kWarps) return false;
     *share = {sms, true};
     return true;
   }
-  const int rounds = pairs / kWarps / share->ctas;  // whole ones
-  const bool alone = bits == 4 && share->ctas <= sms;
-  return rounds >= (bits == 8 ? 1 : 2) || steps > (alone ? 8 : 4);
+  if (!two) {
+    if (pairs <= 1.1 * sms) return steps > (bits == 4 ? 8 : 4);
+    if (bits != 4 || !plain || steps > 4) return true;
+    return steps > 2 ? share->dealt : pairs > 4 * sms;
+  }
+  const double rounds = pairs / (2.0 * sms * kWarps);
+  const int whole = (int)rounds;
+  if (bits == 4) return steps > 4 || whole >= 2;
+  if (bits == 8) return steps > 4 || whole >= (steps > 3 ? 5 : plain || steps <= 2 ? 1 : 2);
+  if (steps <= 4) return plain || whole >= 2;
+  if (plain) return share->dealt && rounds < (steps <= 6 ? 2.5 : 1.4);
+  if (!share->dealt) return steps <= 6 ? whole >= 2 : whole < 3;
+  return rounds - whole < 0.4 && (steps <= 6 ? whole >= 2 : whole == 1);
 }
 template <bool DEALT>
 __device__ __forceinline__ long long first_row(int warp) {

@@ -86,7 +86,7 @@ int launch(const void* mat, const void* vec_half, void* res_half, int rows, int 
   if (!aligned16(mat) || !aligned16(vec_half)) return HQ_ERR_MISALIGNED;
   if ((size_t)n * 2 > 226 * 1024) return HQ_ERR_TOO_LARGE;  // beyond 113 KiB only one CTA fits an SM
   Share share = share_rows(rows, (size_t)n * BITS / 8, BITS, true);
-  const bool ring = takes_ring(rows, input_steps<BITS>(n), BITS, input_bytes<BITS>(n), &share);
+  const bool ring = takes_ring(rows, input_steps<BITS>(n), BITS, input_bytes<BITS>(n), true, &share);
   const int grid = share.ctas;
   const size_t smem = smem_request((ring ? kRing : 0) + input_bytes<BITS>(n), grid);
   // the launcher of the reference rounds both parameters to fp16 (gemv.cu:21-22)

@@ -72,6 +72,21 @@ def test_one_ring_per_sm(hq, dev, bits, n, per_warp, one):
         assert ("Lb1EE" in name) == (one is not False) and blocks == (sms if one else 2 * sms)
 
 
+@pytest.mark.parametrize("n", [1280, 1800, 2048, 2056, 4096])
+def test_fp16_rows_from_registers(hq, dev, n):
+    """Layers whose last round of pairs is nearly full: each piece's next loads follow its product, to a row's end inside,
+    at and behind a turn of four steps."""
+    import torch
+    from launches import launched
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    rows = 2 * int(31 * sms) + 1
+    mat, w, x = _layer(16, rows, n, dev)
+    call = _calls(hq, 16, mat, x, rows)[1]
+    assert torch.equal(call(), (w @ x.double()).half())
+    ((name, _),) = launched(call)
+    assert "Lb0EE" in name
+
+
 @pytest.mark.parametrize("bits,n", [(16, 60032), (8, 90112), (4, 115712)])
 def test_rows_too_long_for_the_ring(hq, dev, bits, n):
     """Inputs that leave the ring no room come from registers, up to the longest vector that the calls take."""
