@@ -11,7 +11,8 @@
 //    as they are and six windows of them (kPair).  Inputs are pre-scaled by the matching powers of two.
 //  * An input is split into bf16 pieces by truncation, two for fp16, three for fp32, which hold it
 //    exactly; piece i is column i of B, so both input types cost the same and every product is exact.
-//    fp32 inputs are scaled by the largest exponent of their 128 (a quad of groups).
+//    fp32 inputs are scaled by the largest exponent of their 128 (a quad of groups); their sums are held as
+//    2^-8 of their value, so only what is below 2^-118 loses bits on the way.
 //  * The affine part is factored: sum (s*q - z)*x = s*sum(q*x) - z*sum(x).
 //  * A warp owns 32 columns and takes four groups (a quad) at a time: lane (g, t) multiplies
 //    columns 4g .. 4g + 3 of group t.  NB warps side by side, W / NB in turn along K.
@@ -252,7 +253,7 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
         for (int r = 0; r < 4; r++) m = max(m, __float_as_uint(x[r]) & 0x7fffffffu);
         e = max(0, (int)(__reduce_max_sync(0xffffffffu, m) >> 23) - 126);  // all of them below 2^e
       }
-      if (lane == 0) sums[i] = make_float2(sum, F16IN ? 1.f : pow2f(e - 13));
+      if (lane == 0) sums[i] = make_float2(sum, F16IN ? 1.f : pow2f(min(e, 128) - 1));  // (129: an infinity, or no number)
       const int top = F16IN ? 110 : 126 - e;
       const float slo = pow2f(top - plo), shi = pow2f(top - phi);
       unsigned char* const quad = table + (size_t)i * kQuadBytes<F16IN> + (j & 3) * 4;
@@ -339,7 +340,7 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
           }
           // lane = column of the warp
           float q = t == 0 ? s[0] : t == 1 ? s[1] : t == 2 ? s[2] : s[3];
-          q *= F16IN ? pow2f(23) : pow2f(20);
+          q *= F16IN ? pow2f(23) : pow2f(8);
           const int col = (block * NB + cw) * kColsPerWarp + lane;
           // (fp16 inputs: the reference rounds both parameters to fp16, kernels.h:121-122)
           const float sc = F16IN ? __half2float(__float2half_rn(par.x)) : par.x;

@@ -40,20 +40,27 @@ def test_divisions(hq, dev, N, K, half):
     assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24 + want.abs() * 2.0 ** -22 + 2.0 ** -22).all())
 
 
-@pytest.mark.parametrize("exponent", [-110, -60, -1, 0, 60, 110])
-def test_fp32_inputs_of_any_exponent(hq, dev, exponent):
+@pytest.mark.parametrize("exponent,K", [(-123, 2048), (-110, 2048), (-60, 2048), (-1, 2048), (0, 2048), (60, 2048), (110, 2048),
+                                        (-123, 32), (0, 32), (118, 32)])
+def test_fp32_inputs_of_any_exponent(hq, dev, exponent, K):
     """Inputs are split exactly and scaled by their largest exponent: the bound above holds for tiny and huge
-    ones, also beside ones of another size (every 256 inputs 2^-20 of the others)."""
+    ones, also beside ones of another size (every 256 inputs 2^-20 of the others, single ones 2^-12).  The sums are
+    held as 2^-8 of their value: below 2^-118 an addition may lose 2^-142, a quantum of fp32 times 2^8.  (Large scales
+    with small inputs: an atomic addition takes what is below 2^-126 for zero.)"""
     import torch
-    N, K = 516, 2048
+    N = 516
     g, mat, scales, zeros, codes = _layer(hq, dev, N, K)
-    x = torch.randn(K, generator=g, device=dev) * 2.0 ** exponent
+    scales, zeros = (v * 2.0 ** (16 if exponent < 0 else 0) for v in (scales, zeros))
+    x = torch.randn(K, generator=g, device=dev).abs() * 2.0 ** exponent
     x[256:512] *= 2.0 ** -20
-    out = torch.zeros(N, device=dev)
-    hq.vecquant3matmul(x, mat, out, scales, zeros, K * 3 // 32, N)
-    want = scales.double() * (x.double() @ codes) - zeros.double() * x.double().sum()
-    size = scales.double() * (x.double().abs() @ codes) + zeros.double() * x.double().abs().sum()
-    assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24).all())
+    x[5::37] *= 2.0 ** -12
+    for x in (x, x * torch.randint(0, 2, (K,), generator=g, device=dev).mul(2).sub(1)):
+        out = torch.zeros(N, device=dev)
+        hq.vecquant3matmul(x, mat, out, scales, zeros, K * 3 // 32, N)
+        want = scales.double() * (x.double() @ codes) - zeros.double() * x.double().sum()
+        size = scales.double() * (x.double().abs() @ codes) + zeros.double() * x.double().abs().sum()
+        bound = size * K * 2.0 ** -24 + scales.double() * (K // 16 + 8) * 2.0 ** -142 + (K // 128 + 1) * 2.0 ** -126
+        assert bool(((out.double() - want).abs() <= bound).all())
 
 
 @pytest.mark.parametrize("half", [True, False])
