@@ -17,15 +17,17 @@
 //  * A warp owns 32 columns and takes four groups (a quad) at a time: lane (g, t) multiplies
 //    columns 4g .. 4g + 3 of group t.  NB warps side by side, W / NB in turn along K.
 //  * One CTA per SM takes an equal range of (block of 32 NB columns, quads) steps; sums go to mul
-//    (the reference API accumulates into it) once per range and block, one atomicAdd per column.
+//    (the reference API accumulates into it) once per range and block, an atomicAdd per column from each of
+//    the W / NB warps along K.
 //  * Words come by cp.async, two quads ahead per warp, eight lanes to a 128-byte line: with a quarter-warp
 //    over four lines a read of 226 MB took 57 us, with whole lines 35 (the copy rate).
 //
 // What bounds it: the logic pipe (two cycles an operation, 22 of them for 32 weights), 56 %, and HBM.
 // us in replayed graphs, sums of fp16 products in registers, a group ahead (before) -> this
-// form, fp16 (fp32) inputs: 49152 x 12288 50.3 -> 40.9 (72.7 -> 41.9), 28672 x 8192 24.5 -> 18.3 (30.3 -> 18.7), 8192 x
-// 8192 9.8 -> 7.4 (11.3 -> 7.6), 4096 x 4096 3.8 -> 3.2 (4.3 -> 3.2), 1024 x 4096 3.3 -> 2.4 (2.9 -> 2.4), 512 x
-// 1024 2.4 -> 1.8 (2.1 -> 1.8); 300 layers of 512 to 49152 columns, 1024 to 16384 inputs 0.78, worst 1.07 (768 x 9408).
+// form, fp16 (fp32) inputs, words from HBM: 49152 x 12288 50.4 -> 40.6 (73.0 -> 41.7), 28672 x 8192 24.7 -> 18.2 (30.5 -> 18.6),
+// 8192 x 8192 9.9 -> 7.4 (11.5 -> 7.7), 4096 x 4096 4.0 -> 3.8 (4.9 -> 3.8), 1024 x 4096 3.5 -> 2.7 (3.2 -> 2.7), 512 x
+// 1024 2.3 -> 1.9 (2.3 -> 1.8); 499 layers of 512 to 32768 columns, 1024 to 16384 inputs 0.81, 8 of them above 1.02, worst 1.10
+// (fp16 4644 x 1984 2.80 -> 3.08).
 // Error against fp64 sums: 5e-4 to 1.1e-3 -> 1e-7 to 2.5e-7 (fp32 inputs 1e-7 to 5.7e-7 -> 1e-7 to 2.1e-7).
 // Taken back: windows by multiplications on the other pipe (49152 x 12288 45.1 -> 54.6).
 #include <limits.h>
@@ -448,9 +450,14 @@ int q3_gemv_launch(const void* vec, const int32_t* mat, float* mul, const float*
   const int n16 = narrow(16), n20 = narrow(20);
   const long long l16 = longest(16, 16 >> n16), l20 = longest(20, 20 >> n20);
   const bool wide = 20 * l20 <= 16 * l16;
-  // Layers of up to half a step for every SM start sooner with 8 warps (512 x 1024, graphs, 2.5 -> 2.0 us).
-  const long long u8 = (long long)((width + 255) / 256) * p.slice_quads;
-  if (2 * u8 <= slots) return q3_gemv_go<F16IN, 8, 8>(vec, mat, mul, scales, zeros, p, slices, stream);
+  // 8 warps start sooner, and a layer of few steps, a step being W / 8 of theirs, wastes less of its last one: us
+  // in graphs, words from HBM, 16 or 20 warps -> 8, at steps of 8 of 0.2 (512 x 1024) 2.5 -> 1.9, 1.7 (1408 x 5440,
+  // fp32) 2.93 -> 2.89, 2.4 (4096 x 4096, fp32) 4.05 -> 3.80, 2.5 (11148 x 1088, fp32) 4.00 -> 3.57, 2.9 (1808 x 6784, fp32)
+  // 4.00 -> 3.44, 4.5 (4096 x 5376) 4.76 -> 4.43.  One step of 20 warps is the better at 2 to 2.5 (1.05); with more than five
+  // steps too few words are on their way (1.02 to 1.06 up to seven, then 1.2).
+  const long long l8 = longest(8, 8);
+  if (l8 <= 5 && 8 * l8 <= min(16 * l16, 20 * l20))
+    return q3_gemv_go<F16IN, 8, 8>(vec, mat, mul, scales, zeros, p, slices, stream);
   switch (wide ? 3 + n20 : n16) {
     case 0: return q3_gemv_go<F16IN, 16, 16>(vec, mat, mul, scales, zeros, p, slices, stream);
     case 1: return q3_gemv_go<F16IN, 16, 8>(vec, mat, mul, scales, zeros, p, slices, stream);

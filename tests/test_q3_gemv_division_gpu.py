@@ -5,10 +5,13 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# N, K, at 148 SMs: 8 warps; 16 warps, one step; 20 warps (11008: ranges of four steps); 16 warps, eight
-# side by side (4100 columns of 33 quads); two slices of K, the second of them shorter
-SIZES = [(4, 32), (260, 160), (512, 1024), (3200, 3040), (8804, 1280), (5116, 4288), (11008, 4096), (4100, 4160),
-         (516, 16416), (1028, 33024)]
+# warps of a CTA, those of them side by side (at 148 SMs), columns, inputs: ranges of one step, of several and into the next block;
+# more than 16384 inputs are two slices of K
+FORMS = [(8, 8, 4, 32), (8, 8, 260, 160), (8, 8, 512, 1024), (8, 8, 5116, 4288), (8, 8, 4100, 4160),
+         (16, 16, 1612, 13632), (16, 16, 804, 26144), (16, 8, 1548, 15136), (16, 8, 3308, 16448),
+         (16, 4, 572, 14016), (16, 4, 1544, 16800),
+         (20, 20, 3200, 3040), (20, 20, 8804, 1280), (20, 20, 11008, 4096), (20, 20, 516, 16416), (20, 20, 1028, 33024),
+         (20, 10, 944, 10752), (20, 10, 820, 11424), (20, 10, 264, 24736), (20, 5, 684, 13344), (20, 5, 2312, 19008)]
 
 
 def _layer(hq, dev, N, K):
@@ -22,22 +25,28 @@ def _layer(hq, dev, N, K):
 
 
 @pytest.mark.parametrize("half", [True, False])
-@pytest.mark.parametrize("N,K", SIZES)
-def test_divisions(hq, dev, N, K, half):
+@pytest.mark.parametrize("warps,beside,N,K", FORMS)
+def test_divisions(hq, dev, warps, beside, N, K, half):
     """Products are exact, so what differs from fp64 is the order of fp32 sums: K * 2^-24 of the sum of
-    the products' magnitudes at most, whatever the inputs' exponents (here 2^-8 to 2^8)."""
+    the products' magnitudes at most, whatever the inputs' exponents (here 2^-8 to 2^8).  Inputs of one sign too: a piece
+    of theirs that went missing would be 2^-9 of them (the third of fp32 inputs 2^-17, seen with the fewest inputs)."""
     import torch
+    from launches import launched
     g, mat, scales, zeros, codes = _layer(hq, dev, N, K)
     x = torch.randn(K, generator=g, device=dev) * torch.exp2(torch.randint(-8, 9, (K,), generator=g, device=dev).float())
-    x = x.half() if half else x
     call = hq.vecquant3matmul_faster if half else hq.vecquant3matmul
     s, z = (scales.half().double(), zeros.half().double()) if half else (scales.double(), zeros.double())
     start = torch.randn(N, generator=g, device=dev)
-    out = start.clone()
-    call(x, mat, out, scales, zeros, K * 3 // 32, N)
-    want = start.double() + s * (x.double() @ codes) - z * x.double().sum()
-    size = s * (x.double().abs() @ codes) + z * x.double().abs().sum()
-    assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24 + want.abs() * 2.0 ** -22 + 2.0 ** -22).all())
+    for x in (x, x.abs()):
+        x = x.half() if half else x
+        out = start.clone()
+        call(x, mat, out, scales, zeros, K * 3 // 32, N)
+        want = start.double() + s * (x.double() @ codes) - z * x.double().sum()
+        size = s * (x.double().abs() @ codes) + z * x.double().abs().sum()
+        assert bool(((out.double() - want).abs() <= size * K * 2.0 ** -24 + want.abs() * 2.0 ** -22 + 2.0 ** -22).all())
+    ((name, _),) = launched(lambda: call(x, mat, out, scales, zeros, K * 3 // 32, N))
+    if torch.cuda.get_device_properties(dev).multi_processor_count == 148:
+        assert f"q3_gemv_kernelILb{int(half)}ELi{warps}ELi{beside}EE" in name, name
 
 
 @pytest.mark.parametrize("exponent,K", [(-123, 2048), (-110, 2048), (-60, 2048), (-1, 2048), (0, 2048), (60, 2048), (110, 2048),
