@@ -156,6 +156,11 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
   unsigned char* const table = smem_raw + W * kDepth * kSlot;
   float2* const sums = reinterpret_cast<float2*>(table + (size_t)p.staged * KW * kQuadBytes<F16IN>);
 
+  // extents of the caller's buffers, used only by the index-checked build
+  const size_t mat_bytes = (size_t)p.groups * 3 * p.width * 4, vec_bytes = (size_t)p.groups * 32 * (F16IN ? 2 : 4);
+  const size_t column_bytes = (size_t)p.width * 4;
+  (void)mat_bytes; (void)vec_bytes; (void)column_bytes;
+
   pdl_launch_dependents();
   // The lines of the first steps on their way to L2 while the kernel before drains, where a CTA has three
   // steps or more (8192 x 8192 8.2 -> 7.4 us, 12288 x 16384 17.5 -> 16.3; one step, 1184 x 6976, 2.6 -> 3.0).
@@ -163,8 +168,10 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
 #pragma unroll
     for (int d = 0; d < kDepth - 1; d++) {
       const int row = (q_lo + (k0 + d) * KW) * 12 + tid, col = b0 * NB * kColsPerWarp;
-      if (k0 + d < p.steps && tid < 12 * KW && row < g_hi * 3)
-        prefetch_l2(mat + (size_t)row * p.width + col, (uint32_t)min(NB * kColsPerWarp, p.width - col) * 4u);
+      const uint32_t bytes = (uint32_t)min(NB * kColsPerWarp, p.width - col) * 4u;
+      if (k0 + d < p.steps && tid < 12 * KW && row < g_hi * 3 &&
+          HQ_IN_BOUNDS(mat + (size_t)row * p.width + col, bytes, mat, mat_bytes, 1101))
+        prefetch_l2(mat + (size_t)row * p.width + col, bytes);
     }
   }
   pdl_wait();
@@ -189,7 +196,8 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
   aim();
   auto request = [&](int slot) {
     const uint32_t dst = ring_in + slot * kSlot;
-    if (rows_left > 0) {
+    if (rows_left > 0 && HQ_IN_BOUNDS(src, 16, mat, mat_bytes, 1102) &&
+        HQ_IN_BOUNDS(src + 2 * row, 16, mat, mat_bytes, 1103)) {
       copy_16(dst, src);
       copy_16(dst + 512, src + row);
       copy_16(dst + 1024, src + 2 * row);
@@ -206,7 +214,7 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
   float2 par = make_float2(0.f, 0.f), par_next = par;
   auto parameters = [&](int of) {
     const int col = (of * NB + cw) * kColsPerWarp + lane;
-    if (col >= p.width) return make_float2(0.f, 0.f);
+    if (col >= p.width || !HQ_IN_BOUNDS(scales + col, 4, scales, column_bytes, 1104)) return make_float2(0.f, 0.f);
     const float s = ld_ordered_f32(scales + col);
     return make_float2(s, ld_ordered_f32(zeros + col));
   };
@@ -229,6 +237,9 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
         raw[2 * h] = raw[2 * h + 1] = (In)0.f;
         if (i < staged * KW && group + 2 * h < g_hi) {
           const size_t at = (size_t)(group + 2 * h) * 32;
+          if (!HQ_IN_BOUNDS(mine_lo + at, sizeof(In), vec, vec_bytes, 1105) ||
+              !HQ_IN_BOUNDS(mine_hi + at, sizeof(In), vec, vec_bytes, 1106))
+            continue;
           if constexpr (F16IN) {
             raw[2 * h] = ld_dependent_f16(mine_lo + at);
             raw[2 * h + 1] = ld_dependent_f16(mine_hi + at);
@@ -347,7 +358,7 @@ q3_gemv_kernel(const void* vec, const int32_t* mat, float* mul, const float* sca
           // (fp16 inputs: the reference rounds both parameters to fp16, kernels.h:121-122)
           const float sc = F16IN ? __half2float(__float2half_rn(par.x)) : par.x;
           const float nz = F16IN ? __half2float(__float2half_rn(-par.y)) : -par.y;
-          if (col < p.width) atomicAdd(&mul[col], fmaf(sc, q, nz * sumx));
+          if (col < p.width && HQ_IN_BOUNDS(mul + col, 4, mul, column_bytes, 1107)) atomicAdd(&mul[col], fmaf(sc, q, nz * sumx));
 #pragma unroll
           for (int i = 0; i < 4; i++) acc0[i] = acc1[i] = 0.f;
           sumx = 0.f;

@@ -109,3 +109,40 @@ def test_fused_nf4_rows_checked(hq, dev, checked, rows, n, act):
         v = v[0::2] * v[1::2] * torch.sigmoid(v[1::2])
     assert float((y[0].double() - v).norm() / v.norm()) < TOL_F16
     assert _violations(checked)[0] == 0, _violations(checked)
+
+
+# every division of the kernel, a quad, a block and a second slice of K that are not full
+@pytest.mark.parametrize("half", [True, False])
+@pytest.mark.parametrize("N,K", [(4, 32), (260, 160), (732, 864), (5116, 4288), (3200, 3040), (572, 14016), (820, 11424), (684, 13344),
+                                 (516, 16416), (3308, 16448), (804, 26144)])
+def test_q3_gemv_checked(hq, dev, checked, N, K, half):
+    import torch
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    mat = torch.randint(-2**31, 2**31, (K * 3 // 32, N), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    scales = torch.rand(N, generator=g, device=dev) * 0.01 + 0.001
+    x = torch.randn(K, generator=g, device=dev)
+    codes = hq.vecquant3_dequant(mat, torch.ones(N, device=dev), torch.zeros(N, device=dev), K * 3 // 32, N)
+    out = torch.zeros(N, device=dev)
+    (hq.vecquant3matmul_faster if half else hq.vecquant3matmul)(x.half() if half else x, mat, out, scales, scales, K * 3 // 32, N)
+    want = scales.double() * (x.double() @ codes.double() - x.double().sum())
+    assert float((out.double() - want).norm() / want.norm()) < TOL_F16
+    assert _violations(checked)[0] == 0, _violations(checked)
+
+
+@pytest.mark.parametrize("bits", [16, 8, 4])
+@pytest.mark.parametrize("rows,steps,more", [(37, 1, -1), (299, 4, 1), (301, 12, 1), (9177, 9, -1), (19001, 2, 1)])
+def test_row_mat_vecs_checked(hq, dev, checked, bits, rows, steps, more):
+    """By ring and from registers, an odd row, rows that end inside a step; RMSNorm and a gated activation too."""
+    import torch
+    from test_row_stream_gpu import STEP, _calls, _layer
+    n = STEP[bits] * steps + more * (128 // bits)
+    mat, w, x = _layer(bits, rows, n, dev)
+    for call in _calls(hq, bits, mat, x, rows):
+        assert torch.equal(call(), (w @ x.double()).half())
+    fmt, kw = {16: ("f16", {}), 8: ("int8", dict(scale=1.0, zero_point=-2.0)), 4: ("int4", dict(scale=1.0, zero_point=7.0))}[bits]
+    gamma = torch.full((n,), 0.01, device=dev).half()
+    y = hq.gemv_fused(fmt, x, mat[:rows - 1], rows // 2, gamma=gamma, act=1, **kw)
+    v = w[:rows - 1] @ (x.double() * torch.rsqrt((x.double() ** 2).mean() + 1e-5) * gamma.double())
+    v = v[0::2] * v[1::2] * torch.sigmoid(v[1::2])
+    assert float((y.double() - v).norm() / v.norm()) < TOL_F16
+    assert _violations(checked)[0] == 0, _violations(checked)
